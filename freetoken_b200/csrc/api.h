@@ -317,6 +317,8 @@ int ftk_paged_attention_ex(const void* q, const void* k_slab, const void* v_slab
 // size 128, pages of a multiple of 16 tokens; n_tokens = rows of q.  ftk_attention_tc_fits says whether
 // the sizes are taken.
 int ftk_attention_tc_fits(int head_dim, int page_size, int group);
+// The same for heads of 64 and 256, which these kernels take without a bias by distance and a soft cap (256: form 0 only).
+int ftk_attention_tc_heads_fit(int head_dim, int page_size, int group);
 int ftk_paged_attention_tc(const void* q, const void* k_slab, const void* v_slab, const int32_t* block_table,
                            int bt_stride, const int32_t* seg_info, int n_segs, const int32_t* items, int n_items,
                            float* part_o, float* part_ml, int n_slots, void* out, int n_tokens, int n_q_heads,

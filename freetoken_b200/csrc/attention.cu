@@ -1058,6 +1058,7 @@ static int launch_bf16(const AttnParams& p, cudaStream_t s) {
 
 #include "attention_tc.cuh"
 #include "attention_tc2.cuh"
+#include "attention_tc256.cuh"
 
 using namespace ftk;
 
@@ -1081,6 +1082,10 @@ int ftk_attention_tc_set_status(int code) {
 
 extern "C" int ftk_attention_tc_fits(int head_dim, int page_size, int group) {
   return attention_tc_fits(head_dim, page_size, group) ? 1 : 0;
+}
+
+extern "C" int ftk_attention_tc_heads_fit(int head_dim, int page_size, int group) {
+  return attention_tc_heads_fit(head_dim, page_size, group) ? 1 : 0;
 }
 
 extern "C" int ftk_attention_tc_few_fits(int head_dim, int page_size, int group) {
@@ -1114,11 +1119,17 @@ static int paged_attention_tc_impl(const void* q, const void* k_slab, const void
   FTK_REQUIRE(q && k_slab && v_slab && block_table && seg_info && items && out, "paged_attention_tc: null pointer");
   FTK_REQUIRE(n_q_heads >= 1 && n_kv_heads >= 1 && n_q_heads % n_kv_heads == 0, "paged_attention_tc: %d query heads, %d KV heads",
               n_q_heads, n_kv_heads);
-  FTK_REQUIRE(attention_tc_fits(head_dim, page_size, n_q_heads / n_kv_heads),
-              "paged_attention_tc: head size %d, pages of %d, %d heads per KV head: takes head size 128, pages of a "
-              "multiple of 16, at most 128 heads per KV head", head_dim, page_size, n_q_heads / n_kv_heads);
-  FTK_REQUIRE(!few || attention_tc_few_fits(head_dim, page_size, n_q_heads / n_kv_heads),
-              "paged_attention_tc: tiles of 16 rows take at most 16 heads per KV head, got %d", n_q_heads / n_kv_heads);
+  const int kv_split = extras && extras->kv_split > 1 ? extras->kv_split : 1;
+  FTK_REQUIRE(n_q_heads / n_kv_heads % kv_split == 0 && (long long)n_kv_heads * kv_split <= 65535,
+              "paged_attention_tc: %d query heads per KV head cannot be split %d ways", n_q_heads / n_kv_heads, kv_split);
+  const int n_heads = n_kv_heads * kv_split, group = n_q_heads / n_heads;  // KV heads as the work list counts them
+  const bool plain = !(extras && (extras->dist_bias || extras->softcap > 0.f));
+  FTK_REQUIRE(attention_tc_fits(head_dim, page_size, group) || (plain && attention_tc_heads_fit(head_dim, page_size, group)),
+              "paged_attention_tc: head size %d, pages of %d, %d heads per KV head: takes head size 128 (64 and 256 without a "
+              "bias by distance and a soft cap), pages of a multiple of 16, at most 128 heads per KV head", head_dim, page_size, group);
+  FTK_REQUIRE(form == kTcSingle || head_dim <= kTcD, "paged_attention_tc: heads of %d run in single tiles of 128 rows", head_dim);
+  FTK_REQUIRE(!few || attention_tc_few_fits(kTcD, page_size, group),
+              "paged_attention_tc: tiles of 16 rows take at most 16 heads per KV head, got %d", group);
   FTK_REQUIRE(n_tokens >= 1 && n_items >= 0 && n_segs >= 1 && num_pages >= 1 && bt_stride >= 1,
               "paged_attention_tc: bad sizes");
   // (one slab for keys and values: the rows zeroed before a window's first key lie in the key stage itself, which the
@@ -1134,13 +1145,12 @@ static int paged_attention_tc_impl(const void* q, const void* k_slab, const void
   p.block_table = block_table; p.bt_stride = bt_stride;
   p.seg_info = seg_info; p.n_segs = n_segs; p.items = items; p.n_items = n_items;
   p.part_o = part_o; p.part_ml = part_ml; p.n_slots = n_slots;
-  p.Hq = n_q_heads; p.Hkv = n_kv_heads; p.G = n_q_heads / n_kv_heads; p.D = head_dim; p.P = page_size;
+  p.Hq = n_q_heads; p.Hkv = n_heads; p.G = group; p.D = head_dim; p.P = page_size;
   p.num_pages = num_pages; p.tile_rows = pair ? 2 * kTcRows : few ? kTcFewRows : kTcRows; p.scale = scale; p.window = window;
   p.sel = nullptr; p.sel_stride = 0; p.block_size = 0; p.arrivals = nullptr;
   p.dist_bias = extras ? extras->dist_bias : nullptr;
   p.dist_len = extras ? extras->dist_len : 0;
-  p.slab_heads = n_kv_heads; p.kv_split = 1;
-  FTK_REQUIRE(!extras || extras->kv_split <= 1, "paged_attention_tc: KV heads are not split for the tcgen05 kernels");
+  p.slab_heads = n_kv_heads; p.kv_split = kv_split;
   p.has_sink = extras ? extras->has_sink : 0;
   p.sink = extras ? extras->sink_logit : 0.f;
   p.sink_heads = extras ? extras->sink_heads : nullptr;
@@ -1156,16 +1166,21 @@ static int paged_attention_tc_impl(const void* q, const void* k_slab, const void
                                            : "attention: tcgen05, 128-row query tiles, soft cap");
   else if (p.dist_bias) note_variant(few ? "attention: tcgen05, tiles of at most 16 rows, bias by distance"
                                     : "attention: tcgen05, 128-row query tiles, bias by distance");
+  else if (head_dim == kTcWideD) note_variant("attention: tcgen05, 128-row query tiles, heads of 256");
+  else if (head_dim == 64) note_variant(pair ? "attention: tcgen05, two 128-row query tiles per CTA, heads of 64"
+                                        : few ? "attention: tcgen05, tiles of at most 16 rows, heads of 64"
+                                              : "attention: tcgen05, 128-row query tiles, heads of 64");
   else if (window > 0 || p.has_sink) note_variant("attention: tcgen05, 128-row query tiles, window or sink");
   else
   note_variant(pair ? "attention: tcgen05, two 128-row query tiles per CTA"
                : few ? "attention: tcgen05, tiles of at most 16 rows, one softmax warp"
                      : "attention: tcgen05, 128-row query tiles");
-  const int rc = pair ? launch_attention_tc2(p, n_tokens, s) : launch_attention_tc(p, n_tokens, s);
+  const int rc = head_dim == kTcWideD ? launch_attention_tc_wide(p, n_tokens, s)
+                 : pair ? launch_attention_tc2(p, n_tokens, s) : launch_attention_tc(p, n_tokens, s);
   FTK_REQUIRE(rc == 0, "paged_attention_tc: cannot set up the kernel (%d)", rc);
   FTK_LAUNCH_CHECK("paged_attention_tc");
   if (n_slots > 0) {
-    dim3 grid(n_items, n_kv_heads);
+    dim3 grid(n_items, n_heads);
     // a CTA merges its share of a tile's rows, a warp a row at a time (three trips to memory one after the
     // other): tiles of 128 and 256 rows get as many warps as a tile cut in two has rows per CTA / 4
     const int threads = p.tile_rows >= 128 ? 512 : 128;  // (96 registers a thread)

@@ -1,4 +1,4 @@
-// Paged causal attention on the 5th-generation tensor cores (tcgen05), bfloat16, head size 128: long
+// Paged causal attention on the 5th-generation tensor cores (tcgen05), bfloat16, head size 128 (or 64): long
 // steps and decode steps.  Included by attention.cu after AttnParams / Item / load_item.
 //
 // A tile is 128 query rows: the `group` query heads of one KV head for 128 / group consecutive tokens
@@ -42,7 +42,8 @@ constexpr int kTcThreads = 224;
 constexpr int kTcHalf = 128 * 64 * 2;       // bytes of a [128 rows x 64 elements] swizzle-atom column
 constexpr int kTcTile = 2 * kTcHalf;        // a [128 x 128] bfloat16 tile
 constexpr int kTcStages = 3;                // key and value tiles in flight
-constexpr int kTcSmem = (1 + 2 * kTcStages) * kTcTile + 1024;  // Q, K and V stages
+constexpr int kTcSmemOf(int d) { return (1 + 2 * kTcStages) * (kTcTile * d / kTcD) + 1024; }  // Q, K and V stages
+constexpr int kTcSmem = kTcSmemOf(kTcD);
 constexpr int kTcPCol = 3 * kTcKeys;        // tensor memory: S x2 (128 columns each), O (128), P x2 (64 each)
 
 __device__ __forceinline__ void tmem_ld32(uint32_t addr, float (&v)[32]) {
@@ -282,7 +283,7 @@ __device__ __forceinline__ void clear_outside(float (&v)[128], int key0, int lo,
 
 // Softmax and epilogue of a tile's rows 0..15 by one warp (the warp of TMEM lanes 0..31), for tiles
 // that have no more rows: thread t has rows t / 4 and t / 4 + 8 and a quarter of their columns.
-template <bool BIASED, int CAPPED>
+template <bool BIASED, int CAPPED, int D>
 __device__ __forceinline__ void attention_tc_few_rows(const AttnParams& p, uint32_t tmem, int lane, int n_work, int n_rounds,
                                                       uint64_t* s_full, uint64_t* s_empty, uint64_t* p_full,
                                                       uint64_t* pv_done, uint64_t* o_free, volatile int* abortp,
@@ -406,7 +407,7 @@ __device__ __forceinline__ void attention_tc_few_rows(const AttnParams& p, uint3
         }
         tc_fence_after();
 #pragma unroll 1
-        for (int k = 0; k < 4; ++k) {
+        for (int k = 0; k < D / 32; ++k) {
           float o[16];
           tmem_ld_16rows_32cols(tmem + (uint32_t)(2 * kTcKeys + 32 * k), o);
           tmem_ld_wait();
@@ -465,11 +466,11 @@ __device__ __forceinline__ void attention_tc_few_rows(const AttnParams& p, uint3
       const bool live = n_tiles > 0;
       const float inv_a = live && l_a > 0.f ? 1.f / l_a : 0.f, inv_b = live && l_b > 0.f ? 1.f / l_b : 0.f;
       const int tok_a = it.q_start + it.tok0 + ra / G, tok_b = it.q_start + it.tok0 + rb / G;
-      __nv_bfloat16* dst_a = (__nv_bfloat16*)p.out + ((size_t)tok_a * p.Hq + kvh * G + ra % G) * kTcD;
-      __nv_bfloat16* dst_b = (__nv_bfloat16*)p.out + ((size_t)tok_b * p.Hq + kvh * G + rb % G) * kTcD;
+      __nv_bfloat16* dst_a = (__nv_bfloat16*)p.out + ((size_t)tok_a * p.Hq + kvh * G + ra % G) * D;
+      __nv_bfloat16* dst_b = (__nv_bfloat16*)p.out + ((size_t)tok_b * p.Hq + kvh * G + rb % G) * D;
       const size_t slot0 = ((size_t)(it.base + it.split) * p.Hkv + kvh) * p.tile_rows;
 #pragma unroll 1
-      for (int k = 0; k < 4; ++k) {
+      for (int k = 0; k < D / 32; ++k) {
         float o[16];
         if (live) {
           tmem_ld_16rows_32cols(tmem + (uint32_t)(2 * kTcKeys + 32 * k), o);
@@ -485,8 +486,8 @@ __device__ __forceinline__ void attention_tc_few_rows(const AttnParams& p, uint3
             if (ra < R) *reinterpret_cast<uint32_t*>(dst_a + col) = tc_pack(o[4 * i] * inv_a, o[4 * i + 1] * inv_a);
             if (rb < R) *reinterpret_cast<uint32_t*>(dst_b + col) = tc_pack(o[4 * i + 2] * inv_b, o[4 * i + 3] * inv_b);
           } else {
-            if (ra < R) *reinterpret_cast<float2*>(p.part_o + (slot0 + ra) * kTcD + col) = make_float2(o[4 * i], o[4 * i + 1]);
-            if (rb < R) *reinterpret_cast<float2*>(p.part_o + (slot0 + rb) * kTcD + col) = make_float2(o[4 * i + 2], o[4 * i + 3]);
+            if (ra < R) *reinterpret_cast<float2*>(p.part_o + (slot0 + ra) * D + col) = make_float2(o[4 * i], o[4 * i + 1]);
+            if (rb < R) *reinterpret_cast<float2*>(p.part_o + (slot0 + rb) * D + col) = make_float2(o[4 * i + 2], o[4 * i + 3]);
           }
         }
       }
@@ -510,10 +511,12 @@ __device__ __forceinline__ void attention_tc_few_rows(const AttnParams& p, uint3
   }
 }
 
-template <bool FEW, bool BIASED = false, int CAPPED = kCapNone>
+template <bool FEW, bool BIASED = false, int CAPPED = kCapNone, int D = kTcD>
 __global__ void __launch_bounds__(kTcThreads)
 attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                     const __grid_constant__ CUtensorMap map_v, AttnParams p) {
+  constexpr int kHalves = D / 64, kTile = kHalves * kTcHalf;  // 64-column parts of a row; bytes of a tile
+  constexpr uint32_t kLoaders = 8 * kHalves, kLoaderMask = (1u << kLoaders) - 1u;  // lanes of a loading warp: one per box
   extern __shared__ unsigned char dyn_smem[];
   __shared__ uint64_t q_full, q_empty, o_free, k_full[kTcStages], k_empty[kTcStages], v_full[kTcStages], v_empty[kTcStages], s_full[2], s_empty[2],
       p_full[2], pv_done[2];
@@ -534,7 +537,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   };
   const uint32_t base = (smem_addr(dyn_smem) + 1023u) & ~1023u;
   unsigned char* tiles = dyn_smem + (base - smem_addr(dyn_smem));
-  const uint32_t q_s = base, k_s = base + kTcTile, v_s = base + (1 + kTcStages) * kTcTile;
+  const uint32_t q_s = base, k_s = base + kTile, v_s = base + (1 + kTcStages) * kTile;
 
   if (threadIdx.x == 0) {
     mbar_init(&q_full, 1);
@@ -552,7 +555,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (FEW) {  // query rows that no load writes must not hold whatever the kernel before left there
-    for (int i = threadIdx.x; i < kTcTile / 16; i += kTcThreads) reinterpret_cast<uint4*>(tiles)[i] = make_uint4(0u, 0u, 0u, 0u);
+    for (int i = threadIdx.x; i < kTile / 16; i += kTcThreads) reinterpret_cast<uint4*>(tiles)[i] = make_uint4(0u, 0u, 0u, 0u);
     fence_async_smem();
   }
   if (warp == 1) tmem_alloc(&tmem_slot, 512);
@@ -584,12 +587,12 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     // one warp made the keys wait for the value stage.)
     // Values that are the keys (one slab given for both): the key tile serves both products.  The value loader
     // has nothing to do, and a key stage is free again once the second product has read it.
-    if (lane < 16 && !(warp == 6 && p.k == p.v)) {
-      const int kv = warp == 6, box = lane >> 1, h = lane & 1;
+    if (lane < kLoaders && !(warp == 6 && p.k == p.v)) {
+      const int kv = warp == 6, box = lane / kHalves, h = lane % kHalves;
       const CUtensorMap* map = kv ? &map_v : &map_k;
       uint64_t* full = kv ? v_full : k_full;
       uint64_t* empty = kv ? v_empty : k_empty;
-      unsigned char* stage0 = tiles + (kv ? 1 + kTcStages : 1) * kTcTile + h * kTcHalf + box * 2048;
+      unsigned char* stage0 = tiles + (kv ? 1 + kTcStages : 1) * kTile + h * kTcHalf + box * 2048;
       bool ok = true;
       bool waited = false;  // for the kernel before this one (decode steps)
       int g = 0;   // tiles of all pieces so far: stage g & 1
@@ -604,13 +607,13 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         // the queries go out once the products of the piece before have read theirs: before the first key
         // tile, or (decode steps) after the key tiles that may go out before the kernel before this one is over
         auto load_queries = [&]() -> bool {
-          if (!__all_sync(0x0000ffffu, mbar_wait(&q_empty, (uint32_t)(qi & 1) ^ 1u, abortp))) {
+          if (!__all_sync(kLoaderMask, mbar_wait(&q_empty, (uint32_t)(qi & 1) ^ 1u, abortp))) {
             if (lane == 0) fail(210);
             return false;
           }
           if (lane == 0) {
-            mbar_expect_tx(&q_full, (uint32_t)(2 * 128 * G * (p.tile_rows / G)));  // two boxes of (64, group, tokens per tile)
-            for (int hh = 0; hh < 2; ++hh)  // (d, head, token): rows land as token-major, head-minor
+            mbar_expect_tx(&q_full, (uint32_t)(kHalves * 128 * G * (p.tile_rows / G)));  // boxes of (64, group, tokens per tile)
+            for (int hh = 0; hh < kHalves; ++hh)  // (d, head, token): rows land as token-major, head-minor
               tma_load_3d(tiles + hh * kTcHalf, &map_q, &q_full, hh * 64, kvh * G, it.q_start + it.tok0);
           }
           return true;
@@ -618,6 +621,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         const int q_at = FEW ? min(n_tiles - 1, 1) : 0;
         const int fresh_from = it.kv_len - it.q_len;  // first position that this step wrote
         const int32_t* bt = p.block_table + (size_t)it.bt_row * p.bt_stride;
+        const int slab_head = kvh / p.kv_split;
         // this lane's page of tile j: looked up one tile ahead, so that the answer is there when the stage is free
         auto page_of = [&](int j) {
           const int key = it.kb + j * kTcKeys + 16 * box;
@@ -638,7 +642,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
           const int key = key0 + 16 * box;
           const int page = page_next;
           page_next = page_of(j + 1);
-          const int row = (page * p.Hkv + kvh) * p.P + (key + it.shift(p, key)) % p.P;
+          const int row = (page * p.slab_heads + slab_head) * p.P + (key + it.shift(p, key)) % p.P;
           if (FEW && !waited && (key0 + kTcKeys > fresh_from || (!kv && j == q_at))) {
             pdl_wait();
             waited = true;
@@ -647,14 +651,14 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             ok = false;
             break;
           }
-          if (!__all_sync(0x0000ffffu, mbar_wait(&empty[st], par, abortp))) {
+          if (!__all_sync(kLoaderMask, mbar_wait(&empty[st], par, abortp))) {
             if (lane == 0) fail(201 + kv);
             ok = false;
             break;
           }
-          if (lane == 0) mbar_expect_tx(&full[st], (uint32_t)n_box * 2 * 2048);
-          __syncwarp(0x0000ffffu);
-          if (box < n_box) tma_load_2d(stage0 + st * kTcTile, map, &full[st], h * 64, row);
+          if (lane == 0) mbar_expect_tx(&full[st], (uint32_t)n_box * kHalves * 2048);
+          __syncwarp(kLoaderMask);
+          if (box < n_box) tma_load_2d(stage0 + st * kTile, map, &full[st], h * 64, row);
         }
         ++qi;
       }
@@ -662,7 +666,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (lane 0); the warp zeroes value rows past the end
     constexpr uint32_t idesc_qk = instr_desc(kTcKeys);
-    constexpr uint32_t idesc_pv = instr_desc(kTcD) | (1u << 16);  // B (values) MN-major
+    constexpr uint32_t idesc_pv = instr_desc(D) | (1u << 16);  // B (values) MN-major
     const bool tied = p.k == p.v;  // the value tile is the key tile (same boxes, same layout in shared memory)
     const int v_tile0 = tied ? 1 : 1 + kTcStages;  // first value stage, in tiles from `tiles`
     bool ok = true;
@@ -692,9 +696,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
           if (lane == 0) {
             const uint32_t d = tmem + (uint32_t)(st * kTcKeys);
 #pragma unroll
-            for (int kk = 0; kk < 8; ++kk) {  // 16 elements of the head dimension per MMA
+            for (int kk = 0; kk < 4 * kHalves; ++kk) {  // 16 elements of the head dimension per MMA
               const uint64_t a = smem_desc(q_s + (kk >> 2) * kTcHalf) + 2 * (kk & 3);
-              const uint64_t b = smem_desc(k_s + ks * kTcTile + (kk >> 2) * kTcHalf) + 2 * (kk & 3);
+              const uint64_t b = smem_desc(k_s + ks * kTile + (kk >> 2) * kTcHalf) + 2 * (kk & 3);
               tc_mma(d, a, b, idesc_qk, kk != 0);
             }
             if (!tied) tc_commit(&k_empty[ks]);
@@ -723,9 +727,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             const int first = key0 + it.shift(p, key0);
             const int from = max(0, p.keep_first - first), dead = min(kTcKeys, it.lo - first);
             if (dead > from) {
-              for (int x = lane; x < (dead - from) * 16; x += 32) {
-                const int r = from + x / 16, h = (x / 8) & 1, c = x & 7;
-                *reinterpret_cast<uint4*>(tiles + (v_tile0 + vs) * kTcTile + h * kTcHalf + r * 128 + c * 16) =
+              for (int x = lane; x < (dead - from) * 8 * kHalves; x += 32) {
+                const int r = from + x / (8 * kHalves), h = (x / 8) % kHalves, c = x & 7;
+                *reinterpret_cast<uint4*>(tiles + (v_tile0 + vs) * kTile + h * kTcHalf + r * 128 + c * 16) =
                     make_uint4(0u, 0u, 0u, 0u);
               }
               fence_async_smem();
@@ -734,9 +738,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
           if (live < kTcKeys) {
             // the value rows past the end of the request: zero, whatever the page holds there (the rest of
             // the last loaded box) and whatever the stage held before (boxes that were not loaded)
-            for (int x = lane; x < (kTcKeys - live) * 16; x += 32) {
-              const int r = live + x / 16, h = (x / 8) & 1, c = x & 7;
-              *reinterpret_cast<uint4*>(tiles + (v_tile0 + vs) * kTcTile + h * kTcHalf + r * 128 + c * 16) =
+            for (int x = lane; x < (kTcKeys - live) * 8 * kHalves; x += 32) {
+              const int r = live + x / (8 * kHalves), h = (x / 8) % kHalves, c = x & 7;
+              *reinterpret_cast<uint4*>(tiles + (v_tile0 + vs) * kTile + h * kTcHalf + r * 128 + c * 16) =
                   make_uint4(0u, 0u, 0u, 0u);
             }
             fence_async_smem();
@@ -748,7 +752,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk) {  // 16 keys per MMA
               const uint32_t a = tmem + (uint32_t)(kTcPCol + st * (kTcKeys / 2) + kk * 8);
-              const uint64_t b = smem_desc_mn((tied ? k_s : v_s) + vs * kTcTile + kk * 2048, kTcHalf);
+              const uint64_t b = smem_desc_mn((tied ? k_s : v_s) + vs * kTile + kk * 2048, kTcHalf);
               tc_mma_ts(d, a, b, idesc_pv, (i | kk) != 0);
             }
             tc_commit(tied ? &k_empty[vs] : &v_empty[vs]);
@@ -763,7 +767,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   } else if (FEW) {
     // ------------------------------------------------------------ softmax and epilogue of rows 0..15 by one warp
     if ((warp & 3) == 0) {
-      attention_tc_few_rows<BIASED, CAPPED>(p, tmem, lane, n_work, n_rounds, s_full, s_empty, p_full, pv_done, &o_free, abortp, &abort_flag);
+      attention_tc_few_rows<BIASED, CAPPED, D>(p, tmem, lane, n_work, n_rounds, s_full, s_empty, p_full, pv_done, &o_free, abortp, &abort_flag);
     }
   } else {
     // ------------------------------------------------------------ softmax and epilogue (warps 2..5), one row per thread
@@ -884,7 +888,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         }
         tc_fence_after();
 #pragma unroll 1
-        for (int c = 0; c < 4; ++c) {
+        for (int c = 0; c < D / 32; ++c) {
           float o[32];
           tmem_ld32(lane_addr + 2 * kTcKeys + c * 32, o);
 #pragma unroll
@@ -948,9 +952,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         // (a sink in the denominator: e^sink relative to the running maximum, which is in the exp2 domain)
         const float lt = l + (p.has_sink ? exp2f((p.sink_heads ? __ldg(p.sink_heads + kvh * G + r % G) : p.sink) * 1.4426950408889634f - m_used) : 0.f);
         const float inv = lt > 0.f ? 1.f / lt : 0.f;
-        __nv_bfloat16* dst = (__nv_bfloat16*)p.out + ((size_t)tok * p.Hq + kvh * G + r % G) * kTcD;
+        __nv_bfloat16* dst = (__nv_bfloat16*)p.out + ((size_t)tok * p.Hq + kvh * G + r % G) * D;
 #pragma unroll 1
-        for (int c = 0; c < 4; ++c) {
+        for (int c = 0; c < D / 32; ++c) {
           float o[32];
           if (live) tmem_ld32(lane_addr + 2 * kTcKeys + c * 32, o);
           if (r < R) {
@@ -968,13 +972,13 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       } else {
         const size_t slot = ((size_t)(it.base + it.split) * p.Hkv + kvh) * p.tile_rows + r;
 #pragma unroll 1
-        for (int c = 0; c < 4; ++c) {
+        for (int c = 0; c < D / 32; ++c) {
           float o[32];
           if (live) tmem_ld32(lane_addr + 2 * kTcKeys + c * 32, o);
           if (r < R) {
 #pragma unroll
             for (int q4 = 0; q4 < 8; ++q4)
-              *reinterpret_cast<float4*>(p.part_o + slot * kTcD + c * 32 + q4 * 4) =
+              *reinterpret_cast<float4*>(p.part_o + slot * D + c * 32 + q4 * 4) =
                   live ? make_float4(o[4 * q4], o[4 * q4 + 1], o[4 * q4 + 2], o[4 * q4 + 3]) : make_float4(0.f, 0.f, 0.f, 0.f);
           }
         }
@@ -1011,6 +1015,12 @@ inline bool attention_tc_fits(int head_dim, int page_size, int group) {
   return head_dim == kTcD && page_size >= 16 && page_size % 16 == 0 && group >= 1 && group <= kTcRows;
 }
 
+// Heads of 64 (one 64-column part a row instead of two, the same kernels: 16 heads on 4, 2,048 tokens 169 -> 34 us against
+// mma.sync) and of 256 (attention_tc256.cuh): no bias by distance, no soft cap.
+inline bool attention_tc_heads_fit(int head_dim, int page_size, int group) {
+  return (head_dim == 64 || head_dim == 256) && attention_tc_fits(kTcD, page_size, group);
+}
+
 // Tiles of at most 16 rows (decode steps) on the same kernel with one softmax warp: the same sizes, at most
 // 16 query heads per KV head.
 constexpr int kTcFewRows = 16;
@@ -1020,6 +1030,7 @@ inline bool attention_tc_few_fits(int head_dim, int page_size, int group) {
 
 // `p.tile_rows` is 128, or 16 for the few-rows form.
 inline int launch_attention_tc(const AttnParams& p, int n_tokens, cudaStream_t s) {
+  const int D = p.D;
   static bool configured = false;
   if (!configured) {
     if (cudaFuncSetAttribute(attention_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem) != cudaSuccess ||
@@ -1028,7 +1039,9 @@ inline int launch_attention_tc(const AttnParams& p, int n_tokens, cudaStream_t s
         cudaFuncSetAttribute(attention_tc_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem) != cudaSuccess ||
         cudaFuncSetAttribute(attention_tc_kernel<false, false, kCapBounded>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem) != cudaSuccess ||
         cudaFuncSetAttribute(attention_tc_kernel<false, false, kCapAny>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem) != cudaSuccess ||
-        cudaFuncSetAttribute(attention_tc_kernel<true, false, kCapAny>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem) != cudaSuccess)
+        cudaFuncSetAttribute(attention_tc_kernel<true, false, kCapAny>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem) != cudaSuccess ||
+        cudaFuncSetAttribute(attention_tc_kernel<false, false, kCapNone, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem) != cudaSuccess ||
+        cudaFuncSetAttribute(attention_tc_kernel<true, false, kCapNone, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem) != cudaSuccess)
       return 2;
     configured = true;
   }
@@ -1036,15 +1049,15 @@ inline int launch_attention_tc(const AttnParams& p, int n_tokens, cudaStream_t s
   CUtensorMap mq, mk, mv;
   {
     // queries [T, Hq, D] seen as (d, head, token); a box is (64, group, tokens per tile)
-    const uint64_t dims[3] = {(uint64_t)kTcD, (uint64_t)p.Hq, (uint64_t)n_tokens};
-    const uint64_t strides[2] = {(uint64_t)kTcD * 2, (uint64_t)p.Hq * kTcD * 2};
+    const uint64_t dims[3] = {(uint64_t)D, (uint64_t)p.Hq, (uint64_t)n_tokens};
+    const uint64_t strides[2] = {(uint64_t)D * 2, (uint64_t)p.Hq * D * 2};
     const uint32_t box[3] = {64, (uint32_t)p.G, (uint32_t)(p.tile_rows / p.G)};
     if (!make_map(&mq, p.q, 3, dims, strides, box)) return 4;
   }
   {
     // a slab [pages, Hkv, P, D] seen as rows of D; a box is 16 rows of one page x 64 elements
-    const uint64_t dims[2] = {(uint64_t)kTcD, (uint64_t)p.num_pages * p.Hkv * p.P};
-    const uint64_t strides[1] = {(uint64_t)kTcD * 2};
+    const uint64_t dims[2] = {(uint64_t)D, (uint64_t)p.num_pages * p.slab_heads * p.P};
+    const uint64_t strides[1] = {(uint64_t)D * 2};
     const uint32_t box[2] = {64, 16};
     if (!make_map(&mk, p.k, 2, dims, strides, box) || !make_map(&mv, p.v, 2, dims, strides, box)) return 4;
   }
@@ -1056,7 +1069,11 @@ inline int launch_attention_tc(const AttnParams& p, int n_tokens, cudaStream_t s
   }
   const long long n_work = (long long)p.n_items * p.Hkv;  // one CTA per SM, each takes every sms-th piece of work
   const int grid = (int)(n_work < sms ? n_work : sms);
-  if (p.tile_rows == kTcFewRows && p.softcap > 0.f) {
+  if (D == 64) {
+    if (p.softcap > 0.f || p.dist_bias) return 5;
+    if (p.tile_rows == kTcFewRows) FTK_LAUNCH((attention_tc_kernel<true, false, kCapNone, 64>), grid, kTcThreads, kTcSmemOf(64), s, mq, mk, mv, p);
+    else FTK_LAUNCH((attention_tc_kernel<false, false, kCapNone, 64>), grid, kTcThreads, kTcSmemOf(64), s, mq, mk, mv, p);
+  } else if (p.tile_rows == kTcFewRows && p.softcap > 0.f) {
     FTK_LAUNCH((attention_tc_kernel<true, false, kCapAny>), grid, kTcThreads, kTcSmem, s, mq, mk, mv, p);
   } else if (p.softcap > 0.f && soft_cap_bounded(p.softcap)) {
     FTK_LAUNCH((attention_tc_kernel<false, false, kCapBounded>), grid, kTcThreads, kTcSmem, s, mq, mk, mv, p);

@@ -30,10 +30,12 @@ constexpr int kTc2Threads = 384;                                  // a warpgroup
 constexpr int kTc2RegsFew = 72, kTc2RegsMany = 216;                // of 384 x 168: what 128 threads give, 256 take
 constexpr int kTc2Smem = (2 + 2 * kTc2Stages) * kTcTile + 1024;    // Q_A, Q_B, K and V stages
 
-template <int CAPPED>
+template <int CAPPED, int D = kTcD>
 __global__ void __launch_bounds__(kTc2Threads, 1)
 attention_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                      const __grid_constant__ CUtensorMap map_v, AttnParams p) {
+  constexpr int kHalves = D / 64, kTile = kHalves * kTcHalf;  // 64-column parts of a row; bytes of a tile
+  constexpr uint32_t kLoaders = 8 * kHalves, kLoaderMask = (1u << kLoaders) - 1u;  // lanes of a loading warp: one per box
   extern __shared__ unsigned char dyn_smem[];
   __shared__ uint64_t q_full, q_empty, o_free[2], k_full[kTc2Stages], k_empty[kTc2Stages], v_full[kTc2Stages],
       v_empty[kTc2Stages], s_full[2], p_full[2], pv_done[2];
@@ -48,7 +50,7 @@ attention_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
   };
   const uint32_t base = (smem_addr(dyn_smem) + 1023u) & ~1023u;
   unsigned char* tiles = dyn_smem + (base - smem_addr(dyn_smem));
-  const uint32_t q_s = base, k_s = base + 2 * kTcTile, v_s = base + (2 + kTc2Stages) * kTcTile;
+  const uint32_t q_s = base, k_s = base + 2 * kTile, v_s = base + (2 + kTc2Stages) * kTile;
 
   if (threadIdx.x == 0) {
     mbar_init(&q_full, 1);
@@ -84,12 +86,12 @@ attention_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
   regs_give<kTc2RegsFew>();  // (warp 3 only fills the warpgroup)
   if (warp == 0 || warp == 2) {
     // ------------------------------------------------------------ TMA producers: warp 0 keys (and queries), warp 2 values
-    if (lane < 16) {
-      const int kv = warp == 2, box = lane >> 1, h = lane & 1;
+    if (lane < kLoaders) {
+      const int kv = warp == 2, box = lane / kHalves, h = lane % kHalves;
       const CUtensorMap* map = kv ? &map_v : &map_k;
       uint64_t* full = kv ? v_full : k_full;
       uint64_t* empty = kv ? v_empty : k_empty;
-      unsigned char* stage0 = tiles + (kv ? 2 + kTc2Stages : 2) * kTcTile + h * kTcHalf + box * 2048;
+      unsigned char* stage0 = tiles + (kv ? 2 + kTc2Stages : 2) * kTile + h * kTcHalf + box * 2048;
       bool ok = true;
       int g = 0;   // key tiles of all pieces so far
       int qi = 0;  // pieces with tiles so far
@@ -101,22 +103,23 @@ attention_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         const int n_tiles = tiles_of(it);
         if (n_tiles == 0) continue;
         if (!kv) {  // the queries, once the products of the piece before have read theirs
-          if (!__all_sync(0x0000ffffu, mbar_wait(&q_empty, (uint32_t)(qi & 1) ^ 1u, abortp))) {
+          if (!__all_sync(kLoaderMask, mbar_wait(&q_empty, (uint32_t)(qi & 1) ^ 1u, abortp))) {
             if (lane == 0) fail(310);
             ok = false;
             break;
           }
           if (lane == 0) {
             const int n_q = it.ntok > tpt ? 2 : 1;  // tile B only when the piece has tokens for it
-            mbar_expect_tx(&q_full, (uint32_t)(n_q * 2 * 128 * G * tpt));
+            mbar_expect_tx(&q_full, (uint32_t)(n_q * kHalves * 128 * G * tpt));
             for (int x = 0; x < n_q; ++x)
-              for (int hh = 0; hh < 2; ++hh)  // (d, head, token): rows land as token-major, head-minor
-                tma_load_3d(tiles + x * kTcTile + hh * kTcHalf, &map_q, &q_full, hh * 64, kvh * G,
+              for (int hh = 0; hh < kHalves; ++hh)  // (d, head, token): rows land as token-major, head-minor
+                tma_load_3d(tiles + x * kTile + hh * kTcHalf, &map_q, &q_full, hh * 64, kvh * G,
                             it.q_start + it.tok0 + x * tpt);
           }
         }
         ++qi;
         const int32_t* bt = p.block_table + (size_t)it.bt_row * p.bt_stride;
+        const int slab_head = kvh / p.kv_split;
         for (int j = 0; j < n_tiles && ok; ++j, ++g) {
           const int st = g % kTc2Stages;
           const uint32_t par = ((g / kTc2Stages) & 1) ^ 1;
@@ -129,22 +132,22 @@ attention_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             page = slot < p.bt_stride ? bt[slot] : 0;
             if (page < 0 || page >= p.num_pages) page = 0;
           }
-          const int row = (page * p.Hkv + kvh) * p.P + key % p.P;
-          if (!__all_sync(0x0000ffffu, mbar_wait(&empty[st], par, abortp))) {
+          const int row = (page * p.slab_heads + slab_head) * p.P + key % p.P;
+          if (!__all_sync(kLoaderMask, mbar_wait(&empty[st], par, abortp))) {
             if (lane == 0) fail(301 + kv);
             ok = false;
             break;
           }
-          if (lane == 0) mbar_expect_tx(&full[st], (uint32_t)n_box * 2 * 2048);
-          __syncwarp(0x0000ffffu);
-          if (box < n_box) tma_load_2d(stage0 + st * kTcTile, map, &full[st], h * 64, row);
+          if (lane == 0) mbar_expect_tx(&full[st], (uint32_t)n_box * kHalves * 2048);
+          __syncwarp(kLoaderMask);
+          if (box < n_box) tma_load_2d(stage0 + st * kTile, map, &full[st], h * 64, row);
         }
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (lane 0); the warp zeroes value rows past the end
     constexpr uint32_t idesc_qk = instr_desc(kTcKeys);
-    constexpr uint32_t idesc_pv = instr_desc(kTcD) | (1u << 16);  // B (values) MN-major
+    constexpr uint32_t idesc_pv = instr_desc(D) | (1u << 16);  // B (values) MN-major
     bool ok = true;
     int g0 = 0;  // key tiles of the pieces before this one
     int qi = 0;  // pieces with tiles before this one
@@ -171,9 +174,9 @@ attention_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         if (lane == 0) {
           const uint32_t d = tmem + (uint32_t)(x * kTcKeys);
 #pragma unroll
-          for (int kk = 0; kk < 8; ++kk) {  // 16 elements of the head dimension per MMA
-            const uint64_t a = smem_desc(q_s + x * kTcTile + (kk >> 2) * kTcHalf) + 2 * (kk & 3);
-            const uint64_t b = smem_desc(k_s + ks * kTcTile + (kk >> 2) * kTcHalf) + 2 * (kk & 3);
+          for (int kk = 0; kk < 4 * kHalves; ++kk) {  // 16 elements of the head dimension per MMA
+            const uint64_t a = smem_desc(q_s + x * kTile + (kk >> 2) * kTcHalf) + 2 * (kk & 3);
+            const uint64_t b = smem_desc(k_s + ks * kTile + (kk >> 2) * kTcHalf) + 2 * (kk & 3);
             tc_mma(d, a, b, idesc_qk, kk != 0);
           }
           tc_commit(&s_full[x]);
@@ -195,9 +198,9 @@ attention_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
           if (live < kTcKeys) {
             // the value rows past the end of the request: zero, whatever the page holds there and
             // whatever the stage held before
-            for (int z = lane; z < (kTcKeys - live) * 16; z += 32) {
-              const int r = live + z / 16, h = (z / 8) & 1, c = z & 7;
-              *reinterpret_cast<uint4*>(tiles + (2 + kTc2Stages + vs) * kTcTile + h * kTcHalf + r * 128 + c * 16) =
+            for (int z = lane; z < (kTcKeys - live) * 8 * kHalves; z += 32) {
+              const int r = live + z / (8 * kHalves), h = (z / 8) % kHalves, c = z & 7;
+              *reinterpret_cast<uint4*>(tiles + (2 + kTc2Stages + vs) * kTile + h * kTcHalf + r * 128 + c * 16) =
                   make_uint4(0u, 0u, 0u, 0u);
             }
             fence_async_smem();
@@ -211,7 +214,7 @@ attention_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk) {  // 16 keys per MMA
             const uint32_t a = tmem + (uint32_t)(x * kTcKeys + kk * 8);
-            const uint64_t b = smem_desc_mn(v_s + vs * kTcTile + kk * 2048, kTcHalf);
+            const uint64_t b = smem_desc_mn(v_s + vs * kTile + kk * 2048, kTcHalf);
             tc_mma_ts(d, a, b, idesc_pv, (j | kk) != 0);
           }
           tc_commit(&pv_done[x]);
@@ -323,7 +326,7 @@ attention_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
           }
           tc_fence_after();
 #pragma unroll 1
-          for (int c = 0; c < 4; ++c) {
+          for (int c = 0; c < D / 32; ++c) {
             float o[32];
             tmem_ld32(o_addr + c * 32, o);
 #pragma unroll
@@ -373,9 +376,9 @@ attention_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         const int tok = it.q_start + it.tok0 + X * tpt + r / G;
         if (it.nsplit == 1) {
           const float inv = l > 0.f ? 1.f / l : 0.f;
-          __nv_bfloat16* dst = (__nv_bfloat16*)p.out + ((size_t)tok * p.Hq + kvh * G + r % G) * kTcD;
+          __nv_bfloat16* dst = (__nv_bfloat16*)p.out + ((size_t)tok * p.Hq + kvh * G + r % G) * D;
 #pragma unroll 1
-          for (int c = 0; c < 4; ++c) {
+          for (int c = 0; c < D / 32; ++c) {
             float o[32];
             if (live) tmem_ld32(o_addr + c * 32, o);
             if (r < R) {
@@ -394,13 +397,13 @@ attention_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
           // the rows of tile B follow those of tile A in the piece's slot of partial sums
           const size_t slot = ((size_t)(it.base + it.split) * p.Hkv + kvh) * p.tile_rows + X * tpt * G + r;
 #pragma unroll 1
-          for (int c = 0; c < 4; ++c) {
+          for (int c = 0; c < D / 32; ++c) {
             float o[32];
             if (live) tmem_ld32(o_addr + c * 32, o);
             if (r < R) {
 #pragma unroll
               for (int q4 = 0; q4 < 8; ++q4)
-                *reinterpret_cast<float4*>(p.part_o + slot * kTcD + c * 32 + q4 * 4) =
+                *reinterpret_cast<float4*>(p.part_o + slot * D + c * 32 + q4 * 4) =
                     live ? make_float4(o[4 * q4], o[4 * q4 + 1], o[4 * q4 + 2], o[4 * q4 + 3]) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
           }
@@ -433,26 +436,28 @@ attention_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
 
 // 256 query rows per piece of work; otherwise what the one-tile kernel takes.
 inline int launch_attention_tc2(const AttnParams& p, int n_tokens, cudaStream_t s) {
+  const int D = p.D;
   static bool configured = false;
   if (!configured) {
     if (cudaFuncSetAttribute(attention_tc2_kernel<kCapNone>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTc2Smem) != cudaSuccess ||
         cudaFuncSetAttribute(attention_tc2_kernel<kCapBounded>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTc2Smem) != cudaSuccess ||
-        cudaFuncSetAttribute(attention_tc2_kernel<kCapAny>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTc2Smem) != cudaSuccess)
+        cudaFuncSetAttribute(attention_tc2_kernel<kCapAny>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTc2Smem) != cudaSuccess ||
+        cudaFuncSetAttribute(attention_tc2_kernel<kCapNone, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTc2Smem) != cudaSuccess)
       return 2;
     configured = true;
   }
   CUtensorMap mq, mk, mv;
   {
     // queries [T, Hq, D] seen as (d, head, token); a box is (64, group, tokens per tile)
-    const uint64_t dims[3] = {(uint64_t)kTcD, (uint64_t)p.Hq, (uint64_t)n_tokens};
-    const uint64_t strides[2] = {(uint64_t)kTcD * 2, (uint64_t)p.Hq * kTcD * 2};
+    const uint64_t dims[3] = {(uint64_t)D, (uint64_t)p.Hq, (uint64_t)n_tokens};
+    const uint64_t strides[2] = {(uint64_t)D * 2, (uint64_t)p.Hq * D * 2};
     const uint32_t box[3] = {64, (uint32_t)p.G, (uint32_t)(kTcRows / p.G)};
     if (!make_map(&mq, p.q, 3, dims, strides, box)) return 4;
   }
   {
     // a slab [pages, Hkv, P, D] seen as rows of D; a box is 16 rows of one page x 64 elements
-    const uint64_t dims[2] = {(uint64_t)kTcD, (uint64_t)p.num_pages * p.Hkv * p.P};
-    const uint64_t strides[1] = {(uint64_t)kTcD * 2};
+    const uint64_t dims[2] = {(uint64_t)D, (uint64_t)p.num_pages * p.slab_heads * p.P};
+    const uint64_t strides[1] = {(uint64_t)D * 2};
     const uint32_t box[2] = {64, 16};
     if (!make_map(&mk, p.k, 2, dims, strides, box) || !make_map(&mv, p.v, 2, dims, strides, box)) return 4;
   }
@@ -464,7 +469,10 @@ inline int launch_attention_tc2(const AttnParams& p, int n_tokens, cudaStream_t 
   }
   const long long n_work = (long long)p.n_items * p.Hkv;
   const int grid = (int)(n_work < sms ? n_work : sms);
-  if (p.softcap > 0.f && soft_cap_bounded(p.softcap)) FTK_LAUNCH(attention_tc2_kernel<kCapBounded>, grid, kTc2Threads, kTc2Smem, s, mq, mk, mv, p);
+  if (D == 64) {
+    if (p.softcap > 0.f) return 5;
+    FTK_LAUNCH((attention_tc2_kernel<kCapNone, 64>), grid, kTc2Threads, (kTc2Smem - 1024) / 2 + 1024, s, mq, mk, mv, p);
+  } else if (p.softcap > 0.f && soft_cap_bounded(p.softcap)) FTK_LAUNCH(attention_tc2_kernel<kCapBounded>, grid, kTc2Threads, kTc2Smem, s, mq, mk, mv, p);
   else if (p.softcap > 0.f) FTK_LAUNCH(attention_tc2_kernel<kCapAny>, grid, kTc2Threads, kTc2Smem, s, mq, mk, mv, p);
   else FTK_LAUNCH(attention_tc2_kernel<kCapNone>, grid, kTc2Threads, kTc2Smem, s, mq, mk, mv, p);
   return 0;

@@ -124,6 +124,7 @@ _SIGNATURES = {
     "ftk_table_route": [_vp, _vp, _i, _i, _i, _i, _f, _vp, _vp, _vp],
     "ftk_scale_f32": [_vp, ctypes.c_longlong, _f, _vp],
     "ftk_attention_tc_fits": [_i, _i, _i],
+    "ftk_attention_tc_heads_fit": [_i, _i, _i],
     "ftk_paged_attention_tc": [_vp, _vp, _vp, _vp, _i, _vp, _i, _vp, _i, _vp, _vp, _i, _vp,
                                _i, _i, _i, _i, _i, _i, _f, _i, _vp],
     "ftk_paged_attention_tc_ex": [_vp, _vp, _vp, _vp, _i, _vp, _i, _vp, _i, _vp, _vp, _i, _vp,
@@ -496,7 +497,7 @@ def paged_attention(q: torch.Tensor, k_slab: torch.Tensor, v_slab: torch.Tensor,
     ``v_slab`` may be ``k_slab`` itself (values that are the keys): each key tile is then brought in once.
     ``kv_split > 1`` (more query heads per KV head than a tile has rows): every KV head is taken as that many
     heads of the same keys with a share of its query heads each; the work list and the scratch are then made for
-    ``Hkv * kv_split`` heads.  Not with the tcgen05 kernels.
+    ``Hkv * kv_split`` heads.
     Of the tcgen05 kernels the ones with one query tile a piece (128 rows, or at most 16) take the bias; with
     one slab for keys and values their key tile in shared memory serves both products.
 
@@ -533,8 +534,8 @@ def paged_attention(q: torch.Tensor, k_slab: torch.Tensor, v_slab: torch.Tensor,
         sink_heads, sink = _dev(sink, "sink", torch.float32), 0.0
     kv_split = max(1, int(kv_split))
     Hv = Hkv * kv_split
-    if kv_split > 1 and ((Hq // Hkv) % kv_split or sel is not None or tile_rows in (128, 256) or few_rows):
-        raise KernelError("paged_attention: kv_split must divide the query heads per KV head (no tcgen05, no selection)")
+    if kv_split > 1 and ((Hq // Hkv) % kv_split or sel is not None):
+        raise KernelError("paged_attention: kv_split must divide the query heads per KV head (no selection)")
     if part_o is not None and (part_o.shape[1:] != (Hv, tile_rows, D) or part_ml is None
                                or part_ml.shape != (n_slots, Hv, tile_rows, 2)):
         raise KernelError("paged_attention: scratch shapes do not match tile_rows / heads")
@@ -544,7 +545,7 @@ def paged_attention(q: torch.Tensor, k_slab: torch.Tensor, v_slab: torch.Tensor,
         # bfloat16 steps on the tcgen05 kernels: one query tile per CTA, a pair of them, or tiles of a few rows
         if sel is not None or q.dtype != torch.bfloat16:
             raise KernelError("paged_attention: the tcgen05 kernels take bfloat16 without block selection")
-        if window or sink is not None or dist_bias is not None or softcap:
+        if window or sink is not None or dist_bias is not None or softcap or kv_split > 1:
             # the form with one 128-row query tile a piece takes a window, a sink and a bias by distance (a bias not
             # together with a window); the form for tiles of at most 16 rows takes the bias alone
             if (window or sink is not None) and (tile_rows != 128 or few_rows):
@@ -553,7 +554,7 @@ def paged_attention(q: torch.Tensor, k_slab: torch.Tensor, v_slab: torch.Tensor,
                 raise KernelError("paged_attention: of the tcgen05 kernels the ones with one query tile a piece take a "
                                   "distance bias [Hq, L] (no window)")
             ex = _AttnExtras(_dev(dist_bias, "dist_bias", torch.float32), dist_bias.shape[1] if dist_bias is not None else 0,
-                             1, 0 if sink is None else 1, 0.0 if sink is None else float(sink), sink_heads, softcap,
+                             kv_split, 0 if sink is None else 1, 0.0 if sink is None else float(sink), sink_heads, softcap,
                              keep_first)
             what = "soft cap" if softcap else "distance bias" if dist_bias is not None else "window or sink"
             _check(_lib().ftk_paged_attention_tc_ex(
@@ -621,6 +622,12 @@ def paged_attention(q: torch.Tensor, k_slab: torch.Tensor, v_slab: torch.Tensor,
 def attention_tc_fits(head_dim: int, page_size: int, group: int) -> bool:
     """Whether the tcgen05 attention kernel (tiles of 128 query rows) takes these sizes."""
     return bool(_lib().ftk_attention_tc_fits(head_dim, page_size, group))
+
+
+def attention_tc_heads_fit(head_dim: int, page_size: int, group: int) -> bool:
+    """Whether the tcgen05 attention kernels take these sizes for heads of another size than 128: 64 in every form, 256 in
+    tiles of 128 rows; neither with a bias by distance or a soft cap (``csrc/attention_tc.cuh: attention_tc_heads_fit``)."""
+    return head_dim in (64, 256) and attention_tc_fits(128, page_size, group)
 
 
 def attention_tc_few_fits(head_dim: int, page_size: int, group: int) -> bool:

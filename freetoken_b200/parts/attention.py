@@ -48,7 +48,7 @@ TC_MIN_DECODE_SPAN = 0   # decode steps go there from this length of the longest
 def attention_kernel_form(dtype: torch.dtype, decode_only: bool = False, group: int = 1, n_tokens: int = 0,
                           head_dim: int = 0, page_size: int = 0, window: Optional[int] = None,
                           longest_span: int = 0, one_tile_only: bool = False, no_few: bool = False,
-                          window_on_tc: bool = False) -> Tuple[int, bool]:
+                          window_on_tc: bool = False, plain_scores: bool = False) -> Tuple[int, bool]:
     """``(query rows one attention CTA handles, the tcgen05 kernel's form for few rows)``.
 
     16 rows in the 32-bit kernel.  bfloat16 steps whose sizes the tcgen05 kernels take: 128 rows for
@@ -64,20 +64,26 @@ def attention_kernel_form(dtype: torch.dtype, decode_only: bool = False, group: 
     25 for eight, 74 to 93 against 105 to 111 for 64).  Otherwise 16 rows for decode steps
     of small groups and 64 in the bfloat16 mma.sync kernels.  ``one_tile_only``: of the tcgen05 kernels only
     the ones with a single query tile a piece may be chosen (they are the ones that take a bias by distance);
-    ``no_few``: nor the form for tiles of at most 16 rows (a window or a sink: the 128-row form alone takes them)."""
+    ``no_few``: nor the form for tiles of at most 16 rows (a window or a sink: the 128-row form alone takes them).
+    ``plain_scores`` (no bias by distance, no soft cap): heads of 64 and 256 go to the tcgen05 kernels too, 256 in the
+    128-row form alone, for decode steps as well."""
     if dtype != torch.bfloat16:
         return 16, False
     sized = bool(head_dim and page_size)
+    other = sized and plain_scores and ops.attention_tc_heads_fit(head_dim, page_size, group)
+    if other and head_dim > 128:
+        return (128, False) if decode_only or n_tokens >= TC_MIN_TOKENS else (64, False)
+    fits_as = 128 if other else head_dim  # (heads of 64: every form that heads of 128 have)
     if window is not None:  # (of the tcgen05 kernels the one with a single 128-row tile a piece takes a window)
         one_tile_only = no_few = True
     if decode_only:
         if sized and (not no_few or (window is not None and window_on_tc)) and longest_span >= TC_MIN_DECODE_SPAN:
-            if not no_few and ops.attention_tc_few_fits(head_dim, page_size, group):
+            if not no_few and ops.attention_tc_few_fits(fits_as, page_size, group):
                 return 16, True
-            if ops.attention_tc_fits(head_dim, page_size, group):
+            if ops.attention_tc_fits(fits_as, page_size, group):
                 return 128, False
         return (16 if group <= 16 else 64), False
-    tc = sized and ops.attention_tc_fits(head_dim, page_size, group)
+    tc = sized and ops.attention_tc_fits(fits_as, page_size, group)
     if tc and not one_tile_only and (n_tokens >= TC_PAIR_MIN_TOKENS or
                (n_tokens >= TC_PAIR_MIN_TOKENS_LONG and longest_span >= TC_PAIR_MIN_SPAN)):
         return 256, False
@@ -238,7 +244,8 @@ class GQAttention(Mixer):
         special = has_sink or self.window is not None
         return attention_kernel_form(self.env.dtype, decode_only, self.plan_group, n_tokens,
                                      self.pad_dim if sized else 0, page_size, self.window, longest_span,
-                                     one_tile_only=special or self.log_dist_bias, no_few=special, window_on_tc=True)
+                                     one_tile_only=special or self.log_dist_bias, no_few=special, window_on_tc=True,
+                                     plain_scores=not self.log_dist_bias)
 
     def tile_rows(self, decode_only: bool, n_tokens: int = 0, page_size: int = 0, longest_span: int = 0) -> int:
         return self.kernel_form(decode_only, n_tokens, page_size, longest_span)[0]
@@ -255,6 +262,7 @@ class GQAttention(Mixer):
         rows, few_rows = self.kernel_form(builder.decode_only, n_tokens, page_size, builder.longest_span())
         if rows >= 128 and not few_rows and not builder.decode_only and n_tokens >= TC_PAIR_MIN_TOKENS_LONG \
                 and self.sink is None and not self.learned_sink and not self.log_dist_bias and self.window is None \
+                and self.pad_dim <= 128 \
                 and hasattr(builder, "cheaper_attention_rows"):
             # one or two query tiles a piece: whichever work list the kernel is estimated to get through sooner
             rows = builder.cheaper_attention_rows(self.plan_group, self.window, self.plan_kv_heads, self.pad_dim)

@@ -21,7 +21,8 @@ Without a query latent (``q_rank = None``) the queries are a plain projection of
 the input projection.
 
 ``kv_rank + rot_dim`` may be at most 256 (the attention kernels' largest head); the tcgen05 kernels take it
-when it is 128.  The reference has no such layer.
+when it is 64, 128 or 256.  There the heads are taken in groups that fill a tile's 128 rows (:func:`tile_split`).  The
+reference has no such layer.
 """
 
 from __future__ import annotations
@@ -37,6 +38,27 @@ from ..kernels import ops
 from .attention import attention_kernel_form
 from .base import MIXERS, BuildEnv, Mixer, StepState
 from .rope import shared_position
+
+
+TC_SPLIT_GAIN = 1.1  # heads are split into more groups for a tcgen05 step when that fills so many times the rows of a tile
+
+
+def rows_filled(heads: int, split: int, rows: int = 128) -> int:
+    """Rows of a tile of ``rows`` that whole tokens fill when ``heads`` are taken in ``split`` groups."""
+    group = heads // split
+    return rows // group * group if group <= rows else 0
+
+
+def tile_split(heads: int) -> int:
+    """In how many groups a tcgen05 step takes ``heads`` query heads on one KV head.  Every group reads the keys again (from
+    L2), so the fewest groups that fit are taken unless more fill a tile better: 48 heads fill 96 of 128 rows, three times 16
+    all of them, a quarter fewer tiles."""
+    fits = [s for s in range(1, heads + 1) if heads % s == 0 and heads // s <= 128]
+    best = fits[0]
+    for s in fits[1:]:
+        if rows_filled(heads, s) >= TC_SPLIT_GAIN * rows_filled(heads, best):
+            best = s
+    return best
 
 
 @MIXERS.register("latent_attention")
@@ -84,6 +106,8 @@ class LatentAttention(Mixer):
         most = 16 if env.dtype != torch.bfloat16 else 64  # query heads on the one KV head that a tile's rows take
         self.kv_split = next(s for s in range(1, self.n_heads + 1) if self.n_heads % s == 0 and self.n_heads // s <= most)
         self.plan_group = self.n_heads // self.kv_split
+        self._tc_split = tile_split(self.n_heads)
+        self._tc_decode_split = next(s for s in range(1, self.n_heads + 1) if self.n_heads % s == 0 and self.n_heads // s <= 128)
         self._w_uk: Optional[torch.Tensor] = None
         self._w_uv: Optional[torch.Tensor] = None
 
@@ -124,22 +148,33 @@ class LatentAttention(Mixer):
         return rows + DEAL_MOST_PIECES * 148 * 256 * (self.pad_dim + 2) * 4
 
     # ------------------------------------------------------------------ step
+    def step_split(self, decode_only: bool, rows: int) -> int:
+        """The groups that a step whose attention runs in tiles of ``rows`` rows takes the heads in."""
+        if rows < 128:
+            return self.kv_split
+        return self._tc_decode_split if decode_only else self._tc_split
+
     def kernel_form(self, decode_only: bool, n_tokens: int = 0, page_size: int = 0, longest_span: int = 0):
         # (keys that are the values, a window and a sink together: the tiles of 16 / 64 rows take them, and of the
-        # tcgen05 kernels the one with a single 128-row tile a piece, whose head is 128 wide)
-        sized = self.kv_split == 1
-        return attention_kernel_form(self.env.dtype, decode_only, self.plan_group, n_tokens, self.pad_dim if sized else 0,
-                                     page_size, self.window, longest_span, one_tile_only=True, no_few=True)
+        # tcgen05 kernels the ones with a single 128-row tile a piece)
+        group = self.n_heads // (self._tc_decode_split if decode_only else self._tc_split)
+        rows, few = attention_kernel_form(self.env.dtype, decode_only, group, n_tokens, self.pad_dim, page_size, self.window,
+                                          longest_span, one_tile_only=True, no_few=True, plain_scores=True)
+        if rows < 128:
+            rows, few = attention_kernel_form(self.env.dtype, decode_only, self.plan_group, n_tokens)
+        return rows, few
 
     def plan_key(self, decode_only: bool = False, n_tokens: int = 0, page_size: int = 0, longest_span: int = 0):
         rows, few = self.kernel_form(decode_only, n_tokens, page_size, longest_span)
-        return ("attention", self.plan_group, rows, self.window, self.kv_split, self.pad_dim, few)
+        split = self.step_split(decode_only, rows)
+        return ("attention", self.n_heads // split, rows, self.window, split, self.pad_dim, few)
 
     def prepare(self, builder) -> None:
         n_tokens = sum(q for q, _ in builder.seg_lens)
         page_size = builder.engine.config.page_size if builder.engine is not None else 0
         rows, few = self.kernel_form(builder.decode_only, n_tokens, page_size, builder.longest_span())
-        self._step_plan = builder.attention_plan(self.plan_group, rows, self.window, self.kv_split, self.pad_dim, few)
+        split = self.step_split(builder.decode_only, rows)
+        self._step_plan = builder.attention_plan(self.n_heads // split, rows, self.window, split, self.pad_dim, few)
 
     def forward(self, h: torch.Tensor, step: StepState, cache: Any, writes_cache: bool) -> torch.Tensor:
         if not writes_cache:
@@ -164,7 +199,7 @@ class LatentAttention(Mixer):
         o = ws.get("latent.o", (T, H, P), dt, (cap, H, P))
         ops.paged_attention(qa, slab, slab, cache.block_table, step.seg_info, len(step.segments), plan.items_dev,
                             plan.n_items, plan.part_o, plan.part_ml, o, self._step_plan[2], self.scale, self.window,
-                            few_rows=self._step_plan[6], kv_split=self.kv_split, sink=self.params.get("sink"))
+                            few_rows=self._step_plan[6], kv_split=self._step_plan[4], sink=self.params.get("sink"))
         ov = ws.get("latent.ov", (T, H, Dv), dt, (cap, H, Dv))
         ops.heads_linear(o[:, :, :C], self._w_uv, ov)
         if self.head_gate:
