@@ -34,6 +34,8 @@ from ..errors import ConfigError
 from ..kernels import ops
 from .base import MIXERS, BuildEnv, Mixer, StepState
 
+CHUNK_MIN_TOKENS = 16  # steps in which some request brings so many tokens go in chunks where they can
+
 UNIT_EPS = 1e-6  # inside the root of the unit norms of q and k: fixed by the design
 
 
@@ -104,7 +106,8 @@ class GatedDelta(Mixer):
         item = 4 if self.env.dtype == torch.float32 else 2
         H, D, Dv = self.n_heads, self.head_dim, self.v_dim
         own = (self.proj_rows + self.conv_dim + H * Dv + self.hidden + (H * Dv if self.gate_rank else 0)) * item
-        return n_tokens * (own + (H * Dv + (H * D if self.decay_rank else 0)) * 4)
+        chunks = 0 if self.decay_rank else ops.delta_chunk_scratch(self.env.dtype, n_tokens, self.env.max_decode_rows, H, self.n_kv_heads, D, Dv)
+        return n_tokens * (own + (H * Dv + (H * D if self.decay_rank else 0)) * 4) + chunks
 
     def forward(self, h: torch.Tensor, step: StepState, cache: Any, writes_cache: bool) -> torch.Tensor:
         if not writes_cache:
@@ -124,9 +127,16 @@ class GatedDelta(Mixer):
             ops.linear_f32(a, self.params["decay_proj.weight"], z)
             a = None
         o32 = ws.get("delta.o32", (T, H, Dv), torch.float32, (cap, H, Dv))
+        args = dict(z=z)
+        if z is None and h.is_cuda and max(seg.q_len for seg in step.segments) >= CHUNK_MIN_TOKENS:
+            sizes = (H, self.n_kv_heads, D, Dv)
+            n = ops.delta_chunk_scratch(dt, T, n_segs, *sizes)
+            if n:
+                most = ops.delta_chunk_scratch(dt, cap, max(n_segs, self.env.max_decode_rows), *sizes)
+                args = dict(scratch=ws.get("delta.chunks", (n,), torch.uint8, (most,)))
         ops.delta_scan(qkv[:, : self.k_col], qkv[:, self.k_col: self.v_col], qkv[:, self.v_col:],
                        proj[:, self.b_col: self.a_col], a, self.params["A_log"], self.params["dt_bias"],
-                       D ** -0.5, UNIT_EPS, cache.tensors["s"], step.state_slots, step.seg_info, n_segs, o32, z=z)
+                       D ** -0.5, UNIT_EPS, cache.tensors["s"], step.state_slots, step.seg_info, n_segs, o32, **args)
         gate = proj[:, self.g_col: self.b_col]
         if self.gate_rank:
             low, gate = gate, ws.get("delta.gate", (T, H * Dv), dt, (cap, H * Dv))

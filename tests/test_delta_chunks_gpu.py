@@ -1,0 +1,135 @@
+"""The gated delta rule in chunks against the recurrence in float64, beside the kernel that takes a
+request's tokens one after the other."""
+
+import pytest
+import torch
+
+from freetoken_b200.kernels import ops
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+EPS = 1e-6
+
+
+def problem(lens, H, G, D, Dv, seed=0, a_log=-1.0, same_keys=False):
+    """lens: (tokens of this step, tokens after it) per request."""
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=g)  # noqa: E731
+    T = sum(n for n, _ in lens)
+    wide = rnd(T, 2 * G * D + H * Dv + 8).to(torch.bfloat16)
+    if same_keys:
+        wide[:, G * D:2 * G * D] = wide[:1, G * D:2 * G * D]
+    info, q0 = [], 0
+    for i, (n, kv) in enumerate(lens):
+        info.append([q0, n, kv, i])
+        q0 += n
+    state = rnd(len(lens) + 2, H, Dv, D) * 0.3
+    return dict(q=wide[:, :G * D], k=wide[:, G * D:2 * G * D], v=wide[:, 2 * G * D:2 * G * D + H * Dv], b=rnd(T, H).to(torch.bfloat16),
+                a=rnd(T, H).to(torch.bfloat16), a_log=rnd(H) * 0.5 + a_log, dt_bias=rnd(H) - 1.0, state=state,
+                slots=torch.randperm(len(lens) + 1, device=DEV, generator=g)[:len(lens)].to(torch.int32) + 1,
+                info=torch.tensor(info, dtype=torch.int32, device=DEV), T=T, sizes=(H, G, D, Dv))
+
+
+def run(p, chunks):
+    H, G, D, Dv = p["sizes"]
+    out = torch.full((p["T"], H, Dv), float("nan"), device=DEV)
+    state = p["state"].clone()
+    n = ops.delta_chunk_scratch(torch.bfloat16, p["T"], len(p["info"]), H, G, D, Dv)
+    scratch = torch.full((n,), 255, dtype=torch.uint8, device=DEV) if chunks else None
+    ops.variant_counts(reset=True)
+    ops.delta_scan(p["q"], p["k"], p["v"], p["b"], p["a"], p["a_log"], p["dt_bias"], D ** -0.5, EPS, state, p["slots"], p["info"],
+                   len(p["info"]), out, scratch=scratch)
+    assert bool(ops.variant_counts().get("delta rule: chunks of 32 tokens")) == chunks
+    return out, state
+
+
+def exact(p):
+    H, G, D, Dv = p["sizes"]
+    f = lambda x: x.double()  # noqa: E731
+    unit = lambda x: (x * torch.rsqrt((x * x).sum(-1, keepdim=True) + EPS)).repeat_interleave(H // G, dim=1)  # noqa: E731
+    q, k, v = unit(f(p["q"]).view(-1, G, D)) * D ** -0.5, unit(f(p["k"]).view(-1, G, D)), f(p["v"]).reshape(-1, H, Dv)
+    beta = torch.sigmoid(f(p["b"]))
+    g = torch.exp(-torch.exp(f(p["a_log"])) * torch.nn.functional.softplus(f(p["a"]) + f(p["dt_bias"]), threshold=1e9))
+    out, state = torch.empty(p["T"], H, Dv, dtype=torch.float64, device=DEV), p["state"].double()
+    for i, (q0, n, kv, _) in enumerate(p["info"].tolist()):
+        slot = int(p["slots"][i])
+        S = torch.zeros(H, Dv, D, dtype=torch.float64, device=DEV) if n == kv else state[slot].clone()
+        for t in range(q0, q0 + n):
+            S = S * g[t][:, None, None]
+            u = beta[t][:, None] * (v[t] - (S @ k[t][:, :, None])[..., 0])
+            S = S + u[:, :, None] * k[t][:, None, :]
+            out[t] = (S @ q[t][:, :, None])[..., 0]
+        state[slot] = S
+    return out, state
+
+
+def off(x, want):
+    return float((x.double() - want).norm() / want.norm())
+
+
+MIXED = [(1, 1), (31, 31), (32, 40), (33, 33), (1, 9), (64, 100), (65, 65), (95, 95), (2, 2)]
+
+
+@pytest.mark.parametrize("H,G,D,Dv", [(4, 2, 128, 128), (6, 1, 64, 16), (3, 3, 64, 48), (8, 8, 128, 32), (16, 4, 64, 64), (2, 1, 128, 80)])
+@pytest.mark.parametrize("lens,a_log,same", [(MIXED, -1.0, False), ([(300, 300)], -1.0, False), ([(129, 200), (40, 40)], 2.5, False),
+                                             ([(200, 200)], -6.0, True)])
+def test_chunks_against_the_recurrence(H, G, D, Dv, lens, a_log, same):
+    """Ordinary decays, decays of e^-12 a token and of nearly one, and keys that are all the same."""
+    p = problem(lens, H, G, D, Dv, seed=H + Dv, a_log=a_log, same_keys=same)
+    want, want_state = exact(p)
+    (out, state), (out1, state1) = run(p, True), run(p, False)
+    # both add a few dozen 32-bit roundings of 2^-24 to a state that decays: 1e-6 with room; and the chunks lose nothing
+    for got, plain, w in ((out, out1, want), (state, state1, want_state)):
+        assert torch.isfinite(got).all()
+        assert off(got, w) < 1e-6, (off(got, w), off(plain, w))
+        # (keys that are all the same: every entry of the chunk's triangle counts, and is rounded)
+        assert off(got, w) <= max((1.4 if same else 1.1) * off(plain, w), 1e-7), (off(got, w), off(plain, w))
+    torch.testing.assert_close(out.double(), want, rtol=1e-4, atol=2e-5)
+    untouched = [s for s in range(state.shape[0]) if s not in p["slots"].tolist()]
+    assert torch.equal(state[untouched], p["state"][untouched])
+
+
+@pytest.mark.parametrize("a_log", [-6.0, -1.0])
+def test_a_long_prompt_loses_no_precision(a_log):
+    p = problem([(2048, 2048)], 4, 2, 128, 64, seed=5, a_log=a_log)
+    want, want_state = exact(p)
+    (out, state), (out1, state1) = run(p, True), run(p, False)
+    slots = p["slots"].tolist()
+    state, state1, want_state = state[slots], state1[slots], want_state[slots]
+    assert off(out, want) <= off(out1, want)
+    assert off(state, want_state) <= off(state1, want_state)
+
+
+def test_a_prompt_cut_anywhere():
+    whole = problem([(200, 200)], 4, 2, 128, 32, seed=2)
+    want, want_state = run(whole, True)
+    for cuts in ((32, 168), (1, 199), (100, 100), (33, 31, 136)):
+        state, at, outs = whole["state"].clone(), 0, []
+        for n in cuts:
+            part = {k: (v[at:at + n] if k in ("q", "k", "v", "b", "a") else v) for k, v in whole.items()}
+            part.update(T=n, state=state, info=torch.tensor([[0, n, at + n, 0]], dtype=torch.int32, device=DEV))
+            out, state = run(part, True)
+            outs.append(out)
+            at += n
+        torch.testing.assert_close(torch.cat(outs), want, rtol=1e-5, atol=2e-6)
+        torch.testing.assert_close(state, want_state, rtol=1e-5, atol=2e-6)
+
+
+def test_what_is_not_taken_goes_token_by_token():
+    assert ops.delta_chunk_scratch(torch.float32, 64, 1, 4, 2, 128, 64) == 0
+    for H, G, D, Dv in ((4, 2, 96, 64), (4, 2, 128, 40), (4, 2, 256, 64)):
+        assert ops.delta_chunk_scratch(torch.bfloat16, 64, 1, H, G, D, Dv) == 0
+        assert ops._lib().ftk_delta_chunk_scratch(1, 64, 1, H, G, D, Dv) == 0
+    for T, S in ((1, 1), (31, 1), (33, 2), (2048, 7)):
+        assert ops.delta_chunk_scratch(torch.bfloat16, T, S, 4, 2, 128, 64) == ops._lib().ftk_delta_chunk_scratch(1, T, S, 4, 2, 128, 64)
+    p = problem([(40, 40)], 4, 2, 128, 32)
+    p["k"] = torch.cat([p["k"], p["k"][:, :4]], dim=1)[:, :256]  # rows of 260: no 16-byte copies
+    out, _ = run(dict(p, k=p["k"].contiguous()), True)
+    assert p["k"].stride(0) % 8
+    scratch = torch.empty(ops.delta_chunk_scratch(torch.bfloat16, 40, 1, 4, 2, 128, 32), dtype=torch.uint8, device=DEV)
+    got, state = torch.empty_like(out), p["state"].clone()
+    ops.variant_counts(reset=True)
+    ops.delta_scan(p["q"], p["k"], p["v"], p["b"], p["a"], p["a_log"], p["dt_bias"], 128 ** -0.5, EPS, state, p["slots"], p["info"], 1, got,
+                   scratch=scratch)
+    assert not ops.variant_counts().get("delta rule: chunks of 32 tokens")
+    torch.testing.assert_close(got, out, rtol=1e-4, atol=2e-5)
