@@ -193,7 +193,7 @@ _SIGNATURES = {
     "ftk_ssm_output": [_vp, _vp, ctypes.c_longlong, _vp, _vp, ctypes.c_longlong, _i, _vp, _i, _f, _vp, _i, _i, _i, _vp],
     "ftk_norm_mean": [ctypes.POINTER(_vp), ctypes.POINTER(_vp), _i, _i, _f, _vp, _i, _i, _vp],
 }
-_bound = False
+_bound: Any = None  # the library, its signatures declared
 _launches = 0
 
 
@@ -209,14 +209,14 @@ def count_launches(n: int) -> None:
 
 def _lib():
     global _bound
-    lib = library.load()
-    if not _bound:
+    if _bound is None:
+        lib = library.load()
         for name, args in _SIGNATURES.items():
             fn = getattr(lib, name)
             fn.argtypes = args
             fn.restype = _i
-        _bound = True
-    return lib
+        _bound = lib
+    return _bound
 
 
 def _check(status: int, name: str, launches: int = 1) -> None:
@@ -228,7 +228,8 @@ def _check(status: int, name: str, launches: int = 1) -> None:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    # (the handle itself: torch.cuda.current_stream() makes a stream object of it first, 3 us a launch)
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _code(t: torch.Tensor, what: str) -> int:
@@ -242,13 +243,13 @@ def _code(t: torch.Tensor, what: str) -> int:
 def _dev(t: Optional[torch.Tensor], what: str, dtype: Optional[torch.dtype] = None) -> Optional[int]:
     if t is None:
         return None
+    if t.is_cuda and t.is_contiguous() and (dtype is None or t.dtype == dtype):
+        return t.data_ptr()
     if not t.is_cuda:
         raise KernelError(f"{what}: tensor is on '{t.device}', the kernels run on a CUDA device only")
     if not t.is_contiguous():
         raise KernelError(f"{what}: tensor must be contiguous")
-    if dtype is not None and t.dtype != dtype:
-        raise KernelError(f"{what}: expected {dtype}, got {t.dtype}")
-    return t.data_ptr()
+    raise KernelError(f"{what}: expected {dtype}, got {t.dtype}")
 
 
 def read_status() -> int:
@@ -422,41 +423,41 @@ def norm_rope_store(x: torch.Tensor, head_dim: int, rotary_dim: int, positions: 
     """
     T = x.shape[0]
     n_total = x.shape[1] // head_dim
-    arr = (_Section * len(sections))()
-    keep = []
-    for i, s in enumerate(sections):
-        if s["first_head"] + s["n_heads"] > n_total:
+    arr = (_Section * len(sections))()  # (zeros: what a section does not name stays as it is)
+    for sec, s in zip(arr, sections):
+        first, n, get = s["first_head"], s["n_heads"], s.get
+        if first + n > n_total:
             raise KernelError("norm_rope_store: section exceeds the heads of x")
-        arr[i].first_head = s["first_head"]
-        arr[i].n_heads = s["n_heads"]
-        arr[i].norm_weight = _dev(s.get("norm_weight"), "norm_weight", torch.float32)
-        arr[i].rotate = 1 if s.get("rotate") else 0
-        dense, slab = s.get("dense_out"), s.get("slab")
+        sec.first_head, sec.n_heads = first, n
+        weight, bias, pos_scale, dense, slab = get("norm_weight"), get("bias"), get("pos_scale"), get("dense_out"), get("slab")
+        if weight is not None:
+            sec.norm_weight = _dev(weight, "norm_weight", torch.float32)
+        if get("rotate"):
+            sec.rotate = 1
         if (dense is None) == (slab is None):
             raise KernelError("norm_rope_store: a section needs exactly one of dense_out and slab")
-        dst_dim = int(s.get("dst_head_dim") or head_dim)
-        arr[i].dst_head_dim = dst_dim if dst_dim != head_dim else 0
-        bias, pos_scale = s.get("bias"), s.get("pos_scale")
-        if bias is not None and bias.numel() != s["n_heads"] * head_dim:
-            raise KernelError("norm_rope_store: a section's bias must hold n_heads * head_dim entries")
-        arr[i].bias = _dev(bias, "bias", torch.float32)
-        arr[i].pos_scale = _dev(pos_scale, "pos_scale", torch.float32)
-        arr[i].pos_scale_len = pos_scale.numel() if pos_scale is not None else 0
+        dst_dim = int(get("dst_head_dim") or head_dim)
+        if dst_dim != head_dim:
+            sec.dst_head_dim = dst_dim
+        if bias is not None:
+            if bias.numel() != n * head_dim:
+                raise KernelError("norm_rope_store: a section's bias must hold n_heads * head_dim entries")
+            sec.bias = _dev(bias, "bias", torch.float32)
+        if pos_scale is not None:
+            sec.pos_scale, sec.pos_scale_len = _dev(pos_scale, "pos_scale", torch.float32), pos_scale.numel()
         if dense is not None:
-            if dense.dtype != x.dtype or dense.numel() != T * s["n_heads"] * dst_dim:
+            if dense.dtype != x.dtype or dense.numel() != T * n * dst_dim:
                 raise KernelError("norm_rope_store: dense_out has the wrong dtype or size")
-            arr[i].dense_out = _dev(dense, "dense_out")
+            sec.dense_out = _dev(dense, "dense_out")
         else:
-            if slab.dtype != x.dtype or slab.dim() != 4 or slab.shape[1] != s["n_heads"] \
-                    or slab.shape[3] != dst_dim:
+            shape = slab.shape
+            if slab.dtype != x.dtype or len(shape) != 4 or shape[1] != n or shape[3] != dst_dim:
                 raise KernelError("norm_rope_store: slab must be [pages, n_heads, page_size, head_dim]")
-            arr[i].slab = _dev(slab, "slab")
-            arr[i].slot_map = _dev(s["slot_map"], "slot_map", torch.int32)
-            if s["slot_map"].shape[0] < T:
+            slots = s["slot_map"]
+            sec.slab, sec.slot_map = _dev(slab, "slab"), _dev(slots, "slot_map", torch.int32)
+            if slots.shape[0] < T:
                 raise KernelError("norm_rope_store: slot_map shorter than the tokens")
-            arr[i].num_pages = slab.shape[0]
-            arr[i].page_size = slab.shape[2]
-        keep.append(s)
+            sec.num_pages, sec.page_size = shape[0], shape[2]
     if rotary_dim:
         if rope_table is None or rope_table.shape[1] != rotary_dim:
             raise KernelError("norm_rope_store: rope_table must be [max_pos, rotary_dim]")
@@ -789,7 +790,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[t
             and _room(x) >= P * K and _room(out) >= P * N):
         torch.matmul(x.as_strided((P, K), (K, 1)), w.t(), out=out.as_strided((P, N), (N, 1)))
     else:
-        torch.matmul(x, w.t(), out=out)
+        torch.mm(x, w.t(), out=out)
 
 
 def linear_f32(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:

@@ -111,6 +111,9 @@ class BuildEnv:
     shared: Dict[Any, Any] = field(default_factory=dict)  # parts shared by spec (rope tables)
 
 
+MOST_VIEWS = 1024  # views of work buffers that a workspace keeps to hand out again
+
+
 class Workspace:
     """Named device buffers that live as long as the engine.
 
@@ -123,9 +126,14 @@ class Workspace:
     def __init__(self, device: torch.device):
         self.device = device
         self._buffers: Dict[Any, torch.Tensor] = {}
+        self._views: Dict[Any, torch.Tensor] = {}  # the views handed out since the last allocation
 
     def get(self, name: str, shape: Tuple[int, ...], dtype: torch.dtype,
             max_shape: Optional[Tuple[int, ...]] = None) -> torch.Tensor:
+        key = (name, shape, dtype)
+        view = self._views.get(key)
+        if view is not None:
+            return view
         n = 1
         for s in shape:
             n *= s
@@ -140,7 +148,11 @@ class Workspace:
                 cap = max(cap, n)
             buf = torch.empty(max(cap, 1), dtype=dtype, device=self.device)
             self._buffers[name] = buf
-        return buf[:n].view(shape)
+            self._views.clear()
+        if len(self._views) >= MOST_VIEWS:  # (steps of ever other lengths)
+            self._views.clear()
+        view = self._views[key] = buf[:n].view(shape)
+        return view
 
     def nbytes(self) -> int:
         return sum(b.numel() * b.element_size() for b in self._buffers.values())
