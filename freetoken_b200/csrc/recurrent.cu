@@ -13,6 +13,7 @@
 //      L would lie, so that step 3 never reads a slot that its last chunk is writing;
 //   3. every chunk runs the recurrence from its start state and writes its tokens' outputs; a
 //      segment's last chunk leaves the final state in the slot.
+// (Sizes that gla_chunks.cuh takes go there instead: the same three steps as matrix products.)
 // The recurrence itself is the plain one, token by token, so the result differs from a pure scan only
 // by the rounding of step 2's sums.
 //
@@ -109,11 +110,12 @@ __device__ __forceinline__ void rotated4(const R* row, const float* cs, int d, i
   }
 }
 
-__device__ __forceinline__ float decay_of(float z, float inv_tau) {
+__device__ __forceinline__ float log_decay_of(float z, float inv_tau) {
   // sigmoid(z)^(1 / tau) = exp(-softplus(-z) / tau)
-  const float sp = z > 0.f ? log1pf(expf(-z)) : -z + log1pf(expf(z));
-  return expf(-sp * inv_tau);
+  const float sp = fmaxf(-z, 0.f) + log1pf(expf(-fabsf(z)));
+  return -sp * inv_tau;
 }
+__device__ __forceinline__ float decay_of(float z, float inv_tau) { return expf(log_decay_of(z, inv_tau)); }
 
 __global__ void gla_decay_kernel(float* z, const float* __restrict__ bias, long long n, int hd, float inv_tau) {
   pdl_wait();
@@ -529,8 +531,15 @@ __global__ void gla_carry_kernel(GlaArgs a) {
   }
 }
 
+}  // namespace ftk
+
+#include "gla_chunks.cuh"
+
+namespace ftk {
+
 template <typename T, int DPT>
-static int launch_gla(GlaArgs a, bool any_single, bool any_multi, cudaStream_t s) {
+static int launch_gla(GlaArgs a, bool any_single, bool any_multi, int longest_chunk, cudaStream_t s) {
+  const bool products = any_multi && sizeof(T) == 2 && gla_chunks_fit(a, longest_chunk);
   const int Dp = DPT * kGlaSlices;
   constexpr int kGlaCols = 32 * gla_cols_per_thread(DPT);
   const int dv_real = a.Dv - a.ones_col;  // the column of ones rides in the block of the first columns
@@ -551,7 +560,7 @@ static int launch_gla(GlaArgs a, bool any_single, bool any_multi, cudaStream_t s
     cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     cudaFuncSetAttribute(k3, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   }
-  if (any_multi && !a.a_head) {  // the decays of all of the step's tokens, once, where the logits lay
+  if (any_multi && !products && !a.a_head) {  // the decays of all of the step's tokens, once, where the logits lay
     const long long n = (long long)a.n_tokens * a.H * a.D;
     const unsigned blocks = (unsigned)((n + 255) / 256 < 148 * 16 ? (n + 255) / 256 : 148 * 16);
     FTK_LAUNCH(gla_decay_kernel, blocks, 256, 0, s, a.z, a.z_bias, n, a.H * a.D, a.inv_tau);
@@ -562,6 +571,7 @@ static int launch_gla(GlaArgs a, bool any_single, bool any_multi, cudaStream_t s
     FTK_LAUNCH(k0, grid, threads, smem, s, a);
     FTK_LAUNCH_CHECK("gla_scan (one chunk per request)");
   }
+  if (products) return launch_gla_chunks(a, s);
   if (any_multi) {
     FTK_LAUNCH(k1, grid, threads, smem, s, a);
     FTK_LAUNCH_CHECK("gla_scan (chunk contributions)");
@@ -587,6 +597,21 @@ extern "C" int ftk_gla_scan(const void* q, long long q_stride, const void* k, lo
                             float* decay_prod, float* out, int n_tokens, int n_heads, int dim, int vdim,
                             const float* k_fac, const float* a_head, int a_head_stride, int ones_col, float* out_ones,
                             int qk_div, const float* rope, int n_rot, int rope_neighbours, int max_pos, void* stream) {
+  return ftk_gla_scan_chunks(q, q_stride, k, k_stride, v, v_stride, dtype, z, z_bias, tau, q_scale, state, n_slots, state_slots,
+                             seg_info, n_segs, chunks, n_chunks, seg_chunks, any_single, any_multi, carry, decay_prod, out,
+                             n_tokens, n_heads, dim, vdim, k_fac, a_head, a_head_stride, ones_col, out_ones, qk_div, rope, n_rot,
+                             rope_neighbours, max_pos, 0, stream);
+}
+
+extern "C" int ftk_gla_scan_chunks(const void* q, long long q_stride, const void* k, long long k_stride, const void* v,
+                            long long v_stride, int dtype, float* z, const float* z_bias, float tau,
+                            float q_scale, float* state, int n_slots, const int32_t* state_slots,
+                            const int32_t* seg_info, int n_segs, const int32_t* chunks, int n_chunks,
+                            const int32_t* seg_chunks, int any_single, int any_multi, float* carry,
+                            float* decay_prod, float* out, int n_tokens, int n_heads, int dim, int vdim,
+                            const float* k_fac, const float* a_head, int a_head_stride, int ones_col, float* out_ones,
+                            int qk_div, const float* rope, int n_rot, int rope_neighbours, int max_pos, int longest_chunk,
+                            void* stream) {
   FTK_REQUIRE(dtype_ok(dtype), "gla_scan: bad dtype %d", dtype);
   FTK_REQUIRE(n_tokens >= 0 && n_segs >= 0 && n_chunks >= 0, "gla_scan: bad counts");
   if (n_tokens == 0 || n_chunks == 0) return 0;
@@ -614,10 +639,11 @@ extern "C" int ftk_gla_scan(const void* q, long long q_stride, const void* k, lo
   a.k_fac = k_fac; a.a_head = a_head; a.ones_col = ones_col; a.out_ones = out_ones; a.qk_div = qk_div;
   a.out = out; a.H = n_heads; a.D = dim; a.Dv = vdim; a.n_tokens = n_tokens;
   cudaStream_t s = (cudaStream_t)stream;
-  note_variant(any_multi ? "gla_scan: chunks side by side" : "gla_scan: one chunk per request");
+  note_variant(!any_multi ? "gla_scan: one chunk per request"
+               : dtype == FTK_BF16 && gla_chunks_fit(a, longest_chunk) ? "gla_scan: chunks as products" : "gla_scan: chunks side by side");
   const bool f32 = dtype == FTK_F32;
-  if (dim <= 32) return f32 ? launch_gla<float, 8>(a, any_single, any_multi, s) : launch_gla<__nv_bfloat16, 8>(a, any_single, any_multi, s);
-  if (dim <= 64) return f32 ? launch_gla<float, 16>(a, any_single, any_multi, s) : launch_gla<__nv_bfloat16, 16>(a, any_single, any_multi, s);
-  if (dim <= 128) return f32 ? launch_gla<float, 32>(a, any_single, any_multi, s) : launch_gla<__nv_bfloat16, 32>(a, any_single, any_multi, s);
-  return f32 ? launch_gla<float, 64>(a, any_single, any_multi, s) : launch_gla<__nv_bfloat16, 64>(a, any_single, any_multi, s);
+  if (dim <= 32) return f32 ? launch_gla<float, 8>(a, any_single, any_multi, longest_chunk, s) : launch_gla<__nv_bfloat16, 8>(a, any_single, any_multi, longest_chunk, s);
+  if (dim <= 64) return f32 ? launch_gla<float, 16>(a, any_single, any_multi, longest_chunk, s) : launch_gla<__nv_bfloat16, 16>(a, any_single, any_multi, longest_chunk, s);
+  if (dim <= 128) return f32 ? launch_gla<float, 32>(a, any_single, any_multi, longest_chunk, s) : launch_gla<__nv_bfloat16, 32>(a, any_single, any_multi, longest_chunk, s);
+  return f32 ? launch_gla<float, 64>(a, any_single, any_multi, longest_chunk, s) : launch_gla<__nv_bfloat16, 64>(a, any_single, any_multi, longest_chunk, s);
 }

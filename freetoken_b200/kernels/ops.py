@@ -182,6 +182,9 @@ _SIGNATURES = {
     "ftk_gla_scan": [_vp, ctypes.c_longlong, _vp, ctypes.c_longlong, _vp, ctypes.c_longlong, _i, _vp, _vp, _f, _f,
                      _vp, _i, _vp, _vp, _i, _vp, _i, _vp, _i, _i, _vp, _vp, _vp, _i, _i, _i, _i, _vp, _vp, _i, _i, _vp, _i,
                      _vp, _i, _i, _i, _vp],
+    "ftk_gla_scan_chunks": [_vp, ctypes.c_longlong, _vp, ctypes.c_longlong, _vp, ctypes.c_longlong, _i, _vp, _vp, _f, _f,
+                     _vp, _i, _vp, _vp, _i, _vp, _i, _vp, _i, _i, _vp, _vp, _vp, _i, _i, _i, _i, _vp, _vp, _i, _i, _vp, _i,
+                     _vp, _i, _i, _i, _i, _vp],
     "ftk_hyper_step": [_vp, ctypes.c_longlong, _i, _i, _i, _vp, _vp, _i, _vp, _vp, _vp, _vp, _f, _vp, _i, _vp, _vp],
     "ftk_conv_act": [_vp, ctypes.c_longlong, _i, _vp, _vp, _i, _i, _vp, _i, _vp, _vp, _i, _vp, _i, _i, _vp],
     "ftk_delta_scan_chunks": [_vp, ctypes.c_longlong, _vp, ctypes.c_longlong, _vp, ctypes.c_longlong, _vp, ctypes.c_longlong,
@@ -1162,12 +1165,12 @@ def gla_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: Optional[torc
              any_multi: bool, carry: Optional[torch.Tensor], decay_prod: Optional[torch.Tensor],
              out: torch.Tensor, k_fac: Optional[torch.Tensor] = None, a_head: Optional[torch.Tensor] = None,
              ones_col: bool = False, out_ones: Optional[torch.Tensor] = None, qk_div: int = 1,
-             rope_table: Optional[torch.Tensor] = None, neighbours: bool = False) -> None:
+             rope_table: Optional[torch.Tensor] = None, neighbours: bool = False, chunk: int = 0) -> None:
     """Gated linear attention of the step's tokens, per (request, head):
     ``S <- diag(a_t) S + k_t v_t^T``, ``o_t = S^T (q_t q_scale)``, ``a_t = sigmoid(z_t + z_bias)^(1 / tau)``.
 
     ``q, k [T, H * D]`` and ``v [T, H * Dv]`` of the engine's dtype (views of adjacent columns of a wider
-    tensor are fine); ``z [T, H * D]`` float32 (overwritten with the decays when a segment has several chunks); ``state [slots, H, D, Dv]`` float32, read from and left in
+    tensor are fine); ``z [T, H * D]`` float32 (overwritten when a segment has several chunks); ``state [slots, H, D, Dv]`` float32, read from and left in
     the slot ``state_slots[segment]`` (a segment with ``kv_len == q_len`` starts from zero);
     ``chunks [n, 4]`` / ``seg_chunks [S, 2]`` from :func:`freetoken_b200.parts.gla.chunk_list`; ``carry
     [n, H, D, Dv]`` and ``decay_prod [n, H, D]`` float32 scratch for segments of several chunks;
@@ -1185,7 +1188,10 @@ def gla_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: Optional[torc
 
     ``rope_table [max_pos, n_rot]`` (cos then sin, with ``a_head`` only): the first ``n_rot`` dimensions of every query and
     key are rotated by the token's position as they are read, in 32 bits (they are never rounded); pairs as in
-    :func:`norm_rope_store`."""
+    :func:`norm_rope_store`.
+
+    ``chunk`` (0: not known): no chunk of the list is longer.  Chunks of 32 to 64 tokens may then go as matrix products
+    (``csrc/gla_chunks.cuh``), with ``z`` and ``out`` as scratch on the way."""
     T = out.shape[0]
     H, D, Dv = state.shape[1], state.shape[2], state.shape[3]
     qk_div = int(qk_div)
@@ -1215,7 +1221,7 @@ def gla_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: Optional[torc
     if chunks.numel() < 4 * n_chunks or seg_chunks.numel() < 2 * n_segs:
         raise KernelError("gla_scan: chunk lists too short")
     launches = (1 if any_single else 0) + ((4 if a_head is None else 3) if any_multi else 0)
-    _check(_lib().ftk_gla_scan(
+    _check(_lib().ftk_gla_scan_chunks(
         q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), _code(q, "q"),
         _dev(z, "z", torch.float32), _dev(z_bias, "z_bias", torch.float32), float(tau), float(q_scale),
         _dev(state, "state", torch.float32), state.shape[0], _dev(state_slots, "state_slots", torch.int32),
@@ -1226,7 +1232,7 @@ def gla_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: Optional[torc
         _dev(a_head, "a_head", torch.float32), 0 if one_row else H, 1 if ones_col else 0,
         _dev(out_ones, "out_ones", torch.float32), qk_div, _dev(rope_table, "rope_table", torch.float32),
         rope_table.shape[1] if rope_table is not None else 0, 1 if neighbours else 0,
-        rope_table.shape[0] if rope_table is not None else 0, _stream()), "gla_scan", max(1, launches))
+        rope_table.shape[0] if rope_table is not None else 0, int(chunk), _stream()), "gla_scan", max(1, launches))
 
 
 # --------------------------------------------------------------------------- short convolution, depth mix

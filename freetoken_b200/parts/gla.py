@@ -147,10 +147,11 @@ class GatedLinearAttention(Mixer):
             carry = ws.get("gla.carry", (n_chunks, H, D, Dv), torch.float32, (most, H, D, Dv))
             decay = ws.get("gla.decay", (n_chunks, H, D), torch.float32, (most, H, D))
         o32 = ws.get("gla.o32", (T, H, Dv), torch.float32, (cap, H, Dv))
+        known = dict(chunk=self.chunk) if h.is_cuda else {}
         ops.gla_scan(proj[:, : self.k_row], proj[:, self.k_row: self.v_row], proj[:, self.v_row: self.g_row], z,
                      self.params["decay_proj.bias"], self.tau, self.q_scale, cache.tensors["s"], step.state_slots,
                      step.seg_info, len(step.segments), tensors[name], n_chunks, tensors[name + ".segments"],
-                     single, multi, carry, decay, o32)
+                     single, multi, carry, decay, o32, **known)
         o = ws.get("gla.o", (T, H, Dv), dt, (cap, H, Dv))
         ops.gated_heads(o32, proj[:, self.g_row: self.a_row], o, Dv, "silu", self.params["norm.weight"], self.eps)
         out = ws.get("gla.out", (T, self.hidden), dt, (cap, self.hidden))

@@ -105,10 +105,11 @@ class Retention(Mixer):
             carry = ws.get("gla.carry", (n_chunks, H, D, Dv), torch.float32, (most, H, D, Dv))
             decay = ws.get("gla.decay", (n_chunks, H, D), torch.float32, (most, H, D))
         o32 = ws.get("retention.o32", (T, H, Dv), torch.float32, (cap, H, Dv))
+        known = dict(chunk=self.chunk) if h.is_cuda else {}
         ops.gla_scan(proj[:, : self.k_row], proj[:, self.k_row: self.v_row], proj[:, self.v_row: self.g_row], None, None,
                      1.0, D ** -0.5, cache.tensors["s"], step.state_slots, step.seg_info, len(step.segments), tensors[name],
                      n_chunks, tensors[name + ".segments"], single, multi, carry, decay, o32, a_head=self._decay,
-                     rope_table=self.position.table(), neighbours=bool(getattr(self.position, "interleaved", False)))
+                     rope_table=self.position.table(), neighbours=bool(getattr(self.position, "interleaved", False)), **known)
         o = ws.get("retention.o", (T, H, Dv), dt, (cap, H, Dv))
         ops.gated_heads(o32, proj[:, self.g_row:], o, Dv, "silu", self._ones, self.eps)
         out = ws.get("retention.out", (T, self.hidden), dt, (cap, self.hidden))
