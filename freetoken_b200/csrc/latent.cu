@@ -133,6 +133,59 @@ __global__ void latent_query_rotate_kernel(const T* __restrict__ q, int n_heads,
   }
 }
 
+// The same for bfloat16 rows whose offsets allow 16-byte accesses: a thread takes eight adjacent values of a head's rotated part
+// (or of the zeros behind it) and, where the pairs are halves apart, the eight they are turned with.  No shared memory and no
+// barrier: the kernel above has two values in flight a thread between two barriers, and is bound by that latency (2,048 tokens,
+// 48 heads, 64 rotated values, 25 MB in and out: 28.4 us, this one 8.6 us).
+__global__ void __launch_bounds__(256) latent_query_rotate_vec_kernel(const __nv_bfloat16* __restrict__ q, int n_heads, int flat_dim,
+                                                                      int rot_dim, int n_rot, int interleaved,
+                                                                      const int32_t* __restrict__ positions,
+                                                                      const float* __restrict__ table, int max_pos,
+                                                                      __nv_bfloat16* __restrict__ q_out, int kv_rank, int pad_dim,
+                                                                      int n_vecs) {
+  pdl_wait();
+  pdl_trigger();
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= n_vecs) return;
+  const int per_row = (pad_dim - kv_rank) >> 3, row = i / per_row, d = (i - row * per_row) * 8, t = row / n_heads;
+  uint4 res = make_uint4(0u, 0u, 0u, 0u);
+  if (d < rot_dim) {
+    const __nv_bfloat16* src = q + (size_t)row * (flat_dim + rot_dim) + flat_dim;
+    res = *reinterpret_cast<const uint4*>(src + d);
+    if (d < n_rot) {
+      const int half = n_rot >> 1, pos = min(max(positions[t], 0), max_pos - 1);
+      const float* tab = table + (size_t)pos * n_rot;
+      const bool low = d < half;
+      const int at = interleaved ? d >> 1 : low ? d : d - half;
+      float c[8], s[8];
+      Vec4<float>::load(tab + at, reinterpret_cast<float (&)[4]>(c[0]));
+      Vec4<float>::load(tab + half + at, reinterpret_cast<float (&)[4]>(s[0]));
+      uint4 other = res;
+      if (!interleaved) {
+        other = *reinterpret_cast<const uint4*>(src + (low ? d + half : d - half));
+        Vec4<float>::load(tab + at + 4, reinterpret_cast<float (&)[4]>(c[4]));
+        Vec4<float>::load(tab + half + at + 4, reinterpret_cast<float (&)[4]>(s[4]));
+      }
+      __nv_bfloat162* v2 = reinterpret_cast<__nv_bfloat162*>(&res);
+      const __nv_bfloat162* o2 = reinterpret_cast<const __nv_bfloat162*>(&other);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float2 v = __bfloat1622float2(v2[u]), o = __bfloat1622float2(o2[u]);
+        float2 y;
+        if (interleaved) {
+          y.x = v.x * c[u] - v.y * s[u];
+          y.y = v.y * c[u] + v.x * s[u];
+        } else {
+          y.x = low ? v.x * c[2 * u] - o.x * s[2 * u] : v.x * c[2 * u] + o.x * s[2 * u];
+          y.y = low ? v.y * c[2 * u + 1] - o.y * s[2 * u + 1] : v.y * c[2 * u + 1] + o.y * s[2 * u + 1];
+        }
+        v2[u] = __floats2bfloat162_rn(y.x, y.y);
+      }
+    }
+  }
+  *reinterpret_cast<uint4*>(q_out + (size_t)row * pad_dim + kv_rank + d) = res;
+}
+
 }  // namespace ftk
 
 using namespace ftk;
@@ -173,14 +226,24 @@ extern "C" int ftk_latent_query_rotate(const void* q, int dtype, int n_heads, in
               pad_dim >= kv_rank + rot_dim && n_tokens >= 0, "latent_query_rotate: bad sizes");
   if (n_tokens == 0 || pad_dim == kv_rank) return 0;
   FTK_REQUIRE(q && positions && q_out && (n_rot == 0 || table), "latent_query_rotate: null pointer");
+  cudaStream_t s = (cudaStream_t)stream;
+  const float* tab = n_rot ? table : nullptr;
+  const long long vecs = (long long)n_tokens * n_heads * ((pad_dim - kv_rank) / 8);
+  const uintptr_t at = (uintptr_t)q | (uintptr_t)q_out | (uintptr_t)tab;
+  if (dtype == FTK_BF16 && (flat_dim | rot_dim | kv_rank | pad_dim) % 8 == 0 && n_rot % (interleaved ? 8 : 16) == 0 && at % 16 == 0 &&
+      vecs <= 0x7fffff00LL) {
+    note_variant("latent_query_rotate: eight values a thread");
+    FTK_LAUNCH(latent_query_rotate_vec_kernel, (unsigned)((vecs + 255) / 256), 256, 0, s, (const __nv_bfloat16*)q, n_heads, flat_dim,
+               rot_dim, n_rot, interleaved, positions, tab, max_pos, (__nv_bfloat16*)q_out, kv_rank, pad_dim, (int)vecs);
+    FTK_LAUNCH_CHECK("latent_query_rotate");
+    return 0;
+  }
   // a block takes a token's heads in groups that give its 128 threads two values each to read and pad_dim - kv_rank to write
   const int per = max(1, min(n_heads, 256 / max(rot_dim, 1)));
   const size_t smem = (size_t)per * rot_dim * sizeof(float) + 16;
   FTK_REQUIRE(smem <= 48 * 1024, "latent_query_rotate: %d rotated values a head do not fit", rot_dim);
   FTK_REQUIRE((n_heads + per - 1) / per <= 65535, "latent_query_rotate: too many heads");
   const dim3 grid(n_tokens, (n_heads + per - 1) / per);
-  cudaStream_t s = (cudaStream_t)stream;
-  const float* tab = n_rot ? table : nullptr;
   if (dtype == FTK_F32)
     FTK_LAUNCH(latent_query_rotate_kernel<float>, grid, 128, smem, s, (const float*)q, n_heads, flat_dim, rot_dim, n_rot,
                interleaved, positions, tab, max_pos, (float*)q_out, kv_rank, pad_dim, per);

@@ -174,6 +174,27 @@ __global__ void head_gate_kernel(T* __restrict__ o, const T* __restrict__ g, lon
   for (int d = lane; d < head_dim; d += 32) row[d] = from_float<T>(to_float(row[d]) * s);
 }
 
+// The same for bfloat16 heads of 8 k elements on 16-byte addresses: a thread takes eight (2,048 tokens, 48 heads of 128, 50 MB in
+// and out: two bytes an access 26.8 us, this 9.5 us).
+__global__ void __launch_bounds__(256) head_gate_vec_kernel(__nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ g, long long g_stride,
+                                                            int n_heads, int per_row, int n_vecs) {
+  pdl_wait();
+  pdl_trigger();
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= n_vecs) return;
+  uint4 raw = *(reinterpret_cast<const uint4*>(o) + i);
+  const int w = i / per_row, t = w / n_heads, h = w - t * n_heads;
+  const float x = to_float(g[t * g_stride + h]);
+  const float s = 1.f / (1.f + expf(-x));
+  __nv_bfloat162* p2 = reinterpret_cast<__nv_bfloat162*>(&raw);
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const float2 f = __bfloat1622float2(p2[u]);
+    p2[u] = __floats2bfloat162_rn(f.x * s, f.y * s);
+  }
+  *(reinterpret_cast<uint4*>(o) + i) = raw;
+}
+
 __global__ void table_route_kernel(const int32_t* __restrict__ token_ids, const int32_t* __restrict__ table, int n_tokens,
                                    int vocab, int top_k, int n_experts, float weight, int32_t* __restrict__ ids,
                                    float* __restrict__ weights) {
@@ -244,7 +265,12 @@ extern "C" int ftk_head_gate(void* o, int dtype, const void* gates, long long ga
   const long long blocks = (warps + 3) / 4;
   FTK_REQUIRE(blocks <= 0x7fffffffLL, "head_gate: too many rows");
   cudaStream_t s = (cudaStream_t)stream;
-  if (dtype == FTK_F32)
+  const long long vecs = warps * (head_dim / 8);
+  if (dtype == FTK_BF16 && head_dim % 8 == 0 && al16(o) && vecs <= 0x7fffff00LL) {
+    note_variant("head_gate: eight values a thread");
+    FTK_LAUNCH(head_gate_vec_kernel, (int)((vecs + 255) / 256), 256, 0, s, (__nv_bfloat16*)o, (const __nv_bfloat16*)gates, gate_stride,
+               n_heads, head_dim / 8, (int)vecs);
+  } else if (dtype == FTK_F32)
     FTK_LAUNCH(head_gate_kernel<float>, (int)blocks, 128, 0, s, (float*)o, (const float*)gates, gate_stride, n_tokens, n_heads, head_dim);
   else
     FTK_LAUNCH(head_gate_kernel<__nv_bfloat16>, (int)blocks, 128, 0, s, (__nv_bfloat16*)o, (const __nv_bfloat16*)gates, gate_stride,
