@@ -157,6 +157,24 @@ typedef struct {
 
 const char* ftk_last_error(void);
 
+// The attention work list of a step (host memory only; csrc/attention_plan.cu).  segments: (q_len, kv_len) per request; items:
+// room for `capacity` items of 8 int32.  Returns how many items the list has (more than `capacity`: nothing was written; call again
+// with room for them), or -1 for arguments that no step has.  est_us: the launch's estimated time, -1 where there is none.
+typedef struct {
+  int tokens_per_tile, tile_rows;
+  int window;                // -1: none
+  int keep_first;
+  int n_kv_heads, sm_count, max_splits, min_split_keys;
+  int fixed_splits;          // -1: none
+  int sparse_block, sparse_topk;  // 0: all keys
+  int key_tile, split_quantum;
+  int deal_most_cuts, deal_search_limit, deal_most_pieces;
+  double fixed_cost_keys, split_cost_keys;
+  double us_per_key_tile, fixed_us, split_us, launch_us;  // us_per_key_tile 0: the kernel's costs are not given
+} ftk_attention_plan_rules;
+int ftk_attention_plan(const int32_t* segments, int n_segs, const ftk_attention_plan_rules* rules, int32_t* items, int capacity,
+                       int32_t* n_slots, double* est_us);
+
 int ftk_embedding_gather(const void* table, int dtype, const int32_t* ids, int n_tokens, int hidden,
                          int vocab, float* out, void* stream);
 int ftk_add_rmsnorm(const void* x, int x_dtype, float* residual, const float* weight, void* out,

@@ -16,10 +16,13 @@ split, and the tile's first partial slot.
 
 from __future__ import annotations
 
+import ctypes
 from dataclasses import dataclass
 from typing import List, Optional, Sequence, Tuple
 
 import numpy as np
+
+from ..kernels import library
 
 ITEM_INTS = 8
 SPLIT_QUANTUM = 64  # split boundaries are multiples of this many keys (of 128 for the kernel with 128-key tiles)
@@ -148,10 +151,58 @@ def build_plan(segments: Sequence[Tuple[int, int]], group: int, tile_rows: int,
 
     ``sparse = (block_size, topk)`` plans a block-sparse layer: one token per tile (every token has
     its own choice of key blocks) and key ranges that count chosen keys: ``min(topk, visible
-    blocks) * block_size`` of them."""
+    blocks) * block_size`` of them.
+
+    Where the native library is loaded (every engine on a GPU) the list comes from ``csrc/attention_plan.cu``, the same
+    numbers: a step waits for its lists (one prompt of 2,048 tokens over 16 heads of 64 on 4, both forms compared: 0.9 ms of
+    array calls here, 40 us there)."""
     if key_tile is None:
         key_tile = 128 if tile_rows >= 128 else 0
     tpt = 1 if sparse else tokens_per_tile(tile_rows, group)
+    lib = library.loaded()
+    plan = None
+    if lib is not None:
+        plan = _native_plan(lib, segments, tpt, tile_rows, window, n_kv_heads, sm_count, max_splits, min_split_keys, fixed_splits,
+                            sparse, key_tile, costs, keep_first)
+    if plan is None:
+        plan = plain_plan(segments, tpt, tile_rows, window, n_kv_heads, sm_count, max_splits, min_split_keys, fixed_splits, sparse,
+                          key_tile, costs, keep_first)
+    return plan
+
+
+class _Rules(ctypes.Structure):  # ftk_attention_plan_rules
+    _fields_ = [(n, ctypes.c_int) for n in (
+        "tokens_per_tile", "tile_rows", "window", "keep_first", "n_kv_heads", "sm_count", "max_splits", "min_split_keys", "fixed_splits",
+        "sparse_block", "sparse_topk", "key_tile", "split_quantum", "deal_most_cuts", "deal_search_limit", "deal_most_pieces")] + [
+        (n, ctypes.c_double) for n in ("fixed_cost_keys", "split_cost_keys", "us_per_key_tile", "fixed_us", "split_us", "launch_us")]
+
+
+def _native_plan(lib, segments, tpt, tile_rows, window, n_kv_heads, sm_count, max_splits, min_split_keys, fixed_splits, sparse,
+                 key_tile, costs, keep_first) -> Optional[AttentionPlan]:
+    seg = np.array(segments, dtype=np.int32).reshape(-1, 2)
+    block, topk = sparse or (0, 0)
+    priced = (costs.us_per_key_tile, costs.fixed_us, costs.split_us) if costs is not None else (0.0, 0.0, 0.0)
+    rules = _Rules(tpt, tile_rows, -1 if window is None else window, keep_first, n_kv_heads, sm_count, max_splits, min_split_keys,
+                   -1 if fixed_splits is None else fixed_splits, block, topk, key_tile, SPLIT_QUANTUM, DEAL_MOST_CUTS,
+                   DEAL_SEARCH_LIMIT, DEAL_MOST_PIECES, FIXED_COST_KEYS, SPLIT_COST_KEYS, *priced, LAUNCH_US)
+    n_slots, est = ctypes.c_int32(), ctypes.c_double()
+    room = 1024
+    while True:
+        items = np.empty((room, ITEM_INTS), dtype=np.int32)
+        n = lib.ftk_attention_plan(ctypes.c_void_p(seg.ctypes.data), seg.shape[0], ctypes.byref(rules), ctypes.c_void_p(items.ctypes.data),
+                                   room, ctypes.byref(n_slots), ctypes.byref(est))
+        if n <= room:
+            break
+        room = n
+    if n < 0:
+        return None
+    return AttentionPlan(items=items[:n], n_items=n, n_slots=n_slots.value, tokens_per_tile=tpt, max_splits=max_splits,
+                         est_us=est.value if est.value >= 0.0 else None)
+
+
+def plain_plan(segments, tpt, tile_rows, window, n_kv_heads, sm_count, max_splits, min_split_keys, fixed_splits, sparse, key_tile,
+               costs, keep_first) -> AttentionPlan:
+    """:func:`build_plan` without the native library: the statement that it is held to."""
     # tiles: segment, first token, tokens, first key, one past the last key
     seg_q = np.asarray([q for q, _ in segments], dtype=np.int64).reshape(-1)
     seg_kv = np.asarray([kv for _, kv in segments], dtype=np.int64).reshape(-1)

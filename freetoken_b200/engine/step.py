@@ -91,6 +91,7 @@ class StepBuilder:
     def __init__(self, engine, seg_lens: Sequence[Tuple[int, int]], fixed: bool, sm_count: int):
         self.engine = engine
         self.seg_lens = list(seg_lens)  # (q_len, kv_len) per segment
+        self._segments = np.array(self.seg_lens, dtype=np.int32).reshape(-1, 2)  # the same for the work lists
         self.fixed = fixed
         self.sm_count = sm_count
         self.sections: List[Tuple[str, np.ndarray]] = []
@@ -138,7 +139,7 @@ class StepBuilder:
         costs = None
         if tile_rows >= 128 and not self.fixed:  # what a piece costs these kernels: for the cuts and for est_us
             costs = TC_TWO_TILE_COSTS if tile_rows == 256 else TC_ONE_TILE_COSTS
-        return build_plan(self.seg_lens, group, tile_rows, window, n_kv_heads,
+        return build_plan(self._segments, group, tile_rows, window, n_kv_heads,
                           sm_count=self.sm_count if per_sm == 2 else max(1, self.sm_count // 2),
                           fixed_splits=self.fixed_splits(n_kv_heads, per_sm, None if window is None else window + keep_first)
                           if self.fixed else None,
@@ -164,7 +165,7 @@ class StepBuilder:
         """Work list of a block-sparse layer: one token per tile, key ranges over chosen keys."""
         key = ("sparse_attention", group, tile_rows, n_kv_heads, head_dim, block_size, topk)
         if key not in self.plans:
-            plan = build_plan(self.seg_lens, group, tile_rows, None, n_kv_heads, sm_count=self.sm_count,
+            plan = build_plan(self._segments, group, tile_rows, None, n_kv_heads, sm_count=self.sm_count,
                               fixed_splits=self.fixed_splits(n_kv_heads) if self.fixed else None,
                               sparse=(block_size, topk))
             self.plans[key] = plan

@@ -155,5 +155,10 @@ def load() -> ctypes.CDLL:
         return lib
 
 
+def loaded() -> Optional[ctypes.CDLL]:
+    """The library if it is loaded already (nothing is built for callers that can do without)."""
+    return _lib
+
+
 def library_path() -> Optional[str]:
     return _lib_path
