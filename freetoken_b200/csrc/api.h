@@ -275,20 +275,20 @@ int ftk_ssm_output(const float* o32, const void* x, long long x_stride, const fl
 // o = S^T q, with beta = sigmoid(b), g = exp(-exp(a_log) softplus(a + dt_bias)), q and k made unit vectors per head
 // (x / sqrt(sum x^2 + unit_eps), q then times q_scale).  q, k hold n_kv_heads heads of `dim`; state [n_slots, n_heads,
 // vdim, dim] float32 (column by column); out [T, n_heads, vdim] float32.
-// The same for portions of bfloat16 prompts in chunks of 32 tokens (one decay a head, keys of 64 or 128
-// channels, value channels in multiples of 16): ftk_delta_chunk_scratch says how many bytes of scratch, 0 where the sizes are
-// not taken.
-long long ftk_delta_chunk_scratch(int dtype, int n_tokens, int n_segs, int n_heads, int n_kv_heads, int dim, int vdim);
-int ftk_delta_scan_chunks(const void* q, long long q_stride, const void* k, long long k_stride, const void* v, long long v_stride,
-                          const void* b, long long b_stride, const void* a, long long a_stride, int dtype, const float* a_log,
-                          const float* dt_bias, float q_scale, float unit_eps, float* state, int n_slots, const int32_t* state_slots,
-                          const int32_t* seg_info, int n_segs, float* out, int n_tokens, int n_heads, int n_kv_heads, int dim,
-                          int vdim, void* scratch, long long scratch_bytes, void* stream);
 int ftk_delta_scan(const void* q, long long q_stride, const void* k, long long k_stride, const void* v, long long v_stride,
                    const void* b, long long b_stride, const void* a, long long a_stride, float* z, int dtype, const float* a_log,
                    const float* dt_bias, float q_scale, float unit_eps, float* state, int n_slots,
                    const int32_t* state_slots, const int32_t* seg_info, int n_segs, float* out, int n_tokens,
                    int n_heads, int n_kv_heads, int dim, int vdim, void* stream);
+// The same for portions of bfloat16 prompts in chunks of 32 tokens (one decay a head, keys of 64 or 128 channels, value channels in
+// multiples of 16): of the n_segs requests the n_long that bring long_from tokens and more; the others go token by token, in a
+// launch before.  ftk_delta_chunk_scratch says how many bytes of scratch n_long requests take, 0 where the sizes are not taken.
+long long ftk_delta_chunk_scratch(int dtype, int n_tokens, int n_long, int n_heads, int n_kv_heads, int dim, int vdim);
+int ftk_delta_scan_chunks(const void* q, long long q_stride, const void* k, long long k_stride, const void* v, long long v_stride,
+                          const void* b, long long b_stride, const void* a, long long a_stride, int dtype, const float* a_log,
+                          const float* dt_bias, float q_scale, float unit_eps, float* state, int n_slots, const int32_t* state_slots,
+                          const int32_t* seg_info, int n_segs, float* out, int n_tokens, int n_heads, int n_kv_heads, int dim,
+                          int vdim, int long_from, int n_long, void* scratch, long long scratch_bytes, void* stream);
 // (z [n_tokens, n_heads * dim] float32 instead of a: logits of one decay per head and key channel; dt_bias is then
 // [n_heads * dim].  When a segment has several tokens z is overwritten with the decays.)
 // Short causal convolution over time with a residual (shortconv.cu): out[t, c] = x[t, c] + sum_j w[c, j] *

@@ -47,6 +47,7 @@ struct DeltaArgs {
   int wide;  // q, k and v rows allow 16-byte copies
   float* z;  // CH: decay logits [T, H * D], or (z_is_decay) the decays; dt_bias is then [H * D]
   int z_is_decay;
+  int shorter_than;  // requests of so many tokens and more are left alone (0: none is)
 };
 
 __device__ __forceinline__ float delta_softplus(float z) { return z > 0.f ? z + log1pf(expf(-z)) : log1pf(expf(z)); }
@@ -124,6 +125,7 @@ __global__ void __launch_bounds__(kDeltaThreads) delta_scan_kernel(DeltaArgs a) 
   const int D = a.D, Dv = a.Dv;
   const int q_start = a.seg_info[seg * 4], q_len = a.seg_info[seg * 4 + 1], kv_len = a.seg_info[seg * 4 + 2];
   if (q_len <= 0 || q_start < 0 || q_start + q_len > a.n_tokens || kv_len < q_len) return;
+  if (a.shorter_than > 0 && q_len >= a.shorter_than) return;
   const int slot = a.state_slots[seg];
   if (slot < 0 || slot >= a.n_slots) return;
   const int hqk = h / (a.H / a.G);
@@ -484,15 +486,10 @@ static int launch_delta(DeltaArgs a, cudaStream_t s) {
   return launch_delta_sized<T, 32, 8>(a, s);
 }
 
-}  // namespace ftk
-
-using namespace ftk;
-
-extern "C" int ftk_delta_scan(const void* q, long long q_stride, const void* k, long long k_stride, const void* v,
-                              long long v_stride, const void* b, long long b_stride, const void* a, long long a_stride,
-                              float* z, int dtype, const float* a_log, const float* dt_bias, float q_scale, float unit_eps,
-                              float* state, int n_slots, const int32_t* state_slots, const int32_t* seg_info, int n_segs,
-                              float* out, int n_tokens, int n_heads, int n_kv_heads, int dim, int vdim, void* stream) {
+int delta_scan_tokens(const void* q, long long q_stride, const void* k, long long k_stride, const void* v, long long v_stride, const void* b,
+                      long long b_stride, const void* a, long long a_stride, float* z, int dtype, const float* a_log, const float* dt_bias,
+                      float q_scale, float unit_eps, float* state, int n_slots, const int32_t* state_slots, const int32_t* seg_info,
+                      int n_segs, float* out, int n_tokens, int n_heads, int n_kv_heads, int dim, int vdim, int shorter_than, void* stream) {
   FTK_REQUIRE(dtype_ok(dtype), "delta_scan: bad dtype %d", dtype);
   FTK_REQUIRE(n_tokens >= 0 && n_segs >= 0, "delta_scan: bad counts");
   if (n_tokens == 0 || n_segs == 0) return 0;
@@ -504,10 +501,21 @@ extern "C" int ftk_delta_scan(const void* q, long long q_stride, const void* k, 
   DeltaArgs d;
   d.q = q; d.k = k; d.v = v; d.b = b; d.a = a;
   d.q_stride = q_stride; d.k_stride = k_stride; d.v_stride = v_stride; d.b_stride = b_stride; d.a_stride = a_stride;
-  d.z = z; d.z_is_decay = 0;
+  d.z = z; d.z_is_decay = 0; d.shorter_than = shorter_than;
   d.a_log = a_log; d.dt_bias = dt_bias; d.q_scale = q_scale; d.unit_eps = unit_eps;
   d.state = state; d.n_slots = n_slots; d.state_slots = state_slots; d.seg_info = seg_info; d.n_segs = n_segs;
   d.out = out; d.n_tokens = n_tokens; d.H = n_heads; d.G = n_kv_heads; d.D = dim; d.Dv = vdim;
   cudaStream_t s = (cudaStream_t)stream;
   return dtype == FTK_F32 ? launch_delta<float>(d, s) : launch_delta<__nv_bfloat16>(d, s);
+}
+
+}  // namespace ftk
+
+extern "C" int ftk_delta_scan(const void* q, long long q_stride, const void* k, long long k_stride, const void* v,
+                              long long v_stride, const void* b, long long b_stride, const void* a, long long a_stride,
+                              float* z, int dtype, const float* a_log, const float* dt_bias, float q_scale, float unit_eps,
+                              float* state, int n_slots, const int32_t* state_slots, const int32_t* seg_info, int n_segs,
+                              float* out, int n_tokens, int n_heads, int n_kv_heads, int dim, int vdim, void* stream) {
+  return ftk::delta_scan_tokens(q, q_stride, k, k_stride, v, v_stride, b, b_stride, a, a_stride, z, dtype, a_log, dt_bias, q_scale, unit_eps, state,
+                                n_slots, state_slots, seg_info, n_segs, out, n_tokens, n_heads, n_kv_heads, dim, vdim, 0, stream);
 }

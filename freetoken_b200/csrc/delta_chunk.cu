@@ -21,6 +21,12 @@
 
 namespace ftk {
 
+// (delta.cu: the requests of fewer tokens than shorter_than, token by token)
+int delta_scan_tokens(const void* q, long long q_stride, const void* k, long long k_stride, const void* v, long long v_stride, const void* b,
+                      long long b_stride, const void* a, long long a_stride, float* z, int dtype, const float* a_log, const float* dt_bias,
+                      float q_scale, float unit_eps, float* state, int n_slots, const int32_t* state_slots, const int32_t* seg_info,
+                      int n_segs, float* out, int n_tokens, int n_heads, int n_kv_heads, int dim, int vdim, int shorter_than, void* stream);
+
 constexpr int kDcTokens = 32;                 // tokens a chunk
 // scratch of one (chunk, head): rows s of T^T and (A T)^T, columns t in the order of dc_place, then per token beta, beta c rk, c rq, (c_C / c) rk, then c_C
 constexpr int kDcMats = kDcTokens * 2 * kDcTokens;
@@ -35,6 +41,7 @@ struct DeltaChunkArgs {
   const int32_t* state_slots; const int32_t* seg_info; int n_segs;
   float* out; int n_tokens, H, G, D, Dv;
   unsigned char* scratch;
+  int long_from, n_long, n_chunks;  // requests of long_from tokens and more go in chunks: n_long of them; the chunks that scratch holds
 };
 
 __device__ __forceinline__ void dc_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
@@ -71,7 +78,7 @@ __device__ __forceinline__ float dc_high(uint32_t w) { return __uint_as_float(w 
 // chunks of a segment; 0 for one that the kernels leave alone
 __device__ __forceinline__ int dc_chunks(const DeltaChunkArgs& a, int seg) {
   const int q_start = a.seg_info[seg * 4], q_len = a.seg_info[seg * 4 + 1], kv_len = a.seg_info[seg * 4 + 2];
-  if (q_len <= 0 || q_start < 0 || q_start + q_len > a.n_tokens || kv_len < q_len) return 0;
+  if (q_len < a.long_from || q_start < 0 || q_start + q_len > a.n_tokens || kv_len < q_len) return 0;
   return (q_len + kDcTokens - 1) / kDcTokens;
 }
 
@@ -267,17 +274,28 @@ __global__ void __launch_bounds__(2 * NV * KS) delta_chunk_kernel(DeltaChunkArgs
   constexpr int kThreads = 2 * NV * KS, CG = NV / 4, NT = 4 / KS, DT = D / (8 * KS), LD = D + 8;
   extern __shared__ __align__(16) unsigned char dc_smem[];
   DcShared<D, NV, KS>& sh = *reinterpret_cast<DcShared<D, NV, KS>*>(dc_smem);
-  const int seg = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * NV;
+  const int h = blockIdx.y, col0 = blockIdx.z * NV;
   const int tid = threadIdx.x, lane = tid & 31;
-  const int n_chunks = dc_chunks(a, seg);
-  if (n_chunks == 0) return;
+  // the block's request: the blockIdx.x-th of those that go in chunks (every warp looks for it)
+  int seg = -1, n_chunks = 0, before = 0, left = blockIdx.x;  // before: chunks of the requests in front of it
+  for (int i0 = 0; i0 < a.n_segs && seg < 0; i0 += 32) {
+    const int n = i0 + lane < a.n_segs ? dc_chunks(a, i0 + lane) : 0;
+    const unsigned some = __ballot_sync(0xffffffffu, n > 0);
+    const int at = left < __popc(some) ? (int)__fns(some, 0, left + 1) : 32;  // its lane
+    left -= __popc(some);
+    int sum = lane < at ? n : 0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    before += sum;
+    if (at < 32) {
+      seg = i0 + at;
+      n_chunks = __shfl_sync(0xffffffffu, n, at);
+    }
+  }
+  if (seg < 0) return;
   const int q_start = a.seg_info[seg * 4], q_len = a.seg_info[seg * 4 + 1], kv_len = a.seg_info[seg * 4 + 2];
   const int slot = a.state_slots[seg];
   if (slot < 0 || slot >= a.n_slots) return;
-  int before = 0;  // chunks of the segments before this one
-  for (int i0 = 0; i0 < seg; i0 += 32) before += i0 + lane < seg ? dc_chunks(a, i0 + lane) : 0;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
   const int hqk = h / (a.H / a.G);
   auto fetch = [&](int ch) {
     DcStage<D, NV>& st = sh.stage[ch & 1];
@@ -458,8 +476,7 @@ __global__ void __launch_bounds__(2 * NV * KS) delta_chunk_kernel(DeltaChunkArgs
 
 template <int D, int NV, int KS>
 static int launch_delta_chunks_as(const DeltaChunkArgs& a, cudaStream_t s) {
-  const int n_chunks = a.n_tokens / kDcTokens + a.n_segs;
-  const dim3 grid(a.n_segs, a.H, (a.Dv + NV - 1) / NV);
+  const dim3 grid(a.n_long, a.H, (a.Dv + NV - 1) / NV);
   const size_t smem = sizeof(DcShared<D, NV, KS>);
   static_assert(sizeof(DcShared<D, NV, KS>) <= 227 * 1024, "shared memory");
   auto kern = delta_chunk_kernel<D, NV, KS>;
@@ -470,9 +487,9 @@ static int launch_delta_chunks_as(const DeltaChunkArgs& a, cudaStream_t s) {
     auto prep = delta_prep_kernel<D, 8>;
     FTK_REQUIRE(cudaFuncSetAttribute(prep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(8 * sl)) == cudaSuccess,
                 "delta_scan (chunks): cannot set up the kernel");
-    FTK_LAUNCH(prep, dim3(n_chunks, a.G), 256, 8 * sl, s, a);
+    FTK_LAUNCH(prep, dim3(a.n_chunks, a.G), 256, 8 * sl, s, a);
   } else {
-    FTK_LAUNCH((delta_prep_kernel<D, 4>), dim3(n_chunks, a.G), 128, 4 * sl, s, a);
+    FTK_LAUNCH((delta_prep_kernel<D, 4>), dim3(a.n_chunks, a.G), 128, 4 * sl, s, a);
   }
   FTK_LAUNCH_CHECK("delta_scan (chunks, triangles)");
   FTK_LAUNCH(kern, grid, 2 * NV * KS, smem, s, a);
@@ -486,7 +503,7 @@ static int launch_delta_chunks_as(const DeltaChunkArgs& a, cudaStream_t s) {
 // other splits of the channels: 440 to 470 us at 48 heads.  (Token by token: 860 us at 48 heads, 538 at 16.)
 template <int D>
 static int launch_delta_chunks(const DeltaChunkArgs& a, cudaStream_t s) {
-  const long long blocks = (long long)a.n_segs * a.H * ((a.Dv + 15) / 16);
+  const long long blocks = (long long)a.n_long * a.H * ((a.Dv + 15) / 16);
   return blocks > 2 * 148 ? launch_delta_chunks_as<D, 48, 4>(a, s) : launch_delta_chunks_as<D, 16, 4>(a, s);
 }
 
@@ -494,7 +511,7 @@ static int launch_delta_chunks(const DeltaChunkArgs& a, cudaStream_t s) {
 
 using namespace ftk;
 
-// Bytes of scratch for steps of n_tokens tokens and n_segs requests, or 0 where the sizes are not taken.
+// Bytes of scratch for steps of n_tokens tokens of which n_segs requests go in chunks, or 0 where the sizes are not taken.
 extern "C" long long ftk_delta_chunk_scratch(int dtype, int n_tokens, int n_segs, int n_heads, int n_kv_heads, int dim, int vdim) {
   if (dtype != FTK_BF16 || (dim != 64 && dim != 128) || vdim < 16 || vdim % 16 || vdim > 65535 * 16 || n_heads < 1 || n_heads > 65535 ||
       n_kv_heads < 1 || n_heads % n_kv_heads || n_tokens < 1 || n_segs < 1)
@@ -506,9 +523,11 @@ extern "C" int ftk_delta_scan_chunks(const void* q, long long q_stride, const vo
                                      long long v_stride, const void* b, long long b_stride, const void* a, long long a_stride,
                                      int dtype, const float* a_log, const float* dt_bias, float q_scale, float unit_eps, float* state,
                                      int n_slots, const int32_t* state_slots, const int32_t* seg_info, int n_segs, float* out,
-                                     int n_tokens, int n_heads, int n_kv_heads, int dim, int vdim, void* scratch, long long scratch_bytes,
-                                     void* stream) {
-  const long long need = ftk_delta_chunk_scratch(dtype, n_tokens, n_segs, n_heads, n_kv_heads, dim, vdim);
+                                     int n_tokens, int n_heads, int n_kv_heads, int dim, int vdim, int long_from, int n_long, void* scratch,
+                                     long long scratch_bytes, void* stream) {
+  FTK_REQUIRE(long_from >= 1 && n_long >= 1 && n_long <= n_segs, "delta_scan (chunks): %d of %d requests of %d tokens and more", n_long,
+              n_segs, long_from);
+  const long long need = ftk_delta_chunk_scratch(dtype, n_tokens, n_long, n_heads, n_kv_heads, dim, vdim);
   FTK_REQUIRE(need > 0, "delta_scan (chunks): type %d, heads of %d x %d, %d tokens are not taken", dtype, dim, vdim, n_tokens);
   FTK_REQUIRE(q && k && v && b && a && a_log && dt_bias && state && state_slots && seg_info && out && scratch,
               "delta_scan (chunks): null pointer");
@@ -524,6 +543,13 @@ extern "C" int ftk_delta_scan_chunks(const void* q, long long q_stride, const vo
   d.state = state; d.n_slots = n_slots; d.state_slots = state_slots; d.seg_info = seg_info; d.n_segs = n_segs;
   d.out = out; d.n_tokens = n_tokens; d.H = n_heads; d.G = n_kv_heads; d.D = dim; d.Dv = vdim;
   d.scratch = (unsigned char*)scratch;
+  d.long_from = long_from; d.n_long = n_long; d.n_chunks = n_tokens / kDcTokens + n_long;
+  if (n_long < n_segs) {
+    const int rc = delta_scan_tokens(q, q_stride, k, k_stride, v, v_stride, b, b_stride, a, a_stride, nullptr, dtype, a_log, dt_bias, q_scale,
+                                     unit_eps, state, n_slots, state_slots, seg_info, n_segs, out, n_tokens, n_heads, n_kv_heads, dim, vdim,
+                                     long_from, stream);
+    if (rc) return rc;
+  }
   note_variant("delta rule: chunks of 32 tokens");
   return dim == 64 ? launch_delta_chunks<64>(d, (cudaStream_t)stream) : launch_delta_chunks<128>(d, (cudaStream_t)stream);
 }

@@ -188,7 +188,7 @@ _SIGNATURES = {
     "ftk_hyper_step": [_vp, ctypes.c_longlong, _i, _i, _i, _vp, _vp, _i, _vp, _vp, _vp, _vp, _f, _vp, _i, _vp, _vp],
     "ftk_conv_act": [_vp, ctypes.c_longlong, _i, _vp, _vp, _i, _i, _vp, _i, _vp, _vp, _i, _vp, _i, _i, _vp],
     "ftk_delta_scan_chunks": [_vp, ctypes.c_longlong, _vp, ctypes.c_longlong, _vp, ctypes.c_longlong, _vp, ctypes.c_longlong,
-                              _vp, ctypes.c_longlong, _i, _vp, _vp, _f, _f, _vp, _i, _vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _vp,
+                              _vp, ctypes.c_longlong, _i, _vp, _vp, _f, _f, _vp, _i, _vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _i, _vp,
                               ctypes.c_longlong, _vp],
     "ftk_delta_scan": [_vp, ctypes.c_longlong, _vp, ctypes.c_longlong, _vp, ctypes.c_longlong, _vp, ctypes.c_longlong,
                        _vp, ctypes.c_longlong, _vp, _i, _vp, _vp, _f, _f, _vp, _i, _vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _vp],
@@ -1619,18 +1619,19 @@ def ssm_output(o32: torch.Tensor, x: torch.Tensor, d_skip: torch.Tensor, z: torc
                                  int(norm_groups), float(eps), _dev(out, "out"), T, H, P, _stream()), "ssm_output")
 
 
-def delta_chunk_scratch(dtype: torch.dtype, n_tokens: int, n_segs: int, n_heads: int, n_kv_heads: int, dim: int, vdim: int) -> int:
-    """Bytes of scratch with which :func:`delta_scan` may take a step of so many tokens and requests in chunks; 0 where the
-    sizes are not taken (as ``ftk_delta_chunk_scratch`` says)."""
-    if dtype != torch.bfloat16 or dim not in (64, 128) or vdim < 16 or vdim % 16 or n_heads % n_kv_heads or n_tokens < 1 or n_segs < 1:
+def delta_chunk_scratch(dtype: torch.dtype, n_tokens: int, n_long: int, n_heads: int, n_kv_heads: int, dim: int, vdim: int) -> int:
+    """Bytes of scratch with which :func:`delta_scan` may take ``n_long`` requests of a step of so many tokens in chunks; 0 where
+    the sizes are not taken (as ``ftk_delta_chunk_scratch`` says)."""
+    if dtype != torch.bfloat16 or dim not in (64, 128) or vdim < 16 or vdim % 16 or n_heads % n_kv_heads or n_tokens < 1 or n_long < 1:
         return 0
-    return (n_tokens // 32 + n_segs) * n_heads * (32 * 64 * 4 + 4 * 32 * 4 + 16)
+    return (n_tokens // 32 + n_long) * n_heads * (32 * 64 * 4 + 4 * 32 * 4 + 16)
 
 
 def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, b_raw: torch.Tensor, a_raw: Optional[torch.Tensor],
                a_log: torch.Tensor, dt_bias: torch.Tensor, q_scale: float, unit_eps: float, state: torch.Tensor,
                state_slots: torch.Tensor, seg_info: torch.Tensor, n_segs: int, out: torch.Tensor,
-               z: Optional[torch.Tensor] = None, scratch: Optional[torch.Tensor] = None) -> None:
+               z: Optional[torch.Tensor] = None, scratch: Optional[torch.Tensor] = None, long_from: int = 1,
+               n_long: Optional[int] = None) -> None:
     """The gated delta rule over the step's tokens, per (request, head), a request's tokens in order:
     ``S <- g S``, ``u = beta (v - S^T k)``, ``S <- S + k u^T``, ``o = S^T q``, with ``beta = sigmoid(b_raw)``,
     ``g = exp(-exp(a_log) softplus(a_raw + dt_bias))``, and ``q``, ``k`` first made unit vectors per head
@@ -1645,8 +1646,9 @@ def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, b_raw: torch.T
     ``g[d] = exp(-exp(a_log) softplus(z[d] + dt_bias[d]))``, on the rows of ``S`` that belong to key channels; when a segment
     has several tokens, ``z`` is overwritten with the decays.
 
-    ``scratch`` (bytes on the device, :func:`delta_chunk_scratch` of them): the tokens may go in chunks of 32
-    where the sizes and alignments allow it, which pays for steps whose requests bring many tokens (``csrc/delta_chunk.cu``)."""
+    ``scratch`` (bytes on the device, :func:`delta_chunk_scratch` of them): where the sizes and alignments allow it, the
+    ``n_long`` requests (None: all) that bring ``long_from`` tokens and more go in chunks of 32 tokens, and the others token by
+    token beside them (``csrc/delta_chunk.cu``)."""
     T, H, Dv = out.shape
     D = state.shape[3]
     if (a_raw is None) == (z is None) or (z is not None and z.shape != (T, H * D)):
@@ -1660,14 +1662,16 @@ def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, b_raw: torch.T
     as_ = _cols(a_raw, "delta_scan: a_raw", (T, H), q.dtype) if z is None else 0
     if a_log.shape != (H,) or dt_bias.shape != ((H,) if z is None else (H * D,)):
         raise KernelError("delta_scan: a_log must be [H], dt_bias [H] (or [H * D] with a decay per channel)")
-    if scratch is not None and z is None and 0 < delta_chunk_scratch(q.dtype, T, n_segs, H, G, D, Dv) <= scratch.numel() \
+    n_long = n_segs if n_long is None else int(n_long)
+    if scratch is not None and z is None and 0 < delta_chunk_scratch(q.dtype, T, n_long, H, G, D, Dv) <= scratch.numel() \
             and (qs | ks | vs) % 8 == 0 and (q.data_ptr() | k.data_ptr() | v.data_ptr() | out.data_ptr() | scratch.data_ptr()) % 16 == 0:
         _check(_lib().ftk_delta_scan_chunks(
             q.data_ptr(), qs, k.data_ptr(), ks, v.data_ptr(), vs, b_raw.data_ptr(), bs, a_raw.data_ptr(), as_, _code(q, "q"),
             _dev(a_log, "a_log", torch.float32), _dev(dt_bias, "dt_bias", torch.float32), float(q_scale), float(unit_eps),
             _dev(state, "state", torch.float32), state.shape[0], _dev(state_slots, "state_slots", torch.int32),
             _dev(seg_info, "seg_info", torch.int32), n_segs, _dev(out, "out", torch.float32), T, H, G, D, Dv,
-            _dev(scratch, "scratch", torch.uint8), scratch.numel(), _stream()), "delta_scan (chunks)", 2)
+            int(long_from), n_long, _dev(scratch, "scratch", torch.uint8), scratch.numel(), _stream()), "delta_scan (chunks)",
+            2 + (n_long < n_segs))
         return
     _check(_lib().ftk_delta_scan(
         q.data_ptr(), qs, k.data_ptr(), ks, v.data_ptr(), vs, b_raw.data_ptr(), bs,

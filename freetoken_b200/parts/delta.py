@@ -25,7 +25,8 @@ slot of the cache manager's state pool; both start from zero.  The reference has
 
 from __future__ import annotations
 
-from typing import Any, Dict
+import math
+from typing import Any, Dict, Sequence
 
 import torch
 
@@ -34,9 +35,39 @@ from ..errors import ConfigError
 from ..kernels import ops
 from .base import MIXERS, BuildEnv, Mixer, StepState
 
-CHUNK_MIN_TOKENS = 16  # steps in which some request brings so many tokens go in chunks where they can
+CHUNK_MIN_TOKENS = 80  # no request of fewer tokens goes in chunks: see chunks_pay
+SMS = 148
 
 UNIT_EPS = 1e-6  # inside the root of the unit norms of q and k: fixed by the design
+
+
+def chunks_pay(lens: Sequence[int], beside: bool, n_heads: int, head_dim: int, v_dim: int) -> bool:
+    """Whether requests of ``lens`` tokens are through sooner in chunks (``csrc/delta_chunk.cu``) than token by token
+    (``csrc/delta.cu``); ``beside``: the step has others, which then take a launch of their own.
+
+    Both kernels are chains (of chunks, of tokens) until a step has more blocks than the GPU holds at once, then waves or a rate.
+    Fitted to timings of both (heads of 64 and 128, 4 to 48 of them, 1 to 32 requests of 32 to 2,048 tokens, 16 to 256 value
+    channels).  One request, 48 heads of 128, token by token against chunks: 37 and 40 us for 64 tokens, 43 and 44 for 80, 51 and
+    46 for 96, 63 and 50 for 128, 227 and 120 for 512; 16 heads of 64: 23 and 26, 29 and 28, 32 and 28, 41 and 30, 139 and 54.
+    Many requests fill the GPU token by token as well: 32 heads of 128, four of 256 tokens 162 and 177, eight of 512 612 and 644;
+    48 heads, eight of 128 tokens 248 and 247, two of 512 311 and 220."""
+    longest = max(lens)
+    states = sum(lens) / longest * n_heads  # (request, head) pairs at work, on average
+    wide = head_dim > 64
+    rounds = lambda cols: math.ceil(states * -(-v_dim // cols) / SMS)  # noqa: E731  (blocks of so many value columns an SM)
+    chunks = -(-longest // 32)
+    if states * -(-v_dim // 16) <= 2 * SMS:  # (as csrc/delta_chunk.cu: launch_delta_chunks)
+        in_chunks = 22.5 + chunks * (2.6 if wide else 1.7) * (1.0 if rounds(16) == 1 else 1.5 if wide else 2.1)
+    else:
+        in_chunks = (22.0 + rounds(48) * (4.5 + 5.2 * chunks)) if wide else (17.0 + rounds(48) * (3.0 + 3.5 * chunks))
+    in_chunks += 0.014 * states * chunks + (6.0 if beside else 0.0)
+    if wide and states * v_dim >= 32 * SMS:  # (as csrc/delta.cu: launch_delta)
+        token = (0.43, 0.61, 1.2)[rounds(64) - 1] if rounds(64) < 4 else 0.305 * rounds(64)
+    elif wide:
+        token = 0.27 if rounds(16) == 1 else 0.34
+    else:
+        token = 0.26 if rounds(16) <= 2 else max(0.36, 0.086 * rounds(16))
+    return in_chunks < 8.0 + longest * token
 
 
 @MIXERS.register("gated_delta")
@@ -128,12 +159,14 @@ class GatedDelta(Mixer):
             a = None
         o32 = ws.get("delta.o32", (T, H, Dv), torch.float32, (cap, H, Dv))
         args = dict(z=z)
-        if z is None and h.is_cuda and max(seg.q_len for seg in step.segments) >= CHUNK_MIN_TOKENS:
+        long = [seg.q_len for seg in step.segments if seg.q_len >= CHUNK_MIN_TOKENS] if z is None and h.is_cuda else []
+        n_long = len(long)
+        if long and chunks_pay(long, n_long < n_segs, H, D, Dv):
             sizes = (H, self.n_kv_heads, D, Dv)
-            n = ops.delta_chunk_scratch(dt, T, n_segs, *sizes)
+            n = ops.delta_chunk_scratch(dt, T, n_long, *sizes)
             if n:
                 most = ops.delta_chunk_scratch(dt, cap, max(n_segs, self.env.max_decode_rows), *sizes)
-                args = dict(scratch=ws.get("delta.chunks", (n,), torch.uint8, (most,)))
+                args = dict(scratch=ws.get("delta.chunks", (n,), torch.uint8, (most,)), long_from=CHUNK_MIN_TOKENS, n_long=n_long)
         ops.delta_scan(qkv[:, : self.k_col], qkv[:, self.k_col: self.v_col], qkv[:, self.v_col:],
                        proj[:, self.b_col: self.a_col], a, self.params["A_log"], self.params["dt_bias"],
                        D ** -0.5, UNIT_EPS, cache.tensors["s"], step.state_slots, step.seg_info, n_segs, o32, **args)

@@ -133,3 +133,62 @@ def test_what_is_not_taken_goes_token_by_token():
                    scratch=scratch)
     assert not ops.variant_counts().get("delta rule: chunks of 32 tokens")
     torch.testing.assert_close(got, out, rtol=1e-4, atol=2e-5)
+
+
+def scan(p, out=None, eps=EPS, **kw):
+    """One call with scratch for what is asked for; outputs start as NaN, scratch as 0xff."""
+    H, G, D, Dv = p["sizes"]
+    out = torch.full((p["T"], H, Dv), float("nan"), device=DEV) if out is None else out
+    state = p["state"].clone()
+    if kw:
+        n = ops.delta_chunk_scratch(torch.bfloat16, p["T"], kw["n_long"], H, G, D, Dv)
+        kw["scratch"] = torch.full((n,), 255, dtype=torch.uint8, device=DEV)
+    ops.variant_counts(reset=True)
+    ops.delta_scan(p["q"], p["k"], p["v"], p["b"], p["a"], p["a_log"], p["dt_bias"], D ** -0.5, eps, state, p["slots"], p["info"],
+                   len(p["info"]), out, **kw)
+    return out, state
+
+
+@pytest.mark.parametrize("H,G,D,Dv", [(4, 2, 128, 128), (6, 1, 64, 48)])
+@pytest.mark.parametrize("lens", [[(1, 9), (64, 100), (5, 5), (1, 1), (96, 300), (63, 63), (2, 40)], [(200, 200)] + [(1, 30)] * 40,
+                                  [(1, 30)] * 33 + [(64, 64)] + [(1, 5)] * 31 + [(70, 70)]])
+def test_only_the_long_requests_of_a_step_go_in_chunks(H, G, D, Dv, lens):
+    """A decoding request is the same, bit for bit, with and without a long neighbour: it stays token by token."""
+    p = problem(lens, H, G, D, Dv, seed=D + len(lens))
+    is_long = [n >= 64 for n, _ in lens]
+    out, state = scan(p, long_from=64, n_long=sum(is_long))
+    assert ops.variant_counts().get("delta rule: chunks of 32 tokens")
+    (chunks, chunk_state), (tokens, token_state) = run(p, True), run(p, False)
+    for i, (q0, n, _, _) in enumerate(p["info"].tolist()):
+        slot, rows = int(p["slots"][i]), slice(q0, q0 + n)
+        want, want_state = (chunks, chunk_state) if is_long[i] else (tokens, token_state)
+        assert torch.equal(out[rows], want[rows]) and torch.equal(state[slot], want_state[slot]), (i, n)
+    rest = [s for s in range(state.shape[0]) if s not in p["slots"].tolist()]
+    assert torch.equal(state[rest], p["state"][rest])
+
+
+def test_a_layer_takes_a_step_apart(monkeypatch):
+    """The part hands over the number of its long requests, and no scratch where there is none."""
+    from freetoken_b200.config.spec import PartSpec
+    from freetoken_b200.parts import MIXERS, BuildEnv, Segment, StepState, Workspace
+    from freetoken_b200.parts.delta import CHUNK_MIN_TOKENS
+
+    calls = []
+    real = ops.delta_scan
+    monkeypatch.setattr(ops, "delta_scan", lambda *a, **kw: (calls.append({k: v for k, v in kw.items() if k != "scratch"}), real(*a, **kw)))
+    env = BuildEnv(dtype=torch.bfloat16, device=torch.device(DEV), max_seq_len=512, max_step_tokens=512, workspace=Workspace(torch.device(DEV)))
+    part = MIXERS.build(PartSpec("gated_delta", dict(hidden=64, n_heads=4, n_kv_heads=2, head_dim=64, v_head_dim=64, taps=1, eps=1e-6)), env)
+    part.bind({n: torch.zeros(s.shape, device=DEV, dtype=torch.float32 if s.dtype == "float32" else torch.bfloat16)
+               for n, s in part.param_specs().items()})
+    for lens, n_long in (([1, CHUNK_MIN_TOKENS, 1, CHUNK_MIN_TOKENS - 1, 200], 2), ([1, 1, CHUNK_MIN_TOKENS - 1], 0)):
+        info, q0 = [], 0
+        for n in lens:
+            info.append([q0, n, n, 0])
+            q0 += n
+        step = StepState(n_tokens=q0, segments=[Segment(i, a, n, kv) for i, (a, n, kv, _) in enumerate(info)], token_ids=None, positions=None,
+                         seg_info=torch.tensor(info, dtype=torch.int32, device=DEV),
+                         state_slots=torch.arange(len(lens), dtype=torch.int32, device=DEV), logit_rows=None, n_logit_rows=0,
+                         attention_plans={}, decode_only=False)
+        cache = type("C", (), dict(tensors={"s": torch.zeros(len(lens), 4, 64, 64, device=DEV)}))
+        part.forward(torch.zeros(q0, 64, dtype=torch.bfloat16, device=DEV), step, cache, True)
+        assert calls.pop() == (dict(long_from=CHUNK_MIN_TOKENS, n_long=n_long) if n_long else dict(z=None))
