@@ -405,10 +405,10 @@ __global__ void __launch_bounds__(2 * NV * KS) delta_chunk_kernel(DeltaChunkArgs
     }
     __syncthreads();
     // [T; A T] X, again a token's two rows as a pair
-    // (this thread's tokens all lie in front of the bound, and what a row has behind its token is zero)
-    const int upto = 8 * NT * (kr + 1);
-#pragma unroll 8
-    for (int e = 0; e < upto; ++e) {
+    // (rows in front of `own` count for all of this thread's tokens; of the rest a token takes those up to itself: what T has behind it
+    // is zero, but a later token's X may be anything, and its infinities and NaNs must not reach back)
+    const int own = 8 * NT * kr;
+    auto term = [&](int e, bool all) {
       float y[4];
       dc_load4(&sh.x[e][c0], y);
       uint64_t x[NT];
@@ -422,12 +422,16 @@ __global__ void __launch_bounds__(2 * NV * KS) delta_chunk_kernel(DeltaChunkArgs
         }
       }
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const uint64_t y2 = dc_pair(y[j], y[j]);
+      for (int i = 0; i < NT; ++i) {
+        if (!all && e > own + tg + 8 * i) continue;
 #pragma unroll
-        for (int i = 0; i < NT; ++i) dc_fma2(r[i][j], x[i], y2);
+        for (int j = 0; j < 4; ++j) dc_fma2(r[i][j], x[i], dc_pair(y[j], y[j]));
       }
-    }
+    };
+#pragma unroll 8
+    for (int e = 0; e < own; ++e) term(e, true);
+#pragma unroll
+    for (int e = 0; e < 8 * NT; ++e) term(own + e, false);
 #pragma unroll
     for (int i = 0; i < NT; ++i) {
       const int t = tg + 8 * (kr * NT + i), tok = ch * kDcTokens + t;

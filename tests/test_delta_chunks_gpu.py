@@ -192,3 +192,20 @@ def test_a_layer_takes_a_step_apart(monkeypatch):
         cache = type("C", (), dict(tensors={"s": torch.zeros(len(lens), 4, 64, 64, device=DEV)}))
         part.forward(torch.zeros(q0, 64, dtype=torch.bfloat16, device=DEV), step, cache, True)
         assert calls.pop() == (dict(long_from=CHUNK_MIN_TOKENS, n_long=n_long) if n_long else dict(z=None))
+
+
+@pytest.mark.parametrize("H,G,D,Dv", [(4, 2, 128, 48), (6, 1, 64, 16)])
+@pytest.mark.parametrize("what", ["q", "k", "v", "a", "b"])
+@pytest.mark.parametrize("at,value", [(0, float("nan")), (5, float("inf")), (17, float("nan")), (31, float("-inf")), (38, float("nan"))])
+def test_a_value_that_is_no_number_reaches_no_earlier_token(H, G, D, Dv, what, at, value):
+    """Nor another request, or a request's other outputs than those that the recurrence hands it to."""
+    p = problem([(40, 50), (33, 33)], H, G, D, Dv, seed=at)
+    clean, clean_state = run(p, True)
+    bad = dict(p, **{what: p[what].clone()})
+    bad[what][at, 3 if what in "ab" else slice(None, None, 2)] = value
+    out, state = run(bad, True)
+    tokens, token_state = run(bad, False)
+    assert torch.equal(out[:at], clean[:at]) and torch.equal(out[40:], clean[40:])
+    assert torch.equal(state[p["slots"][1]], clean_state[p["slots"][1]])
+    # where the token-by-token kernel has numbers, there are numbers
+    assert torch.isfinite(out[torch.isfinite(tokens)]).all()
