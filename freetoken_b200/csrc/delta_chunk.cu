@@ -163,7 +163,8 @@ __global__ void __launch_bounds__(32 * W) delta_prep_kernel(DeltaChunkArgs a) {
   }
   __syncthreads();
   const int t = lane;
-  const float rk = rsqrtf(kk[t][t] + a.unit_eps), rq = rsqrtf(s2q[t] + a.unit_eps) * a.q_scale;
+  // (rows that do not exist are zeros: with unit_eps = 0 they would have no unit vector)
+  const float rk = t < nb ? rsqrtf(kk[t][t] + a.unit_eps) : 0.f, rq = t < nb ? rsqrtf(s2q[t] + a.unit_eps) * a.q_scale : 0.f;
   const size_t tok = (size_t)(q_start + min(t, nb - 1));
   for (int hh = warp; hh < per; hh += W) {
     const int h = g * per + hh;

@@ -209,3 +209,15 @@ def test_a_value_that_is_no_number_reaches_no_earlier_token(H, G, D, Dv, what, a
     assert torch.equal(state[p["slots"][1]], clean_state[p["slots"][1]])
     # where the token-by-token kernel has numbers, there are numbers
     assert torch.isfinite(out[torch.isfinite(tokens)]).all()
+
+
+@pytest.mark.parametrize("H,G,D,Dv", [(4, 2, 128, 48), (6, 1, 64, 16)])
+@pytest.mark.parametrize("lens", [[(33, 33), (1, 7), (95, 200)], [(64, 64)]])
+def test_unit_vectors_without_a_floor(H, G, D, Dv, lens):
+    """unit_eps = 0, which vectors that are not zero allow: also where the last chunk is not full."""
+    p = problem(lens, H, G, D, Dv, seed=3)
+    (out, state), (plain, plain_state) = scan(p, eps=0.0, n_long=len(lens)), scan(p, eps=0.0)
+    # (the same sums as with the usual floor of 1e-6 under squares of about D: the bound of the first test above)
+    assert torch.isfinite(plain).all() and torch.isfinite(plain_state).all()
+    torch.testing.assert_close(out, plain, rtol=1e-4, atol=2e-5)
+    torch.testing.assert_close(state, plain_state, rtol=1e-4, atol=2e-5)
