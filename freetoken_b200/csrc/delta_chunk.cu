@@ -293,7 +293,8 @@ __global__ void __launch_bounds__(2 * NV * KS) delta_chunk_kernel(DeltaChunkArgs
       n_chunks = __shfl_sync(0xffffffffu, n, at);
     }
   }
-  if (seg < 0) return;
+  // (a table whose requests overlap, or more of them long than the caller said: chunks that no scratch was laid out for)
+  if (seg < 0 || before + n_chunks > a.n_chunks) return;
   const int q_start = a.seg_info[seg * 4], q_len = a.seg_info[seg * 4 + 1], kv_len = a.seg_info[seg * 4 + 2];
   const int slot = a.state_slots[seg];
   if (slot < 0 || slot >= a.n_slots) return;

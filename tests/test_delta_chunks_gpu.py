@@ -221,3 +221,22 @@ def test_unit_vectors_without_a_floor(H, G, D, Dv, lens):
     assert torch.isfinite(plain).all() and torch.isfinite(plain_state).all()
     torch.testing.assert_close(out, plain, rtol=1e-4, atol=2e-5)
     torch.testing.assert_close(state, plain_state, rtol=1e-4, atol=2e-5)
+
+
+def test_requests_that_overlap_stay_within_scratch():
+    """A table that names more chunks than the tokens allow: what scratch holds is worked on, the rest is left alone."""
+    p = problem([(96, 96)] * 4, 4, 2, 128, 48)
+    _, clean = run(p, True)
+    p["info"][:, 0] = 0  # (four requests over the same 96 tokens of a step of 96: three chunks each, room for 96 / 32 + 4 = 7)
+    p = {k: (v[:96] if k in ("q", "k", "v", "b", "a") else v) for k, v in p.items()}
+    p["T"] = 96
+    n = ops.delta_chunk_scratch(torch.bfloat16, 96, 4, 4, 2, 128, 48)
+    guarded = torch.full((2 * n,), 171, dtype=torch.uint8, device=DEV)
+    H, G, D, Dv = p["sizes"]
+    out, state = torch.empty(96, H, Dv, device=DEV), p["state"].clone()
+    ops.delta_scan(p["q"], p["k"], p["v"], p["b"], p["a"], p["a_log"], p["dt_bias"], D ** -0.5, EPS, state, p["slots"], p["info"], 4, out,
+                   scratch=guarded)
+    slots = p["slots"].long()
+    assert torch.equal(state[slots[0]], clean[slots[0]]) and torch.equal(state[slots[1]], state[slots[0]])
+    assert torch.equal(state[slots[2:]], p["state"][slots[2:]])  # (chunks 6 to 11: past the scratch)
+    assert bool((guarded[n:] == 171).all())
