@@ -645,11 +645,7 @@ __global__ void __launch_bounds__(256, 2) gla_out_kernel(GlaArgs a) {
 #pragma unroll
       for (int i = 0; i < 8; ++i) step4(acc[i], &sh.q[tg + 8 * i][half * (D / 2) + 8 * st + d], y);
     }
-    if (st == 1 && tid < kGcTokens) {  // P has come: the rest of the 16-byte words on the diagonal
-      for (int s = tid + 1; s <= (tid | 3); ++s) sh.p[tid][s] = 0.f;
-    }
   }
-  static_assert(kStages >= 4, "a barrier between P's last words and their readers");
 #pragma unroll 1
   for (int s = 4 * half; s < n; s += 8) {
     uint64_t y[4][TC / 2];
@@ -662,9 +658,24 @@ __global__ void __launch_bounds__(256, 2) gla_out_kernel(GlaArgs a) {
         y[e][j + 1] = gc_pair(gc_low(w.y), gc_high(w.y));
       }
     }
+    // (a row takes the tokens up to its own: nothing of a later one, infinite or NaN, may reach it; what P's 16-byte words hold
+    // behind the diagonal was never written)
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
-      if (8 * i + 7 >= s) step4(acc[i], &sh.p[tg + 8 * i][s], y);  // (rows before s: zeros)
+    for (int i = 0; i < 8; ++i) {
+      if (8 * i > s) {
+        step4(acc[i], &sh.p[tg + 8 * i][s], y);
+      } else if (8 * i + 7 >= s) {
+        const int behind = tg + 8 * i - s;
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (e <= behind) {
+            const float f = sh.p[tg + 8 * i][s + e];
+            const uint64_t f2 = gc_pair(f, f);
+#pragma unroll
+            for (int j = 0; j < TC / 2; ++j) gc_fma2(acc[i][j], f2, y[e][j]);
+          }
+      }
+    }
   }
   // the upper threads' sums go through shared memory, where the stages lay
   __syncthreads();

@@ -113,3 +113,26 @@ def test_what_stays_token_by_token(kw):
     out, state, taken = run(p, kw["chunk"])
     want, want_state = exact(p)
     assert not taken and rel(out, want) <= 1e-6 and rel(state[p["slots"].long()], want_state[p["slots"].long()]) <= 1e-6
+
+
+@pytest.mark.parametrize("kw", [dict(D=128, Dv=128, chunk=64), dict(D=64, Dv=64, chunk=50), dict(D=64, Dv=96, chunk=64, decay="head", div=2)], ids=str)
+@pytest.mark.parametrize("what", ["q", "k", "v", "decay"])
+@pytest.mark.parametrize("at,value", [(0, float("nan")), (6, float("inf")), (21, float("nan")), (49, float("-inf")), (63, float("nan")), (129, float("nan"))])
+def test_a_value_that_is_no_number_reaches_no_earlier_token(kw, what, at, value):
+    """Nor another request: a later token counts for nothing, not for zero times what it holds."""
+    p = problem([(130, 150), (70, 70)], H=2, **kw)
+    clean, clean_state, taken = run(p, kw["chunk"])
+    name = what if what != "decay" else "z" if p["a_head"] is None else "a_head"
+    if name == "a_head" and value == value:
+        value = float("nan")  # (a decay itself, not its logit)
+    bad = dict(p, **{name: p[name].clone()})
+    if name in ("q", "k", "v"):  # (their rows stay views of the same wide rows)
+        cols = dict(q=p["q"], k=p["k"], v=p["v"])[name]
+        bad[name] = torch.empty(cols.shape[0], cols.stride(0), dtype=cols.dtype, device=DEV)[:, : cols.shape[1]].copy_(cols)
+    bad[name][at, ::2] = value
+    out, state, bad_taken = run(bad, kw["chunk"])
+    tokens, _, _ = run(bad, 0)
+    assert taken and bad_taken
+    assert torch.equal(out[:at], clean[:at]) and torch.equal(out[130:], clean[130:])
+    assert torch.equal(state[p["slots"][1]], clean_state[p["slots"][1]])
+    assert torch.isfinite(out[torch.isfinite(tokens)]).all()
