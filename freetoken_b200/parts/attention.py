@@ -48,7 +48,7 @@ TC_MIN_DECODE_SPAN = 0   # decode steps go there from this length of the longest
 def attention_kernel_form(dtype: torch.dtype, decode_only: bool = False, group: int = 1, n_tokens: int = 0,
                           head_dim: int = 0, page_size: int = 0, window: Optional[int] = None,
                           longest_span: int = 0, one_tile_only: bool = False, no_few: bool = False,
-                          window_on_tc: bool = False, plain_scores: bool = False) -> Tuple[int, bool]:
+                          window_on_tc: bool = False, plain_scores: bool = False, n_kv_heads: int = 1) -> Tuple[int, bool]:
     """``(query rows one attention CTA handles, the tcgen05 kernel's form for few rows)``.
 
     16 rows in the 32-bit kernel.  bfloat16 steps whose sizes the tcgen05 kernels take: 128 rows for
@@ -66,7 +66,9 @@ def attention_kernel_form(dtype: torch.dtype, decode_only: bool = False, group: 
     the ones with a single query tile a piece may be chosen (they are the ones that take a bias by distance);
     ``no_few``: nor the form for tiles of at most 16 rows (a window or a sink: the 128-row form alone takes them).
     ``plain_scores`` (no bias by distance, no soft cap): heads of 64 and 256 go to the tcgen05 kernels too, 256 in the
-    128-row form alone, for decode steps as well."""
+    128-row form alone, for decode steps as well (against 16-row tiles of mma.sync, a layer of 16 heads on 4 of 256: 36 against
+    39 microseconds for one request of 2,048 tokens, 50 against 66 for eight, 113 against 182 for 64; 16 on 16: 45 and 50, 96 and
+    106, 314 and 481; 16 on one: 35 and 47, 43 and 59, 70 and 98); heads of 64 with a window where :func:`window_64_pays`."""
     if dtype != torch.bfloat16:
         return 16, False
     sized = bool(head_dim and page_size)
@@ -77,6 +79,8 @@ def attention_kernel_form(dtype: torch.dtype, decode_only: bool = False, group: 
     if window is not None:  # (of the tcgen05 kernels the one with a single 128-row tile a piece takes a window)
         one_tile_only = no_few = True
     if decode_only:
+        if other and window is not None and not window_64_pays(n_tokens * n_kv_heads, min(window, longest_span)):
+            return (16 if group <= 16 else 64), False
         if sized and (not no_few or (window is not None and window_on_tc)) and longest_span >= TC_MIN_DECODE_SPAN:
             if not no_few and ops.attention_tc_few_fits(fits_as, page_size, group):
                 return 16, True
@@ -90,6 +94,17 @@ def attention_kernel_form(dtype: torch.dtype, decode_only: bool = False, group: 
     if tc and n_tokens >= TC_MIN_TOKENS:
         return 128, False
     return 64, False
+
+
+def window_64_pays(pairs: int, keys: int) -> bool:
+    """Whether a decode step of heads of 64 over windows of ``keys`` keys is faster on the tcgen05 kernel's 128-row tiles than on
+    16-row tiles of mma.sync; ``pairs``: (request, KV head) pairs.  A piece costs the former some 4 microseconds beside its keys,
+    one CTA an SM, so it wins with long windows, with few pairs, and where the pairs fill one to three rounds of the SMs.  A layer of
+    32 heads on 8, mma.sync against tcgen05: windows of 1,024, 31 and 27 us for one request, 47 and 43 for 16, 55 and 61 for 24,
+    78 and 74 for 48, 92 and 113 for 64, 139 and 148 for 128; of 128, 29 and 31 for 8, 39 and 61 for 64; of 512, 37 and 35 for 8,
+    45 and 51 for 24, 66 and 78 for 64; of 4,096, 66 and 53 for 8, 168 and 131 for 32."""
+    rounds = -(-pairs // 148)
+    return keys >= 4096 or (keys >= 512 and pairs <= 64) or (keys >= 1024 and rounds <= 3 and pairs >= 0.85 * 148 * rounds)
 
 
 def attention_tile_rows(dtype: torch.dtype, decode_only: bool = False, group: int = 1, n_tokens: int = 0,
@@ -245,7 +260,7 @@ class GQAttention(Mixer):
         return attention_kernel_form(self.env.dtype, decode_only, self.plan_group, n_tokens,
                                      self.pad_dim if sized else 0, page_size, self.window, longest_span,
                                      one_tile_only=special or self.log_dist_bias, no_few=special, window_on_tc=True,
-                                     plain_scores=not self.log_dist_bias)
+                                     plain_scores=not self.log_dist_bias, n_kv_heads=self.plan_kv_heads)
 
     def tile_rows(self, decode_only: bool, n_tokens: int = 0, page_size: int = 0, longest_span: int = 0) -> int:
         return self.kernel_form(decode_only, n_tokens, page_size, longest_span)[0]
