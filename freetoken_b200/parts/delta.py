@@ -137,8 +137,14 @@ class GatedDelta(Mixer):
         item = 4 if self.env.dtype == torch.float32 else 2
         H, D, Dv = self.n_heads, self.head_dim, self.v_dim
         own = (self.proj_rows + self.conv_dim + H * Dv + self.hidden + (H * Dv if self.gate_rank else 0)) * item
-        chunks = 0 if self.decay_rank else ops.delta_chunk_scratch(self.env.dtype, n_tokens, self.env.max_decode_rows, H, self.n_kv_heads, D, Dv)
-        return n_tokens * (own + (H * Dv + (H * D if self.decay_rank else 0)) * 4) + chunks
+        return n_tokens * (own + (H * Dv + (H * D if self.decay_rank else 0)) * 4) + self.chunk_scratch(n_tokens, n_tokens // CHUNK_MIN_TOKENS)[1]
+
+    def chunk_scratch(self, n_tokens: int, n_long: int):
+        """``(chunks, bytes)`` of what ``n_long`` requests of a step of so many tokens need to go in chunks (0 bytes: they do not)."""
+        if self.decay_rank:
+            return 0, 0
+        return n_tokens // 32 + n_long, ops.delta_chunk_scratch(self.env.dtype, n_tokens, n_long, self.n_heads, self.n_kv_heads,
+                                                               self.head_dim, self.v_dim)
 
     def forward(self, h: torch.Tensor, step: StepState, cache: Any, writes_cache: bool) -> torch.Tensor:
         if not writes_cache:
@@ -162,11 +168,10 @@ class GatedDelta(Mixer):
         long = [seg.q_len for seg in step.segments if seg.q_len >= CHUNK_MIN_TOKENS] if z is None and h.is_cuda else []
         n_long = len(long)
         if long and chunks_pay(long, n_long < n_segs, H, D, Dv):
-            sizes = (H, self.n_kv_heads, D, Dv)
-            n = ops.delta_chunk_scratch(dt, T, n_long, *sizes)
-            if n:
-                most = ops.delta_chunk_scratch(dt, cap, max(n_segs, self.env.max_decode_rows), *sizes)
-                args = dict(scratch=ws.get("delta.chunks", (n,), torch.uint8, (most,)), long_from=CHUNK_MIN_TOKENS, n_long=n_long)
+            chunks, n = self.chunk_scratch(T, n_long)
+            if n:  # (a row a chunk: layers of other sizes have a buffer of their own, and no step asks for more rows)
+                row, most = n // chunks, self.chunk_scratch(cap, cap // CHUNK_MIN_TOKENS)[0]
+                args = dict(scratch=ws.get("delta.chunks", (chunks, row), torch.uint8, (most, row)), long_from=CHUNK_MIN_TOKENS, n_long=n_long)
         ops.delta_scan(qkv[:, : self.k_col], qkv[:, self.k_col: self.v_col], qkv[:, self.v_col:],
                        proj[:, self.b_col: self.a_col], a, self.params["A_log"], self.params["dt_bias"],
                        D ** -0.5, UNIT_EPS, cache.tensors["s"], step.state_slots, step.seg_info, n_segs, o32, **args)

@@ -240,3 +240,35 @@ def test_requests_that_overlap_stay_within_scratch():
     assert torch.equal(state[slots[0]], clean[slots[0]]) and torch.equal(state[slots[1]], state[slots[0]])
     assert torch.equal(state[slots[2:]], p["state"][slots[2:]])  # (chunks 6 to 11: past the scratch)
     assert bool((guarded[n:] == 171).all())
+
+
+def test_layers_of_different_sizes_share_a_workspace():
+    """Each has scratch of its own from its first step on, with room for the largest: nothing that a step was given moves later."""
+    from freetoken_b200.config.spec import PartSpec
+    from freetoken_b200.parts import MIXERS, BuildEnv, Segment, StepState, Workspace
+
+    env = BuildEnv(dtype=torch.bfloat16, device=torch.device(DEV), max_seq_len=512, max_step_tokens=480, workspace=Workspace(torch.device(DEV)),
+                   max_decode_rows=2)
+    layers = []
+    for heads in (2, 6):
+        part = MIXERS.build(PartSpec("gated_delta", dict(hidden=64, n_heads=heads, n_kv_heads=2, head_dim=64, v_head_dim=16, taps=1, eps=1e-6)), env)
+        part.bind({n: torch.zeros(s.shape, device=DEV, dtype=torch.float32 if s.dtype == "float32" else torch.bfloat16)
+                   for n, s in part.param_specs().items()})
+        layers.append(part)
+
+    def step(lens):
+        info = [[sum(lens[:i]), n, n, 0] for i, n in enumerate(lens)]
+        T = sum(lens)
+        s = StepState(n_tokens=T, segments=[Segment(i, a, n, kv) for i, (a, n, kv, _) in enumerate(info)], token_ids=None, positions=None,
+                      seg_info=torch.tensor(info, dtype=torch.int32, device=DEV), state_slots=torch.arange(len(lens), dtype=torch.int32, device=DEV),
+                      logit_rows=None, n_logit_rows=0, attention_plans={}, decode_only=False)
+        for part in layers:
+            cache = type("C", (), dict(tensors={"s": torch.zeros(len(lens), part.n_heads, 16, 64, device=DEV)}))
+            part.forward(torch.zeros(T, 64, dtype=torch.bfloat16, device=DEV), s, cache, True)
+        return {k: b.data_ptr() for k, b in env.workspace._buffers.items() if k[0] == "delta.chunks"}
+
+    first = step([200])
+    assert len(first) == 2
+    assert step([80] * 6) == first and step([480]) == first and step([81] * 5) == first  # (as many requests as fit in a step)
+    assert sum(b.numel() for k, b in env.workspace._buffers.items() if k[0] == "delta.chunks") == sum(
+        p.chunk_scratch(480, 6)[1] for p in layers)
