@@ -239,7 +239,11 @@ __global__ void __launch_bounds__(32 * kFewWarps) moe_gemm_few_kernel(const T* _
 }
 
 // Which of them: by the mean number of rows an expert has (the counts are on the device), and 16-byte (bfloat16: 8-byte)
-// loads where rows and bases allow them.
+// loads where rows and bases allow them.  Up to 4 rows the kernel for few rows: 16 experts of 1,024 x 1,408 in 32 bits with 1, 2
+// and 4 rows each 49 + 31, 50 + 35 and 68 + 46 us for the two products, against 111 + 84 of the tiles at 5 (and at 1 to 16) rows.  Up
+// to 32 rows tiles of 32 rows, one an expert: 113 + 86 us at 32 rows; at 33 an expert has two of them, twice that, and tiles of 64
+// take 169 + 117.  The mean can mislead: 256 rows of 64 experts' four each on one of them are 33 tiles of eight rows, 146 + 133 us
+// (the kernels of 32-row tiles before these: 180 + 201).
 template <typename T, bool GATED>
 static int launch_moe_gemm(const void* x, const void* w, const int32_t* offsets, int n_experts, int K, int N, int w_rows,
                            const int32_t* routes, const float* weights, int n_routes, int act, float alpha, float limit, void* out,
@@ -255,7 +259,8 @@ static int launch_moe_gemm(const void* x, const void* w, const int32_t* offsets,
     return 0; \
   } while (0)
   constexpr int cols = GATED ? kTiledCols / 2 : kTiledCols;
-  if (wide && n_routes <= 4 * n_experts)
+  // (tiles of a few rows are the most: with so many experts that a grid cannot hold them, larger ones)
+  if (wide && n_routes <= 4 * n_experts && grid_of(kFewRows, 1).y <= 65535u)
     FTK_MOE_GEMM((moe_gemm_few_kernel<T, GATED>), kFewRows, (GATED ? 1 : 2) * kFewPairs * kFewWarps, 32 * kFewWarps);
   if (wide && n_routes <= 32 * n_experts) FTK_MOE_GEMM((moe_gemm_kernel<T, GATED, 32, true>), 32, cols, kTiledThreads);
   if (wide) FTK_MOE_GEMM((moe_gemm_kernel<T, GATED, 64, true>), 64, cols, kTiledThreads);

@@ -41,3 +41,15 @@ def test_expert_products(dtype, hidden, inter, rows, act):
     torch.testing.assert_close(a.double(), want, **tol)
     down = torch.einsum("rk,rnk->rn", a.double(), w2.double()[e]) * weights.double()[routes.long()][:, None]
     torch.testing.assert_close(y.double(), down, **tol)
+
+
+def test_more_experts_than_a_grid_has_tiles_of_few_rows():
+    """44,000 experts of four rows: 66,000 tiles of eight rows do not fit a grid, 49,500 of 32 rows do."""
+    E, K, I = 44000, 8, 4
+    g = torch.Generator(device=DEV).manual_seed(1)
+    x, w1 = torch.randn(4 * E, K, device=DEV, generator=g), torch.randn(E, 2 * I, K, device=DEV, generator=g)
+    offsets = torch.arange(0, 4 * E + 1, 4, dtype=torch.int32, device=DEV)
+    a = torch.full((4 * E, I), float("nan"), device=DEV)
+    ops.moe_gemm1_act(x, w1, offsets, "silu", 1.702, 7.0, a)
+    gu = torch.einsum("erk,enk->ern", x.view(E, 4, K).double(), w1.double()).view(4 * E, 2 * I)
+    torch.testing.assert_close(a.double(), gu[:, :I] * torch.sigmoid(gu[:, :I]) * gu[:, I:], rtol=1e-5, atol=2e-5)  # (8 terms in 32 bits)
