@@ -232,16 +232,10 @@ int ftk_gla_scan(const void* q, long long q_stride, const void* k, long long k_s
                  const int32_t* chunks, int n_chunks, const int32_t* seg_chunks, int any_single, int any_multi,
                  float* carry, float* decay_prod, float* out, int n_tokens, int n_heads, int dim, int vdim,
                  const float* k_fac, const float* a_head, int a_head_stride, int ones_col, float* out_ones, int qk_div,
-                 const float* rope, int n_rot, int rope_neighbours, int max_pos, void* stream);
-// The same for a caller that knows its chunks: none longer than longest_chunk tokens (0: not known).  From 32 to 64, bfloat16 rows
-// of 64 or 128 key and 64 to 128 value channels go as matrix products; z and out's rows then serve as scratch on the way.
-int ftk_gla_scan_chunks(const void* q, long long q_stride, const void* k, long long k_stride, const void* v,
-                 long long v_stride, int dtype, float* z, const float* z_bias, float tau, float q_scale,
-                 float* state, int n_slots, const int32_t* state_slots, const int32_t* seg_info, int n_segs,
-                 const int32_t* chunks, int n_chunks, const int32_t* seg_chunks, int any_single, int any_multi,
-                 float* carry, float* decay_prod, float* out, int n_tokens, int n_heads, int dim, int vdim,
-                 const float* k_fac, const float* a_head, int a_head_stride, int ones_col, float* out_ones, int qk_div,
-                 const float* rope, int n_rot, int rope_neighbours, int max_pos, int longest_chunk, void* stream);
+                 const float* rope, int n_rot, int rope_neighbours, int max_pos, int longest_chunk, int* launches, void* stream);
+// (longest_chunk: no chunk of the list is longer; 0: not known.  From 32 to 64, bfloat16 rows of 64 or 128 key and 64 to 128 value
+// channels go as matrix products; z and out's rows then serve as scratch on the way.  launches, in host memory or null: how many
+// kernels the call has launched)
 // (a_head_stride 0: a_head [n_heads], the same decays for every token.  rope [max_pos, n_rot] cos || sin: queries and keys
 // are rotated by their position, in 32 bits, as they are read; pairs of neighbours or of halves of the n_rot dimensions.)
 // (qk_div > 1: head h reads the queries and keys of head h / qk_div, and q, k hold n_heads / qk_div heads; with a_head)

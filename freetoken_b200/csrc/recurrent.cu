@@ -538,8 +538,7 @@ __global__ void gla_carry_kernel(GlaArgs a) {
 namespace ftk {
 
 template <typename T, int DPT>
-static int launch_gla(GlaArgs a, bool any_single, bool any_multi, int longest_chunk, cudaStream_t s) {
-  const bool products = any_multi && sizeof(T) == 2 && gla_chunks_fit(a, longest_chunk);
+static int launch_gla(GlaArgs a, bool any_single, bool any_multi, bool products, cudaStream_t s) {
   const int Dp = DPT * kGlaSlices;
   constexpr int kGlaCols = 32 * gla_cols_per_thread(DPT);
   const int dv_real = a.Dv - a.ones_col;  // the column of ones rides in the block of the first columns
@@ -556,9 +555,11 @@ static int launch_gla(GlaArgs a, bool any_single, bool any_multi, int longest_ch
   auto k1 = gla_chunk_kernel<T, DPT, 1>;
   auto k3 = gla_chunk_kernel<T, DPT, 3>;
   if (smem > 48 * 1024) {
-    cudaFuncSetAttribute(k0, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(k3, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (any_single) cudaFuncSetAttribute(k0, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (any_multi && !products) {
+      cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      cudaFuncSetAttribute(k3, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    }
   }
   if (any_multi && !products && !a.a_head) {  // the decays of all of the step's tokens, once, where the logits lay
     const long long n = (long long)a.n_tokens * a.H * a.D;
@@ -596,22 +597,9 @@ extern "C" int ftk_gla_scan(const void* q, long long q_stride, const void* k, lo
                             const int32_t* seg_chunks, int any_single, int any_multi, float* carry,
                             float* decay_prod, float* out, int n_tokens, int n_heads, int dim, int vdim,
                             const float* k_fac, const float* a_head, int a_head_stride, int ones_col, float* out_ones,
-                            int qk_div, const float* rope, int n_rot, int rope_neighbours, int max_pos, void* stream) {
-  return ftk_gla_scan_chunks(q, q_stride, k, k_stride, v, v_stride, dtype, z, z_bias, tau, q_scale, state, n_slots, state_slots,
-                             seg_info, n_segs, chunks, n_chunks, seg_chunks, any_single, any_multi, carry, decay_prod, out,
-                             n_tokens, n_heads, dim, vdim, k_fac, a_head, a_head_stride, ones_col, out_ones, qk_div, rope, n_rot,
-                             rope_neighbours, max_pos, 0, stream);
-}
-
-extern "C" int ftk_gla_scan_chunks(const void* q, long long q_stride, const void* k, long long k_stride, const void* v,
-                            long long v_stride, int dtype, float* z, const float* z_bias, float tau,
-                            float q_scale, float* state, int n_slots, const int32_t* state_slots,
-                            const int32_t* seg_info, int n_segs, const int32_t* chunks, int n_chunks,
-                            const int32_t* seg_chunks, int any_single, int any_multi, float* carry,
-                            float* decay_prod, float* out, int n_tokens, int n_heads, int dim, int vdim,
-                            const float* k_fac, const float* a_head, int a_head_stride, int ones_col, float* out_ones,
                             int qk_div, const float* rope, int n_rot, int rope_neighbours, int max_pos, int longest_chunk,
-                            void* stream) {
+                            int* launches, void* stream) {
+  if (launches) *launches = 0;
   FTK_REQUIRE(dtype_ok(dtype), "gla_scan: bad dtype %d", dtype);
   FTK_REQUIRE(n_tokens >= 0 && n_segs >= 0 && n_chunks >= 0, "gla_scan: bad counts");
   if (n_tokens == 0 || n_chunks == 0) return 0;
@@ -639,11 +627,12 @@ extern "C" int ftk_gla_scan_chunks(const void* q, long long q_stride, const void
   a.k_fac = k_fac; a.a_head = a_head; a.ones_col = ones_col; a.out_ones = out_ones; a.qk_div = qk_div;
   a.out = out; a.H = n_heads; a.D = dim; a.Dv = vdim; a.n_tokens = n_tokens;
   cudaStream_t s = (cudaStream_t)stream;
-  note_variant(!any_multi ? "gla_scan: one chunk per request"
-               : dtype == FTK_BF16 && gla_chunks_fit(a, longest_chunk) ? "gla_scan: chunks as products" : "gla_scan: chunks side by side");
+  const bool products = any_multi && dtype == FTK_BF16 && gla_chunks_fit(a, longest_chunk);
+  note_variant(!any_multi ? "gla_scan: one chunk per request" : products ? "gla_scan: chunks as products" : "gla_scan: chunks side by side");
+  if (launches) *launches = (any_single ? 1 : 0) + (products ? 3 : any_multi ? (a_head ? 3 : 4) : 0);
   const bool f32 = dtype == FTK_F32;
-  if (dim <= 32) return f32 ? launch_gla<float, 8>(a, any_single, any_multi, longest_chunk, s) : launch_gla<__nv_bfloat16, 8>(a, any_single, any_multi, longest_chunk, s);
-  if (dim <= 64) return f32 ? launch_gla<float, 16>(a, any_single, any_multi, longest_chunk, s) : launch_gla<__nv_bfloat16, 16>(a, any_single, any_multi, longest_chunk, s);
-  if (dim <= 128) return f32 ? launch_gla<float, 32>(a, any_single, any_multi, longest_chunk, s) : launch_gla<__nv_bfloat16, 32>(a, any_single, any_multi, longest_chunk, s);
-  return f32 ? launch_gla<float, 64>(a, any_single, any_multi, longest_chunk, s) : launch_gla<__nv_bfloat16, 64>(a, any_single, any_multi, longest_chunk, s);
+  if (dim <= 32) return f32 ? launch_gla<float, 8>(a, any_single, any_multi, products, s) : launch_gla<__nv_bfloat16, 8>(a, any_single, any_multi, products, s);
+  if (dim <= 64) return f32 ? launch_gla<float, 16>(a, any_single, any_multi, products, s) : launch_gla<__nv_bfloat16, 16>(a, any_single, any_multi, products, s);
+  if (dim <= 128) return f32 ? launch_gla<float, 32>(a, any_single, any_multi, products, s) : launch_gla<__nv_bfloat16, 32>(a, any_single, any_multi, products, s);
+  return f32 ? launch_gla<float, 64>(a, any_single, any_multi, products, s) : launch_gla<__nv_bfloat16, 64>(a, any_single, any_multi, products, s);
 }

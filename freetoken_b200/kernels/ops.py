@@ -181,10 +181,7 @@ _SIGNATURES = {
     "ftk_mlstm_output": [_vp, _vp, _vp, _vp, ctypes.c_longlong, _vp, _f, _vp, _i, _i, _i, _i, _vp],
     "ftk_gla_scan": [_vp, ctypes.c_longlong, _vp, ctypes.c_longlong, _vp, ctypes.c_longlong, _i, _vp, _vp, _f, _f,
                      _vp, _i, _vp, _vp, _i, _vp, _i, _vp, _i, _i, _vp, _vp, _vp, _i, _i, _i, _i, _vp, _vp, _i, _i, _vp, _i,
-                     _vp, _i, _i, _i, _vp],
-    "ftk_gla_scan_chunks": [_vp, ctypes.c_longlong, _vp, ctypes.c_longlong, _vp, ctypes.c_longlong, _i, _vp, _vp, _f, _f,
-                     _vp, _i, _vp, _vp, _i, _vp, _i, _vp, _i, _i, _vp, _vp, _vp, _i, _i, _i, _i, _vp, _vp, _i, _i, _vp, _i,
-                     _vp, _i, _i, _i, _i, _vp],
+                     _vp, _i, _i, _i, _i, _vp, _vp],
     "ftk_hyper_step": [_vp, ctypes.c_longlong, _i, _i, _i, _vp, _vp, _i, _vp, _vp, _vp, _vp, _f, _vp, _i, _vp, _vp],
     "ftk_conv_act": [_vp, ctypes.c_longlong, _i, _vp, _vp, _i, _i, _vp, _i, _vp, _vp, _i, _vp, _i, _i, _vp],
     "ftk_delta_scan_chunks": [_vp, ctypes.c_longlong, _vp, ctypes.c_longlong, _vp, ctypes.c_longlong, _vp, ctypes.c_longlong,
@@ -218,6 +215,8 @@ def _lib():
             fn = getattr(lib, name)
             fn.argtypes = args
             fn.restype = _i
+        lib.ftk_delta_chunk_scratch.argtypes = [_i] * 7
+        lib.ftk_delta_chunk_scratch.restype = ctypes.c_longlong
         _bound = lib
     return _bound
 
@@ -634,7 +633,7 @@ def attention_tc_fits(head_dim: int, page_size: int, group: int) -> bool:
 def attention_tc_heads_fit(head_dim: int, page_size: int, group: int) -> bool:
     """Whether the tcgen05 attention kernels take these sizes for heads of another size than 128: 64 in every form, 256 in
     tiles of 128 rows; neither with a bias by distance or a soft cap (``csrc/attention_tc.cuh: attention_tc_heads_fit``)."""
-    return head_dim in (64, 256) and attention_tc_fits(128, page_size, group)
+    return bool(_lib().ftk_attention_tc_heads_fit(head_dim, page_size, group))
 
 
 def attention_tc_few_fits(head_dim: int, page_size: int, group: int) -> bool:
@@ -1220,8 +1219,8 @@ def gla_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: Optional[torc
         raise KernelError("gla_scan: scratch for segments of several chunks is missing or too small")
     if chunks.numel() < 4 * n_chunks or seg_chunks.numel() < 2 * n_segs:
         raise KernelError("gla_scan: chunk lists too short")
-    launches = (1 if any_single else 0) + ((4 if a_head is None else 3) if any_multi else 0)
-    _check(_lib().ftk_gla_scan_chunks(
+    launches = ctypes.c_int()
+    _check(_lib().ftk_gla_scan(
         q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), _code(q, "q"),
         _dev(z, "z", torch.float32), _dev(z_bias, "z_bias", torch.float32), float(tau), float(q_scale),
         _dev(state, "state", torch.float32), state.shape[0], _dev(state_slots, "state_slots", torch.int32),
@@ -1232,7 +1231,8 @@ def gla_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: Optional[torc
         _dev(a_head, "a_head", torch.float32), 0 if one_row else H, 1 if ones_col else 0,
         _dev(out_ones, "out_ones", torch.float32), qk_div, _dev(rope_table, "rope_table", torch.float32),
         rope_table.shape[1] if rope_table is not None else 0, 1 if neighbours else 0,
-        rope_table.shape[0] if rope_table is not None else 0, int(chunk), _stream()), "gla_scan", max(1, launches))
+        rope_table.shape[0] if rope_table is not None else 0, int(chunk), ctypes.addressof(launches), _stream()), "gla_scan", 0)
+    count_launches(launches.value)
 
 
 # --------------------------------------------------------------------------- short convolution, depth mix
@@ -1619,12 +1619,17 @@ def ssm_output(o32: torch.Tensor, x: torch.Tensor, d_skip: torch.Tensor, z: torc
                                  int(norm_groups), float(eps), _dev(out, "out"), T, H, P, _stream()), "ssm_output")
 
 
+DELTA_CHUNK = 32  # tokens a chunk
+# of a chunk and head: rows of T and A T, four factors a token, the chunk's decay (csrc/delta_chunk.cu: kDcBytes)
+DELTA_CHUNK_BYTES = DELTA_CHUNK * 2 * DELTA_CHUNK * 4 + 4 * DELTA_CHUNK * 4 + 16
+
+
 def delta_chunk_scratch(dtype: torch.dtype, n_tokens: int, n_long: int, n_heads: int, n_kv_heads: int, dim: int, vdim: int) -> int:
     """Bytes of scratch with which :func:`delta_scan` may take ``n_long`` requests of a step of so many tokens in chunks; 0 where
-    the sizes are not taken (as ``ftk_delta_chunk_scratch`` says)."""
+    the sizes are not taken (what ``ftk_delta_chunk_scratch`` says, without the library: engines on any device size their buffers)."""
     if dtype != torch.bfloat16 or dim not in (64, 128) or vdim < 16 or vdim % 16 or n_heads % n_kv_heads or n_tokens < 1 or n_long < 1:
         return 0
-    return (n_tokens // 32 + n_long) * n_heads * (32 * 64 * 4 + 4 * 32 * 4 + 16)
+    return (n_tokens // DELTA_CHUNK + n_long) * n_heads * DELTA_CHUNK_BYTES
 
 
 def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, b_raw: torch.Tensor, a_raw: Optional[torch.Tensor],

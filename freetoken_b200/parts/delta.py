@@ -55,7 +55,7 @@ def chunks_pay(lens: Sequence[int], beside: bool, n_heads: int, head_dim: int, v
     states = sum(lens) / longest * n_heads  # (request, head) pairs at work, on average
     wide = head_dim > 64
     rounds = lambda cols: math.ceil(states * -(-v_dim // cols) / SMS)  # noqa: E731  (blocks of so many value columns an SM)
-    chunks = -(-longest // 32)
+    chunks = -(-longest // ops.DELTA_CHUNK)
     if states * -(-v_dim // 16) <= 2 * SMS:  # (as csrc/delta_chunk.cu: launch_delta_chunks)
         in_chunks = 22.5 + chunks * (2.6 if wide else 1.7) * (1.0 if rounds(16) == 1 else 1.5 if wide else 2.1)
     else:
@@ -143,7 +143,7 @@ class GatedDelta(Mixer):
         """``(chunks, bytes)`` of what ``n_long`` requests of a step of so many tokens need to go in chunks (0 bytes: they do not)."""
         if self.decay_rank:
             return 0, 0
-        return n_tokens // 32 + n_long, ops.delta_chunk_scratch(self.env.dtype, n_tokens, n_long, self.n_heads, self.n_kv_heads,
+        return n_tokens // ops.DELTA_CHUNK + n_long, ops.delta_chunk_scratch(self.env.dtype, n_tokens, n_long, self.n_heads, self.n_kv_heads,
                                                                self.head_dim, self.v_dim)
 
     def forward(self, h: torch.Tensor, step: StepState, cache: Any, writes_cache: bool) -> torch.Tensor:

@@ -1,9 +1,11 @@
-"""Which attention kernel a decode step of windowed heads of 64 goes to: the rule against timings of both kernels."""
+"""Which attention kernels take which heads, and where a decode step of windowed heads of 64 goes: the rule against timings of both
+kernels."""
 
 import pytest
 import torch
 
 from freetoken_b200.config.spec import PartSpec
+from freetoken_b200.kernels import ops
 from freetoken_b200.parts import MIXERS, BuildEnv, Workspace
 
 
@@ -20,3 +22,11 @@ def test_windowed_heads_of_64(heads, kv, n, window, span, mma_us, tc_us):
     part = MIXERS.build(PartSpec("gqa_attention", dict(hidden=64, n_heads=heads, n_kv_heads=kv, head_dim=64, eps=1e-6,
                                                        position=PartSpec("none"), window=window)), env)
     assert part.kernel_form(True, n, 16, span) == ((128, False) if tc_us < mma_us else (16, False))
+
+
+@pytest.mark.parametrize("head_dim", [16, 32, 64, 96, 128, 192, 256])
+@pytest.mark.parametrize("page,group", [(16, 1), (16, 128), (16, 129), (8, 4), (64, 6), (24, 4)])
+def test_heads_of_the_tensor_core_kernels(head_dim, page, group):
+    fits = page % 16 == 0 and group <= 128
+    assert ops.attention_tc_fits(head_dim, page, group) == (fits and head_dim == 128)
+    assert ops.attention_tc_heads_fit(head_dim, page, group) == (fits and head_dim in (64, 256))

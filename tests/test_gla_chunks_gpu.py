@@ -136,3 +136,15 @@ def test_a_value_that_is_no_number_reaches_no_earlier_token(kw, what, at, value)
     assert torch.equal(out[:at], clean[:at]) and torch.equal(out[130:], clean[130:])
     assert torch.equal(state[p["slots"][1]], clean_state[p["slots"][1]])
     assert torch.isfinite(out[torch.isfinite(tokens)]).all()
+
+
+@pytest.mark.parametrize("lens,chunk,kw,launches", [
+    ([(130, 130), (1, 9)], 64, dict(D=64, Dv=64), 4), ([(130, 130)], 64, dict(D=64, Dv=64), 3), ([(1, 9)], 64, dict(D=64, Dv=64), 1),
+    ([(130, 130), (1, 9)], 16, dict(D=64, Dv=64), 5), ([(130, 130)], 64, dict(D=64, Dv=64, decay="head"), 3),
+    ([(130, 130)], 16, dict(D=64, Dv=64, decay="head"), 3)], ids=str)
+def test_launches_are_counted(lens, chunk, kw, launches):
+    """Single chunks one, products three, chunks side by side three and one for the decays of channels."""
+    p = problem(lens, H=2, chunk=chunk, **kw)
+    before = ops.launch_count()
+    run(p, chunk)
+    assert ops.launch_count() - before == launches
