@@ -64,16 +64,6 @@ __device__ __forceinline__ uint32_t dc_lds(const __nv_bfloat16* p) { return *rei
 
 // Where row t of T, and right behind it row t of A T, lies among 64: a thread takes tokens that are eight apart.
 __host__ __device__ constexpr int dc_place(int t) { return t % 8 * 8 + t / 8 * 2; }
-__device__ __forceinline__ uint64_t dc_pair(float x, float y) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
-  return r;
-}
-__device__ __forceinline__ void dc_unpair(uint64_t p, float& x, float& y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(p)); }
-__device__ __forceinline__ void dc_fma2(uint64_t& d, uint64_t a, uint64_t b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b)); }
-// the two bfloat16 of a word
-__device__ __forceinline__ float dc_low(uint32_t w) { return __uint_as_float(w << 16); }
-__device__ __forceinline__ float dc_high(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
 
 // chunks of a segment; 0 for one that the kernels leave alone
 __device__ __forceinline__ int dc_chunks(const DeltaChunkArgs& a, int seg) {
@@ -360,12 +350,12 @@ __global__ void __launch_bounds__(2 * NV * KS) delta_chunk_kernel(DeltaChunkArgs
           dc_load4(sp + (d0 + e) * NV, y);
           uint64_t y2[4];
 #pragma unroll
-          for (int j = 0; j < 4; ++j) y2[j] = dc_pair(y[j], y[j]);
+          for (int j = 0; j < 4; ++j) y2[j] = f2_pair(y[j], y[j]);
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            const uint64_t x = e & 1 ? dc_pair(dc_high(kw[i][e >> 1]), dc_high(qw[i][e >> 1])) : dc_pair(dc_low(kw[i][e >> 1]), dc_low(qw[i][e >> 1]));
+            const uint64_t x = e & 1 ? f2_pair(bf2_high(kw[i][e >> 1]), bf2_high(qw[i][e >> 1])) : f2_pair(bf2_low(kw[i][e >> 1]), bf2_low(qw[i][e >> 1]));
 #pragma unroll
-            for (int j = 0; j < 4; ++j) dc_fma2(acc[i][j], x, y2[j]);
+            for (int j = 0; j < 4; ++j) f2_fma(acc[i][j], x, y2[j]);
           }
         }
       }
@@ -373,7 +363,7 @@ __global__ void __launch_bounds__(2 * NV * KS) delta_chunk_kernel(DeltaChunkArgs
       for (int i = 0; i < 4; ++i) {
         float k4[4], q4[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) dc_unpair(acc[i][j], k4[j], q4[j]);
+        for (int j = 0; j < 4; ++j) f2_unpair(acc[i][j], k4[j], q4[j]);
         float* dst = &sh.part[kr][8 * tg + 2 * i][c0];
         *reinterpret_cast<float4*>(dst) = make_float4(k4[0], k4[1], k4[2], k4[3]);
         *reinterpret_cast<float4*>(dst + NV) = make_float4(q4[0], q4[1], q4[2], q4[3]);
@@ -403,7 +393,7 @@ __global__ void __launch_bounds__(2 * NV * KS) delta_chunk_kernel(DeltaChunkArgs
       *reinterpret_cast<float4*>(&sh.x[t][c0]) = make_float4(fmaf(be, v[0], -bs * k4[0]), fmaf(be, v[1], -bs * k4[1]),
                                                              fmaf(be, v[2], -bs * k4[2]), fmaf(be, v[3], -bs * k4[3]));
 #pragma unroll
-      for (int j = 0; j < 4; ++j) r[i][j] = dc_pair(0.f, os * q4[j]);
+      for (int j = 0; j < 4; ++j) r[i][j] = f2_pair(0.f, os * q4[j]);
     }
     __syncthreads();
     // [T; A T] X, again a token's two rows as a pair
@@ -427,7 +417,7 @@ __global__ void __launch_bounds__(2 * NV * KS) delta_chunk_kernel(DeltaChunkArgs
       for (int i = 0; i < NT; ++i) {
         if (!all && e > own + tg + 8 * i) continue;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) dc_fma2(r[i][j], x[i], dc_pair(y[j], y[j]));
+        for (int j = 0; j < 4; ++j) f2_fma(r[i][j], x[i], f2_pair(y[j], y[j]));
       }
     };
 #pragma unroll 8
@@ -439,7 +429,7 @@ __global__ void __launch_bounds__(2 * NV * KS) delta_chunk_kernel(DeltaChunkArgs
       const int t = tg + 8 * (kr * NT + i), tok = ch * kDcTokens + t;
       float u[4], o[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) dc_unpair(r[i][j], u[j], o[j]);
+      for (int j = 0; j < 4; ++j) f2_unpair(r[i][j], u[j], o[j]);
       const float ks = st.vec[3 * kDcTokens + t];
       *reinterpret_cast<float4*>(&sh.u[t][c0]) = make_float4(ks * u[0], ks * u[1], ks * u[2], ks * u[3]);
       if (live && tok < q_len)
@@ -457,9 +447,9 @@ __global__ void __launch_bounds__(2 * NV * KS) delta_chunk_kernel(DeltaChunkArgs
       dc_load4(&sh.u[e][c0], y);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const uint64_t y2 = dc_pair(y[j], y[j]);
+        const uint64_t y2 = f2_pair(y[j], y[j]);
 #pragma unroll
-        for (int i = 0; i < DT / 2; ++i) dc_fma2(add[i][j], dc_pair(dc_low(w[i]), dc_high(w[i])), y2);
+        for (int i = 0; i < DT / 2; ++i) f2_fma(add[i][j], f2_pair(bf2_low(w[i]), bf2_high(w[i])), y2);
       }
     }
 #pragma unroll
@@ -467,7 +457,7 @@ __global__ void __launch_bounds__(2 * NV * KS) delta_chunk_kernel(DeltaChunkArgs
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         float x, y;
-        dc_unpair(add[i / 2][j], x, y);
+        f2_unpair(add[i / 2][j], x, y);
         s[i][j] = fmaf(whole, s[i][j], x);
         s[i + 1][j] = fmaf(whole, s[i + 1][j], y);
       }
@@ -506,7 +496,9 @@ static int launch_delta_chunks_as(const DeltaChunkArgs& a, cudaStream_t s) {
 // Columns a block.  16, twelve warps' worth of 48 shared out over three blocks, while that leaves SMs without a third block; else
 // 48 with twelve warps, three a scheduler.  Chunk kernel alone, 2,048 tokens of 128 key channels, 16 heads of 128 (128 blocks of
 // 16 columns): 282 us, blocks of 48 columns 385; 48 heads (384 and 144 blocks): 435 and 387 us.  Blocks of 32 and 64 columns and
-// other splits of the channels: 440 to 470 us at 48 heads.  (Token by token: 860 us at 48 heads, 538 at 16.)
+// other splits of the channels: 440 to 470 us at 48 heads.  (Token by token: 860 us at 48 heads, 538 at 16.)  48 divides neither 64
+// nor 128: of 64 value columns a third of the second block's work is for nothing, and 48 heads with four requests of 256 tokens take
+// 175 us against 162 token by token; such steps do not come here (parts/delta.py: chunks_pay).
 template <int D>
 static int launch_delta_chunks(const DeltaChunkArgs& a, cudaStream_t s) {
   const long long blocks = (long long)a.n_long * a.H * ((a.Dv + 15) / 16);

@@ -28,23 +28,6 @@ namespace ftk {
 
 constexpr int kGcTokens = 64, kGcBlock = 16, kGcBlocks = kGcTokens / kGcBlock;
 
-__device__ __forceinline__ uint64_t gc_pair(float x, float y) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
-  return r;
-}
-__device__ __forceinline__ void gc_unpair(uint64_t p, float& x, float& y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(p)); }
-__device__ __forceinline__ void gc_fma2(uint64_t& d, uint64_t a, uint64_t b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b)); }
-__device__ __forceinline__ uint64_t gc_add2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ uint64_t gc_mul2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
 // hi + lo <- (hi + lo) (x + xlo): products of given decays are kept in two words until they are used.  (The same decay at every
 // token would otherwise leave the same error at every step, 64 times a chunk.  Decays from logits are summed up as logarithms.)
 __device__ __forceinline__ void gc_times(float& hi, float& lo, float x, float xlo) {
@@ -57,8 +40,6 @@ __device__ __forceinline__ void gc_settle(float& hi, float& lo) {
   lo = lo - (s - hi);
   hi = s;
 }
-__device__ __forceinline__ float gc_low(uint32_t w) { return __uint_as_float(w << 16); }
-__device__ __forceinline__ float gc_high(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
 
 // What a block of the two chunk kernels works on; false for a chunk that is not theirs.
 struct GcChunk { int seg, tok0, n, place, n_seg_chunks, slot; size_t row0; int pos0; };
@@ -75,8 +56,8 @@ __device__ __forceinline__ bool gc_chunk(const GlaArgs& a, int c, GcChunk& x) {
   return x.slot >= 0 && x.slot < a.n_slots;
 }
 __device__ __forceinline__ void gc_widen(const uint4& w, float (&y)[8]) {
-  y[0] = gc_low(w.x); y[1] = gc_high(w.x); y[2] = gc_low(w.y); y[3] = gc_high(w.y);
-  y[4] = gc_low(w.z); y[5] = gc_high(w.z); y[6] = gc_low(w.w); y[7] = gc_high(w.w);
+  y[0] = bf2_low(w.x); y[1] = bf2_high(w.x); y[2] = bf2_low(w.y); y[3] = bf2_high(w.y);
+  y[4] = bf2_low(w.z); y[5] = bf2_high(w.z); y[6] = bf2_low(w.w); y[7] = bf2_high(w.w);
 }
 // Eight adjacent elements of a row, rotated (every load issued before the first is used, where the pairs allow it).
 __device__ __forceinline__ void gc_rotated8(const GlaArgs& a, const __nv_bfloat16* row, int pos, int d, float (&y)[8]) {
@@ -150,13 +131,13 @@ __device__ __forceinline__ void gc_pairs(const float* k, const float* q, const f
         ulonglong2 m = *reinterpret_cast<const ulonglong2*>(mid + d);
         if (between > 1) {
           const ulonglong2 m1 = *reinterpret_cast<const ulonglong2*>(mid + D + d);
-          m.x = gc_mul2(m.x, m1.x);
-          m.y = gc_mul2(m.y, m1.y);
+          m.x = f2_mul(m.x, m1.x);
+          m.y = f2_mul(m.y, m1.y);
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          kv[i].x = gc_mul2(kv[i].x, m.x);
-          kv[i].y = gc_mul2(kv[i].y, m.y);
+          kv[i].x = f2_mul(kv[i].x, m.x);
+          kv[i].y = f2_mul(kv[i].y, m.y);
         }
       }
 #pragma unroll
@@ -164,8 +145,8 @@ __device__ __forceinline__ void gc_pairs(const float* k, const float* q, const f
         const ulonglong2 qv = *reinterpret_cast<const ulonglong2*>(q + t * LD + d);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          gc_fma2(acc[4 * t + i], qv.x, kv[i].x);
-          gc_fma2(acc[4 * t + i], qv.y, kv[i].y);
+          f2_fma(acc[4 * t + i], qv.x, kv[i].x);
+          f2_fma(acc[4 * t + i], qv.y, kv[i].y);
         }
       }
     }
@@ -174,7 +155,7 @@ __device__ __forceinline__ void gc_pairs(const float* k, const float* q, const f
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
     float x, y;
-    gc_unpair(acc[i], x, y);
+    f2_unpair(acc[i], x, y);
     sums[i] = x + y;
   }
   gc_scatter_sums(sums, place);
@@ -363,8 +344,8 @@ __global__ void __launch_bounds__(2 * D, 256 / D) gla_local_kernel(GlaArgs a) {
         if (m == u) continue;
         const ulonglong2 l = *reinterpret_cast<const ulonglong2*>(&sh.lam4[4 * b + m][d]);
         ulonglong2& y = m > u ? kv : qv;
-        y.x = gc_mul2(y.x, l.x);
-        y.y = gc_mul2(y.y, l.y);
+        y.x = f2_mul(y.x, l.x);
+        y.y = f2_mul(y.y, l.y);
       }
       *reinterpret_cast<ulonglong2*>(&sh.k[t][d]) = kv;
       *reinterpret_cast<ulonglong2*>(&sh.q[t][d]) = qv;
@@ -398,8 +379,8 @@ __global__ void __launch_bounds__(2 * D, 256 / D) gla_local_kernel(GlaArgs a) {
       ulonglong2 qv = *reinterpret_cast<const ulonglong2*>(&sh.q[t][d]);
       for (int m = 0; m < t / kGcBlock; ++m) {
         const ulonglong2 l = *reinterpret_cast<const ulonglong2*>(&sh.lam[m][d]);
-        qv.x = gc_mul2(qv.x, l.x);
-        qv.y = gc_mul2(qv.y, l.y);
+        qv.x = f2_mul(qv.x, l.x);
+        qv.y = f2_mul(qv.y, l.y);
       }
       *reinterpret_cast<ulonglong2*>(a.z + ((x.row0 + t) * a.H + h) * D + d) = qv;
     }
@@ -425,10 +406,10 @@ __global__ void __launch_bounds__(2 * D, 256 / D) gla_local_kernel(GlaArgs a) {
         const ulonglong2 l0 = *reinterpret_cast<const ulonglong2*>(&sh.lam[b][dg]), l1 = *reinterpret_cast<const ulonglong2*>(&sh.lam[b][dg + 4]);
 #pragma unroll
         for (int j = 0; j < TC; ++j) {
-          acc[0][j] = gc_mul2(acc[0][j], l0.x);
-          acc[1][j] = gc_mul2(acc[1][j], l0.y);
-          acc[2][j] = gc_mul2(acc[2][j], l1.x);
-          acc[3][j] = gc_mul2(acc[3][j], l1.y);
+          acc[0][j] = f2_mul(acc[0][j], l0.x);
+          acc[1][j] = f2_mul(acc[1][j], l0.y);
+          acc[2][j] = f2_mul(acc[2][j], l1.x);
+          acc[3][j] = f2_mul(acc[3][j], l1.y);
         }
       }
 #pragma unroll 4
@@ -443,12 +424,12 @@ __global__ void __launch_bounds__(2 * D, 256 / D) gla_local_kernel(GlaArgs a) {
         }
 #pragma unroll
         for (int j = 0; j < TC; ++j) {
-          const float v = j & 1 ? gc_high(w[j >> 1]) : gc_low(w[j >> 1]);
-          const uint64_t v2 = gc_pair(v, v);
-          gc_fma2(acc[0][j], k0.x, v2);
-          gc_fma2(acc[1][j], k0.y, v2);
-          gc_fma2(acc[2][j], k1.x, v2);
-          gc_fma2(acc[3][j], k1.y, v2);
+          const float v = j & 1 ? bf2_high(w[j >> 1]) : bf2_low(w[j >> 1]);
+          const uint64_t v2 = f2_pair(v, v);
+          f2_fma(acc[0][j], k0.x, v2);
+          f2_fma(acc[1][j], k0.y, v2);
+          f2_fma(acc[2][j], k1.x, v2);
+          f2_fma(acc[3][j], k1.y, v2);
         }
       }
     }
@@ -457,7 +438,7 @@ __global__ void __launch_bounds__(2 * D, 256 / D) gla_local_kernel(GlaArgs a) {
     for (int i = 0; i < 4; ++i) {
       float lo[TC], hi[TC];
 #pragma unroll
-      for (int j = 0; j < TC; ++j) gc_unpair(acc[i][j], lo[j], hi[j]);
+      for (int j = 0; j < TC; ++j) f2_unpair(acc[i][j], lo[j], hi[j]);
 #pragma unroll
       for (int j = 0; j < TC; j += 4) {
         if (cg + 16 * j >= a.Dv) continue;
@@ -620,9 +601,9 @@ __global__ void __launch_bounds__(256, 2) gla_out_kernel(GlaArgs a) {
     Vec4<float>::load(at, f);
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      const uint64_t f2 = gc_pair(f[e], f[e]);
+      const uint64_t f2 = f2_pair(f[e], f[e]);
 #pragma unroll
-      for (int j = 0; j < TC / 2; ++j) gc_fma2(row[j], f2, y[e][j]);
+      for (int j = 0; j < TC / 2; ++j) f2_fma(row[j], f2, y[e][j]);
     }
   };
 #pragma unroll 1
@@ -654,8 +635,8 @@ __global__ void __launch_bounds__(256, 2) gla_out_kernel(GlaArgs a) {
 #pragma unroll
       for (int j = 0; j < TC / 2; j += 2) {
         const uint2 w = *reinterpret_cast<const uint2*>(&sh.v[s + e][cg + 32 * j]);
-        y[e][j] = gc_pair(gc_low(w.x), gc_high(w.x));
-        y[e][j + 1] = gc_pair(gc_low(w.y), gc_high(w.y));
+        y[e][j] = f2_pair(bf2_low(w.x), bf2_high(w.x));
+        y[e][j + 1] = f2_pair(bf2_low(w.y), bf2_high(w.y));
       }
     }
     // (a row takes the tokens up to its own: nothing of a later one, infinite or NaN, may reach it; what P's 16-byte words hold
@@ -670,9 +651,9 @@ __global__ void __launch_bounds__(256, 2) gla_out_kernel(GlaArgs a) {
         for (int e = 0; e < 4; ++e)
           if (e <= behind) {
             const float f = sh.p[tg + 8 * i][s + e];
-            const uint64_t f2 = gc_pair(f, f);
+            const uint64_t f2 = f2_pair(f, f);
 #pragma unroll
-            for (int j = 0; j < TC / 2; ++j) gc_fma2(acc[i][j], f2, y[e][j]);
+            for (int j = 0; j < TC / 2; ++j) f2_fma(acc[i][j], f2, y[e][j]);
           }
       }
     }
@@ -692,7 +673,7 @@ __global__ void __launch_bounds__(256, 2) gla_out_kernel(GlaArgs a) {
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int j = 0; j < TC / 2; ++j) acc[i][j] = gc_add2(acc[i][j], other[(i * (TC / 2) + j) * 128]);
+    for (int j = 0; j < TC / 2; ++j) acc[i][j] = f2_add(acc[i][j], other[(i * (TC / 2) + j) * 128]);
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const int t = tg + 8 * i;
@@ -702,8 +683,8 @@ __global__ void __launch_bounds__(256, 2) gla_out_kernel(GlaArgs a) {
     for (int j = 0; j < TC / 2; j += 2) {
       if (cg + 32 * j >= Dv) continue;
       float4 f;
-      gc_unpair(acc[i][j], f.x, f.y);
-      gc_unpair(acc[i][j + 1], f.z, f.w);
+      f2_unpair(acc[i][j], f.x, f.y);
+      f2_unpair(acc[i][j + 1], f.z, f.w);
       *reinterpret_cast<float4*>(o + 32 * j) = f;
     }
   }
