@@ -130,7 +130,7 @@ class Workspace:
 
     def get(self, name: str, shape: Tuple[int, ...], dtype: torch.dtype,
             max_shape: Optional[Tuple[int, ...]] = None) -> torch.Tensor:
-        key = (name, shape, dtype)
+        key = (name, tuple(shape), dtype)
         view = self._views.get(key)
         if view is not None:
             return view
