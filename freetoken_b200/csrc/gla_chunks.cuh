@@ -508,6 +508,8 @@ struct GcOut {
   float p[kGcTokens][LP];
   uint16_t v[kGcTokens][16 * TC];  // (bfloat16)
   float dec[kGcTokens];
+  float next[16 * TC];             // a row of the state behind the chunk
+  int odd;                         // whether a value of the chunk is infinite or NaN
 };
 // 8 tokens (eight apart: their rows lie in different banks) x TC columns (fours, 64 apart) a thread, and two threads for them: each takes half of
 // the channels and half of the tokens (sums of 96 terms instead of 192, and 16 warps an SM).  Bound by the fmas.  The start state
@@ -554,6 +556,10 @@ __global__ void __launch_bounds__(256, 2) gla_out_kernel(GlaArgs a) {
   for (int i = tid; i < kGcTokens * (kGcTokens / 4); i += kThreads) {  // (what lies behind the diagonal was not written)
     const int t = i / (kGcTokens / 4), s = i % (kGcTokens / 4) * 4;
     gla_cp16(&sh.p[t][s], t < n ? pin + (size_t)t * a.H * Dv + s : pin, t < n && s <= t);
+  }
+  if (4 * tid < Dv) {
+    const float* next = x.place + 1 < x.n_seg_chunks && c + 1 < a.n_chunks ? start + (size_t)a.H * D * Dv : a.state + ((size_t)x.slot * a.H + h) * D * Dv;
+    gla_cp16(&sh.next[4 * tid], next + 4 * tid, true);
   }
   fetch(1);  // (and P and V)
   fetch(2);
@@ -626,36 +632,54 @@ __global__ void __launch_bounds__(256, 2) gla_out_kernel(GlaArgs a) {
 #pragma unroll
       for (int i = 0; i < 8; ++i) step4(acc[i], &sh.q[tg + 8 * i][half * (D / 2) + 8 * st + d], y);
     }
+    if (st == 1 && tid < kGcTokens) {  // P has come: the rest of the 16-byte words on the diagonal
+      for (int s = tid + 1; s <= (tid | 3); ++s) sh.p[tid][s] = 0.f;
+    } else if (st == 1 && tid < kGcTokens + 32) {
+      // Whether one of the chunk's values is infinite or NaN: what the chunk adds to its column of the state is then not finite,
+      // nor is the state behind the chunk, of which one row tells.  (A row of P must then stop at its own token: what it has
+      // behind is zero, and zero times such a value is NaN.)
+      float y[4] = {0.f, 0.f, 0.f, 0.f};
+      if (4 * (tid - kGcTokens) < Dv) Vec4<float>::load(&sh.next[4 * (tid - kGcTokens)], y);
+      const bool odd = __any_sync(0xffffffffu, !(fabsf(y[0]) < INFINITY && fabsf(y[1]) < INFINITY && fabsf(y[2]) < INFINITY && fabsf(y[3]) < INFINITY));
+      if (tid == kGcTokens) sh.odd = odd;
+    }
   }
+  static_assert(kStages >= 4, "a barrier between P's last words, the flag and their readers");
+  if (sh.odd) {  // token by token, each row up to its own
 #pragma unroll 1
-  for (int s = 4 * half; s < n; s += 8) {
-    uint64_t y[4][TC / 2];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
+    for (int s = 4 * half; s < n; s += (s & 3) == 3 ? 5 : 1) {
+      uint64_t y[TC / 2];
 #pragma unroll
       for (int j = 0; j < TC / 2; j += 2) {
-        const uint2 w = *reinterpret_cast<const uint2*>(&sh.v[s + e][cg + 32 * j]);
-        y[e][j] = f2_pair(bf2_low(w.x), bf2_high(w.x));
-        y[e][j + 1] = f2_pair(bf2_low(w.y), bf2_high(w.y));
+        const uint2 w = *reinterpret_cast<const uint2*>(&sh.v[s][cg + 32 * j]);
+        y[j] = f2_pair(bf2_low(w.x), bf2_high(w.x));
+        y[j + 1] = f2_pair(bf2_low(w.y), bf2_high(w.y));
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (tg + 8 * i < s) continue;
+        const float f = sh.p[tg + 8 * i][s];
+        const uint64_t f2 = f2_pair(f, f);
+#pragma unroll
+        for (int j = 0; j < TC / 2; ++j) f2_fma(acc[i][j], f2, y[j]);
       }
     }
-    // (a row takes the tokens up to its own: nothing of a later one, infinite or NaN, may reach it; what P's 16-byte words hold
-    // behind the diagonal was never written)
+  } else {
+#pragma unroll 1
+    for (int s = 4 * half; s < n; s += 8) {
+      uint64_t y[4][TC / 2];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      if (8 * i > s) {
-        step4(acc[i], &sh.p[tg + 8 * i][s], y);
-      } else if (8 * i + 7 >= s) {
-        const int behind = tg + 8 * i - s;
+      for (int e = 0; e < 4; ++e) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
-          if (e <= behind) {
-            const float f = sh.p[tg + 8 * i][s + e];
-            const uint64_t f2 = f2_pair(f, f);
-#pragma unroll
-            for (int j = 0; j < TC / 2; ++j) f2_fma(acc[i][j], f2, y[e][j]);
-          }
+        for (int j = 0; j < TC / 2; j += 2) {
+          const uint2 w = *reinterpret_cast<const uint2*>(&sh.v[s + e][cg + 32 * j]);
+          y[e][j] = f2_pair(bf2_low(w.x), bf2_high(w.x));
+          y[e][j + 1] = f2_pair(bf2_low(w.y), bf2_high(w.y));
+        }
       }
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (8 * i + 7 >= s) step4(acc[i], &sh.p[tg + 8 * i][s], y);  // (rows before s: zeros)
     }
   }
   // the upper threads' sums go through shared memory, where the stages lay
