@@ -67,6 +67,23 @@ def prepare_chunks(builder, chunk: int) -> Tuple[str, int, bool, bool]:
     return (name,) + found[name]
 
 
+def longest_chunk(segments, chunk: int, n_heads: int, head_dim: int) -> int:
+    """What :func:`ops.gla_scan` is told of a step's chunks: ``chunk`` (no chunk is longer, and long portions may go as matrix
+    products), or 0 where the token-by-token kernels are faster: a product costs a chunk of 64 tokens whatever it holds, which
+    tells for heads of 64 once the step has more (chunk, head) blocks than the GPU takes at once.  Token by token against products, 16 heads of
+    64 x 64: 32 requests of 65 tokens 106 and 120 us (one decay a head 101 and 122), of 80 tokens 125 and 122 (120 and 124), of 129
+    tokens 170 and 161; 16 requests of 65 tokens 86 and 75; 64 heads, 16 requests of 65 tokens 167 and 190, of 96 196 and 200, of 129 269
+    and 265.  Heads of 128: 48 heads, one request of 65 tokens 102 and 75, four 135 and 142, 32 867 and 814."""
+    tokens = chunks = 0
+    for seg in segments:
+        if seg.q_len > chunk:
+            tokens += seg.q_len
+            chunks += -(-seg.q_len // chunk)
+    if head_dim <= 64 and chunks * n_heads > 4 * 148 and tokens <= 0.6 * 64 * chunks:
+        return 0
+    return chunk
+
+
 @MIXERS.register("gated_linear_attention")
 class GatedLinearAttention(Mixer):
     """params: ``hidden``, ``n_heads``, ``head_dim`` (keys and queries), ``v_head_dim``, ``tau``, ``decay_rank``
@@ -147,7 +164,7 @@ class GatedLinearAttention(Mixer):
             carry = ws.get("gla.carry", (n_chunks, H, D, Dv), torch.float32, (most, H, D, Dv))
             decay = ws.get("gla.decay", (n_chunks, H, D), torch.float32, (most, H, D))
         o32 = ws.get("gla.o32", (T, H, Dv), torch.float32, (cap, H, Dv))
-        known = dict(chunk=self.chunk) if h.is_cuda else {}
+        known = dict(chunk=longest_chunk(step.segments, self.chunk, H, D)) if h.is_cuda else {}
         ops.gla_scan(proj[:, : self.k_row], proj[:, self.k_row: self.v_row], proj[:, self.v_row: self.g_row], z,
                      self.params["decay_proj.bias"], self.tau, self.q_scale, cache.tensors["s"], step.state_slots,
                      step.seg_info, len(step.segments), tensors[name], n_chunks, tensors[name + ".segments"],

@@ -29,7 +29,7 @@ from ..config.spec import ParamSpec, PartSpec, StateNeed
 from ..errors import ConfigError
 from ..kernels import ops
 from .base import MIXERS, BuildEnv, Mixer, StepState
-from .gla import DEFAULT_CHUNK, prepare_chunks
+from .gla import DEFAULT_CHUNK, longest_chunk, prepare_chunks
 
 
 @MIXERS.register("mamba2")
@@ -122,7 +122,7 @@ class Mamba2(Mixer):
             decay = ws.get("mamba2.decay", (n_chunks, H, N), f32, (most, H, N))
         o32 = ws.get("mamba2.o32", (T, H, P), f32, (cap, H, P))
         # queries C, keys B times the step size, values x: where the convolution left them
-        known = dict(chunk=self.chunk) if h.is_cuda else {}
+        known = dict(chunk=longest_chunk(step.segments, self.chunk, H, N)) if h.is_cuda else {}
         ops.gla_scan(xbc[:, I + self.bc:], xbc[:, I: I + self.bc], xbc[:, :I], None, None, 1.0, 1.0, cache.tensors["s"],
                      step.state_slots, step.seg_info, n_segs, tensors[name], n_chunks, tensors[name + ".segments"],
                      single, multi, carry, decay, o32, k_fac=step_size, a_head=dec, qk_div=H // self.groups, **known)

@@ -25,7 +25,7 @@ from ..config.spec import ParamSpec, PartSpec, StateNeed
 from ..errors import ConfigError
 from ..kernels import ops
 from .base import MIXERS, BuildEnv, Mixer, StepState
-from .gla import DEFAULT_CHUNK, prepare_chunks
+from .gla import DEFAULT_CHUNK, longest_chunk, prepare_chunks
 from .rope import shared_position
 
 
@@ -105,7 +105,7 @@ class Retention(Mixer):
             carry = ws.get("gla.carry", (n_chunks, H, D, Dv), torch.float32, (most, H, D, Dv))
             decay = ws.get("gla.decay", (n_chunks, H, D), torch.float32, (most, H, D))
         o32 = ws.get("retention.o32", (T, H, Dv), torch.float32, (cap, H, Dv))
-        known = dict(chunk=self.chunk) if h.is_cuda else {}
+        known = dict(chunk=longest_chunk(step.segments, self.chunk, H, D)) if h.is_cuda else {}
         ops.gla_scan(proj[:, : self.k_row], proj[:, self.k_row: self.v_row], proj[:, self.v_row: self.g_row], None, None,
                      1.0, D ** -0.5, cache.tensors["s"], step.state_slots, step.seg_info, len(step.segments), tensors[name],
                      n_chunks, tensors[name + ".segments"], single, multi, carry, decay, o32, a_head=self._decay,
