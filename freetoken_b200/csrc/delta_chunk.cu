@@ -10,7 +10,8 @@
 // K^T U, which are 32-bit fmas on the CUDA cores over register tiles.  Decays are running products, never differences of
 // logarithms.  The state is rounded once a chunk instead of once a token pair.
 //
-// What bounds it: the fma pipe, where the token-by-token kernel is bound by the chain of sums, shuffles and updates that a token
+// What bounds it: shared memory (75 % busy) and the fma pipe (49 %) between four barriers a chunk, with one block an SM, where the
+// token-by-token kernel is bound by the chain of sums, shuffles and updates that a token
 // pair cannot start before the one before has ended.  q and k stay bfloat16 in shared memory, eight to a 16-byte load, and are
 // widened in registers, and fmas go two at a time (fma.rn.f32x2): with 4 x 4 tiles over 32-bit copies the kernel was bound by
 // shared memory (87 % busy, 503 us at 48 heads).  The same products on mma.sync, the state in three bfloat16 pieces, took 384 us
@@ -373,6 +374,7 @@ __global__ void __launch_bounds__(2 * NV * KS) delta_chunk_kernel(DeltaChunkArgs
     // this thread's tokens from here on: tg + 8 (kr NT + i)
     uint64_t r[NT][4];
     const int place = 8 * tg + 2 * NT * kr;
+    bool odd = false;  // an infinite or NaN X
 #pragma unroll
     for (int i = 0; i < NT; ++i) {
       float k4[4], q4[4];
@@ -390,17 +392,16 @@ __global__ void __launch_bounds__(2 * NV * KS) delta_chunk_kernel(DeltaChunkArgs
       const float be = st.vec[t], bs = st.vec[kDcTokens + t], os = st.vec[2 * kDcTokens + t];
       float v[4];
       Vec4<__nv_bfloat16>::load(st.v + t * NV + c0, v);
-      *reinterpret_cast<float4*>(&sh.x[t][c0]) = make_float4(fmaf(be, v[0], -bs * k4[0]), fmaf(be, v[1], -bs * k4[1]),
-                                                             fmaf(be, v[2], -bs * k4[2]), fmaf(be, v[3], -bs * k4[3]));
+      const float4 xt = make_float4(fmaf(be, v[0], -bs * k4[0]), fmaf(be, v[1], -bs * k4[1]), fmaf(be, v[2], -bs * k4[2]), fmaf(be, v[3], -bs * k4[3]));
+      *reinterpret_cast<float4*>(&sh.x[t][c0]) = xt;
+      odd |= !(fabsf(xt.x) < INFINITY && fabsf(xt.y) < INFINITY && fabsf(xt.z) < INFINITY && fabsf(xt.w) < INFINITY);
 #pragma unroll
       for (int j = 0; j < 4; ++j) r[i][j] = f2_pair(0.f, os * q4[j]);
     }
-    __syncthreads();
-    // [T; A T] X, again a token's two rows as a pair
-    // (rows in front of `own` count for all of this thread's tokens; of the rest a token takes those up to itself: what T has behind it
-    // is zero, but a later token's X may be anything, and its infinities and NaNs must not reach back)
-    const int own = 8 * NT * kr;
-    auto term = [&](int e, bool all) {
+    odd = __syncthreads_or(odd);
+    // [T; A T] X, again a token's two rows as a pair.  This thread's tokens all lie in front of 8 NT (kr + 1), and what a row has behind
+    // its token is zero.  But zero times an infinity or NaN is NaN: with such an X in the chunk a row stops at its own token.
+    auto term = [&](int e, bool to_own) {
       float y[4];
       dc_load4(&sh.x[e][c0], y);
       uint64_t x[NT];
@@ -415,15 +416,19 @@ __global__ void __launch_bounds__(2 * NV * KS) delta_chunk_kernel(DeltaChunkArgs
       }
 #pragma unroll
       for (int i = 0; i < NT; ++i) {
-        if (!all && e > own + tg + 8 * i) continue;
+        if (to_own && e > tg + 8 * (kr * NT + i)) continue;
 #pragma unroll
         for (int j = 0; j < 4; ++j) f2_fma(r[i][j], x[i], f2_pair(y[j], y[j]));
       }
     };
+    const int upto = 8 * NT * (kr + 1);
+    if (!odd) {
 #pragma unroll 8
-    for (int e = 0; e < own; ++e) term(e, true);
-#pragma unroll
-    for (int e = 0; e < 8 * NT; ++e) term(own + e, false);
+      for (int e = 0; e < upto; ++e) term(e, false);
+    } else {
+#pragma unroll 1
+      for (int e = 0; e < upto; ++e) term(e, true);
+    }
 #pragma unroll
     for (int i = 0; i < NT; ++i) {
       const int t = tg + 8 * (kr * NT + i), tok = ch * kDcTokens + t;
