@@ -246,7 +246,8 @@ __device__ __forceinline__ float4 f32_four(const float* p, bool vec) {
 // What bounds it: in decode steps the trips to memory that wait for one another (work item, block table, keys), in prompts the
 // shared memory pipe.  So a key's row is looked up once (by the last warp, a chunk ahead), not once per element; a chunk's rows
 // are fetched sixteen bytes a thread into registers while the chunk before is worked on; and scores and products read four keys'
-// or four elements' words at a time.  Every sum keeps its order: results are the same, bit for bit, as with the plain loops.  16
+// or four elements' words at a time.  Every sum keeps its order: results are the same, bit for bit, as with the plain loops before
+// (compared once, 504 calls: heads of 16 to 256, windows, sinks, one slab or two, cut and uncut).  16
 // heads on 4 of 64 / 128 / 256, 1,500 tokens: 1,993 / 2,793 / 4,393 -> 1,362 / 1,410 / 3,258 us; 16 tokens of decode over 2,000
 // keys (merge included): 148 / 249 / 419 -> 97 / 96 / 235 us.
 template <int COLS>

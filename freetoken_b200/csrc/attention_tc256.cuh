@@ -12,7 +12,7 @@
 //          round.  Separate slabs: one key tile and one value tile.
 // What bounds it: per key tile 16 products of 128 x 128 x 16 and 8 of 128 x 256 x 16, about 1.4 us of the tensor pipe at
 // the rate this pipe takes them from one thread; the softmax (4 warps, a row a thread) runs under them.  48 heads on one
-// cached row of 256, 2,048 tokens: 1,502 us on mma.sync (64-row tiles), 166 us here (620 TFLOP/s).
+// cached row of 256, 2,048 tokens: 1,502 us on mma.sync (64-row tiles), 166 us here (620 TFLOP/s, the tensor pipe 36 % busy).
 // It takes a window, kept first tokens and a sink; no bias by distance, no soft cap.  A KV head may be taken as `kv_split`
 // heads of the same keys: 48 heads on one row fill 96 of a tile's 128 rows, three times 16 heads fill all of them.
 #pragma once

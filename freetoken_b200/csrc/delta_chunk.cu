@@ -10,7 +10,7 @@
 // K^T U, which are 32-bit fmas on the CUDA cores over register tiles.  Decays are running products, never differences of
 // logarithms.  The state is rounded once a chunk instead of once a token pair.
 //
-// What bounds it: shared memory (75 % busy) and the fma pipe (49 %) between four barriers a chunk, with one block an SM, where the
+// What bounds it: shared memory (77 % busy) and the fma pipe (50 %) between four barriers a chunk, with one block an SM, where the
 // token-by-token kernel is bound by the chain of sums, shuffles and updates that a token
 // pair cannot start before the one before has ended.  q and k stay bfloat16 in shared memory, eight to a 16-byte load, and are
 // widened in registers, and fmas go two at a time (fma.rn.f32x2): with 4 x 4 tiles over 32-bit copies the kernel was bound by

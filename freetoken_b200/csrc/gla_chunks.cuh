@@ -18,9 +18,9 @@
 // token become two, over register tiles, and the decays are products of at most 9 factors instead of a running product.
 //
 // 48 heads of 128 x 128, 2,048 tokens, a decay per channel, each kernel with its wait for the one before: decays 53 us,
-// contributions 226, carry 99 and outputs 359 token by token; 208, 85 and 132 for these three.  The layer 973 -> 686 us, with
+// contributions 226, carry 99 and outputs 359 token by token; 207, 84 and 137 for these three.  The layer 973 -> 690 us, with
 // one decay a head 949 -> 653; 16 heads 371 -> 231, 16 heads of 64 181 -> 134, 300 tokens 212 -> 159.  Against 64 bits the
-// outputs are off by 1.0e-7 either way, and by 2.8e-7 instead of 7.0e-6 where the decays are close to 1.  The fmas alone would
+// outputs are off by 1.0e-7 either way, and by 3.0e-7 instead of 3.6e-6 where the decays are close to 1.  The fmas alone would
 // take 100 us at 1.9 GHz.
 #pragma once
 
@@ -163,8 +163,8 @@ __device__ __forceinline__ void gc_pairs(const float* k, const float* q, const f
   if (on && t < rows) *reinterpret_cast<float2*>(pout + t * prow + 2 * (place & 1)) = make_float2(sums[0], sums[1]);
 }
 
-// What bounds it: the fmas and shared memory about equally, with 2 blocks an SM and a barrier between the passes (fma pipe 41 %
-// busy).  A third of a block's time goes by before its first products, on loads and decays; the logits come through shared
+// What bounds it: the fmas and shared memory about equally, with 2 blocks an SM and a barrier between the passes (fma pipe 45 %
+// busy, shared memory 47 %).  A third of a block's time goes by before its first products, on loads and decays; the logits come through shared
 // memory so that the decays are a loop of four instead of 32 copies of the code (a block's first pass 38,000 -> 28,000 cycles).
 template <int D, int TC>
 __global__ void __launch_bounds__(2 * D, 256 / D) gla_local_kernel(GlaArgs a) {
@@ -714,8 +714,10 @@ __global__ void __launch_bounds__(256, 2) gla_out_kernel(GlaArgs a) {
   }
 }
 
-// Whether a step's long portions go as products (the chunks are the host's: none may be longer than 64).
-// Shorter chunks than 32 would leave more than half of a product's rows empty.
+// Whether a step's long portions go as products (the chunks are the host's: none may be longer than 64; where they do not pay the
+// host names no length, parts/gla.py: longest_chunk).  Shorter chunks than 32 would leave more than half of a product's rows empty.  A
+// layer, token by token against products, one request of 65, 128 and 256 tokens: 48 heads of 128 159 and 130, 167 and 138, 177 and
+// 155 us; 16 heads of 64 87 and 65, 87 and 69, 95 and 69; one decay a head, 16 heads of 64 61 and 57, 61 and 61, 62 and 62.
 inline bool gla_chunks_fit(const GlaArgs& a, int longest_chunk) {
   const uintptr_t at = (uintptr_t)a.q | (uintptr_t)a.k | (uintptr_t)a.v | (uintptr_t)a.out | (uintptr_t)a.carry | (uintptr_t)a.state | (a.a_head ? 0 : (uintptr_t)a.z);
   return (a.D == 64 || a.D == 128) && a.Dv >= 64 && a.Dv <= 128 && a.Dv % 8 == 0 && !a.ones_col && longest_chunk >= 32 &&
