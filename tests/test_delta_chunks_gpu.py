@@ -82,8 +82,9 @@ def test_chunks_against_the_recurrence(H, G, D, Dv, lens, a_log, same):
     for got, plain, w in ((out, out1, want), (state, state1, want_state)):
         assert torch.isfinite(got).all()
         assert off(got, w) < 1e-6, (off(got, w), off(plain, w))
-        # (keys that are all the same: every entry of the chunk's triangle counts, and is rounded)
-        assert off(got, w) <= max((1.4 if same else 1.1) * off(plain, w), 1e-7), (off(got, w), off(plain, w))
+        # (keys that are all the same: every entry of the chunk's triangle counts, and is rounded: measured 1.18 to 1.24 times; all
+        # others 0.6 to 1.02 times, or below two units of 2^-24)
+        assert off(got, w) <= max((1.3 if same else 1.1) * off(plain, w), 1e-7), (off(got, w), off(plain, w))
     torch.testing.assert_close(out.double(), want, rtol=1e-4, atol=2e-5)
     untouched = [s for s in range(state.shape[0]) if s not in p["slots"].tolist()]
     assert torch.equal(state[untouched], p["state"][untouched])

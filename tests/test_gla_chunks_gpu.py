@@ -97,10 +97,11 @@ def test_against_the_recurrence(kw):
     plain, plain_state, other = run(p, 0)
     assert taken and not other
     # every path does 32-bit sums of at most D + 64 terms a chunk; decays are products of up to 64 factors: 2^-24 each, and
-    # random signs leave a few units of it; the token-by-token kernels measure 1e-7 to 3e-7
+    # random signs leave a few units of it; both ways measure 0.3e-7 to 1.6e-7, and where decays are close to one the token-by-token
+    # kernels 3.6e-6 and the products 3.0e-7
     used = p["slots"].long()
     for x, o, w in ((out, plain, want), (state[used], plain_state[used], want_state[used])):
-        assert rel(x, w) <= max(1e-6, 1.25 * rel(o, w)), (rel(x, w), rel(o, w))
+        assert rel(x, w) <= max(2e-7, 1.1 * rel(o, w)), (rel(x, w), rel(o, w))
     rest = [s for s in range(state.shape[0]) if s not in used.tolist()]
     assert torch.equal(state[rest], p["state"][rest])
 
