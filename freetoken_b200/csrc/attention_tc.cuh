@@ -129,21 +129,6 @@ __device__ __forceinline__ void tmem_st_16rows_16words(uint32_t addr, const uint
                : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
-// Shared-memory descriptor of an MN-major operand with 128-byte swizzle: 64 elements of the MN side
-// are contiguous (128 bytes), eight k rows make a 1024-byte group (stride byte offset), the next 64
-// MN elements lie `lbo` bytes further (leading byte offset).
-__device__ __forceinline__ uint64_t smem_desc_mn(uint32_t addr, uint32_t lbo) {
-  uint64_t d = 0;
-  d |= (uint64_t)((addr >> 4) & 0x3fff);
-  d |= (uint64_t)((lbo >> 4) & 0x3fff) << 16;
-  d |= (uint64_t)(1024 >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
-
 __device__ __forceinline__ float tc_exp2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));

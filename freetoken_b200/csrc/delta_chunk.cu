@@ -1,24 +1,28 @@
-// The gated delta rule in chunks of 32 tokens, for portions of bfloat16 prompts with one decay a head (delta.cu runs
-// everything else token by token).
+// The gated delta rule in chunks, for portions of bfloat16 prompts with one decay a head (delta.cu runs everything else token
+// by token).  Chunks of 32 tokens go two at a time.
 //
-// With S the state as the chunk finds it, c_t = g_1 ... g_t and c_t / c_s the decays behind token s,
+// With S the state as 64 tokens find it, c_t = g_1 ... g_t and c_t / c_s the decays behind token s,
 //   u_t = beta_t (v_t - c_t S^T k_t - sum_(s < t) (c_t / c_s) (k_s . k_t) u_s)
 //   o_t = c_t S^T q_t + sum_(s <= t) (c_t / c_s) (k_s . q_t) u_s            S <- c_C S + sum_s (c_C / c_s) k_s u_s^T,
 // so U = T X with X = beta (V - c K S), T = (I + L)^-1, L_ts = beta_t (c_t / c_s) (k_s . k_t), and O = c Q S + A T X.  T, A T and
-// the factors of a token depend on the chunk alone: delta_prep_kernel makes them for all chunks side by side (the decays in 64
-// bits: where a state lives for hundreds of tokens, their rounding is most of what a result is off).  What is left to do in order (delta_chunk_kernel) is three products a chunk, [K; Q] S, [T; A T] X and
-// K^T U, which are 32-bit fmas on the CUDA cores over register tiles.  Decays are running products, never differences of
-// logarithms.  The state is rounded once a chunk instead of once a token pair.
+// the factors of a token depend on the chunks alone: delta_prep_kernel makes them for all chunks side by side (the decays in 64
+// bits: where a state lives for hundreds of tokens, their rounding is most of what a result is off), T from the inverses of
+// its two blocks of 32.  What is left to do in order (delta_chunk_kernel) is three products: [K; Q] S, [T; A T] X and K^T U.
+// Decays are running products, never differences of logarithms.  The state is rounded once in 64 tokens.
 //
-// What bounds it: shared memory (77 % busy) and the fma pipe (50 %) between four barriers a chunk, with one block an SM, where the
-// token-by-token kernel is bound by the chain of sums, shuffles and updates that a token
-// pair cannot start before the one before has ended.  q and k stay bfloat16 in shared memory, eight to a 16-byte load, and are
-// widened in registers, and fmas go two at a time (fma.rn.f32x2): with 4 x 4 tiles over 32-bit copies the kernel was bound by
-// shared memory (87 % busy, 503 us at 48 heads).  The same products on mma.sync, the state in three bfloat16 pieces, took 384 us
-// there: that pipe takes a 16 x 8 x 16 product in some 24 cycles, and three pieces make that no faster than the fma pipe.
-// 2,048 tokens of one request, both kernels together (token by token -> chunks): 48 heads of 128 x 128 860 -> 405 us, 16 heads
-// 538 -> 282.  Distance from 64 bits there: 2.0e-7 -> 1.6e-7, with decays near one 2.5e-6 -> 2.3e-7.
-#include "common.cuh"
+// The three products run on tcgen05, in 32 bits: K and Q are bfloat16 as they lie, and S, T, X and U are taken apart into three
+// bfloat16 numbers each, whose sum is exactly the 32-bit one (cut off, not rounded: 8 bits a piece).  Of T X the six products
+// that reach 2^-24 are taken.  The tensor core's accumulator cuts off instead of rounding (measured: a bias of half a unit a step of
+// 16; one step, and two, are as close to 64 bits as a chain of as many fmas), so the products of the leading pieces are chains of two
+// steps, added up in registers; the other pieces' are 2^-8 smaller.
+//
+// What bounds it: the chain of a chunk pair, product, registers, shared memory, product, which no other block can hide: the
+// tensor pipe is at work about half of the time.  With 64 columns a block, 48 heads of 128 x 128: 5.0 us a pair (product 0.8, registers 1.1, product 0.8, registers
+// 0.7, product 0.5, registers 1.0); 16 columns a block, 16 heads: 2.9.
+// 2,048 tokens of one request, prep and chunks together (token by token, 32-bit fmas on the CUDA cores in chunks of 32, now): 48 heads of
+// 128 x 128 869, 431 and 228 us, 16 heads 563, 282 and 123; 16 heads of 64 x 64 535, 292 and 110.  Distance from 64 bits, token by token
+// and now: 2.5e-7 and 1.5e-7, with decays near one 2.4e-6 and 1.8e-7, with decays of e^-12 1.2e-7 and 1.1e-7.
+#include "tc_common.cuh"
 
 namespace ftk {
 
@@ -28,10 +32,14 @@ int delta_scan_tokens(const void* q, long long q_stride, const void* k, long lon
                       float q_scale, float unit_eps, float* state, int n_slots, const int32_t* state_slots, const int32_t* seg_info,
                       int n_segs, float* out, int n_tokens, int n_heads, int n_kv_heads, int dim, int vdim, int shorter_than, void* stream);
 
-constexpr int kDcTokens = 32;                 // tokens a chunk
-// scratch of one (chunk, head): rows s of T^T and (A T)^T, columns t in the order of dc_place, then per token beta, beta c rk, c rq, (c_C / c) rk, then c_C
-constexpr int kDcMats = kDcTokens * 2 * kDcTokens;
-constexpr int kDcBytes = kDcMats * 4 + 4 * kDcTokens * 4 + 16;
+__device__ int g_delta_status[4];  // [0] first error code of a wait that ran out, [1] block; 0 = fine
+
+constexpr int kDcTokens = 64;  // tokens of the two chunks that go together
+// Scratch of 64 tokens: a key head's [K; Q] as the tensor core reads it (per 64 channels 128 rows of 128 bytes, swizzled), then a
+// head's [T; A T] the same way (three pieces of 128 rows of 64 tokens), per token beta, beta c rk, c rq, (c_C / c) rk, and c_C.
+constexpr int kDcImage = 128 * 128;  // bytes of 128 rows
+constexpr int kDcHeadBytes = 3 * kDcImage + 4 * kDcTokens * 4 + 16;
+__host__ __device__ constexpr long long dc_row_bytes(int H, int G, int D) { return (long long)G * (D / 64) * kDcImage + (long long)H * kDcHeadBytes; }
 
 struct DeltaChunkArgs {
   const __nv_bfloat16* q; const __nv_bfloat16* k; const __nv_bfloat16* v; const __nv_bfloat16* b; const __nv_bfloat16* a;
@@ -41,52 +49,59 @@ struct DeltaChunkArgs {
   float* state; int n_slots;
   const int32_t* state_slots; const int32_t* seg_info; int n_segs;
   float* out; int n_tokens, H, G, D, Dv;
-  unsigned char* scratch;
-  int long_from, n_long, n_chunks;  // requests of long_from tokens and more go in chunks: n_long of them; the chunks that scratch holds
+  unsigned char* scratch; long long row_bytes;
+  int long_from, n_long, n_chunks;  // requests of long_from tokens and more go in chunks: n_long of them; the rows (of 64 tokens) that scratch holds
 };
 
-__device__ __forceinline__ void dc_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-// The same added to d by 32-bit additions (products of bfloat16 rows are exact; the tensor core's own additions do not round
-// to nearest).
-__device__ __forceinline__ void dc_mma_add(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  float x[4] = {0.f, 0.f, 0.f, 0.f};
-  dc_mma(x, a, b0, b1);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) d[i] += x[i];
-}
-__device__ __forceinline__ void dc_cp16(void* dst, const void* src, bool valid) {
-  const int n = valid ? 16 : 0;  // fewer source bytes than 16: the rest is written as zeros
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(n));
-}
-__device__ __forceinline__ uint32_t dc_lds(const __nv_bfloat16* p) { return *reinterpret_cast<const uint32_t*>(p); }
-
-// Where row t of T, and right behind it row t of A T, lies among 64: a thread takes tokens that are eight apart.
-__host__ __device__ constexpr int dc_place(int t) { return t % 8 * 8 + t / 8 * 2; }
-
-// chunks of a segment; 0 for one that the kernels leave alone
+// rows of 64 tokens of a segment; 0 for one that the kernels leave alone
 __device__ __forceinline__ int dc_chunks(const DeltaChunkArgs& a, int seg) {
   const int q_start = a.seg_info[seg * 4], q_len = a.seg_info[seg * 4 + 1], kv_len = a.seg_info[seg * 4 + 2];
   if (q_len < a.long_from || q_start < 0 || q_start + q_len > a.n_tokens || kv_len < q_len) return 0;
   return (q_len + kDcTokens - 1) / kDcTokens;
 }
 
-// One block per (chunk, key head): the dots of the chunk's rows once for all heads that share them, then a warp a head.
-// (W warps, four at least: as many as heads share the rows, up to eight)
-template <int D, int W>
-__global__ void __launch_bounds__(32 * W) delta_prep_kernel(DeltaChunkArgs a) {
+// Four warps a head, two heads a block: shared memory of one
+constexpr int kDcBlock = 16, kDcBlocks = kDcTokens / kDcBlock, kDcLine = kDcTokens + 4;
+struct DcTeam {
+  float l[kDcTokens][kDcLine];  // L, then A, then A T (rows of tokens; blocks of 16 above the diagonal are not used)
+  float t[kDcTokens][kDcLine];  // T
+  double g[kDcTokens];          // a token's decay;
+  double upto[kDcTokens], behind[kDcTokens];  // the decays of its 16 tokens up to and with it, and behind it (times 1 / |k|);
+  double total[kDcBlocks];      // of all of each 16
+  float beta[kDcTokens];
+};
+// (the image lies there until the dots are done; from a border of 1,024 bytes on)
+template <int D>
+constexpr size_t dc_prep_smem() { return 1024 + (D / 64 * kDcImage > 2 * (int)sizeof(DcTeam) ? D / 64 * kDcImage : 2 * sizeof(DcTeam)); }
+__device__ __forceinline__ void dc_bulk_store(void* dst, uint32_t src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n\tcp.async.bulk.commit_group;" ::"l"(dst), "r"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void dc_stores_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }  // what they copy has been read
+
+// One block per (64 tokens, key head): the dots of the rows once for all heads that share them, then four warps a head.  T and A T in
+// blocks of 16 x 16, a warp a block, a lane a column and half of the rows: one piece of code of 130 fmas for all of their products.
+// (A lane a column of 64 and everything
+// unrolled: 117 us at 48 heads and 2,048 tokens, the instructions' fetches in the way; now 63.)
+template <int D>
+__global__ void __launch_bounds__(256, 2) delta_prep_kernel(DeltaChunkArgs a) {
+  constexpr int kThreads = 256, kParts = D / 32;
+  extern __shared__ unsigned char dyn_smem[];
+  __shared__ float kk[kDcTokens][kDcTokens + 1], qk[kDcTokens][kDcTokens + 1], srk[kDcTokens], srq[kDcTokens];
+  __shared__ int found[2], abort_flag;
+  __shared__ uint64_t dots_done;
+  __shared__ uint32_t tmem_slot;
+  const uint32_t base = (smem_addr(dyn_smem) + 1023u) & ~1023u;
+  unsigned char* prep_smem = dyn_smem + (base - smem_addr(dyn_smem));
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) {
+    mbar_init(&dots_done, 1);
+    abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) tmem_alloc(&tmem_slot, kParts * kDcTokens);
   pdl_wait();
   pdl_trigger();
-  constexpr int RL = D + 8;
-  __shared__ __align__(16) __nv_bfloat16 sk[kDcTokens * RL], sq[kDcTokens * RL];
-  __shared__ float kk[kDcTokens][kDcTokens + 1], qk[kDcTokens][kDcTokens + 1], s2q[kDcTokens];
-  extern __shared__ __align__(16) unsigned char prep_smem[];
-  float (*sl)[kDcTokens][kDcTokens + 4] = reinterpret_cast<float (*)[kDcTokens][kDcTokens + 4]>(prep_smem);
-  __shared__ int found[2];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (warp == 0) {  // which segment's chunk this is
+  if (warp == 0) {  // which segment's this is
     if (lane == 0) found[0] = -1;
     __syncwarp();
     int before = 0;
@@ -104,172 +119,318 @@ __global__ void __launch_bounds__(32 * W) delta_prep_kernel(DeltaChunkArgs a) {
       if (before > (int)blockIdx.x) break;
     }
   }
+  tc_fence_before();
   __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = tmem_slot;
   const int seg = found[0];
-  if (seg < 0) return;
+  if (seg < 0) {
+    __syncthreads();
+    if (warp == 1) tmem_dealloc(tmem, kParts * kDcTokens);
+    return;
+  }
   const int q_start = a.seg_info[seg * 4] + found[1] * kDcTokens, nb = min(kDcTokens, a.seg_info[seg * 4 + 1] - found[1] * kDcTokens);
   const int g = blockIdx.y, per = a.H / a.G;
-  for (int i = threadIdx.x; i < kDcTokens * (D / 8); i += 32 * W) {
+  unsigned char* row = a.scratch + (size_t)blockIdx.x * a.row_bytes;
+  for (int i = threadIdx.x; i < kDcTokens * (D / 8); i += kThreads) {
     const int t = i / (D / 8), d = i % (D / 8) * 8;
     const size_t tok = (size_t)(q_start + min(t, nb - 1));
     uint4 kv = *reinterpret_cast<const uint4*>(a.k + tok * a.k_stride + (size_t)g * D + d);
     uint4 qv = *reinterpret_cast<const uint4*>(a.q + tok * a.q_stride + (size_t)g * D + d);
     if (t >= nb) kv = qv = make_uint4(0u, 0u, 0u, 0u);
-    *reinterpret_cast<uint4*>(sk + t * RL + d) = kv;
-    *reinterpret_cast<uint4*>(sq + t * RL + d) = qv;
+    unsigned char* im = prep_smem + d / 64 * kDcImage + t * 128 + ((((d >> 3) & 7) ^ (t & 7)) << 4);
+    *reinterpret_cast<uint4*>(im) = kv;
+    *reinterpret_cast<uint4*>(im + kDcTokens * 128) = qv;
   }
+  fence_async_smem();
   __syncthreads();
-  if (warp < 4) {
-    // k_t . k_s and q_t . k_s: warp w takes tokens s = 8 w .. 8 w + 7 of both, for all t
-    const int gr = lane >> 2, gc = 2 * (lane & 3);
-    float acc[4][4] = {};
+  // k_t . k_s and q_t . k_s: [K; Q] K^T, chains of two steps in columns of their own
+  if (warp == 0) {
+    if (elect_one()) {
 #pragma unroll
-    for (int kc = 0; kc < D; kc += 16) {
-      const uint32_t b0 = dc_lds(sk + (8 * warp + gr) * RL + kc + gc), b1 = dc_lds(sk + (8 * warp + gr) * RL + kc + gc + 8);
-#pragma unroll
-      for (int m = 0; m < 4; ++m) {  // rows 0-15 and 16-31 of k, then of q
-        const __nv_bfloat16* r = (m < 2 ? sk : sq) + (16 * (m & 1) + gr) * RL + kc + gc;
-        const uint32_t af[4] = {dc_lds(r), dc_lds(r + 8 * RL), dc_lds(r + 8), dc_lds(r + 8 * RL + 8)};
-        dc_mma_add(acc[m], af, b0, b1);
+      for (int k = 0; k < D / 16; ++k) {
+        const uint64_t rows = smem_desc(base + (k >> 2) * kDcImage) + 2 * (k & 3);
+        tc_mma(tmem + (k >> 1) * kDcTokens, rows, rows, instr_desc(kDcTokens), k & 1);
       }
+      tc_commit(&dots_done);
+      if (blockIdx.z == 0)
+        for (int d = 0; d < D / 64; ++d) dc_bulk_store(row + (size_t)(g * (D / 64) + d) * kDcImage, base + d * kDcImage, kDcImage);
     }
-#pragma unroll
-    for (int m = 0; m < 4; ++m) {
-      float (*dst)[kDcTokens + 1] = m < 2 ? kk : qk;
-      const int r = 16 * (m & 1) + gr, c = 8 * warp + gc;
-      dst[r][c] = acc[m][0]; dst[r][c + 1] = acc[m][1];
-      dst[r + 8][c] = acc[m][2]; dst[r + 8][c + 1] = acc[m][3];
-    }
-    // |q|^2, four lanes a token
-    const int t = 8 * warp + gr;
+    __syncwarp();
+  }
+  for (int t0 = 8 * warp; t0 < kDcTokens; t0 += 64) {  // |q|^2, four lanes a token
+    const int t = t0 + (lane >> 2);
     float s = 0.f;
     for (int d = 4 * (lane & 3); d < D; d += 16) {
       float v[4];
-      Vec4<__nv_bfloat16>::load(sq + t * RL + d, v);
-      s = fmaf(v[0], v[0], fmaf(v[1], v[1], fmaf(v[2], v[2], fmaf(v[3], v[3], s))));
+      Vec4<__nv_bfloat16>::load(
+          reinterpret_cast<const __nv_bfloat16*>(prep_smem + d / 64 * kDcImage + (kDcTokens + t) * 128 + ((((d >> 3) & 7) ^ (t & 7)) << 4) + (d & 4) * 2), v);
+      s += fmaf(v[0], v[0], v[1] * v[1]) + fmaf(v[2], v[2], v[3] * v[3]);
     }
     s += __shfl_xor_sync(0xffffffffu, s, 1);
     s += __shfl_xor_sync(0xffffffffu, s, 2);
-    if ((lane & 3) == 0) s2q[t] = s;
+    // (rows that do not exist are zeros: with unit_eps = 0 they would have no unit vector)
+    if ((lane & 3) == 0) srq[t] = t < nb ? rsqrtf(s + a.unit_eps) * a.q_scale : 0.f;
   }
+  if (!mbar_wait(&dots_done, 0, &abort_flag)) {
+    atomicCAS(&g_delta_status[0], 0, 506);
+    abort_flag = 1;
+  }
+  __syncwarp();
+  tc_fence_after();
+  {
+    const int t = (warp & 1) * 32 + lane;
+    float (*dst)[kDcTokens + 1] = warp & 2 ? qk : kk;
+#pragma unroll
+    for (int c = 0; c < kDcTokens / 2; c += 8) {
+      const int s0 = (warp >> 2) * (kDcTokens / 2) + c;
+      float r[kParts][8];
+#pragma unroll
+      for (int m = 0; m < kParts; ++m) tmem_ld8_start(tmem + ((uint32_t)((warp & 3) * 32) << 16) + m * kDcTokens + s0, r[m]);
+      tmem_ld8_finish(r);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        float y = r[0][i] + r[1][i];
+        if constexpr (kParts == 4) y += r[2][i] + r[3][i];
+        dst[t][s0 + i] = y;
+      }
+    }
+  }
+  if (warp == 0) dc_stores_read();
+  tc_fence_before();
   __syncthreads();
-  const int t = lane;
-  // (rows that do not exist are zeros: with unit_eps = 0 they would have no unit vector)
-  const float rk = t < nb ? rsqrtf(kk[t][t] + a.unit_eps) : 0.f, rq = t < nb ? rsqrtf(s2q[t] + a.unit_eps) * a.q_scale : 0.f;
-  const size_t tok = (size_t)(q_start + min(t, nb - 1));
-  for (int hh = warp; hh < per; hh += W) {
+  if (warp == 1) tmem_dealloc(tmem, kParts * kDcTokens);
+  for (int t = threadIdx.x; t < kDcTokens; t += kThreads) srk[t] = t < nb ? rsqrtf(kk[t][t] + a.unit_eps) : 0.f;
+  __syncthreads();
+  // (the warps' blocks of the two teams lie the other way round: the longest chains on different schedulers)
+  const int team = warp >> 2, j = team ? 3 - (warp & 3) : warp & 3, tt = threadIdx.x & 127, col = lane & 15, upper = lane >> 4;
+  DcTeam& sh = reinterpret_cast<DcTeam*>(prep_smem)[team];
+  auto meet = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(1 + team) : "memory"); };
+  const int hh = blockIdx.z * 2 + team;
+  if (hh < per) {
     const int h = g * per + hh;
-    float beta = 0.f;
-    double gt = 1.0;  // (tokens that do not exist add nothing and decay nothing)
-    if (t < nb) {
-      const double z = (double)__bfloat162float(a.a[tok * a.a_stride + h]) + (double)a.dt_bias[h];
-      beta = 1.f / (1.f + expf(-__bfloat162float(a.b[tok * a.b_stride + h])));
-      gt = exp(-exp((double)a.a_log[h]) * (z > 0.0 ? z + log1p(exp(-z)) : log1p(exp(z))));
-    }
-    double c = gt, rest = gt;  // g_1 ... g_t; g_t ... g_C
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const double x = __shfl_up_sync(0xffffffffu, c, o), y = __shfl_down_sync(0xffffffffu, rest, o);
-      if (lane >= o) c *= x;
-      if (lane + o < 32) rest *= y;
-    }
-    double behind = __shfl_down_sync(0xffffffffu, rest, 1);  // g_(t + 1) ... g_C
-    if (lane == 31) behind = 1.0;
-    const double whole = __shfl_sync(0xffffffffu, c, 31);
-    // row t of L (or, later, A), from s = t down
-    auto rows = [&](bool of_a) {
-      double dec = 1.0;
-      __syncwarp();
-#pragma unroll 4
-      for (int s = kDcTokens - 1; s >= 0; --s) {
-        const float rks = __shfl_sync(0xffffffffu, rk, s);
-        const double gs1 = __shfl_sync(0xffffffffu, gt, min(s + 1, 31));
-        if (s < t) dec *= gs1;
-        sl[warp][t][s] = of_a ? (s <= t ? (float)(dec * qk[t][s] * rq * rks) : 0.f)
-                              : (s < t ? (float)(beta * dec * kk[t][s] * rk * rks) : 0.f);
+    unsigned char* image = row + (size_t)a.G * (D / 64) * kDcImage + (size_t)h * kDcHeadBytes;
+    double upto = 1.0, rest = 1.0;
+    if (tt < kDcTokens) {
+      const size_t tok = (size_t)(q_start + min(tt, nb - 1));
+      float beta = 0.f;
+      double gt = 1.0;  // (tokens that do not exist add nothing and decay nothing)
+      if (tt < nb) {
+        const double z = (double)__bfloat162float(a.a[tok * a.a_stride + h]) + (double)a.dt_bias[h];
+        beta = 1.f / (1.f + expf(-__bfloat162float(a.b[tok * a.b_stride + h])));
+        gt = exp(-exp((double)a.a_log[h]) * (z > 0.0 ? z + log1p(exp(-z)) : log1p(exp(z))));
       }
-      __syncwarp();
-    };
-    rows(false);
-    // column `lane` of T: T_tj = -sum_(j <= s < t) L_ts T_sj; then of A T
-    float col[kDcTokens];
-    auto times_row = [&](int r, int n) {  // row r of what sl holds, its first n elements, times the column
-      float x[4] = {0.f, 0.f, 0.f, 0.f};
+      upto = rest = gt;
 #pragma unroll
-      for (int s = 0; s < n; s += 4) {
-        const float4 l = *reinterpret_cast<const float4*>(&sl[warp][r][s]);
-        x[0] = fmaf(l.x, col[s], x[0]);
-        if (s + 1 < n) x[1] = fmaf(l.y, col[s + 1], x[1]);
-        if (s + 2 < n) x[2] = fmaf(l.z, col[s + 2], x[2]);
-        if (s + 3 < n) x[3] = fmaf(l.w, col[s + 3], x[3]);
+      for (int o = 1; o < kDcBlock; o <<= 1) {
+        const double x = __shfl_up_sync(0xffffffffu, upto, o, kDcBlock), y = __shfl_down_sync(0xffffffffu, rest, o, kDcBlock);
+        if (col >= o) upto *= x;
+        if (col + o < kDcBlock) rest *= y;
       }
-      return (x[0] + x[1]) + (x[2] + x[3]);
-    };
-#pragma unroll
-    for (int r = 0; r < kDcTokens; ++r) {
-      const float x = times_row(r, r);
-      col[r] = r == lane ? 1.f : r < lane ? 0.f : -x;
+      rest = __shfl_down_sync(0xffffffffu, rest, 1, kDcBlock);
+      if (col == kDcBlock - 1) { rest = 1.0; sh.total[tt / kDcBlock] = upto; }
+      sh.g[tt] = gt;
+      sh.upto[tt] = upto;
+      sh.behind[tt] = rest * srk[tt];
+      sh.beta[tt] = beta;
     }
-    float* mats = reinterpret_cast<float*>(a.scratch + ((size_t)blockIdx.x * a.H + h) * kDcBytes);
-    float* row = mats + lane * 2 * kDcTokens;
-    rows(true);
+    meet();
+    if (tt < kDcTokens) {
+      for (int m = 0; m < tt / kDcBlock; ++m) upto *= sh.total[m];
+      for (int m = kDcBlocks - 1; m > tt / kDcBlock; --m) rest *= sh.total[m];
+      float* vec = reinterpret_cast<float*>(image + 3 * kDcImage);
+      vec[tt] = sh.beta[tt];
+      vec[kDcTokens + tt] = (float)(sh.beta[tt] * upto * srk[tt]);
+      vec[2 * kDcTokens + tt] = (float)(upto * srq[tt]);
+      vec[3 * kDcTokens + tt] = (float)(rest * srk[tt]);
+      if (tt == 0) vec[4 * kDcTokens] = (float)((sh.total[0] * sh.total[1]) * (sh.total[2] * sh.total[3]));
+    }
+    // L or A, 16 entries of a row a thread and turn
+    auto fill = [&](bool of_a) {
+      const int t = tt & (kDcTokens - 1), own = t / kDcBlock;
+      const float (*dots)[kDcTokens + 1] = of_a ? qk : kk;
+      const double left = of_a ? (double)srq[t] : (double)sh.beta[t] * srk[t];
+#pragma unroll 1
+      for (int m = tt / kDcTokens; m <= own; m += 2) {
+        const bool here = m == own;
+        double f = left;  // the row's factor; in its own 16 tokens times the decays so far, from the token on backwards
+        if (!here) {
+          f *= sh.upto[t];
+          for (int x = m + 1; x < own; ++x) f *= sh.total[x];
+        }
 #pragma unroll
-    for (int r = 0; r < kDcTokens; ++r) *reinterpret_cast<float2*>(row + dc_place(r)) = make_float2(col[r], times_row(r, r + 1));
-    float* vec = mats + kDcMats;
-    vec[t] = beta;
-    vec[kDcTokens + t] = (float)(beta * c * rk);
-    vec[2 * kDcTokens + t] = (float)(c * rq);
-    vec[3 * kDcTokens + t] = (float)(behind * rk);
-    if (t == 0) vec[4 * kDcTokens] = (float)whole;
-    __syncwarp();
+        for (int e = kDcBlock - 4; e >= 0; e -= 4) {
+          float y[4];
+#pragma unroll
+          for (int i = 3; i >= 0; --i) {
+            const int s = kDcBlock * m + e + i;
+            if (here && s < t) f *= sh.g[s + 1];
+            const double x = f * (here ? (double)srk[s] : sh.behind[s]) * (double)dots[t][s];
+            y[i] = s < t || (of_a && s == t) ? (float)x : 0.f;
+          }
+          *reinterpret_cast<float4*>(&sh.l[t][kDcBlock * m + e]) = make_float4(y[0], y[1], y[2], y[3]);
+        }
+      }
+    };
+    fill(false);
+    meet();
+    // this lane's half of a block's rows (every other one: the two that a warp reads at a time lie in different banks) times a column;
+    // `own`: only up to a row's own column
+    auto block_times = [&](const float* rows0, const float (&x)[kDcBlock], bool own, float (&y)[kDcBlock / 2]) {
+#pragma unroll
+      for (int r = 0; r < kDcBlock / 2; ++r) {
+        const float* l = rows0 + (2 * r + upper) * kDcLine;
+        float z[2] = {0.f, 0.f};
+#pragma unroll
+        for (int s = 0; s < kDcBlock; s += 4) {
+          const float4 w = *reinterpret_cast<const float4*>(l + s);
+          const float v[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (!own || s + i <= 2 * r + upper) z[i & 1] = fmaf(v[i], x[s + i], z[i & 1]);
+        }
+        y[r] += z[0] + z[1];
+      }
+    };
+    auto column = [&](int k, int c, float (&x)[kDcBlock]) {  // of block (k, c) of T
+#pragma unroll
+      for (int s = 0; s < kDcBlock; ++s) x[s] = sh.t[kDcBlock * k + s][kDcBlock * c + col];
+    };
+    {
+      // the block's inverse, column by column: T_tj = -sum_(j <= s < t) L_ts T_sj
+      float x[kDcBlock];
+#pragma unroll
+      for (int r = 0; r < kDcBlock; ++r) {
+        float z[2] = {0.f, 0.f};
+#pragma unroll
+        for (int s = 0; s < r; ++s) z[s & 1] = fmaf(sh.l[kDcBlock * j + r][kDcBlock * j + s], x[s], z[s & 1]);
+        x[r] = r == col ? 1.f : r < col ? 0.f : -(z[0] + z[1]);
+      }
+#pragma unroll
+      for (int r = 0; r < kDcBlock; ++r)
+        if (r / (kDcBlock / 2) == upper) sh.t[kDcBlock * j + r][kDcBlock * j + col] = x[r];
+    }
+    meet();
+    // the blocks below it: T_ij = -T_ii sum_(j <= k < i) L_ik T_kj
+#pragma unroll 1
+    for (int i = j + 1; i < kDcBlocks; ++i) {
+      float x[kDcBlock], y[kDcBlock / 2] = {}, z[kDcBlock / 2] = {};
+#pragma unroll 1
+      for (int k = j; k < i; ++k) {
+        column(k, j, x);
+        block_times(&sh.l[kDcBlock * i][kDcBlock * k], x, false, y);
+      }
+#pragma unroll
+      for (int r = 0; r < kDcBlock / 2; ++r) {
+        const float other = __shfl_xor_sync(0xffffffffu, y[r], 16);
+        x[2 * r] = upper ? other : y[r];
+        x[2 * r + 1] = upper ? y[r] : other;
+      }
+      block_times(&sh.t[kDcBlock * i][kDcBlock * i], x, true, z);
+#pragma unroll
+      for (int r = 0; r < kDcBlock / 2; ++r) sh.t[kDcBlock * i + 2 * r + upper][kDcBlock * j + col] = -z[r];
+      __syncwarp();
+    }
+    meet();
+    fill(true);
+    meet();
+    // A T: the blocks (i, c) of this warp, their products (i - c + 1) shared out evenly
+    float y[4][kDcBlock / 2] = {};
+    const int mine[4] = {j == 0 ? 30 : j == 1 ? 20 : j == 2 ? 31 : 32, j == 0 ? 0 : j == 1 ? 10 : j == 2 ? 21 : 11, j == 3 ? 22 : -1, j == 3 ? 33 : -1};
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      if (mine[m] < 0) continue;
+      const int i = mine[m] / 10, c = mine[m] % 10;
+      float x[kDcBlock];
+#pragma unroll 1
+      for (int k = c; k < i; ++k) {
+        column(k, c, x);
+        block_times(&sh.l[kDcBlock * i][kDcBlock * k], x, false, y[m]);
+      }
+      column(i, c, x);
+      block_times(&sh.l[kDcBlock * i][kDcBlock * i], x, true, y[m]);
+    }
+    meet();
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      if (mine[m] < 0) continue;
+#pragma unroll
+      for (int r = 0; r < kDcBlock / 2; ++r) sh.l[kDcBlock * (mine[m] / 10) + 2 * r + upper][kDcBlock * (mine[m] % 10) + col] = y[m][r];
+    }
+    meet();
+    // [T; A T] as the tensor core reads it, eight columns of a row a thread and turn
+#pragma unroll 2
+    for (int e = tt; e < 2 * kDcTokens * 8; e += 128) {
+      const int r = e >> 3, t = r & (kDcTokens - 1), c = (e & 7) * 8;
+      const float* src = r < kDcTokens ? &sh.t[t][c] : &sh.l[t][c];
+      uint4 w[3] = {};
+      if (c / kDcBlock <= t / kDcBlock) {
+        float v[8];
+        Vec4<float>::load(src, reinterpret_cast<float (&)[4]>(v[0]));
+        Vec4<float>::load(src + 4, reinterpret_cast<float (&)[4]>(v[4]));
+        split3(v, w);
+      }
+#pragma unroll
+      for (int m = 0; m < 3; ++m) *reinterpret_cast<uint4*>(image + m * kDcImage + r * 128 + (((e & 7) ^ (r & 7)) << 4)) = w[m];
+    }
+    if (blockIdx.z == 0 && warp == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
 }
 
-// A block owns NV value columns of one (request, head): 2 NV KS threads.  In [K; Q] S a thread has 4 columns of 4 tokens' K and Q
-// rows (tokens eight apart: eight lanes read eight rows, in different banks) over a KS-th of the key channels; the partial sums
-// meet in shared memory, and each of the KS threads goes on with 4 / KS of the tokens.  In the update it keeps D / (8 KS) channels x
-// 4 columns of the state in registers.
+// shared memory of the chunk kernel, from a border of 1,024 bytes on
+template <int NV>
+struct DcPlace {
+  static constexpr int kq = 0, t = kq + 4 * kDcImage;                // [K; Q] of two rows of chunks; the pieces of [T; A T]
+  static constexpr int s = t + 3 * kDcImage;                         // the state's pieces: rows of key channels
+  static constexpr int s_piece = NV == 64 ? kDcImage : 2 * NV;       // (64 columns fill the 128 bytes of a row, 16 columns' three pieces lie in one)
+  static constexpr int x = s + (NV == 64 ? 3 : 1) * kDcImage;        // X's, then U's: rows of tokens
+  static constexpr int x_piece = NV == 64 ? kDcImage / 2 : 2 * NV;
+  static constexpr int o = x + (NV == 64 ? 3 : 1) * kDcImage / 2;    // outputs on their way: rows of tokens, in different banks
+  static constexpr int o_row = NV * 4 + 16;
+  static constexpr int bytes = o + (NV == 64 ? kDcTokens * o_row : 0);
+};
+__device__ __forceinline__ void dc_bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  mbar_expect_tx(bar, bytes);
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes),
+               "r"(smem_addr(bar)) : "memory");
+}
+// A block owns NV value columns of one (request, head).  A thread has a row (a token of K, of Q; a key channel) and 8 or 16 of the
+// columns.  Products, by one thread (columns of NV in tensor memory; each is read before the next is issued, so all use the same):
+//   [K; Q] S      two 16-channel steps of the leading piece each in columns of their own (up to 4), the second and third piece (4, 5)
+//   [T; A T] X    32 tokens each of the leading pieces' product (0, 1), second order (2), third (3)
+//   K^T U         the same
+template <int NV>
+constexpr int dc_threads() { return NV == 64 ? 512 : 256; }
 template <int D, int NV>
-struct DcStage {
-  __nv_bfloat16 k[kDcTokens * (D + 8)], q[kDcTokens * (D + 8)], v[kDcTokens * NV];
-  float m[kDcMats];
-  float vec[4 * kDcTokens + 4];
-};
-template <int D, int NV, int KS>
-struct DcShared {
-  DcStage<D, NV> stage[2];
-  float s[D][NV];                // the state as the chunk finds it
-  float part[KS][64][NV];        // partial sums
-  float x[kDcTokens][NV], u[kDcTokens][NV];
-};
-__device__ __forceinline__ void dc_load4(const float* p, float (&v)[4]) {
-  const float4 t = *reinterpret_cast<const float4*>(p);
-  v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
-}
-template <int N>
-__device__ __forceinline__ void dc_words(const __nv_bfloat16* p, uint32_t (&w)[N]) {  // N = 1, 2 or 4 words, as aligned as that
-  if constexpr (N == 1) {
-    w[0] = *reinterpret_cast<const uint32_t*>(p);
-  } else if constexpr (N == 2) {
-    const uint2 t = *reinterpret_cast<const uint2*>(p);
-    w[0] = t.x; w[1] = t.y;
-  } else {
-    const uint4 t = *reinterpret_cast<const uint4*>(p);
-    w[0] = t.x; w[1] = t.y; w[2] = t.z; w[3] = t.w;
+__global__ void __launch_bounds__(dc_threads<NV>()) delta_chunk_kernel(DeltaChunkArgs a) {
+  constexpr int NH = NV * 128 / dc_threads<NV>(), NG = NH / 8;  // columns a thread, eights of them
+  using At = DcPlace<NV>;
+  extern __shared__ unsigned char dc_smem[];
+  __shared__ uint64_t kq_full[2], t_full, mma_done;
+  __shared__ uint32_t tmem_slot;
+  __shared__ int abort_flag, odd_flag[2], first_odd[NV];  // the first token whose X is no number, per column
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, quad = warp & 3, share = warp >> 2;
+  const uint32_t base = (smem_addr(dc_smem) + 1023u) & ~1023u;
+  unsigned char* tiles = dc_smem + (base - smem_addr(dc_smem));
+  if (tid == 0) {
+    mbar_init(&kq_full[0], 1);
+    mbar_init(&kq_full[1], 1);
+    mbar_init(&t_full, 1);
+    mbar_init(&mma_done, 1);
+    abort_flag = odd_flag[0] = odd_flag[1] = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-}
-
-template <int D, int NV, int KS>
-__global__ void __launch_bounds__(2 * NV * KS) delta_chunk_kernel(DeltaChunkArgs a) {
+  if (tid < NV) first_odd[tid] = kDcTokens;
+  if (warp == 0) tmem_alloc(&tmem_slot, NV == 64 ? 512 : 128);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
   pdl_wait();
   pdl_trigger();
-  constexpr int kThreads = 2 * NV * KS, CG = NV / 4, NT = 4 / KS, DT = D / (8 * KS), LD = D + 8;
-  extern __shared__ __align__(16) unsigned char dc_smem[];
-  DcShared<D, NV, KS>& sh = *reinterpret_cast<DcShared<D, NV, KS>*>(dc_smem);
-  const int h = blockIdx.y, col0 = blockIdx.z * NV;
-  const int tid = threadIdx.x, lane = tid & 31;
+  const uint32_t tmem = tmem_slot, my_tmem = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(share * NH);
+  const int h = blockIdx.y, col0 = blockIdx.z * NV + share * NH;
   // the block's request: the blockIdx.x-th of those that go in chunks (every warp looks for it)
-  int seg = -1, n_chunks = 0, before = 0, left = blockIdx.x;  // before: chunks of the requests in front of it
+  int seg = -1, n_chunks = 0, before = 0, left = blockIdx.x;  // before: rows of the requests in front of it
   for (int i0 = 0; i0 < a.n_segs && seg < 0; i0 += 32) {
     const int n = i0 + lane < a.n_segs ? dc_chunks(a, i0 + lane) : 0;
     const unsigned some = __ballot_sync(0xffffffffu, n > 0);
@@ -285,229 +446,312 @@ __global__ void __launch_bounds__(2 * NV * KS) delta_chunk_kernel(DeltaChunkArgs
     }
   }
   // (a table whose requests overlap, or more of them long than the caller said: chunks that no scratch was laid out for)
-  if (seg < 0 || before + n_chunks > a.n_chunks) return;
-  const int q_start = a.seg_info[seg * 4], q_len = a.seg_info[seg * 4 + 1], kv_len = a.seg_info[seg * 4 + 2];
-  const int slot = a.state_slots[seg];
-  if (slot < 0 || slot >= a.n_slots) return;
-  const int hqk = h / (a.H / a.G);
-  auto fetch = [&](int ch) {
-    DcStage<D, NV>& st = sh.stage[ch & 1];
-    const int t0 = ch * kDcTokens, nb = min(kDcTokens, q_len - t0);
-    constexpr int per = D / 8;
-    for (int i = tid; i < kDcTokens * per; i += kThreads) {
-      const int t = i / per, d = i % per * 8;
-      const bool in = t < nb;
-      const size_t tok = (size_t)(q_start + t0 + (in ? t : 0));
-      dc_cp16(st.k + t * LD + d, a.k + tok * a.k_stride + (size_t)hqk * D + d, in);
-      dc_cp16(st.q + t * LD + d, a.q + tok * a.q_stride + (size_t)hqk * D + d, in);
+  if (seg < 0 || before + n_chunks > a.n_chunks) n_chunks = 0;
+  const int slot = n_chunks ? a.state_slots[seg] : -1;
+  if (slot < 0 || slot >= a.n_slots) n_chunks = 0;
+  if (n_chunks) {
+    const int q_start = a.seg_info[seg * 4], q_len = a.seg_info[seg * 4 + 1], kv_len = a.seg_info[seg * 4 + 2];
+    const unsigned char* rows = a.scratch + (size_t)before * a.row_bytes;
+    const unsigned char* kq_src = rows + (size_t)(h / (a.H / a.G)) * (D / 64) * kDcImage;
+    const unsigned char* head_src = rows + (size_t)a.G * (D / 64) * kDcImage + (size_t)h * kDcHeadBytes;
+    auto load_kq = [&](int ch) {
+      dc_bulk_load(base + At::kq + (ch & 1) * 2 * kDcImage, kq_src + (size_t)ch * a.row_bytes, D / 64 * kDcImage, &kq_full[ch & 1]);
+    };
+    auto load_t = [&](int ch) { dc_bulk_load(base + At::t, head_src + (size_t)ch * a.row_bytes, 3 * kDcImage, &t_full); };
+    int kq_issued = 0, t_issued = 0, kq_seen = 0, t_seen = 0;  // (thread 0)
+    if (tid == 0) {
+      load_kq(0);
+      load_t(0);
+      kq_issued = t_issued = 1;
+      if (n_chunks > 1) { load_kq(1); kq_issued = 2; }
     }
-    for (int i = tid; i < kDcTokens * (NV / 8); i += kThreads) {
-      const int t = i / (NV / 8), d = i % (NV / 8) * 8;
-      const bool in = t < nb && col0 + d < a.Dv;
-      const size_t tok = (size_t)(q_start + t0 + (in ? t : 0));
-      dc_cp16(st.v + t * NV + d, a.v + tok * a.v_stride + (size_t)h * a.Dv + (in ? col0 + d : 0), in);
-    }
-    const unsigned char* src = a.scratch + ((size_t)(before + ch) * a.H + h) * kDcBytes;
-    for (int i = tid; i < kDcMats / 4; i += kThreads) dc_cp16(st.m + 4 * i, src + (size_t)i * 16, true);
-    for (int i = tid; i < kDcTokens + 1; i += kThreads) dc_cp16(st.vec + 4 * i, src + kDcMats * 4 + (size_t)i * 16, true);
-    asm volatile("cp.async.commit_group;\n" ::);
-  };
-  fetch(0);
-  const int c0 = tid % CG * 4, tg = tid / CG % 8, kr = tid / (8 * CG);
-  const int dg = tid / CG * DT;  // the thread's channels of the state
-  const bool live = col0 + c0 < a.Dv;  // (value channels come in multiples of 16)
-  float* sta = a.state + (((size_t)slot * a.H + h) * a.Dv + (live ? col0 + c0 : 0)) * D + dg;
-  const bool fresh = kv_len == q_len;
-  float s[DT][4];
+    const int row = quad * 32 + lane, t = row & (kDcTokens - 1);  // (rows 0 to 63: K's tokens, then Q's)
+    const bool of_k = quad < 2, channel = row < D;
+    // what a token's row needs beside the products, a chunk ahead: its values, beta and factors
+    uint4 v_next[NG];
+    float f_next[3], whole_next;
+    auto fetch = [&](int ch) {
+      const float* vec = reinterpret_cast<const float*>(head_src + (size_t)ch * a.row_bytes + 3 * kDcImage);
+      whole_next = vec[4 * kDcTokens];
+      if (of_k) {
+        const bool in = ch * kDcTokens + t < q_len;
+        const __nv_bfloat16* src = a.v + (size_t)(q_start + (in ? ch * kDcTokens + t : 0)) * a.v_stride + (size_t)h * a.Dv;
 #pragma unroll
-  for (int i = 0; i < DT; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) s[i][j] = !fresh && live ? sta[(size_t)j * D + i] : 0.f;
-#pragma unroll 1
-  for (int ch = 0; ch < n_chunks; ++ch) {
-#pragma unroll
-    for (int i = 0; i < DT; ++i) *reinterpret_cast<float4*>(&sh.s[dg + i][c0]) = make_float4(s[i][0], s[i][1], s[i][2], s[i][3]);
-    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    __syncthreads();  // the chunk's rows have landed, the state lies in shared memory, the chunk before is through
-    if (ch + 1 < n_chunks) fetch(ch + 1);
-    const DcStage<D, NV>& st = sh.stage[ch & 1];
-    {
-      // [K; Q] S, a token's two rows as a pair
-      uint64_t acc[4][4] = {};
-      const __nv_bfloat16* kp = st.k + tg * LD + kr * (D / KS);
-      const __nv_bfloat16* qp = st.q + tg * LD + kr * (D / KS);
-      const float* sp = &sh.s[kr * (D / KS)][c0];
-#pragma unroll 2
-      for (int d0 = 0; d0 < D / KS; d0 += 8) {
-        uint32_t kw[4][4], qw[4][4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          dc_words(kp + 8 * i * LD + d0, kw[i]);
-          dc_words(qp + 8 * i * LD + d0, qw[i]);
-        }
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          float y[4];
-          dc_load4(sp + (d0 + e) * NV, y);
-          uint64_t y2[4];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) y2[j] = f2_pair(y[j], y[j]);
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const uint64_t x = e & 1 ? f2_pair(bf2_high(kw[i][e >> 1]), bf2_high(qw[i][e >> 1])) : f2_pair(bf2_low(kw[i][e >> 1]), bf2_low(qw[i][e >> 1]));
-#pragma unroll
-            for (int j = 0; j < 4; ++j) f2_fma(acc[i][j], x, y2[j]);
-          }
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        float k4[4], q4[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) f2_unpair(acc[i][j], k4[j], q4[j]);
-        float* dst = &sh.part[kr][8 * tg + 2 * i][c0];
-        *reinterpret_cast<float4*>(dst) = make_float4(k4[0], k4[1], k4[2], k4[3]);
-        *reinterpret_cast<float4*>(dst + NV) = make_float4(q4[0], q4[1], q4[2], q4[3]);
-      }
-    }
-    __syncthreads();
-    // this thread's tokens from here on: tg + 8 (kr NT + i)
-    uint64_t r[NT][4];
-    const int place = 8 * tg + 2 * NT * kr;
-    bool odd = false;  // an infinite or NaN X
-#pragma unroll
-    for (int i = 0; i < NT; ++i) {
-      float k4[4], q4[4];
-      dc_load4(&sh.part[0][place + 2 * i][c0], k4);
-      dc_load4(&sh.part[0][place + 2 * i + 1][c0], q4);
-#pragma unroll
-      for (int e = 1; e < KS; ++e) {
-        float y[4], z[4];
-        dc_load4(&sh.part[e][place + 2 * i][c0], y);
-        dc_load4(&sh.part[e][place + 2 * i + 1][c0], z);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) { k4[j] += y[j]; q4[j] += z[j]; }
-      }
-      const int t = tg + 8 * (kr * NT + i);
-      const float be = st.vec[t], bs = st.vec[kDcTokens + t], os = st.vec[2 * kDcTokens + t];
-      float v[4];
-      Vec4<__nv_bfloat16>::load(st.v + t * NV + c0, v);
-      const float4 xt = make_float4(fmaf(be, v[0], -bs * k4[0]), fmaf(be, v[1], -bs * k4[1]), fmaf(be, v[2], -bs * k4[2]), fmaf(be, v[3], -bs * k4[3]));
-      *reinterpret_cast<float4*>(&sh.x[t][c0]) = xt;
-      odd |= !(fabsf(xt.x) < INFINITY && fabsf(xt.y) < INFINITY && fabsf(xt.z) < INFINITY && fabsf(xt.w) < INFINITY);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) r[i][j] = f2_pair(0.f, os * q4[j]);
-    }
-    odd = __syncthreads_or(odd);
-    // [T; A T] X, again a token's two rows as a pair.  This thread's tokens all lie in front of 8 NT (kr + 1), and what a row has behind
-    // its token is zero.  But zero times an infinity or NaN is NaN: with such an X in the chunk a row stops at its own token.
-    auto term = [&](int e, bool to_own) {
-      float y[4];
-      dc_load4(&sh.x[e][c0], y);
-      uint64_t x[NT];
-#pragma unroll
-      for (int i = 0; i < NT; i += 2) {
-        if constexpr (NT == 1) {
-          x[0] = *reinterpret_cast<const uint64_t*>(st.m + e * 2 * kDcTokens + place);
-        } else {
-          const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(st.m + e * 2 * kDcTokens + place + 2 * i);
-          x[i] = w.x; x[i + 1] = w.y;
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < NT; ++i) {
-        if (to_own && e > tg + 8 * (kr * NT + i)) continue;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) f2_fma(r[i][j], x[i], f2_pair(y[j], y[j]));
+        for (int i = 0; i < NG; ++i)
+          v_next[i] = in && col0 + 8 * i < a.Dv ? *reinterpret_cast<const uint4*>(src + col0 + 8 * i) : make_uint4(0u, 0u, 0u, 0u);
+        f_next[0] = vec[t];
+        f_next[1] = vec[kDcTokens + t];
+        f_next[2] = vec[3 * kDcTokens + t];
+      } else {
+        f_next[0] = vec[2 * kDcTokens + t];
       }
     };
-    const int upto = 8 * NT * (kr + 1);
-    if (!odd) {
-#pragma unroll 8
-      for (int e = 0; e < upto; ++e) term(e, false);
-    } else {
+    fetch(0);
+    float* sta = a.state + (((size_t)slot * a.H + h) * a.Dv + col0) * D + row;
+    float s[NH];
+#pragma unroll
+    for (int j = 0; j < NH; ++j) s[j] = channel && kv_len != q_len && col0 + j < a.Dv ? sta[(size_t)j * D] : 0.f;
+    // eight columns as three pieces into row `r` of an operand
+    auto put = [&](int at, int piece, int r, int i, const float (&x)[8]) {
+      uint4 w[3];
+      split3(x, w);
+#pragma unroll
+      for (int m = 0; m < 3; ++m) {
+        const int g8 = share * NG + i;
+        const int off = NV == 64 ? m * piece + ((g8 ^ (r & 7)) << 4) : (((m * NV / 8 + g8) ^ (r & 7)) << 4);
+        *reinterpret_cast<uint4*>(tiles + at + r * 128 + off) = w[m];
+      }
+    };
+    uint32_t phase = 0;
+    bool bad = false;
+    auto wait = [&](uint64_t* bar, uint32_t parity, int code) {
+      if (bad) return;
+      if (!mbar_wait(bar, parity, &abort_flag)) {
+        atomicCAS(&g_delta_status[0], 0, code);
+        abort_flag = 1;
+        bad = true;
+      }
+    };
+    constexpr uint32_t id1 = instr_desc(NV) | kMnMajorB, id2 = instr_desc(2 * NV) | kMnMajorB;
 #pragma unroll 1
-      for (int e = 0; e < upto; ++e) term(e, true);
-    }
+    for (int ch = 0; ch < n_chunks; ++ch) {
+      const uint32_t kq = base + At::kq + (ch & 1) * 2 * kDcImage;
+      if (channel) {
 #pragma unroll
-    for (int i = 0; i < NT; ++i) {
-      const int t = tg + 8 * (kr * NT + i), tok = ch * kDcTokens + t;
-      float u[4], o[4];
+        for (int i = 0; i < NG; ++i) put(At::s, At::s_piece, row, i, reinterpret_cast<const float (&)[8]>(s[8 * i]));
+      }
+      fence_async_smem();
+      tc_fence_before();
+      if (__syncthreads_or(bad)) break;
+      if (warp == 0) {
+        wait(&kq_full[ch & 1], (uint32_t)(ch >> 1) & 1u, 501);
+        ++kq_seen;
+        tc_fence_after();
+        __syncwarp();
+        if (elect_one()) {
+          odd_flag[(ch + 1) & 1] = 0;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) f2_unpair(r[i][j], u[j], o[j]);
-      const float ks = st.vec[3 * kDcTokens + t];
-      *reinterpret_cast<float4*>(&sh.u[t][c0]) = make_float4(ks * u[0], ks * u[1], ks * u[2], ks * u[3]);
-      if (live && tok < q_len)
-        *reinterpret_cast<float4*>(a.out + ((size_t)(q_start + tok) * a.H + h) * a.Dv + col0 + c0) = make_float4(o[0], o[1], o[2], o[3]);
-    }
-    __syncthreads();
-    // S <- c_C S + K^T ((c_C / c) rk U), channels in pairs
-    const float whole = st.vec[4 * kDcTokens];
-    uint64_t add[DT / 2][4] = {};
-#pragma unroll 8
-    for (int e = 0; e < kDcTokens; ++e) {
-      uint32_t w[DT / 2];
-      float y[4];
-      dc_words(st.k + e * LD + dg, w);
-      dc_load4(&sh.u[e][c0], y);
+          for (int k = 0; k < D / 16; ++k) {
+            const uint64_t ad = smem_desc(kq + (k >> 2) * kDcImage) + 2 * (k & 3);
+            const uint32_t bs = base + At::s + k * 2048;
+            tc_mma(tmem + (k >> 1) * NV, ad, smem_desc_mn(bs, kDcImage), id1, k & 1);
+            tc_mma(tmem + 4 * NV, ad, smem_desc_mn(bs + At::s_piece, kDcImage), id2, k != 0);
+          }
+          tc_commit(&mma_done);
+        }
+        __syncwarp();
+      }
+      uint4 v[NG];
+      const float f0 = f_next[0], f1 = f_next[1], f2 = f_next[2], whole = whole_next;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const uint64_t y2 = f2_pair(y[j], y[j]);
+      for (int i = 0; i < NG; ++i) v[i] = v_next[i];
+      if (ch + 1 < n_chunks) fetch(ch + 1);
+      wait(&mma_done, phase, 502);
+      phase ^= 1;
+      __syncwarp();
+      tc_fence_after();
+      float o[NH];  // Q's rows: what the state gives
+      // What a row of T and A T has behind its token is zero, but zero times an infinity or NaN is NaN: such an X goes into the product
+      // as zero, and its column is NaN from its token on.
+      bool odd = false;
 #pragma unroll
-        for (int i = 0; i < DT / 2; ++i) f2_fma(add[i][j], f2_pair(bf2_low(w[i]), bf2_high(w[i])), y2);
+      for (int i = 0; i < NG; ++i) {
+        constexpr int kParts = D / 32;
+        float r[kParts + 2][8], y[8];
+#pragma unroll
+        for (int m = 0; m < kParts; ++m) tmem_ld8_start(my_tmem + m * NV + 8 * i, r[m]);
+        tmem_ld8_start(my_tmem + 4 * NV + 8 * i, r[kParts]);
+        tmem_ld8_start(my_tmem + 5 * NV + 8 * i, r[kParts + 1]);
+        tmem_ld8_finish(r);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          y[j] = r[0][j] + r[1][j];
+          if constexpr (kParts == 4) y[j] += r[2][j] + r[3][j];
+          y[j] += r[kParts][j] + r[kParts + 1][j];
+        }
+        if (of_k) {
+          const uint32_t w[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            y[j] = fmaf(f0, j & 1 ? bf2_high(w[j >> 1]) : bf2_low(w[j >> 1]), -f1 * y[j]);
+            if (!(fabsf(y[j]) < INFINITY)) {
+              odd = true;
+              atomicMin(&first_odd[share * NH + 8 * i + j], t);
+              y[j] = 0.f;
+            }
+          }
+          put(At::x, At::x_piece, row, i, y);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) o[8 * i + j] = f0 * y[j];
+        }
+      }
+      if (odd) odd_flag[ch & 1] = 1;
+      fence_async_smem();
+      tc_fence_before();
+      if (__syncthreads_or(bad)) break;
+      const bool some_odd = odd_flag[ch & 1] != 0;
+      if (warp == 0) {
+        wait(&t_full, (uint32_t)ch & 1u, 503);
+        ++t_seen;
+        tc_fence_after();
+        __syncwarp();
+        if (elect_one()) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const uint64_t t1 = smem_desc(base + At::t) + 2 * k, t2 = smem_desc(base + At::t + kDcImage) + 2 * k,
+                           t3 = smem_desc(base + At::t + 2 * kDcImage) + 2 * k;
+            const uint64_t x1 = smem_desc_mn(base + At::x + k * 2048, kDcImage / 2), x2 = smem_desc_mn(base + At::x + k * 2048 + At::x_piece, kDcImage / 2);
+            tc_mma(tmem + (k >> 1) * NV, t1, x1, id1, k & 1);
+            tc_mma(tmem + 2 * NV, t1, x2, id2, k != 0);
+            tc_mma(tmem + 2 * NV, t2, x1, id2, 1);
+            tc_mma(tmem + 3 * NV, t3, x1, id1, 1);
+          }
+          tc_commit(&mma_done);
+        }
+        __syncwarp();
+      }
+      float u[NH];
+      wait(&mma_done, phase, 504);
+      phase ^= 1;
+      __syncwarp();
+      tc_fence_after();
+#pragma unroll
+      for (int i = 0; i < NG; ++i) {
+        float r[4][8];
+#pragma unroll
+        for (int m = 0; m < 4; ++m) tmem_ld8_start(my_tmem + m * NV + 8 * i, r[m]);
+        tmem_ld8_finish(r);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) u[8 * i + j] = (r[0][j] + r[1][j]) + (r[2][j] + r[3][j]);
+      }
+      if (some_odd) {
+#pragma unroll
+        for (int j = 0; j < NH; ++j)
+          if (t >= first_odd[share * NH + j]) u[j] = NAN;
+      }
+      if (tid == 0 && ch + 1 < n_chunks && !bad) {
+        load_t(ch + 1);
+        ++t_issued;
+      }
+      if (of_k) {
+#pragma unroll
+        for (int j = 0; j < NH; ++j) u[j] *= f2;
+#pragma unroll
+        for (int i = 0; i < NG; ++i) put(At::x, At::x_piece, row, i, reinterpret_cast<const float (&)[8]>(u[8 * i]));
+      }
+      fence_async_smem();
+      tc_fence_before();
+      if (__syncthreads_or(bad)) break;
+      if (some_odd && tid < NV) first_odd[tid] = kDcTokens;
+      if (warp == 0) {
+        tc_fence_after();
+        if (elect_one()) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const uint64_t kt = smem_desc_mn(kq + k * 2048, kDcImage);
+            tc_mma(tmem + (k >> 1) * NV, kt, smem_desc_mn(base + At::x + k * 2048, kDcImage / 2), id1 | kMnMajorA, k & 1);
+            tc_mma(tmem + 2 * NV, kt, smem_desc_mn(base + At::x + k * 2048 + At::x_piece, kDcImage / 2), id2 | kMnMajorA, k != 0);
+          }
+          tc_commit(&mma_done);
+        }
+        __syncwarp();
+      }
+      if (!of_k) {
+        const int tok0 = ch * kDcTokens;
+        float* dst = a.out + ((size_t)(q_start + tok0) * a.H + h) * a.Dv + (int)blockIdx.z * NV;
+        const size_t stride = (size_t)a.H * a.Dv;
+        if constexpr (NV == 64) {  // through shared memory: whole rows of 64 columns, 16 threads a row
+          const int me = share * 64 + t, c = me % 16 * 4;
+#pragma unroll
+          for (int j = 0; j < NH; j += 4)
+            *reinterpret_cast<float4*>(tiles + At::o + t * At::o_row + (share * NH + j) * 4) = make_float4(o[j] + u[j], o[j + 1] + u[j + 1], o[j + 2] + u[j + 2], o[j + 3] + u[j + 3]);
+          asm volatile("bar.sync 1, %0;" ::"n"(dc_threads<NV>() / 2) : "memory");
+          if ((int)blockIdx.z * NV + c < a.Dv) {
+#pragma unroll
+            for (int r = me / 16; r < kDcTokens; r += dc_threads<NV>() / 32)
+              if (tok0 + r < q_len) *reinterpret_cast<float4*>(dst + r * stride + c) = *reinterpret_cast<const float4*>(tiles + At::o + r * At::o_row + c * 4);
+          }
+        } else if (tok0 + t < q_len) {
+#pragma unroll
+          for (int j = 0; j < NH; j += 4)
+            if (col0 + j < a.Dv)
+              *reinterpret_cast<float4*>(dst + t * stride + share * NH + j) = make_float4(o[j] + u[j], o[j + 1] + u[j + 1], o[j + 2] + u[j + 2], o[j + 3] + u[j + 3]);
+        }
+      }
+      wait(&mma_done, phase, 505);
+      phase ^= 1;
+      __syncwarp();
+      tc_fence_after();
+      if (tid == 0 && ch + 2 < n_chunks && !bad) {
+        load_kq(ch + 2);
+        ++kq_issued;
+      }
+#pragma unroll
+      for (int i = 0; i < NG; ++i) {
+        float r[4][8];
+#pragma unroll
+        for (int m = 0; m < 4; ++m) tmem_ld8_start(my_tmem + m * NV + 8 * i, r[m]);
+        tmem_ld8_finish(r);
+        if (channel) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) s[8 * i + j] = fmaf(whole, s[8 * i + j], (r[0][j] + r[1][j]) + (r[2][j] + r[3][j]));
+        }
       }
     }
+    if (tid == 0 && abort_flag) {  // copies still in flight
+      g_delta_status[1] = blockIdx.x;
+      abort_flag = 0;
+      for (; kq_seen < kq_issued; ++kq_seen) mbar_wait(&kq_full[kq_seen & 1], (uint32_t)(kq_seen >> 1) & 1u, &abort_flag);
+      for (; t_seen < t_issued; ++t_seen) mbar_wait(&t_full, (uint32_t)t_seen & 1u, &abort_flag);
+    }
+    if (channel && !bad) {
 #pragma unroll
-    for (int i = 0; i < DT; i += 2)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        float x, y;
-        f2_unpair(add[i / 2][j], x, y);
-        s[i][j] = fmaf(whole, s[i][j], x);
-        s[i + 1][j] = fmaf(whole, s[i + 1][j], y);
-      }
+      for (int j = 0; j < NH; ++j)
+        if (col0 + j < a.Dv) sta[(size_t)j * D] = s[j];
+    }
   }
-  if (live) {
-#pragma unroll
-    for (int i = 0; i < DT; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) sta[(size_t)j * D + i] = s[i][j];
-  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(tmem, NV == 64 ? 512 : 128);
 }
 
-template <int D, int NV, int KS>
+template <int D, int NV>
 static int launch_delta_chunks_as(const DeltaChunkArgs& a, cudaStream_t s) {
-  const dim3 grid(a.n_long, a.H, (a.Dv + NV - 1) / NV);
-  const size_t smem = sizeof(DcShared<D, NV, KS>);
-  static_assert(sizeof(DcShared<D, NV, KS>) <= 227 * 1024, "shared memory");
-  auto kern = delta_chunk_kernel<D, NV, KS>;
-  FTK_REQUIRE(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess,
-              "delta_scan (chunks): cannot set up the kernel");
-  constexpr size_t sl = kDcTokens * (kDcTokens + 4) * sizeof(float);  // a warp's share of the triangles' shared memory
-  if (a.H / a.G > 4) {
-    auto prep = delta_prep_kernel<D, 8>;
-    FTK_REQUIRE(cudaFuncSetAttribute(prep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(8 * sl)) == cudaSuccess,
-                "delta_scan (chunks): cannot set up the kernel");
-    FTK_LAUNCH(prep, dim3(a.n_chunks, a.G), 256, 8 * sl, s, a);
-  } else {
-    FTK_LAUNCH((delta_prep_kernel<D, 4>), dim3(a.n_chunks, a.G), 128, 4 * sl, s, a);
-  }
+  auto prep = delta_prep_kernel<D>;
+  auto kern = delta_chunk_kernel<D, NV>;
+  constexpr int prep_smem = (int)dc_prep_smem<D>(), smem = DcPlace<NV>::bytes + 1024;
+  static_assert(smem <= 227 * 1024, "shared memory");
+  FTK_REQUIRE(cudaFuncSetAttribute(prep, cudaFuncAttributeMaxDynamicSharedMemorySize, prep_smem) == cudaSuccess &&
+                  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess,
+              "delta_scan (chunks): cannot set up the kernels");
+  FTK_LAUNCH(prep, dim3(a.n_chunks, a.G, (a.H / a.G + 1) / 2), 256, prep_smem, s, a);
   FTK_LAUNCH_CHECK("delta_scan (chunks, triangles)");
-  FTK_LAUNCH(kern, grid, 2 * NV * KS, smem, s, a);
+  FTK_LAUNCH(kern, dim3(a.n_long, a.H, (a.Dv + NV - 1) / NV), dc_threads<NV>(), smem, s, a);
   FTK_LAUNCH_CHECK("delta_scan (chunks)");
   return 0;
 }
 
-// Columns a block.  16, twelve warps' worth of 48 shared out over three blocks, while that leaves SMs without a third block; else
-// 48 with twelve warps, three a scheduler.  Chunk kernel alone, 2,048 tokens of 128 key channels, 16 heads of 128 (128 blocks of
-// 16 columns): 282 us, blocks of 48 columns 385; 48 heads (384 and 144 blocks): 435 and 387 us.  Blocks of 32 and 64 columns and
-// other splits of the channels: 440 to 470 us at 48 heads.  (Token by token: 860 us at 48 heads, 538 at 16.)  48 divides neither 64
-// nor 128: of 64 value columns a third of the second block's work is for nothing, and 48 heads with four requests of 256 tokens take
-// 175 us against 162 token by token; such steps do not come here (parts/delta.py: chunks_pay).
+// Columns a block: by the rounds of blocks over the SMs and what a pair of chunks takes, 3.0 us with 16 columns, 5.0 with 64 (and 3 more
+// a block).  16 heads of 128 columns, 2,048 tokens: 123 us with 16 (128 blocks); 48 heads 228 with 64 (96 blocks), three rounds with 16.
 template <int D>
 static int launch_delta_chunks(const DeltaChunkArgs& a, cudaStream_t s) {
-  const long long blocks = (long long)a.n_long * a.H * ((a.Dv + 15) / 16);
-  return blocks > 2 * 148 ? launch_delta_chunks_as<D, 48, 4>(a, s) : launch_delta_chunks_as<D, 16, 4>(a, s);
+  const long long pairs = max(1, a.n_tokens / kDcTokens / a.n_long);  // (of a request, about)
+  auto rounds = [&](int cols) { return ((long long)a.n_long * a.H * ((a.Dv + cols - 1) / cols) + 147) / 148; };
+  return rounds(64) * (3 + 5 * pairs) < rounds(16) * 3 * pairs ? launch_delta_chunks_as<D, 64>(a, s) : launch_delta_chunks_as<D, 16>(a, s);
+}
+
+// What the bounded waits recorded (merged into ftk_read_status).
+int delta_chunk_status(int* out) {
+  int host[4] = {0, 0, 0, 0};
+  if (cudaMemcpyFromSymbol(host, g_delta_status, sizeof(host)) != cudaSuccess) return 2;
+  out[0] = host[0];
+  out[1] = host[1];
+  if (host[0]) {
+    int zero[4] = {0, 0, 0, 0};
+    cudaMemcpyToSymbol(g_delta_status, zero, sizeof(zero));
+  }
+  return 0;
 }
 
 }  // namespace ftk
@@ -519,7 +763,7 @@ extern "C" long long ftk_delta_chunk_scratch(int dtype, int n_tokens, int n_segs
   if (dtype != FTK_BF16 || (dim != 64 && dim != 128) || vdim < 16 || vdim % 16 || vdim > 65535 * 16 || n_heads < 1 || n_heads > 65535 ||
       n_kv_heads < 1 || n_heads % n_kv_heads || n_tokens < 1 || n_segs < 1)
     return 0;
-  return ((long long)n_tokens / kDcTokens + n_segs) * n_heads * kDcBytes;
+  return ((long long)n_tokens / kDcTokens + n_segs) * dc_row_bytes(n_heads, n_kv_heads, dim);
 }
 
 extern "C" int ftk_delta_scan_chunks(const void* q, long long q_stride, const void* k, long long k_stride, const void* v,
@@ -545,7 +789,7 @@ extern "C" int ftk_delta_scan_chunks(const void* q, long long q_stride, const vo
   d.a_log = a_log; d.dt_bias = dt_bias; d.q_scale = q_scale; d.unit_eps = unit_eps;
   d.state = state; d.n_slots = n_slots; d.state_slots = state_slots; d.seg_info = seg_info; d.n_segs = n_segs;
   d.out = out; d.n_tokens = n_tokens; d.H = n_heads; d.G = n_kv_heads; d.D = dim; d.Dv = vdim;
-  d.scratch = (unsigned char*)scratch;
+  d.scratch = (unsigned char*)scratch; d.row_bytes = dc_row_bytes(n_heads, n_kv_heads, dim);
   d.long_from = long_from; d.n_long = n_long; d.n_chunks = n_tokens / kDcTokens + n_long;
   if (n_long < n_segs) {
     const int rc = delta_scan_tokens(q, q_stride, k, k_stride, v, v_stride, b, b_stride, a, a_stride, nullptr, dtype, a_log, dt_bias, q_scale,

@@ -823,6 +823,9 @@ int ftk_moe_gemm2_tc(const void* a, const void* w2, const int32_t* expert_offset
 // out[1] = block, then cleared.  Synchronises with the device.
 int ftk_attention_tc_status(int* out);       // attention.cu
 int ftk_attention_tc_set_status(int code);  // attention.cu
+namespace ftk {
+int delta_chunk_status(int* out);  // delta_chunk.cu
+}  // namespace ftk
 
 // Writes a code into a status word from the host, as a kernel whose wait ran out would: unit 0 = the
 // grouped GEMM's word, 1 = the attention kernel's.  It exists so that the path from a status word to the
@@ -853,6 +856,13 @@ extern "C" int ftk_read_status(int* out) {
     out[0] = attn[0];
     out[1] = attn[1];
     return 0;
+  }
+  for (auto read : {ftk::delta_chunk_status}) {
+    if (read(attn) == 0 && attn[0]) {
+      out[0] = attn[0];
+      out[1] = attn[1];
+      return 0;
+    }
   }
   int host[4] = {0, 0, 0, 0};
   if (cudaMemcpyFromSymbol(host, g_status, sizeof(host)) != cudaSuccess) {

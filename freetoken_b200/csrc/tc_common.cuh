@@ -161,6 +161,13 @@ __device__ __forceinline__ void tc_mma_pair(uint32_t d_tmem, uint64_t a_desc, ui
       "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
+// One lane of a warp that is together, the same one each time.  (Products issued behind it, instead of behind a comparison of the
+// lane's number, leave their thread every 31 instead of every 51 cycles: the compiler sees that their operands are the warp's.)
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(p));
+  return p != 0;
+}
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_commit(uint64_t* bar) {
@@ -209,10 +216,50 @@ __device__ __forceinline__ void tmem_ld16_finish(uint32_t (&r)[16]) {
                :: "memory");
 }
 
+__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
+// Eight columns of a row: started; and the wait for every load so far, to which the registers are tied.
+__device__ __forceinline__ void tmem_ld8_start(uint32_t addr, float (&v)[8]) {
+  uint32_t* r = reinterpret_cast<uint32_t*>(v);
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(addr) : "memory");
+}
+template <int N>
+__device__ __forceinline__ void tmem_ld8_finish(float (&v)[N][8]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) asm volatile("" : "+f"(v[i][j]));
+}
+
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   __nv_bfloat162 t = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&t);
 }
+
+// Two 32-bit numbers in three words of two bfloat16, whose sums they are: rounded to nearest, so that the pieces shrink by 2^-9 and what
+// is left after the second fits the third.  (An infinity leaves a NaN in the second.)
+struct Pieces { uint32_t w[3]; };
+__device__ __forceinline__ Pieces split3(float x, float y) {
+  Pieces p;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    p.w[i] = pack2(x, y);
+    x -= bf2_low(p.w[i]);
+    y -= bf2_high(p.w[i]);
+  }
+  return p;
+}
+// Eight of them as 16 bytes of each piece
+__device__ __forceinline__ void split3(const float (&x)[8], uint4 (&w)[3]) {
+  Pieces p[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) p[j] = split3(x[2 * j], x[2 * j + 1]);
+#pragma unroll
+  for (int m = 0; m < 3; ++m) w[m] = make_uint4(p[0].w[m], p[1].w[m], p[2].w[m], p[3].w[m]);
+}
+constexpr uint32_t kMnMajorA = 1u << 15, kMnMajorB = 1u << 16;  // (in an instruction descriptor)
 
 // Shared-memory matrix descriptor: K-major, 128-byte swizzle, 8-row groups 1024 bytes apart.
 __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
@@ -222,6 +269,18 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
   d |= (uint64_t)(1024 >> 4) << 32;            // stride byte offset: next 8-row group
   d |= (uint64_t)1 << 46;                      // descriptor version of this architecture
   d |= (uint64_t)2 << 61;                      // 128-byte swizzle
+  return d;
+}
+// Shared-memory descriptor of an MN-major operand with 128-byte swizzle: 64 elements of the MN side
+// are contiguous (128 bytes), eight k rows make a 1024-byte group (stride byte offset), the next 64
+// MN elements lie `lbo` bytes further (leading byte offset).
+__device__ __forceinline__ uint64_t smem_desc_mn(uint32_t addr, uint32_t lbo) {
+  uint64_t d = 0;
+  d |= (uint64_t)((addr >> 4) & 0x3fff);
+  d |= (uint64_t)((lbo >> 4) & 0x3fff) << 16;
+  d |= (uint64_t)(1024 >> 4) << 32;
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)2 << 61;
   return d;
 }
 // Instruction descriptor: bf16 x bf16 -> f32, both operands K-major, M = 128, N = n.

@@ -257,7 +257,7 @@ def _dev(t: Optional[torch.Tensor], what: str, dtype: Optional[torch.dtype] = No
 def read_status() -> int:
     """Code left by a kernel whose bounded wait ran out since the last call (0 = none).  Waits
     for the device.  101-104 come from the tensor-core grouped GEMM (producer, accumulator
-    hand-back, operand arrival, accumulator arrival)."""
+    hand-back, operand arrival, accumulator arrival), 501-506 from the delta rule's chunks."""
     out = (ctypes.c_int * 2)()
     status = _lib().ftk_read_status(out)
     if status != 0:
@@ -1619,9 +1619,10 @@ def ssm_output(o32: torch.Tensor, x: torch.Tensor, d_skip: torch.Tensor, z: torc
                                  int(norm_groups), float(eps), _dev(out, "out"), T, H, P, _stream()), "ssm_output")
 
 
-DELTA_CHUNK = 32  # tokens a chunk
-# of a chunk and head: rows of T and A T, four factors a token, the chunk's decay (csrc/delta_chunk.cu: kDcBytes)
-DELTA_CHUNK_BYTES = DELTA_CHUNK * 2 * DELTA_CHUNK * 4 + 4 * DELTA_CHUNK * 4 + 16
+DELTA_CHUNK = 64  # tokens of the two chunks that go together
+DELTA_ROW_BYTES = 128 * 128  # 128 rows of 64 channels or tokens as the tensor core reads them (csrc/delta_chunk.cu: kDcImage)
+# of a head: three pieces of T and A T, four factors a token, the decay of all (csrc/delta_chunk.cu: kDcHeadBytes)
+DELTA_HEAD_BYTES = 3 * DELTA_ROW_BYTES + 4 * DELTA_CHUNK * 4 + 16
 
 
 def delta_chunk_scratch(dtype: torch.dtype, n_tokens: int, n_long: int, n_heads: int, n_kv_heads: int, dim: int, vdim: int) -> int:
@@ -1629,7 +1630,7 @@ def delta_chunk_scratch(dtype: torch.dtype, n_tokens: int, n_long: int, n_heads:
     the sizes are not taken (what ``ftk_delta_chunk_scratch`` says, without the library: engines on any device size their buffers)."""
     if dtype != torch.bfloat16 or dim not in (64, 128) or vdim < 16 or vdim % 16 or n_heads % n_kv_heads or n_tokens < 1 or n_long < 1:
         return 0
-    return (n_tokens // DELTA_CHUNK + n_long) * n_heads * DELTA_CHUNK_BYTES
+    return (n_tokens // DELTA_CHUNK + n_long) * (n_kv_heads * (dim // 64) * DELTA_ROW_BYTES + n_heads * DELTA_HEAD_BYTES)
 
 
 def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, b_raw: torch.Tensor, a_raw: Optional[torch.Tensor],
@@ -1652,7 +1653,7 @@ def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, b_raw: torch.T
     has several tokens, ``z`` is overwritten with the decays.
 
     ``scratch`` (bytes on the device, :func:`delta_chunk_scratch` of them): where the sizes and alignments allow it, the
-    ``n_long`` requests (None: all) that bring ``long_from`` tokens and more go in chunks of 32 tokens, and the others token by
+    ``n_long`` requests (None: all) that bring ``long_from`` tokens and more go in chunks (of 32 tokens, two at a time), and the others token by
     token beside them (``csrc/delta_chunk.cu``)."""
     T, H, Dv = out.shape
     D = state.shape[3]
