@@ -14,18 +14,21 @@
 //   gla_walk_kernel    a thread a state element: S_(c+1) = P_c S_c + L_c over a request's chunks, the start states to where the
 //                      contributions lay, the final state to the slot
 //   gla_out_kernel     a block a (chunk, head): [decayed q | P] [S; V]
-// All 32-bit fmas on the CUDA cores (two at a time, fma.rn.f32x2), 8 x 8 sums a thread.  Three fmas an element of the state and
-// token become two, over register tiles, and the decays are products of at most 9 factors instead of a running product.
+// P's sums are 32-bit fmas on the CUDA cores (two at a time, fma.rn.f32x2); the contributions and the outputs run on tcgen05 with
+// 32-bit operands taken apart into three bfloat16 numbers each (split3).  The decays are products of at most 9 factors instead of a
+// running product.
 //
 // 48 heads of 128 x 128, 2,048 tokens, a decay per channel, each kernel with its wait for the one before: decays 53 us,
-// contributions 226, carry 99 and outputs 359 token by token; 207, 84 and 137 for these three.  The layer 973 -> 690 us, with
-// one decay a head 949 -> 653; 16 heads 371 -> 231, 16 heads of 64 181 -> 134, 300 tokens 212 -> 159.  Against 64 bits the
-// outputs are off by 1.0e-7 either way, and by 3.0e-7 instead of 3.6e-6 where the decays are close to 1.  The fmas alone would
-// take 100 us at 1.9 GHz.
+// contributions 226, carry 99 and outputs 359 token by token; 207, 84 and 137 with all products as 32-bit fmas; 163, 73 and 105 now.  The
+// layer 973 -> 690 -> 600 us, with one decay a head 949 -> 653 -> 589; 16 heads 371 -> 231 -> 205.  Against 64 bits, fmas and now: outputs
+// 1.4e-7 and 1.3e-7, where the decays are close to 1 3.0e-7 and 2.0e-7 (2.3e-7 and 1.5e-7 at the layer's own), states 2.5e-7 and
+// 1.9e-7; with decays of e^-6 a token, where a result is one token's product, 0.9e-7 and 1.0e-7 (the tensor core cuts off).
 #pragma once
+#include "tc_common.cuh"
 
 namespace ftk {
 
+__device__ int g_gla_status[4];  // [0] first error code of a wait that ran out, [1] block; 0 = fine
 constexpr int kGcTokens = 64, kGcBlock = 16, kGcBlocks = kGcTokens / kGcBlock;
 
 // hi + lo <- (hi + lo) (x + xlo): products of given decays are kept in two words until they are used.  (The same decay at every
@@ -105,14 +108,17 @@ __device__ __forceinline__ void gc_scatter_sums(float (&v)[16], int place) {
   }
 }
 
-// TC value columns a thread in the contribution: Dv <= 16 TC
-template <int D, int TC>
+// From a border of 1,024 bytes on.  Once the pairs are done, the keys' three pieces lie over the queries and what follows them.
+template <int D, int VT>  // VT: rows of 64 value columns (with one, the other half of the tile's rows is anything: its results are left alone)
 struct GcLocal {
   static constexpr int LD = D + 4;
-  float k[kGcTokens][LD], q[kGcTokens][LD];
+  unsigned char v[VT * kGcTokens * 128];            // the values (bfloat16) as the tensor core reads them: rows of 64 columns
+  float q[kGcTokens][LD];
   float lam4[kGcTokens / 4][D], lam[kGcBlocks][D];  // the decays of 4 and of 16 tokens,
   float low4[kGcTokens / 4][D], low[kGcBlocks][D];  // and what rounding took from them, or their logarithms
-  uint16_t v[kGcTokens][16 * TC];                   // (bfloat16)
+  float k[kGcTokens][LD];
+  static constexpr int piece = D / 64 * kGcTokens * 128;
+  static_assert(3 * piece <= (kGcTokens * LD + 2 * (kGcTokens / 4 + kGcBlocks) * D) * 4, "room for the keys' pieces");
 };
 
 // The dots of 4 queries and 4 keys whose groups (of 4 or 16 tokens) have `between` others between them, with those decays `mid`
@@ -163,25 +169,44 @@ __device__ __forceinline__ void gc_pairs(const float* k, const float* q, const f
   if (on && t < rows) *reinterpret_cast<float2*>(pout + t * prow + 2 * (place & 1)) = make_float2(sums[0], sums[1]);
 }
 
-// What bounds it: the fmas and shared memory about equally, with 2 blocks an SM and a barrier between the passes (fma pipe 45 %
-// busy, shared memory 47 %).  A third of a block's time goes by before its first products, on loads and decays; the logits come through shared
-// memory so that the decays are a loop of four instead of 32 copies of the code (a block's first pass 38,000 -> 28,000 cycles).
-template <int D, int TC>
+// What bounds it: loads, decays and the pairs' sums on the fma pipe, one after the other between barriers, with two blocks an SM.  The
+// logits come through shared memory so that the decays are a loop of four instead of 32 copies of the code (a block's first pass
+// 38,000 -> 28,000 cycles).  The contribution, as L^T = V^T K, is on tcgen05, keys in three pieces (split3):
+// 207 -> 163 us against fmas.
+template <int D, int VT>
 __global__ void __launch_bounds__(2 * D, 256 / D) gla_local_kernel(GlaArgs a) {
+  constexpr int kThreads = 2 * D, LD = D + 4, kLanes = D / 8;  // lanes a token
+  extern __shared__ unsigned char gc_smem[];
+  __shared__ uint64_t mma_done;
+  __shared__ uint32_t tmem_slot;
+  __shared__ int abort_flag;
+  const uint32_t base = (smem_addr(gc_smem) + 1023u) & ~1023u;
+  GcLocal<D, VT>& sh = *reinterpret_cast<GcLocal<D, VT>*>(gc_smem + (base - smem_addr(gc_smem)));
+  const int c = blockIdx.x / a.H, h = blockIdx.x % a.H, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;  // (heads side by side: whole rows)
+  if (tid == 0) {
+    mbar_init(&mma_done, 1);
+    abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) tmem_alloc(&tmem_slot, 2 * D);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
   pdl_wait();
   pdl_trigger();
-  constexpr int kThreads = 2 * D, LD = D + 4, kLanes = D / 8;  // lanes a token
-  extern __shared__ __align__(16) unsigned char gc_smem[];
-  GcLocal<D, TC>& sh = *reinterpret_cast<GcLocal<D, TC>*>(gc_smem);
-  const int c = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
+  const uint32_t tmem = tmem_slot;
   GcChunk x;
-  if (!gc_chunk(a, c, x)) return;
+  if (!gc_chunk(a, c, x)) {
+    __syncthreads();
+    if (warp == 0) tmem_dealloc(tmem, 2 * D);
+    return;
+  }
   const int n = x.n;
   const __nv_bfloat16* vb = (const __nv_bfloat16*)a.v + (size_t)h * a.Dv;
-  for (int i = tid; i < kGcTokens * 2 * TC; i += kThreads) {
-    const int t = i / (2 * TC), j = i % (2 * TC) * 8;
-    const bool in = t < n && j < a.Dv;
-    gla_cp16(&sh.v[t][j], in ? vb + (x.row0 + t) * a.v_stride + j : vb, in);
+  for (int i = tid; i < kGcTokens * 8 * VT; i += kThreads) {
+    const int t = i / (8 * VT), j = i % (8 * VT);
+    const bool in = t < n && 8 * j < a.Dv;
+    gla_cp16(sh.v + (j >> 3) * (kGcTokens * 128) + t * 128 + (((j & 7) ^ (t & 7)) << 4), in ? vb + (x.row0 + t) * a.v_stride + 8 * j : vb, in);
   }
   gla_cp_commit();
   float* pout = a.out + (x.row0 * a.H + h) * a.Dv;  // P's rows, where the outputs will lie
@@ -396,57 +421,79 @@ __global__ void __launch_bounds__(2 * D, 256 / D) gla_local_kernel(GlaArgs a) {
     }
     a.decay_prod[((size_t)c * a.H + h) * D + tid] = hi;
   }
-  // the chunk's contribution: 8 channels (in pairs) x TC columns (fours, 64 apart) a thread, decayed from block to block
+  // the chunk's contribution: keys decayed to its end, in three pieces; a thread has eight channels of a token of every 16
   {
-    const int cg = tid % 16 * 4, dg = tid / 16 * 8;
-    uint64_t acc[4][TC] = {};
-#pragma unroll 1
+    constexpr int kPass = kThreads / kLanes;  // tokens at a time
+    static_assert(kPass == kGcBlock, "the tokens of a pass lie in one block of 16");
+    const int d = tid % kLanes * 8, t0 = tid / kLanes;
+    uint64_t lam[kGcBlocks - 1][4];
+#pragma unroll
+    for (int b = 1; b < kGcBlocks; ++b)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) lam[b - 1][j] = *reinterpret_cast<const uint64_t*>(&sh.lam[b][d + 2 * j]);
+    __syncthreads();  // the queries and the decays have been read
+    unsigned char* pieces = reinterpret_cast<unsigned char*>(sh.q);
+#pragma unroll
     for (int b = 0; b < kGcBlocks; ++b) {
-      if (b > 0) {
-        const ulonglong2 l0 = *reinterpret_cast<const ulonglong2*>(&sh.lam[b][dg]), l1 = *reinterpret_cast<const ulonglong2*>(&sh.lam[b][dg + 4]);
+      const int t = b * kGcBlock + t0;
+      float y[8];
 #pragma unroll
-        for (int j = 0; j < TC; ++j) {
-          acc[0][j] = f2_mul(acc[0][j], l0.x);
-          acc[1][j] = f2_mul(acc[1][j], l0.y);
-          acc[2][j] = f2_mul(acc[2][j], l1.x);
-          acc[3][j] = f2_mul(acc[3][j], l1.y);
-        }
+      for (int j = 0; j < 4; ++j) {
+        uint64_t kv = *reinterpret_cast<const uint64_t*>(&sh.k[t][d + 2 * j]);
+#pragma unroll
+        for (int m = b + 1; m < kGcBlocks; ++m) kv = f2_mul(kv, lam[m - 1][j]);
+        f2_unpair(kv, y[2 * j], y[2 * j + 1]);
       }
-#pragma unroll 4
-      for (int s = b * kGcBlock; s < (b + 1) * kGcBlock; ++s) {
-        const ulonglong2 k0 = *reinterpret_cast<const ulonglong2*>(&sh.k[s][dg]), k1 = *reinterpret_cast<const ulonglong2*>(&sh.k[s][dg + 4]);
-        uint32_t w[TC / 2];
+      uint4 w[3];
+      split3(y, w);
+      unsigned char* dst = pieces + (d >> 6) * (kGcTokens * 128) + t * 128 + ((((d >> 3) & 7) ^ (t & 7)) << 4);
 #pragma unroll
-        for (int g = 0; g < TC / 4; ++g) {
-          const uint2 t = *reinterpret_cast<const uint2*>(&sh.v[s][cg + 64 * g]);
-          w[2 * g] = t.x;
-          w[2 * g + 1] = t.y;
-        }
-#pragma unroll
-        for (int j = 0; j < TC; ++j) {
-          const float v = j & 1 ? bf2_high(w[j >> 1]) : bf2_low(w[j >> 1]);
-          const uint64_t v2 = f2_pair(v, v);
-          f2_fma(acc[0][j], k0.x, v2);
-          f2_fma(acc[1][j], k0.y, v2);
-          f2_fma(acc[2][j], k1.x, v2);
-          f2_fma(acc[3][j], k1.y, v2);
-        }
-      }
-    }
-    float* dst = a.carry + (((size_t)c * a.H + h) * D + dg) * a.Dv + cg;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      float lo[TC], hi[TC];
-#pragma unroll
-      for (int j = 0; j < TC; ++j) f2_unpair(acc[i][j], lo[j], hi[j]);
-#pragma unroll
-      for (int j = 0; j < TC; j += 4) {
-        if (cg + 16 * j >= a.Dv) continue;
-        *reinterpret_cast<float4*>(dst + (size_t)(2 * i) * a.Dv + 16 * j) = make_float4(lo[j], lo[j + 1], lo[j + 2], lo[j + 3]);
-        *reinterpret_cast<float4*>(dst + (size_t)(2 * i + 1) * a.Dv + 16 * j) = make_float4(hi[j], hi[j + 1], hi[j + 2], hi[j + 3]);
-      }
+      for (int m = 0; m < 3; ++m) *reinterpret_cast<uint4*>(dst + m * sh.piece) = w[m];
     }
   }
+  fence_async_smem();
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    tc_fence_after();
+    if (elect_one()) {
+      constexpr uint32_t id = instr_desc(D) | kMnMajorA | kMnMajorB;
+      const uint32_t v0 = smem_addr(sh.v), k0 = smem_addr(sh.q);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const uint64_t v = smem_desc_mn(v0 + k * 2048, kGcTokens * 128);
+        tc_mma(tmem, v, smem_desc_mn(k0 + k * 2048, kGcTokens * 128), id, k != 0);
+        tc_mma(tmem + D, v, smem_desc_mn(k0 + GcLocal<D, VT>::piece + k * 2048, kGcTokens * 128), id, k != 0);
+        tc_mma(tmem + D, v, smem_desc_mn(k0 + 2 * GcLocal<D, VT>::piece + k * 2048, kGcTokens * 128), id, 1);
+      }
+      tc_commit(&mma_done);
+    }
+    __syncwarp();
+  }
+  if (!mbar_wait(&mma_done, 0, &abort_flag)) {
+    if (atomicCAS(&g_gla_status[0], 0, 602) == 0) g_gla_status[1] = blockIdx.x;
+    abort_flag = 1;
+  }
+  __syncwarp();
+  tc_fence_after();
+  {
+    const int j = (warp & 3) * 32 + lane;  // a value column; 64 channels of it
+    const uint32_t my_tmem = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)((warp >> 2) * 64);
+    float* dst = a.carry + (((size_t)c * a.H + h) * D + (warp >> 2) * 64) * a.Dv + j;
+#pragma unroll 2
+    for (int i = 0; i < 64; i += 8) {
+      float r[2][8];
+      tmem_ld8_start(my_tmem + i, r[0]);
+      tmem_ld8_start(my_tmem + D + i, r[1]);
+      tmem_ld8_finish(r);
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        if (j < a.Dv) dst[(size_t)(i + e) * a.Dv] = r[0][e] + r[1][e];
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(tmem, 2 * D);
 }
 
 // A thread per two state elements of a (segment, head) walks the segment's chunks, the next eight contributions in flight while
@@ -499,219 +546,261 @@ __global__ void __launch_bounds__(256) gla_walk_kernel(GlaArgs a) {
   *reinterpret_cast<float2*>(st) = s;
 }
 
-// Stages of the start state: 16 channels, half of them from each half.
-template <int D, int TC>
-struct GcOut {
-  static constexpr int LD = D + 4, LP = kGcTokens + 4, kStage = 16 * 16 * TC, kBuffers = 4;
-  float q[kGcTokens][LD];
-  float s[kBuffers][kStage];
-  float p[kGcTokens][LP];
-  uint16_t v[kGcTokens][16 * TC];  // (bfloat16)
-  float dec[kGcTokens];
-  float next[16 * TC];             // a row of the state behind the chunk
-  int odd;                         // whether a value of the chunk is infinite or NaN
+// What gla_out_kernel has in shared memory, from a border of 1,024 bytes on: 64 channels of the start state (three pieces of two rows of
+// 64 value columns) and of the queries (three pieces), later P, and the values; all as the tensor core reads them.
+struct GoPlace {
+  static constexpr int tile = 64 * 128;  // 64 rows of 128 bytes
+  static constexpr int s = 0, q = s + 6 * tile, v = q + 3 * tile, bytes = v + 2 * tile;
 };
-// 8 tokens (eight apart: their rows lie in different banks) x TC columns (fours, 64 apart) a thread, and two threads for them: each takes half of
-// the channels and half of the tokens (sums of 96 terms instead of 192, and 16 warps an SM).  Bound by the fmas.  The start state
-// before P and V: small terms first (1.0e-7 off instead of 1.5e-7).  Fours of columns 64 apart: eight together cost two
-// wavefronts a load (167 -> 132 us).
-template <int D, int TC>
+
+// Outputs of a chunk: o^T = S^T q^T + V^T P^T, 128 value columns (rows of the tensor core's tile) x 64 tokens.  Two threads a value column.  S,
+// q and P are taken apart into three bfloat16 numbers each (split3) and the six products that reach 2^-24 are taken (with V, which is
+// bfloat16, three); the leading pieces' products are chains of two steps of 16, added up in registers.  Two blocks an SM; what bounds them is
+// memory's latency (2.7 TB/s: loads, taking apart, products and stores of a block follow one another; the tensor pipe is 13 % busy).
+// 137 -> 105 us against fmas.
+template <int D>
 __global__ void __launch_bounds__(256, 2) gla_out_kernel(GlaArgs a) {
+  constexpr int kStages = D / 64;
+  extern __shared__ unsigned char go_smem[];
+  __shared__ uint64_t mma_done;
+  __shared__ uint32_t tmem_slot;
+  __shared__ int abort_flag, first_odd[128];  // the first token whose value is no number, per column
+  __shared__ float dec[kGcTokens];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, quad = warp & 3, half = warp >> 2;
+  const uint32_t base = (smem_addr(go_smem) + 1023u) & ~1023u;
+  unsigned char* tiles = go_smem + (base - smem_addr(go_smem));
+  if (tid == 0) {
+    mbar_init(&mma_done, 1);
+    abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (tid < 128) first_odd[tid] = kGcTokens;
+  if (warp == 0) tmem_alloc(&tmem_slot, 256);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
   pdl_wait();
   pdl_trigger();
-  using Shared = GcOut<D, TC>;
-  constexpr int kThreads = 256, LD = D + 4, LP = kGcTokens + 4, kStages = D / 16, kBuffers = Shared::kBuffers, kPer = kGcTokens * D / 8 / kThreads;
-  extern __shared__ __align__(16) unsigned char gc_smem[];
-  Shared& sh = *reinterpret_cast<Shared*>(gc_smem);
-  const int c = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
+  const uint32_t tmem = tmem_slot;
+  const int c = blockIdx.x / a.H, h = blockIdx.x % a.H, Dv = a.Dv;
   GcChunk x;
-  if (!gc_chunk(a, c, x)) return;
-  const int n = x.n, Dv = a.Dv;
-  const float* start = a.carry + ((size_t)c * a.H + h) * D * Dv;
-  auto fetch = [&](int st) {  // (a group of copies for every stage, an empty one behind the last)
-    if (st < kStages) {
-      float* to = sh.s[st % kBuffers];
-      for (int i = tid; i < 16 * 4 * TC; i += kThreads) {
-        const int d = i / (4 * TC), j = i % (4 * TC) * 4;
-        const bool in = j < Dv;
-        gla_cp16(to + d * 16 * TC + j, in ? start + (size_t)(8 * st + d + (d >> 3) * (D / 2 - 8)) * Dv + j : start, in);
-      }
-    }
-    gla_cp_commit();
-  };
-  const __nv_bfloat16* vb = (const __nv_bfloat16*)a.v + (size_t)h * Dv;
-  if (!a.a_head) {
-    for (int i = tid; i < kGcTokens * (D / 4); i += kThreads) {
-      const int t = i / (D / 4), d = i % (D / 4) * 4;
-      gla_cp16(&sh.q[t][d], t < n ? a.z + ((x.row0 + t) * a.H + h) * D + d : a.z, t < n);
-    }
-  }
-  fetch(0);  // (and the queries)
-  for (int i = tid; i < kGcTokens * 2 * TC; i += kThreads) {
-    const int t = i / (2 * TC), j = i % (2 * TC) * 8;
-    const bool in = t < n && j < Dv;
-    gla_cp16(&sh.v[t][j], in ? vb + (x.row0 + t) * a.v_stride + j : vb, in);
-  }
-  const float* pin = a.out + (x.row0 * a.H + h) * Dv;
-  for (int i = tid; i < kGcTokens * (kGcTokens / 4); i += kThreads) {  // (what lies behind the diagonal was not written)
-    const int t = i / (kGcTokens / 4), s = i % (kGcTokens / 4) * 4;
-    gla_cp16(&sh.p[t][s], t < n ? pin + (size_t)t * a.H * Dv + s : pin, t < n && s <= t);
-  }
-  if (4 * tid < Dv) {
-    const float* next = x.place + 1 < x.n_seg_chunks && c + 1 < a.n_chunks ? start + (size_t)a.H * D * Dv : a.state + ((size_t)x.slot * a.H + h) * D * Dv;
-    gla_cp16(&sh.next[4 * tid], next + 4 * tid, true);
-  }
-  fetch(1);  // (and P and V)
-  fetch(2);
-  if (a.a_head) {  // one decay for all channels: the queries once more from their rows
-    if (tid < 32) {
-      const double w0 = 2 * tid < n ? a.a_head[(x.row0 + 2 * tid) * a.a_head_stride + h] : 1.f;
-      const double w1 = w0 * (2 * tid + 1 < n ? a.a_head[(x.row0 + 2 * tid + 1) * a.a_head_stride + h] : 1.f);
-      double up = w1;
+  if (gc_chunk(a, c, x)) {
+    const int n = x.n;
+    const float* start = a.carry + ((size_t)c * a.H + h) * D * Dv;
+    const float* pin = a.out + (x.row0 * a.H + h) * Dv;
+    const size_t row = (size_t)a.H * Dv;
+    // eight elements of a row of 128 bytes and more, as they lie in memory, and where they go: rows of `per` eights
+    float sv[4][8], qv[2][8];
+    auto load8 = [](const float* p, bool in, float (&y)[8]) {
+      if (in) {
+        Vec4<float>::load(p, reinterpret_cast<float (&)[4]>(y[0]));
+        Vec4<float>::load(p + 4, reinterpret_cast<float (&)[4]>(y[4]));
+      } else {
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const double y = __shfl_up_sync(0xffffffffu, up, o);
-        if (tid >= o) up *= y;
+        for (int j = 0; j < 8; ++j) y[j] = 0.f;
       }
-      double before = __shfl_up_sync(0xffffffffu, up, 1);
-      if (tid == 0) before = 1.;
-      sh.dec[2 * tid] = (float)(before * w0);
-      sh.dec[2 * tid + 1] = (float)(before * w1);
-    }
+    };
+    auto put8 = [&](int at, int piece, int r, int c8, const float (&y)[8]) {
+      uint4 w[3];
+      split3(y, w);
+      unsigned char* dst = tiles + at + (c8 >> 3) * GoPlace::tile + r * 128 + (((c8 & 7) ^ (r & 7)) << 4);
+#pragma unroll
+      for (int m = 0; m < 3; ++m) *reinterpret_cast<uint4*>(dst + m * piece) = w[m];
+    };
+    auto load_s = [&](int st) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int i = tid + 256 * u, d = i >> 4, c8 = i & 15;
+        load8(start + (size_t)(64 * st + d) * Dv + 8 * c8, 8 * c8 < Dv, sv[u]);
+      }
+    };
     const __nv_bfloat16* qb = (const __nv_bfloat16*)a.q + (size_t)(h / a.qk_div) * D;
-    const int d = tid % (D / 8) * 8, t0 = tid / (D / 8), step = kThreads / (D / 8);
-    uint4 w[kPer];
-    if (!a.rope) {
+    auto load_q = [&](int st) {
 #pragma unroll
-      for (int i = 0; i < kPer; ++i) w[i] = *reinterpret_cast<const uint4*>(qb + (x.row0 + min(t0 + step * i, n - 1)) * a.q_stride + d);
-    }
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < kPer; ++i) {
-      const int t = t0 + step * i;
-      float y[8];
-      if (a.rope) gc_rotated8(a, qb + (x.row0 + min(t, n - 1)) * a.q_stride, x.pos0 + min(t, n - 1), d, y);
-      else gc_widen(w[i], y);
-      const float f = a.q_scale * sh.dec[t];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) y[j] = t < n ? y[j] * f : 0.f;
-      Vec4<float>::store(&sh.q[t][d], reinterpret_cast<float (&)[4]>(y[0]));
-      Vec4<float>::store(&sh.q[t][d + 4], reinterpret_cast<float (&)[4]>(y[4]));
-    }
-  }
-  const int cg = tid % 16 * 4, tg = tid / 16 % 8, half = tid / 128;
-  uint64_t acc[8][TC / 2] = {};
-  // four more of a row's terms: times four rows of columns in pairs
-  auto step4 = [&](uint64_t (&row)[TC / 2], const float* at, const uint64_t (&y)[4][TC / 2]) {
-    float f[4];
-    Vec4<float>::load(at, f);
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const uint64_t f2 = f2_pair(f[e], f[e]);
-#pragma unroll
-      for (int j = 0; j < TC / 2; ++j) f2_fma(row[j], f2, y[e][j]);
-    }
-  };
-#pragma unroll 1
-  for (int st = 0; st < kStages; ++st) {
-    asm volatile("cp.async.wait_group 2;\n" ::: "memory");
-    static_assert(kBuffers == 4, "two stages in flight behind the one that is waited for");
-    __syncthreads();
-    fetch(st + kBuffers - 1);
-    const float* from = sh.s[st % kBuffers] + half * 8 * 16 * TC + cg;
-#pragma unroll
-    for (int d = 0; d < 8; d += 4) {
-      uint64_t y[4][TC / 2];
-#pragma unroll
-      for (int e = 0; e < 4; ++e)
-#pragma unroll
-        for (int j = 0; j < TC / 2; j += 2) {
-          const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(from + (d + e) * 16 * TC + 32 * j);
-          y[e][j] = t.x; y[e][j + 1] = t.y;
-        }
-#pragma unroll
-      for (int i = 0; i < 8; ++i) step4(acc[i], &sh.q[tg + 8 * i][half * (D / 2) + 8 * st + d], y);
-    }
-    if (st == 1 && tid < kGcTokens) {  // P has come: the rest of the 16-byte words on the diagonal
-      for (int s = tid + 1; s <= (tid | 3); ++s) sh.p[tid][s] = 0.f;
-    } else if (st == 1 && tid < kGcTokens + 32) {
-      // Whether one of the chunk's values is infinite or NaN: what the chunk adds to its column of the state is then not finite,
-      // nor is the state behind the chunk, of which one row tells.  (A row of P must then stop at its own token: what it has
-      // behind is zero, and zero times such a value is NaN.)
-      float y[4] = {0.f, 0.f, 0.f, 0.f};
-      if (4 * (tid - kGcTokens) < Dv) Vec4<float>::load(&sh.next[4 * (tid - kGcTokens)], y);
-      const bool odd = __any_sync(0xffffffffu, !(fabsf(y[0]) < INFINITY && fabsf(y[1]) < INFINITY && fabsf(y[2]) < INFINITY && fabsf(y[3]) < INFINITY));
-      if (tid == kGcTokens) sh.odd = odd;
-    }
-  }
-  static_assert(kStages >= 4, "a barrier between P's last words, the flag and their readers");
-  if (sh.odd) {  // token by token, each row up to its own
-#pragma unroll 1
-    for (int s = 4 * half; s < n; s += (s & 3) == 3 ? 5 : 1) {
-      uint64_t y[TC / 2];
-#pragma unroll
-      for (int j = 0; j < TC / 2; j += 2) {
-        const uint2 w = *reinterpret_cast<const uint2*>(&sh.v[s][cg + 32 * j]);
-        y[j] = f2_pair(bf2_low(w.x), bf2_high(w.x));
-        y[j + 1] = f2_pair(bf2_low(w.y), bf2_high(w.y));
-      }
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        if (tg + 8 * i < s) continue;
-        const float f = sh.p[tg + 8 * i][s];
-        const uint64_t f2 = f2_pair(f, f);
-#pragma unroll
-        for (int j = 0; j < TC / 2; ++j) f2_fma(acc[i][j], f2, y[j]);
-      }
-    }
-  } else {
-#pragma unroll 1
-    for (int s = 4 * half; s < n; s += 8) {
-      uint64_t y[4][TC / 2];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-#pragma unroll
-        for (int j = 0; j < TC / 2; j += 2) {
-          const uint2 w = *reinterpret_cast<const uint2*>(&sh.v[s + e][cg + 32 * j]);
-          y[e][j] = f2_pair(bf2_low(w.x), bf2_high(w.x));
-          y[e][j + 1] = f2_pair(bf2_low(w.y), bf2_high(w.y));
+      for (int u = 0; u < 2; ++u) {
+        const int i = tid + 256 * u, t = i >> 3, d = 64 * st + (i & 7) * 8;
+        if (!a.a_head) {
+          load8(a.z + ((x.row0 + t) * a.H + h) * D + d, t < n, qv[u]);
+        } else if (t < n) {  // one decay for all channels: the queries once more from their rows
+          if (a.rope) gc_rotated8(a, qb + (x.row0 + t) * a.q_stride, x.pos0 + t, d, qv[u]);
+          else gc_widen(*reinterpret_cast<const uint4*>(qb + (x.row0 + t) * a.q_stride + d), qv[u]);
+        } else {
+          load8(nullptr, false, qv[u]);
         }
       }
+    };
+    load_s(0);
+    load_q(0);
+    {
+      // The values.  A row of P holds zeros behind its own token, but zero times an infinity or NaN is NaN: such a value goes in as
+      // zero, and its column is NaN from its token on (as its column of the state is).
+      const __nv_bfloat16* vb = (const __nv_bfloat16*)a.v + (size_t)h * Dv;
+      uint4 w[4];
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
-        if (8 * i + 7 >= s) step4(acc[i], &sh.p[tg + 8 * i][s], y);  // (rows before s: zeros)
+      for (int u = 0; u < 4; ++u) {
+        const int i = tid + 256 * u, t = i >> 4, c8 = i & 15;
+        w[u] = t < n && 8 * c8 < Dv ? *reinterpret_cast<const uint4*>(vb + (x.row0 + t) * a.v_stride + 8 * c8) : make_uint4(0u, 0u, 0u, 0u);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int i = tid + 256 * u, t = i >> 4, c8 = i & 15;
+        uint32_t* y = reinterpret_cast<uint32_t*>(&w[u]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const bool lo = (y[j] & 0x7f80u) == 0x7f80u, hi = (y[j] & 0x7f800000u) == 0x7f800000u;
+          if (lo) atomicMin(&first_odd[8 * c8 + 2 * j], t);
+          if (hi) atomicMin(&first_odd[8 * c8 + 2 * j + 1], t);
+          y[j] &= (lo ? 0u : 0xffffu) | (hi ? 0u : 0xffff0000u);
+        }
+        *reinterpret_cast<uint4*>(tiles + GoPlace::v + (c8 >> 3) * GoPlace::tile + t * 128 + (((c8 & 7) ^ (t & 7)) << 4)) = w[u];
+      }
+    }
+    if (a.a_head) {
+      if (tid < 32) {
+        const double w0 = 2 * tid < n ? a.a_head[(x.row0 + 2 * tid) * a.a_head_stride + h] : 1.f;
+        const double w1 = w0 * (2 * tid + 1 < n ? a.a_head[(x.row0 + 2 * tid + 1) * a.a_head_stride + h] : 1.f);
+        double up = w1;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const double y = __shfl_up_sync(0xffffffffu, up, o);
+          if (tid >= o) up *= y;
+        }
+        double before = __shfl_up_sync(0xffffffffu, up, 1);
+        if (tid == 0) before = 1.;
+        dec[2 * tid] = (float)(before * w0);
+        dec[2 * tid + 1] = (float)(before * w1);
+      }
+      __syncthreads();
+    }
+    auto put_stage = [&]() {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int i = tid + 256 * u;
+        put8(GoPlace::s, 2 * GoPlace::tile, i >> 4, i & 15, sv[u]);
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int i = tid + 256 * u;
+        if (a.a_head) {
+          const float f = a.q_scale * dec[i >> 3];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) qv[u][j] *= f;
+        }
+        put8(GoPlace::q, GoPlace::tile, i >> 3, i & 7, qv[u]);
+      }
+    };
+    bool bad = false;
+    uint32_t phase = 0;
+    auto wait = [&]() {
+      if (!bad && !mbar_wait(&mma_done, phase, &abort_flag)) {
+        if (atomicCAS(&g_gla_status[0], 0, 601) == 0) g_gla_status[1] = blockIdx.x;
+        abort_flag = 1;
+        bad = true;
+      }
+      phase ^= 1;
+      __syncwarp();
+      tc_fence_after();
+    };
+    // columns of 64 in tensor memory: two chains of the leading pieces, the second order, the third
+    const uint32_t my_tmem = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(half * 32);
+    constexpr uint32_t id1 = instr_desc(64) | kMnMajorA, id2 = instr_desc(128) | kMnMajorA;
+    float acc[32];
+#pragma unroll
+    for (int j = 0; j < 32; ++j) acc[j] = 0.f;
+    auto add_chains = [&]() {
+#pragma unroll
+      for (int i = 0; i < 32; i += 8) {
+        float r[2][8];
+        tmem_ld8_start(my_tmem + i, r[0]);
+        tmem_ld8_start(my_tmem + 64 + i, r[1]);
+        tmem_ld8_finish(r);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i + j] += r[0][j] + r[1][j];
+      }
+    };
+#pragma unroll 1
+    for (int st = 0; st < kStages; ++st) {
+      put_stage();
+      fence_async_smem();
+      tc_fence_before();
+      __syncthreads();
+      if (warp == 0) {
+        tc_fence_after();
+        if (elect_one()) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const uint64_t s1 = smem_desc_mn(base + GoPlace::s + k * 2048, GoPlace::tile), s2 = smem_desc_mn(base + GoPlace::s + 2 * GoPlace::tile + k * 2048, GoPlace::tile),
+                           s3 = smem_desc_mn(base + GoPlace::s + 4 * GoPlace::tile + k * 2048, GoPlace::tile);
+            const uint64_t q1 = smem_desc(base + GoPlace::q) + 2 * k, q2 = smem_desc(base + GoPlace::q + GoPlace::tile) + 2 * k;
+            tc_mma(tmem + (k >> 1) * 64, s1, q1, id1, k & 1);
+            tc_mma(tmem + 128, s1, q2, id2, st | k);
+            tc_mma(tmem + 128, s2, q1, id2, 1);
+            tc_mma(tmem + 192, s3, q1, id1, 1);
+          }
+          tc_commit(&mma_done);
+        }
+        __syncwarp();
+      }
+      if (st + 1 < kStages) {
+        load_s(st + 1);
+        load_q(st + 1);
+      } else {  // P (what lies behind the diagonal was not written)
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int i = tid + 256 * u, t = i >> 3, s0 = (i & 7) * 8;
+          const float* p = pin + (size_t)min(t, n - 1) * row + s0;
+          load8(p, t < n && s0 + 7 <= t, qv[u]);
+          if (t < n && s0 <= t && s0 + 7 > t) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              if (s0 + j <= t) qv[u][j] = p[j];
+          }
+        }
+      }
+      wait();
+      add_chains();
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int i = tid + 256 * u;
+      put8(GoPlace::q, GoPlace::tile, i >> 3, i & 7, qv[u]);
+    }
+    fence_async_smem();
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+      tc_fence_after();
+      if (elect_one()) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const uint64_t v = smem_desc_mn(base + GoPlace::v + k * 2048, GoPlace::tile);
+          tc_mma(tmem + (k >> 1) * 64, v, smem_desc(base + GoPlace::q) + 2 * k, id1, k & 1);
+          tc_mma(tmem + 128, v, smem_desc(base + GoPlace::q + GoPlace::tile) + 2 * k, id2, 1);
+        }
+        tc_commit(&mma_done);
+      }
+      __syncwarp();
+    }
+    wait();
+    const int j = quad * 32 + lane, odd = first_odd[j];
+    float* o = a.out + (x.row0 * a.H + h) * Dv + j;
+#pragma unroll
+    for (int i = 0; i < 32; i += 8) {
+      float r[4][8];
+#pragma unroll
+      for (int m = 0; m < 4; ++m) tmem_ld8_start(my_tmem + 64 * m + i, r[m]);
+      tmem_ld8_finish(r);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const int t = half * 32 + i + e;
+        const float y = acc[i + e] + ((r[0][e] + r[1][e]) + (r[2][e] + r[3][e]));
+        if (t < n && j < Dv) o[(size_t)t * row] = t >= odd ? NAN : y;
+      }
     }
   }
-  // the upper threads' sums go through shared memory, where the stages lay
+  tc_fence_before();
   __syncthreads();
-  uint64_t* other = reinterpret_cast<uint64_t*>(sh.s) + (tid & 127);
-  static_assert(sizeof(sh.s) >= 128 * 4 * TC * 8, "room for half of the sums");
-  if (half) {
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-      for (int j = 0; j < TC / 2; ++j) other[(i * (TC / 2) + j) * 128] = acc[i][j];
-  }
-  __syncthreads();
-  if (half) return;
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < TC / 2; ++j) acc[i][j] = f2_add(acc[i][j], other[(i * (TC / 2) + j) * 128]);
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int t = tg + 8 * i;
-    if (t >= n) continue;
-    float* o = a.out + ((x.row0 + t) * a.H + h) * Dv + cg;
-#pragma unroll
-    for (int j = 0; j < TC / 2; j += 2) {
-      if (cg + 32 * j >= Dv) continue;
-      float4 f;
-      f2_unpair(acc[i][j], f.x, f.y);
-      f2_unpair(acc[i][j + 1], f.z, f.w);
-      *reinterpret_cast<float4*>(o + 32 * j) = f;
-    }
-  }
+  if (warp == 0) tmem_dealloc(tmem, 256);
 }
 
 // Whether a step's long portions go as products (the chunks are the host's: none may be longer than 64; where they do not pay the
@@ -721,30 +810,42 @@ __global__ void __launch_bounds__(256, 2) gla_out_kernel(GlaArgs a) {
 inline bool gla_chunks_fit(const GlaArgs& a, int longest_chunk) {
   const uintptr_t at = (uintptr_t)a.q | (uintptr_t)a.k | (uintptr_t)a.v | (uintptr_t)a.out | (uintptr_t)a.carry | (uintptr_t)a.state | (a.a_head ? 0 : (uintptr_t)a.z);
   return (a.D == 64 || a.D == 128) && a.Dv >= 64 && a.Dv <= 128 && a.Dv % 8 == 0 && !a.ones_col && longest_chunk >= 32 &&
-         longest_chunk <= kGcTokens && (a.q_stride | a.k_stride | a.v_stride) % 8 == 0 && (at & 15) == 0;
+         longest_chunk <= kGcTokens && (long long)a.n_chunks * a.H <= 0x7fffffff && (a.q_stride | a.k_stride | a.v_stride) % 8 == 0 && (at & 15) == 0;
 }
 
-template <int D, int TC>
+template <int D, int VT>
 static int launch_gla_chunks_as(const GlaArgs& a, cudaStream_t s) {
-  auto local = gla_local_kernel<D, TC>;
-  auto outs = gla_out_kernel<D, TC>;
-  constexpr int sl = (int)sizeof(GcLocal<D, TC>), so = (int)sizeof(GcOut<D, TC>);
+  auto local = gla_local_kernel<D, VT>;
+  auto outs = gla_out_kernel<D>;
+  constexpr int sl = (int)sizeof(GcLocal<D, VT>) + 1024, so = GoPlace::bytes + 1024;
   FTK_REQUIRE(cudaFuncSetAttribute(local, cudaFuncAttributeMaxDynamicSharedMemorySize, sl) == cudaSuccess &&
                   cudaFuncSetAttribute(outs, cudaFuncAttributeMaxDynamicSharedMemorySize, so) == cudaSuccess,
               "gla_scan: cannot set up the chunk kernels");
-  FTK_LAUNCH(local, dim3(a.n_chunks, a.H), 2 * D, sl, s, a);
+  FTK_LAUNCH(local, (unsigned)a.n_chunks * a.H, 2 * D, sl, s, a);
   FTK_LAUNCH_CHECK("gla_scan (chunk products)");
   const size_t DV = (size_t)a.D * a.Dv;
   FTK_LAUNCH(gla_walk_kernel, dim3((unsigned)((DV / 2 + 255) / 256), a.n_segs, a.H), 256, 0, s, a);
   FTK_LAUNCH_CHECK("gla_scan (states)");
-  FTK_LAUNCH(outs, dim3(a.n_chunks, a.H), 256, so, s, a);
+  FTK_LAUNCH(outs, (unsigned)a.n_chunks * a.H, 256, so, s, a);
   FTK_LAUNCH_CHECK("gla_scan (outputs)");
   return 0;
 }
 
+// What the bounded waits recorded (merged into ftk_read_status).
+int gla_chunks_status(int* out) {
+  int host[4] = {0, 0, 0, 0};
+  if (cudaMemcpyFromSymbol(host, g_gla_status, sizeof(host)) != cudaSuccess) return 2;
+  out[0] = host[0];
+  out[1] = host[1];
+  if (host[0]) {
+    int zero[4] = {0, 0, 0, 0};
+    cudaMemcpyToSymbol(g_gla_status, zero, sizeof(zero));
+  }
+  return 0;
+}
+
 inline int launch_gla_chunks(const GlaArgs& a, cudaStream_t s) {
-  if (a.D == 64) return a.Dv <= 64 ? launch_gla_chunks_as<64, 4>(a, s) : launch_gla_chunks_as<64, 8>(a, s);
-  return a.Dv <= 64 ? launch_gla_chunks_as<128, 4>(a, s) : launch_gla_chunks_as<128, 8>(a, s);
+  return a.D == 128 ? launch_gla_chunks_as<128, 2>(a, s) : a.Dv <= 64 ? launch_gla_chunks_as<64, 1>(a, s) : launch_gla_chunks_as<64, 2>(a, s);
 }
 
 }  // namespace ftk
