@@ -1,5 +1,5 @@
-// Grouped expert matrix products on CUDA cores: the true 32-bit path, and the path for sizes the
-// tensor-core kernels refuse.
+// Grouped expert matrix products: the true 32-bit path (on CUDA cores for few rows an expert and for rows without 16-byte loads,
+// else on the tensor cores in three pieces, moe_gemm_split.cuh), and the path for bfloat16 sizes that the tensor-core kernels refuse.
 //
 // Rows are sorted by expert (expert e owns rows [offsets[e], offsets[e+1])); the row counts are
 // only known on the device, so the grid is an upper bound on the row tiles (ceil(R / BM) + experts with rows) and a
@@ -66,12 +66,16 @@ __device__ __forceinline__ T finish(float x, float up, float weight, int act, fl
   return from_float<T>(gated_act(to_float(from_float<T>(x)), to_float(from_float<T>(up)), act, alpha, limit));
 }
 
+}  // namespace ftk
+
+#include "moe_gemm_split.cuh"
+
+namespace ftk {
+
 // Tiles of BM rows x 64 gate and 64 up columns (or 128 columns): 128 threads with BM / 8 rows x 8 columns of sums each, k in
 // steps of 16 through two shared-memory buffers, the next step's 16-byte loads in flight under this step's products.  What
 // bounds it is the FMA pipe: per k a thread reads 16 numbers (four 16-byte loads) for 64 products.  Every sum runs over k in
-// order.  16 experts of 1,024 x 1,408 in 32 bits, 750 tokens in two routes each: 323 us gate/up, 380 us down with the wait for it
-// (27 TFLOP/s; 22 row tiles of 94 rows an expert leave the last wave half empty).  The kernel before (32 x 64 tiles, scalar loads
-// into one buffer) took the two layers of such a step and eight decode steps of four tokens in 8.1 ms, these in 1.6.
+// order.  (27 TFLOP/s in 32 bits, before moe_gemm_split.cuh took those with 16-byte loads.)
 constexpr int kBK = 16, kTiledThreads = 128, kTiledCols = 128;
 template <typename T, bool GATED, int BM, bool WIDE>
 __global__ void __launch_bounds__(kTiledThreads) moe_gemm_kernel(const T* __restrict__ x, const T* __restrict__ w,
@@ -240,9 +244,9 @@ __global__ void __launch_bounds__(32 * kFewWarps) moe_gemm_few_kernel(const T* _
 
 // Which of them: by the mean number of rows an expert has (the counts are on the device), and 16-byte (bfloat16: 8-byte)
 // loads where rows and bases allow them.  Up to 4 rows the kernel for few rows: 16 experts of 1,024 x 1,408 in 32 bits with 1, 2
-// and 4 rows each 49 + 31, 50 + 35 and 68 + 46 us for the two products, against 111 + 84 of the tiles at 5 (and at 1 to 16) rows.  Up
-// to 32 rows tiles of 32 rows, one an expert: 113 + 86 us at 32 rows; at 33 an expert has two of them, twice that, and tiles of 64
-// take 169 + 117.  The mean can mislead: 256 rows of 64 experts' four each on one of them are 33 tiles of eight rows, 146 + 133 us
+// and 4 rows each 49 + 31, 50 + 35 and 68 + 46 us for the two products, against 90 + 43 of the tensor cores' 128-row tiles at 5 to
+// 64 rows.  In bfloat16 up to 32 rows tiles of 32 rows, one an expert; at 33 an expert has two of them, and tiles of 64 are faster.
+// The mean can mislead: 256 rows of 64 experts' four each on one of them are 33 tiles of eight rows, 146 + 133 us
 // (the kernels of 32-row tiles before these: 180 + 201).
 template <typename T, bool GATED>
 static int launch_moe_gemm(const void* x, const void* w, const int32_t* offsets, int n_experts, int K, int N, int w_rows,
@@ -262,8 +266,12 @@ static int launch_moe_gemm(const void* x, const void* w, const int32_t* offsets,
   // (tiles of a few rows are the most: with so many experts that a grid cannot hold them, larger ones)
   if (wide && n_routes <= 4 * n_experts && grid_of(kFewRows, 1).y <= 65535u)
     FTK_MOE_GEMM((moe_gemm_few_kernel<T, GATED>), kFewRows, (GATED ? 1 : 2) * kFewPairs * kFewWarps, 32 * kFewWarps);
-  if (wide && n_routes <= 32 * n_experts) FTK_MOE_GEMM((moe_gemm_kernel<T, GATED, 32, true>), 32, cols, kTiledThreads);
-  if (wide) FTK_MOE_GEMM((moe_gemm_kernel<T, GATED, 64, true>), 64, cols, kTiledThreads);
+  if constexpr (sizeof(T) == 4) {
+    if (wide) return launch_moe_gemm_split<GATED>((const float*)x, (const float*)w, offsets, n_experts, K, N, w_rows, routes, weights, n_routes, act, alpha, limit, (float*)out, s);
+  } else {
+    if (wide && n_routes <= 32 * n_experts) FTK_MOE_GEMM((moe_gemm_kernel<T, GATED, 32, true>), 32, cols, kTiledThreads);
+    if (wide) FTK_MOE_GEMM((moe_gemm_kernel<T, GATED, 64, true>), 64, cols, kTiledThreads);
+  }
   FTK_MOE_GEMM((moe_gemm_kernel<T, GATED, 32, false>), 32, cols, kTiledThreads);
 #undef FTK_MOE_GEMM
 }

@@ -826,6 +826,7 @@ int ftk_attention_tc_set_status(int code);  // attention.cu
 namespace ftk {
 int delta_chunk_status(int* out);  // delta_chunk.cu
 int gla_chunks_status(int* out);   // gla_chunks.cuh
+int moe_gemm_split_status(int* out);  // moe_gemm_split.cuh
 }  // namespace ftk
 
 // Writes a code into a status word from the host, as a kernel whose wait ran out would: unit 0 = the
@@ -858,7 +859,7 @@ extern "C" int ftk_read_status(int* out) {
     out[1] = attn[1];
     return 0;
   }
-  for (auto read : {ftk::delta_chunk_status, ftk::gla_chunks_status}) {
+  for (auto read : {ftk::delta_chunk_status, ftk::gla_chunks_status, ftk::moe_gemm_split_status}) {
     if (read(attn) == 0 && attn[0]) {
       out[0] = attn[0];
       out[1] = attn[1];

@@ -258,7 +258,8 @@ def read_status() -> int:
     """Code left by a kernel whose bounded wait ran out since the last call (0 = none).  Waits
     for the device.  101-104 come from the tensor-core grouped GEMM (producer, accumulator
     hand-back, operand arrival, accumulator arrival), 501-506 from the delta rule's chunks,
-    601 from those of gated linear attention."""
+    601 and 602 from those of gated linear attention, 701 from
+    the 32-bit expert products."""
     out = (ctypes.c_int * 2)()
     status = _lib().ftk_read_status(out)
     if status != 0:
