@@ -678,7 +678,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             break;
           }
           tc_fence_after();
-          if (lane == 0) {
+          if (elect_one()) {
             const uint32_t d = tmem + (uint32_t)(st * kTcKeys);
 #pragma unroll
             for (int kk = 0; kk < 4 * kHalves; ++kk) {  // 16 elements of the head dimension per MMA
@@ -732,7 +732,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
           }
           __syncwarp();
           tc_fence_after();
-          if (lane == 0) {
+          if (elect_one()) {
             const uint32_t d = tmem + 2 * kTcKeys;
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk) {  // 16 keys per MMA

@@ -171,7 +171,7 @@ attention_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         const int g = g0 + j, ks = g % kTc2Stages;
         if (x == 0 && !mbar_wait(&k_full[ks], (uint32_t)(g / kTc2Stages) & 1u, abortp)) return false;
         tc_fence_after();
-        if (lane == 0) {
+        if (elect_one()) {
           const uint32_t d = tmem + (uint32_t)(x * kTcKeys);
 #pragma unroll
           for (int kk = 0; kk < 4 * kHalves; ++kk) {  // 16 elements of the head dimension per MMA
@@ -209,7 +209,7 @@ attention_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         if (j == 0 && !mbar_wait(&o_free[x], (uint32_t)(px[x] & 1) ^ 1u, abortp)) return false;
         __syncwarp();
         tc_fence_after();
-        if (lane == 0) {
+        if (elect_one()) {
           const uint32_t d = tmem + (uint32_t)((2 + x) * kTcKeys);
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk) {  // 16 keys per MMA

@@ -170,7 +170,7 @@ attention_tc_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             break;
           }
           tc_fence_after();
-          if (lane == 0) {
+          if (elect_one()) {
             const uint32_t d = tmem + (uint32_t)((g & 1) * kTcKeys);
             if (s1 > s0) {  // the tile's two steps lie one behind the other
 #pragma unroll
@@ -228,7 +228,7 @@ attention_tc_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
           if (it.ke - key0 < kTcKeys) clear(it.ke - key0, kTcKeys);
           __syncwarp();
           tc_fence_after();
-          if (lane == 0) {
+          if (elect_one()) {
             const uint32_t d = tmem + 2 * kTcKeys;
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk) {  // 16 keys per MMA

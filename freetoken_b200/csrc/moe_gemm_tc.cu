@@ -308,7 +308,7 @@ __global__ void __launch_bounds__(kThreads) moe_gemm_tc_kernel(const __grid_cons
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (of a pair: the leading CTA's)
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       int s = 0;
       uint32_t phase = 0;
       uint32_t acc_phase = 0;  // bit a: phase of accumulator buffer a

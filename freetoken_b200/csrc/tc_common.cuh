@@ -29,8 +29,23 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
       : "=r"(ok) : "r"(smem_addr(bar)), "r"(parity) : "memory");
   return ok != 0;
 }
-// Bounded wait: false when the barrier did not flip within the limit (or another role gave up).
+// Bounded waits: false when the barrier did not flip within the limit (or another role gave up).  The first leaves the asking to the
+// barrier's unit: asked again and again by a tile's softmax threads, it is in the way of products that read shared memory at its full
+// rate (prompt attention 85 -> 81 us, a portion over 32k keys 557 -> 533, the chunks of the delta rule 183 -> 177).
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  for (uint32_t i = 0; i < kSpinLimit / 16; ++i) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(smem_addr(bar)), "r"(parity) : "memory");
+    if (ok) return true;
+    if ((i & 7) == 7 && *abort_flag) return false;
+  }
+  return false;
+}
+__device__ __forceinline__ bool mbar_wait_spin(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
   for (uint32_t i = 0; i < kSpinLimit; ++i) {
     if (mbar_test(bar, parity)) return true;
     if ((i & 63) == 63) {
@@ -162,7 +177,9 @@ __device__ __forceinline__ void tc_mma_pair(uint32_t d_tmem, uint64_t a_desc, ui
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
 // One lane of a warp that is together, the same one each time.  (Products issued behind it, instead of behind a comparison of the
-// lane's number, leave their thread every 31 instead of every 51 cycles: the compiler sees that their operands are the warp's.)
+// lane's number, leave their thread every 31 instead of every 51 cycles: the compiler sees that their operands are the warp's.  A
+// portion over 32k keys 530 -> 496 us, prompt attention 81 -> 78, decode attention of 64 requests 122 -> 116, of eight experts' weights
+// 250 -> 244.)
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(p));
