@@ -90,8 +90,15 @@ class PagedGroup:
         if page != NULL_PAGE:
             self.updates.append((row * self.width + block, page))
 
+    def take_entries(self, row: int, block: int, pages: Sequence[int]) -> None:
+        """:meth:`set_entry` of fresh pages for consecutive blocks from ``block`` on."""
+        self.table_host[row, block:block + len(pages)] = pages
+        at = row * self.width + block
+        self.updates.extend(zip(range(at, at + len(pages)), pages))
+
     def held_pages(self, row: int, n_blocks: int) -> List[int]:
-        return [int(p) for p in self.table_host[row, :n_blocks] if p != NULL_PAGE]
+        pages = self.table_host[row, :n_blocks]
+        return pages[pages != NULL_PAGE].tolist()
 
     def dead_blocks(self, length: int) -> int:
         """Logical blocks no later query can read once the request holds ``length`` tokens."""
@@ -263,9 +270,8 @@ class CacheManager:
             pages = g.held_pages(req.row, n_blocks)
             g.pool.free(pages)
             first = g.first_live.pop(req.row, 0)
-            for b in list(range(min(g.kept_blocks, first, n_blocks))) + list(range(first, n_blocks)):
-                if g.table_host[req.row, b] != NULL_PAGE:
-                    g.set_entry(req.row, b, NULL_PAGE)
+            g.table_host[req.row, :min(g.kept_blocks, first, n_blocks)] = NULL_PAGE
+            g.table_host[req.row, first:n_blocks] = NULL_PAGE
         self.slots.free(req.state_slot)
         self._rows.append(req.row)
 
@@ -312,14 +318,19 @@ class CacheManager:
             plan.kv_lens.append(r.length + n)
             plan.state_slots.append(r.state_slot)
             plan.fresh.append(r.length == 0)
-            pos = np.arange(r.length, r.length + n)
+            pos = None
             for g in self.paged:
                 self._release_dead(g, r)
                 have = max(-(-r.length // self.page_size), g.first_live[r.row])
                 want = -(-(r.length + n) // self.page_size)
                 if want > have:
-                    for b, p in zip(range(have, want), g.pool.alloc(want - have)):
-                        g.set_entry(r.row, b, p)
+                    g.take_entries(r.row, have, g.pool.alloc(want - have))
+                if n == 1:  # (a decode step waits for this: plain numbers instead of arrays of one)
+                    page = int(g.table_host[r.row, r.length // self.page_size])
+                    plan.slot_maps[g.index][t0] = -1 if page == NULL_PAGE else page * self.page_size + r.length % self.page_size
+                    continue
+                if pos is None:
+                    pos = np.arange(r.length, r.length + n)
                 pages = g.table_host[r.row, pos // self.page_size].astype(np.int64)
                 slots = pages * self.page_size + pos % self.page_size
                 # positions whose page a window already passed (long prompt portions) are not stored

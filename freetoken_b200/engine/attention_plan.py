@@ -17,6 +17,7 @@ split, and the tile's first partial slot.
 from __future__ import annotations
 
 import ctypes
+import functools
 from dataclasses import dataclass
 from typing import List, Optional, Sequence, Tuple
 
@@ -41,6 +42,7 @@ class AttentionPlan:
 FIXED_COST_KEYS = 100  # what a CTA's start-up, write-out and merge cost, in keys' worth of time
 
 
+@functools.lru_cache(maxsize=256)
 def wave_splits(base_ctas: int, slots: int, limit: int, span: int = 2048) -> int:
     """Number of key splits (1..limit) with the shortest estimated time.
 

@@ -18,6 +18,7 @@ memory that is left, then the sampler and the CUDA graphs of decode steps
 
 from __future__ import annotations
 
+import functools
 import os
 from dataclasses import dataclass, field
 from typing import Any, Dict, Hashable, List, Optional, Sequence, Tuple
@@ -38,6 +39,12 @@ from .step import StepBuffers, StepBuilder
 
 _TORCH_DTYPE = {"bfloat16": torch.bfloat16, "float32": torch.float32}
 STATUS_CHECK_EVERY = 1024  # steps between two looks at the kernels' status words (a look waits for the device)
+
+
+@functools.lru_cache(maxsize=256)
+def _plan_names(plans: Tuple[Any, ...]) -> Tuple[str, ...]:
+    """A step's work lists in an order of their own, as part of its graph's key (their keys hold None beside numbers)."""
+    return tuple(sorted(map(repr, plans)))
 
 
 @dataclass
@@ -231,14 +238,20 @@ class Engine:
             n = len(e.tokens)
             if n < 1:
                 raise SchedulerError(f"request {e.request_id!r}: an entry needs at least one token")
-            ids = np.asarray(e.tokens, dtype=np.int64)
             if e.device_token is not None:
                 if n != 1:
                     raise SchedulerError(f"request {e.request_id!r}: a token taken from the device stands alone")
-                ids = np.zeros(1, dtype=np.int64)
-            if ids.min() < 0 or ids.max() >= vocab:
-                raise SchedulerError(f"request {e.request_id!r}: token id outside [0, {vocab})")
-            token_ids[t0:t0 + n] = ids
+                token_ids[t0] = 0
+            elif n == 1:  # (a decode step waits for this: plain numbers instead of arrays of one)
+                one = int(e.tokens[0])
+                if not 0 <= one < vocab:
+                    raise SchedulerError(f"request {e.request_id!r}: token id outside [0, {vocab})")
+                token_ids[t0] = one
+            else:
+                ids = np.asarray(e.tokens, dtype=np.int64)
+                if ids.min() < 0 or ids.max() >= vocab:
+                    raise SchedulerError(f"request {e.request_id!r}: token id outside [0, {vocab})")
+                token_ids[t0:t0 + n] = ids
             for w in e.want:
                 if not 0 <= w < n:
                     raise SchedulerError(f"request {e.request_id!r}: wanted place {w} outside its {n} tokens")
@@ -285,16 +298,21 @@ class Engine:
         graphable = (self.use_graphs and decode_only and len(logit_rows) == S
                      and logit_rows == list(range(S)))
         segments: List[Segment] = []
-        seg_info = np.empty((S, 4), dtype=np.int32)
-        positions = np.empty(T, dtype=np.int32)
+        info = []
         q0 = 0
         for i, e in enumerate(entries):
             n = len(e.tokens)
             kv = plan.kv_lens[i]
             segments.append(Segment(e.request_id, q0, n, kv, plan.state_slots[i], plan.fresh[i]))
-            seg_info[i] = (q0, n, kv, plan.rows[i])
-            positions[q0:q0 + n] = np.arange(kv - n, kv)
+            info.append((q0, n, kv, plan.rows[i]))
             q0 += n
+        seg_info = np.array(info, dtype=np.int32)
+        if decode_only:
+            positions = seg_info[:, 2] - 1
+        else:
+            positions = np.empty(T, dtype=np.int32)
+            for q0, n, kv, _ in info:
+                positions[q0:q0 + n] = np.arange(kv - n, kv)
         builder = StepBuilder(self, [(s.q_len, s.kv_len) for s in segments], fixed=graphable,
                               sm_count=self.sm_count)
         builder.add("token_ids", token_ids)
@@ -356,8 +374,7 @@ class Engine:
             return body()
         # one graph per batch size and metadata layout (the attention split count moves with the
         # longest request, which changes the size of the work list a few times over a long decode)
-        key = (S, tuple(arr.size for _, arr in builder.sections), tuple(sorted(map(repr, builder.plans))),
-               builder.longest_span())
+        key = (S, tuple(arr.size for _, arr in builder.sections), _plan_names(tuple(builder.plans)), builder.longest_span())
         recorded_now = key not in self.graphs
         if recorded_now:
             warm = body()  # warm-up: allocates work buffers and library workspaces outside the capture

@@ -24,6 +24,7 @@ import torch
 from .attention_plan import TC_ONE_TILE_COSTS, TC_TWO_TILE_COSTS, AttentionPlan, build_plan, wave_splits
 
 ALIGN = 4  # int32 elements = 16 bytes
+MOST_LAYOUTS = 64  # layouts of steps whose views are kept (decode steps come back to a few)
 
 
 @dataclass
@@ -50,6 +51,7 @@ class StepBuffers:
         self.events: List[Optional[Any]] = [None, None]
         self.turn = 0
         self.last_upload_bytes = 0
+        self._layouts: Dict[Any, Any] = {}  # sections' names and shapes -> their places, and views of the device buffer
 
     def grow(self, need: int) -> None:
         if need <= self.capacity:
@@ -59,30 +61,34 @@ class StepBuffers:
             f"raise max_step_tokens / max_running_req")
 
     def upload(self, sections: List[Tuple[str, np.ndarray]]) -> Dict[str, torch.Tensor]:
-        offsets = []
-        n = 0
-        for _, arr in sections:
-            offsets.append(n)
-            n += -(-max(arr.size, 1) // ALIGN) * ALIGN
-        self.grow(n)
+        layout = tuple((name, arr.shape) for name, arr in sections)
+        known = self._layouts.get(layout)
+        if known is None:
+            places, n = [], 0
+            for _, arr in sections:
+                places.append(slice(n, n + arr.size))
+                n += -(-max(arr.size, 1) // ALIGN) * ALIGN
+            self.grow(n)
+            if len(self._layouts) >= MOST_LAYOUTS:  # (steps of ever other lengths)
+                self._layouts.clear()
+            known = self._layouts[layout] = (
+                n, places, {name: self.dev[at].view(arr.shape) for (name, arr), at in zip(sections, places)}, self.dev[:n],
+                [h[:n] for h in self.host], [[buf[at].reshape(arr.shape) for (_, arr), at in zip(sections, places)] for buf in self.host_np])
+        n, places, views, dev, host, bufs = known
         i = self.turn
         self.turn ^= 1
         if self.events[i] is not None:
             self.events[i].synchronize()
-        buf = self.host_np[i]
-        for (name, arr), off in zip(sections, offsets):
-            buf[off:off + arr.size] = arr.reshape(-1)
+        for (_, arr), to in zip(sections, bufs[i]):
+            to[...] = arr
         self.last_upload_bytes = 4 * n
         if n:
-            self.dev[:n].copy_(self.host[i][:n], non_blocking=True)
+            dev.copy_(host[i], non_blocking=True)
         if self.device.type == "cuda":
-            ev = torch.cuda.Event()
-            ev.record()
-            self.events[i] = ev
-        out = {}
-        for (name, arr), off in zip(sections, offsets):
-            out[name] = self.dev[off:off + arr.size].view(arr.shape)
-        return out
+            if self.events[i] is None:
+                self.events[i] = torch.cuda.Event()
+            self.events[i].record()
+        return dict(views)
 
 
 class StepBuilder:
