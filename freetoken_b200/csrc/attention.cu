@@ -10,7 +10,7 @@
 // fallback for float32 (:45-144).
 //
 // Two implementations share the indexing code below:
-//   * attention_f32_kernel: the true 32-bit path.  One warp per query row, keys in chunks of 32
+//   * attention_f32_kernel: the true 32-bit path.  A warp per one to four query rows, keys in chunks of 32
 //     staged in shared memory, IEEE expf, float32 everywhere.
 //   * attention_bf16_kernel: 64 query rows per CTA on mma.sync m16n8k16 (bf16 in, float32
 //     accumulate), K/V tiles of 64 keys brought in by cp.async through the block table, online
@@ -233,7 +233,7 @@ __device__ __forceinline__ long long kv_row_offset(const AttnParams& p, const It
 }
 
 // ================================================================= float32 path
-constexpr int kF32Rows = 16;   // warps per block = query rows per tile
+constexpr int kF32Rows = 16;   // query rows per tile
 constexpr int kF32Chunk = 32;  // keys per chunk
 
 // Four adjacent floats; `vec`: on a 16-byte boundary.
@@ -241,22 +241,18 @@ __device__ __forceinline__ float4 f32_four(const float* p, bool vec) {
   return vec ? *reinterpret_cast<const float4*>(p) : make_float4(p[0], p[1], p[2], p[3]);
 }
 
-// COLS columns a lane: D <= 32 * COLS.
+// COLS columns a lane: D <= 32 * COLS.  RW rows a warp, so that a key's and a value's words serve as many rows once they are read;
+// a tile of no more rows than the block has warps (a decoding request's) spreads them out.
 //
 // What bounds it: in decode steps the trips to memory that wait for one another (work item, block table, keys), in prompts the
 // shared memory pipe.  So a key's row is looked up once (by the last warp, a chunk ahead), not once per element; a chunk's rows
 // are fetched sixteen bytes a thread into registers while the chunk before is worked on; and scores and products read four keys'
 // or four elements' words at a time.  Every sum keeps its order: results are the same, bit for bit, as with the plain loops before
-// (compared once, 504 calls: heads of 16 to 256, windows, sinks, one slab or two, cut and uncut).  16
-// heads on 4 of 64 / 128 / 256, 1,500 tokens: 1,993 / 2,793 / 4,393 -> 1,362 / 1,410 / 3,258 us; 16 tokens of decode over 2,000
-// keys (merge included): 148 / 249 / 419 -> 97 / 96 / 235 us.
-template <int COLS>
-__global__ void __launch_bounds__(kF32Rows * 32, 2) attention_f32_kernel(AttnParams p) {
-  pdl_wait();
-  pdl_trigger();
-  extern __shared__ __align__(16) float smem[];
-  const Item it = load_item(p, blockIdx.x);
-  if (!it.ok) return;
+// (compared, 504 calls: heads of 16 to 256, windows, sinks, one slab or two, cut and uncut).  16
+// heads on 4 of 64 / 128 / 256, 1,500 tokens: 1,993 / 2,793 / 4,393 us with plain loops, 1,362 / 1,410 / 3,270 with a warp a row, 584 / 939 /
+// 1,709 with two or four rows a warp; 16 tokens of decode over 2,000 keys (merge included): 148 / 249 / 419, 97 / 96 / 235 and 49 / 67 / 123.
+template <int COLS, int WARPS, int RW>
+__device__ __forceinline__ void attention_f32_tile(const AttnParams& p, const Item& it, float* smem) {
   const int kvh = blockIdx.y;
   const int D = p.D, G = p.G;
   const int ld = D + 4;                   // (an odd number of 16-byte words: a warp's rows start in different banks)
@@ -266,7 +262,7 @@ __global__ void __launch_bounds__(kF32Rows * 32, 2) attention_f32_kernel(AttnPar
   float* sv = tied ? sk : sk + kF32Chunk * ld;
   __shared__ long long soff[2][kF32Chunk];  // where a key's row lies (-1: nowhere)
   __shared__ int spos[2][kF32Chunk];        // its position in the sequence (-1: none)
-  constexpr int kThreads = kF32Rows * 32;
+  constexpr int kThreads = WARPS * 32;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int R = it.ntok * G;
   const float* q = (const float*)p.q;
@@ -281,14 +277,14 @@ __global__ void __launch_bounds__(kF32Rows * 32, 2) attention_f32_kernel(AttnPar
     soff[to][lane] = off;
     spos[to][lane] = off >= 0 ? key_position(p, it, kvh, c0 + lane) : -1;
   };
-  if (warp == kF32Rows - 1) look_up(it.kb, 0);
+  if (warp == WARPS - 1) look_up(it.kb, 0);
   for (int i = threadIdx.x; i < R * fours; i += kThreads) {
     const int r = i / fours, d = (i - r * fours) * 4;
     const int tok = it.q_start + it.tok0 + r / G;
     *reinterpret_cast<float4*>(sq + r * D + d) = f32_four(q + ((size_t)tok * p.Hq + kvh * G + r % G) * D + d, vec);
   }
-  // a thread's words of a chunk: at most COLS / 2 of the keys and as many of the values
-  constexpr int kWords = COLS > 2 ? COLS / 2 : 1;
+  // a thread's words of a chunk: at most 8 COLS / WARPS of the keys and as many of the values
+  constexpr int kWords = 8 * COLS / WARPS;
   int row[kWords], at[kWords];
 #pragma unroll
   for (int u = 0; u < kWords; ++u) {
@@ -308,14 +304,22 @@ __global__ void __launch_bounds__(kF32Rows * 32, 2) attention_f32_kernel(AttnPar
       }
     }
   };
-  const bool active = warp < R;
-  const int q_pos = it.kv_len - it.q_len + it.tok0 + warp / G;
-  const int lo_row = p.window > 0 ? q_pos - p.window + 1 : 0;
-  const float* brow = (p.dist_bias && active) ? p.dist_bias + (size_t)(kvh * G + warp % G) * p.dist_len : nullptr;
-  float acc[COLS];
+  const int r0 = warp * RW;  // the warp's rows: r0 .. r0 + RW - 1
+  const bool any = r0 < R;
+  int q_pos[RW], lo_row[RW];
+  const float* brow[RW];
+  float acc[RW][COLS], m[RW], l[RW];
 #pragma unroll
-  for (int i = 0; i < COLS; ++i) acc[i] = 0.f;
-  float m = -INFINITY, l = 0.f;
+  for (int e = 0; e < RW; ++e) {
+    const int r = r0 + e;
+    q_pos[e] = r < R ? it.kv_len - it.q_len + it.tok0 + r / G : -1;
+    lo_row[e] = p.window > 0 ? q_pos[e] - p.window + 1 : 0;
+    brow[e] = (p.dist_bias && r < R) ? p.dist_bias + (size_t)(kvh * G + r % G) * p.dist_len : nullptr;
+    m[e] = -INFINITY;
+    l[e] = 0.f;
+#pragma unroll
+    for (int i = 0; i < COLS; ++i) acc[e][i] = 0.f;
+  }
   __syncthreads();
   if (it.kb < it.ke) fetch(0);
 
@@ -329,77 +333,122 @@ __global__ void __launch_bounds__(kF32Rows * 32, 2) attention_f32_kernel(AttnPar
       *reinterpret_cast<float4*>(sk + row[u] * ld + at[u]) = kr[u];
       if (!tied) *reinterpret_cast<float4*>(sv + row[u] * ld + at[u]) = vr[u];
     }
-    if (more && warp == kF32Rows - 1) look_up(c0 + kF32Chunk, now ^ 1);
+    if (more && warp == WARPS - 1) look_up(c0 + kF32Chunk, now ^ 1);
     __syncthreads();
     if (more) fetch(now ^ 1);
     const int key = lane < nk ? spos[now][lane] : -1;
-    const bool vis = active && key >= 0 && key <= q_pos && (key >= lo_row || key < p.keep_first);
-    float s = -INFINITY;
-    if (vis) {
-      const float* qr = sq + warp * D;
+    if (any) {
+      float dot[RW];
+#pragma unroll
+      for (int e = 0; e < RW; ++e) dot[e] = 0.f;
+      const float* qr = sq + r0 * D;
       const float* key_row = sk + lane * ld;
-      float dot = 0.f;
 #pragma unroll 4
-      for (int d = 0; d < D; d += 4) {
-        const float4 a = *reinterpret_cast<const float4*>(qr + d), b = *reinterpret_cast<const float4*>(key_row + d);
-        dot = fmaf(a.x, b.x, dot);
-        dot = fmaf(a.y, b.y, dot);
-        dot = fmaf(a.z, b.z, dot);
-        dot = fmaf(a.w, b.w, dot);
-      }
-      s = dot * p.scale + dist_bias_at(brow, p.dist_len, q_pos - key);
-      if (p.softcap > 0.f) s = p.softcap * tanhf(s / p.softcap);
-    }
-    const float cm = warp_max(s);
-    if (cm != -INFINITY) {  // something is visible in this chunk
-      const float m_new = fmaxf(m, cm);
-      const float corr = m == -INFINITY ? 0.f : expf(m - m_new);
-      const float pj = vis ? expf(s - m_new) : 0.f;
-      l = l * corr + warp_sum(pj);
-      m = m_new;
+      for (int d = 0; d < D; d += 4) {  // (rows that do not exist: what lies there, never used)
+        const float4 b = *reinterpret_cast<const float4*>(key_row + d);
 #pragma unroll
-      for (int i = 0; i < COLS; ++i) acc[i] *= corr;
-      constexpr int kBatch = COLS > 4 ? 2 : 4;
-      for (int j = 0; j < nk; j += kBatch) {  // (past the last key: rows of zeros)
-        float pb[kBatch], x[kBatch][COLS];
-#pragma unroll
-        for (int u = 0; u < kBatch; ++u) {
-          pb[u] = __shfl_sync(0xffffffffu, pj, j + u);
-#pragma unroll
-          for (int i = 0; i < COLS; ++i) x[u][i] = lane + 32 * i < D ? sv[(j + u) * ld + lane + 32 * i] : 0.f;
+        for (int e = 0; e < RW; ++e) {
+          const float4 a = *reinterpret_cast<const float4*>(qr + e * D + d);
+          dot[e] = fmaf(a.x, b.x, dot[e]);
+          dot[e] = fmaf(a.y, b.y, dot[e]);
+          dot[e] = fmaf(a.z, b.z, dot[e]);
+          dot[e] = fmaf(a.w, b.w, dot[e]);
         }
+      }
+      float pj[RW];
+      bool some = false;  // something is visible in this chunk
 #pragma unroll
-        for (int u = 0; u < kBatch; ++u)
+      for (int e = 0; e < RW; ++e) {
+        const bool vis = key >= 0 && key <= q_pos[e] && (key >= lo_row[e] || key < p.keep_first);
+        float s = -INFINITY;
+        if (vis) {
+          s = dot[e] * p.scale + dist_bias_at(brow[e], p.dist_len, q_pos[e] - key);
+          if (p.softcap > 0.f) s = p.softcap * tanhf(s / p.softcap);
+        }
+        const float cm = warp_max(s);
+        pj[e] = 0.f;
+        if (cm != -INFINITY) {
+          const float m_new = fmaxf(m[e], cm);
+          const float corr = m[e] == -INFINITY ? 0.f : expf(m[e] - m_new);
+          pj[e] = vis ? expf(s - m_new) : 0.f;
+          l[e] = l[e] * corr + warp_sum(pj[e]);
+          m[e] = m_new;
 #pragma unroll
-          for (int i = 0; i < COLS; ++i) acc[i] = pb[u] != 0.f ? fmaf(pb[u], x[u][i], acc[i]) : acc[i];  // (what nobody sees may be anything)
+          for (int i = 0; i < COLS; ++i) acc[e][i] *= corr;
+          some = true;
+        }
+      }
+      if (some) {
+        constexpr int kBatch = COLS > 4 || RW > 1 ? 2 : 4;
+        for (int j = 0; j < nk; j += kBatch) {  // (past the last key: rows of zeros)
+          float x[kBatch][COLS];
+#pragma unroll
+          for (int u = 0; u < kBatch; ++u)
+#pragma unroll
+            for (int i = 0; i < COLS; ++i) x[u][i] = lane + 32 * i < D ? sv[(j + u) * ld + lane + 32 * i] : 0.f;
+#pragma unroll
+          for (int u = 0; u < kBatch; ++u)
+#pragma unroll
+            for (int e = 0; e < RW; ++e) {
+              const float pb = __shfl_sync(0xffffffffu, pj[e], j + u);
+#pragma unroll
+              for (int i = 0; i < COLS; ++i) acc[e][i] = pb != 0.f ? fmaf(pb, x[u][i], acc[e][i]) : acc[e][i];  // (what nobody sees may be anything)
+            }
+        }
       }
     }
     __syncthreads();
   }
-  if (!active) return;
-  const int tok = it.q_start + it.tok0 + warp / G;
-  if (it.nsplit == 1) {
-    float* o = (float*)p.out + ((size_t)tok * p.Hq + kvh * G + warp % G) * D;
-    const float lt = l + sink_term(p, m, kvh * G + warp % G);
-    const float inv = lt > 0.f ? 1.f / lt : 0.f;
+#pragma unroll 1
+  for (int e = 0; e < RW; ++e) {
+    const int r = r0 + e;
+    if (r >= R) return;
+    float me = m[0], le = l[0], o[COLS];
 #pragma unroll
-    for (int i = 0; i < COLS; ++i) {
-      const int d = lane + 32 * i;
-      if (d < D) o[d] = acc[i] * inv;
-    }
-  } else {
-    const size_t slot = ((size_t)(it.base + it.split) * p.Hkv + kvh) * p.tile_rows + warp;
-    float* po = p.part_o + slot * D;
+    for (int i = 0; i < COLS; ++i) o[i] = acc[0][i];
 #pragma unroll
-    for (int i = 0; i < COLS; ++i) {
-      const int d = lane + 32 * i;
-      if (d < D) po[d] = acc[i];
+    for (int f = 1; f < RW; ++f) {
+      if (f != e) continue;
+      me = m[f];
+      le = l[f];
+#pragma unroll
+      for (int i = 0; i < COLS; ++i) o[i] = acc[f][i];
     }
-    if (lane == 0) {
-      p.part_ml[slot * 2] = m;
-      p.part_ml[slot * 2 + 1] = l;
+    const int tok = it.q_start + it.tok0 + r / G;
+    if (it.nsplit == 1) {
+      float* to = (float*)p.out + ((size_t)tok * p.Hq + kvh * G + r % G) * D;
+      const float lt = le + sink_term(p, me, kvh * G + r % G);
+      const float inv = lt > 0.f ? 1.f / lt : 0.f;
+#pragma unroll
+      for (int i = 0; i < COLS; ++i) {
+        const int d = lane + 32 * i;
+        if (d < D) to[d] = o[i] * inv;
+      }
+    } else {
+      const size_t slot = ((size_t)(it.base + it.split) * p.Hkv + kvh) * p.tile_rows + r;
+      float* po = p.part_o + slot * D;
+#pragma unroll
+      for (int i = 0; i < COLS; ++i) {
+        const int d = lane + 32 * i;
+        if (d < D) po[d] = o[i];
+      }
+      if (lane == 0) {
+        p.part_ml[slot * 2] = me;
+        p.part_ml[slot * 2 + 1] = le;
+      }
     }
   }
+}
+
+template <int COLS, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, 16 / WARPS) attention_f32_kernel(AttnParams p) {
+  pdl_wait();
+  pdl_trigger();
+  extern __shared__ __align__(16) float smem[];
+  const Item it = load_item(p, blockIdx.x);
+  if (!it.ok) return;
+  if (it.ntok * p.G <= WARPS) attention_f32_tile<COLS, WARPS, 1>(p, it, smem);  // (a decoding request's few rows: side by side)
+  else attention_f32_tile<COLS, WARPS, kF32Rows / WARPS>(p, it, smem);
 }
 
 // ================================================================= merge of split tiles
@@ -1348,9 +1397,12 @@ static int paged_attention_impl(const void* q, const void* k_slab, const void* v
     FTK_REQUIRE(p.G <= kF32Rows, "paged_attention: %d query heads per KV head exceed the %d-row tile", p.G, kF32Rows);
     const size_t smem = ((size_t)kF32Rows * head_dim + (size_t)kF32Chunk * 2 * (head_dim + 4)) * sizeof(float);
     note_variant(sel ? "attention: float32, block-sparse" : "attention: float32, warp per row");
-    auto kern = head_dim <= 64 ? attention_f32_kernel<2> : head_dim <= 128 ? attention_f32_kernel<4> : attention_f32_kernel<8>;
+    // Four rows a warp for heads of 64, two above: with four rows a head of 128 takes twice the registers for its chunk's words (300
+    // tokens each of four requests 254 us against 177, decode steps 57 against 32).
+    const int warps = head_dim <= 64 ? 4 : 8;
+    auto kern = head_dim <= 64 ? attention_f32_kernel<2, 4> : head_dim <= 128 ? attention_f32_kernel<4, 8> : attention_f32_kernel<8, 8>;
     if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    FTK_LAUNCH(kern, grid, kF32Rows * 32, smem, s, p);
+    FTK_LAUNCH(kern, grid, warps * 32, smem, s, p);
     FTK_LAUNCH_CHECK("paged_attention (float32)");
     if (n_slots > 0) {
       FTK_LAUNCH(attention_merge_kernel<float>, grid, 128, 0, s, p);
