@@ -401,6 +401,9 @@ int ftk_moe_route(const float* x, const float* gate_w, const float* bias, int n_
 // Products of very few tokens (bfloat16): the weights are streamed once by warps of every SM (gemv.cu).
 int ftk_small_linear_fits(int n_tokens, int n_out, int k);
 int ftk_small_linear(const void* x, const void* w, void* out, int n_tokens, int n_out, int k, void* stream);
+// out [n_rows, n] = x [n_rows, k] w^T [n, k] in 32 bits, on the tensor cores in three bfloat16 pieces an operand (moe_gemm_split.cuh);
+// k a multiple of four, operands on 16-byte boundaries.
+int ftk_linear_split(const float* x, const float* w, float* out, int n_rows, int n, int k, void* stream);
 int ftk_moe_small_fits(int n_tokens, int hidden, int inter, int top_k);
 int ftk_moe_small_gate_up(const void* h, const int32_t* ids, const void* w1, void* a, int n_tokens, int top_k,
                           int n_experts, int hidden, int inter, int act, float alpha, float limit, void* stream);

@@ -355,3 +355,15 @@ extern "C" int ftk_moe_gemm2(const void* a, const void* w2, int dtype, const int
   FTK_LAUNCH_CHECK("moe_gemm2");
   return 0;
 }
+
+// out = x w^T in 32 bits, x [n_rows, k], w [n, k], rows side by side (moe_gemm_split.cuh).
+extern "C" int ftk_linear_split(const float* x, const float* w, float* out, int n_rows, int n, int k, void* stream) {
+  FTK_REQUIRE(n_rows >= 0 && n >= 1 && k >= 4 && k % 4 == 0, "linear_split: %d rows of %d x %d", n_rows, n, k);
+  if (n_rows == 0) return 0;
+  FTK_REQUIRE(x && w && out && (((uintptr_t)x | (uintptr_t)w | (uintptr_t)out) & 15) == 0, "linear_split: operands on 16-byte boundaries");
+  note_variant("linear: float32 on the tensor cores");
+  const int rc = launch_moe_gemm_split<false>(x, w, nullptr, 1, k, n, n, nullptr, nullptr, n_rows, 0, 0.f, 0.f, out, (cudaStream_t)stream);
+  FTK_REQUIRE(rc == 0, "linear_split: too many rows (%d)", n_rows);
+  FTK_LAUNCH_CHECK("linear_split");
+  return 0;
+}

@@ -51,7 +51,8 @@ __global__ void __launch_bounds__(kSplitThreads) moe_gemm_split_kernel(const flo
   pdl_wait();
   pdl_trigger();
   const uint32_t tmem = tmem_slot;
-  const ExpertTile tile = find_tile(offsets, n_experts, blockIdx.y, kSplitRows);
+  // (no offsets: one matrix for all n_routes rows, without weights of routes)
+  const ExpertTile tile = offsets ? find_tile(offsets, n_experts, blockIdx.y, kSplitRows) : ExpertTile{0, (int)blockIdx.y * kSplitRows, n_routes};
   if (tile.e >= 0) {
     const int n0 = blockIdx.x * (GATED ? 64 : 128), rows = min(kSplitRows, tile.row_end - tile.row0);
     const float* we = w + (size_t)tile.e * w_rows * K;
@@ -176,7 +177,7 @@ __global__ void __launch_bounds__(kSplitThreads) moe_gemm_split_kernel(const flo
     if (r < rows) {
       const size_t row = (size_t)tile.row0 + r;
       float weight = 1.f;
-      if (!GATED) {
+      if (!GATED && sorted_routes) {
         const int route = sorted_routes[row];
         weight = (route >= 0 && route < n_routes) ? route_weights[route] : 0.f;
       }
@@ -228,7 +229,7 @@ static int launch_moe_gemm_split(const float* x, const float* w, const int32_t* 
                                  const int32_t* routes, const float* weights, int n_routes, int act, float alpha, float limit, float* out,
                                  cudaStream_t s) {
   auto kern = moe_gemm_split_kernel<GATED>;
-  const dim3 grid((N + (GATED ? 63 : 127)) / (GATED ? 64 : 128), (n_routes + kSplitRows - 1) / kSplitRows + (n_experts < n_routes ? n_experts : n_routes));
+  const dim3 grid((N + (GATED ? 63 : 127)) / (GATED ? 64 : 128), (n_routes + kSplitRows - 1) / kSplitRows + (!offsets ? 0 : n_experts < n_routes ? n_experts : n_routes));
   if (grid.y > 65535u) return -1;
   FTK_REQUIRE(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmem) == cudaSuccess,
               "moe_gemm (32 bits): cannot set up the kernel");

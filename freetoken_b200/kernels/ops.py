@@ -145,6 +145,7 @@ _SIGNATURES = {
                       _vp],
     "ftk_small_linear_fits": [_i, _i, _i],
     "ftk_small_linear": [_vp, _vp, _vp, _i, _i, _i, _vp],
+    "ftk_linear_split": [_vp, _vp, _vp, _i, _i, _i, _vp],
     "ftk_moe_small_fits": [_i, _i, _i, _i],
     "ftk_moe_small_gate_up": [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _f, _vp],
     "ftk_moe_small_down": [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp],
@@ -766,11 +767,32 @@ def small_linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
     _check(_lib().ftk_small_linear(_dev(x, "x"), _dev(w, "w"), _dev(out, "out"), T, N, K, _stream()), "small_linear")
 
 
+def linear_split(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
+    """``out = x @ w^T`` in 32 bits on the tensor cores, operands in three bfloat16 numbers each (``csrc/moe_gemm_split.cuh``)."""
+    T, K = x.shape
+    N = w.shape[0]
+    if w.shape != (N, K) or out.shape != (T, N):
+        raise KernelError("linear_split: shapes do not agree")
+    f32 = torch.float32
+    _check(_lib().ftk_linear_split(_dev(x, "x", f32), _dev(w, "w", f32), _dev(out, "out", f32), T, N, K, _stream()), "linear_split")
+
+
+def _split_pays(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> bool:
+    """Whether :func:`linear_split` takes a product, and sooner than the library's: tiles of 128 x 128 take 2 us per 64 of k, one on
+    each SM at a time, and the library's 33 TFLOP/s are behind from about 600,000 results on.  Library and tiles, 1,024 of k: 256 x
+    1,536 36 and 39 us, 512 x 1,536 50 and 39, 861 x 1,536 81 and 39, 861 x 1,024 50 and 38, 64 x 8,192 42 and 34, 2,048 x 8,192 628
+    and 228; 6,144 of k, 192 x 3,072 179 and 164; 256 of k, 2,048 x 256 15 and 18."""
+    T, K = x.shape
+    return (T >= 48 and T * w.shape[0] >= 600000 and K % 4 == 0 and x.dtype == w.dtype == out.dtype == torch.float32
+            and x.is_cuda and x.is_contiguous() and w.is_contiguous() and out.is_contiguous()
+            and (x.data_ptr() | w.data_ptr() | out.data_ptr()) % 16 == 0)
+
+
 def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None) -> None:
     """``out = x @ w^T`` (``x [T, K]``, ``w [N, K]``, ``out [T, N]``): by the library, as in the reference
     (python/freetoken/layers/linear.py:66-70), except for bfloat16 steps of up to four tokens, whose
     product is a stream over the weights that :func:`small_linear` does faster than the library's choice
-    of tile (measured on B200, 3072 x 8192 for one token: see the design notes).
+    of tile (measured on B200, 3072 x 8192 for one token), and large 32-bit products (:func:`linear_split`).
 
     For fewer than 16 rows of bfloat16 and a weight that is at least as long as it is tall, the
     product is taken over 16 rows of the same buffers (the rows past ``T`` hold whatever the
@@ -793,6 +815,8 @@ def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[t
     if (T < P and K >= N and x.dtype == torch.bfloat16 and x.is_cuda and x.is_contiguous() and out.is_contiguous()
             and _room(x) >= P * K and _room(out) >= P * N):
         torch.matmul(x.as_strided((P, K), (K, 1)), w.t(), out=out.as_strided((P, N), (N, 1)))
+    elif x.dtype == torch.float32 and _split_pays(x, w, out):
+        linear_split(x, w, out)
     else:
         torch.mm(x, w.t(), out=out)
 
