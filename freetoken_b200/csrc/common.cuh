@@ -135,6 +135,8 @@ template <typename T>
 struct Vec4;
 template <>
 struct Vec4<float> {
+  using Raw = float4;  // as it lies in memory
+  static __device__ __forceinline__ void unpack(const float4& t, float (&v)[4]) { v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w; }
   static __device__ __forceinline__ void load(const float* p, float (&v)[4]) {
     float4 t = *reinterpret_cast<const float4*>(p);
     v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
@@ -145,10 +147,11 @@ struct Vec4<float> {
 };
 template <>
 struct Vec4<__nv_bfloat16> {
-  static __device__ __forceinline__ void load(const __nv_bfloat16* p, float (&v)[4]) {
-    uint2 t = *reinterpret_cast<const uint2*>(p);
-    __nv_bfloat162 a = *reinterpret_cast<__nv_bfloat162*>(&t.x);
-    __nv_bfloat162 b = *reinterpret_cast<__nv_bfloat162*>(&t.y);
+  using Raw = uint2;
+  static __device__ __forceinline__ void load(const __nv_bfloat16* p, float (&v)[4]) { unpack(*reinterpret_cast<const uint2*>(p), v); }
+  static __device__ __forceinline__ void unpack(const uint2& t, float (&v)[4]) {
+    const __nv_bfloat162 a = *reinterpret_cast<const __nv_bfloat162*>(&t.x);
+    const __nv_bfloat162 b = *reinterpret_cast<const __nv_bfloat162*>(&t.y);
     v[0] = __low2float(a); v[1] = __high2float(a); v[2] = __low2float(b); v[3] = __high2float(b);
   }
   static __device__ __forceinline__ void store(__nv_bfloat16* p, const float (&v)[4]) {

@@ -126,6 +126,27 @@ def test_conv_act_uses_and_advances_the_state(dtype, C, taps, off, bias, act):
         torch.testing.assert_close(st_a.cpu(), st_b, rtol=0, atol=0)
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("C,taps,act", [(512, 4, "silu"), (516, 3, None), (44, 2, "silu")])
+def test_conv_act_rows_on_their_way(dtype, C, taps, act):
+    """Aligned rows (a view of a wider projection) come through a ring of eight: requests around its length, around a tile's 16
+    tokens, shorter than the state (whose rows move up in their slot), and the last thread's columns alone."""
+    lens = [(1, 40), (7, 7), (8, 9), (9, 70), (15, 16), (16, 16), (17, 90), (2, 2), (33, 33), (1, 2)]
+    info, slots, T = segs(lens)
+    x = rnd(T, C + 8, dtype=dtype, seed=1)[:, 8:]
+    w, b = rnd(C, taps, seed=2, scale=0.5), rnd(C, seed=6)
+    st = rnd(len(lens) + 1, taps - 1, C, seed=3)
+    for i, (q, kv) in enumerate(lens):
+        if kv - q < taps - 1:
+            st[i + 1, : taps - 1 - (kv - q)] = 0
+    st_a, st_b = st.clone(), st.clone().cpu()
+    got, want = torch.zeros(T, C, dtype=dtype, device=DEV), torch.zeros(T, C, dtype=dtype)
+    ops.conv_act(x, w, b, act, st_a, slots, info, len(lens), got)
+    ref.conv_act(x.cpu(), w.cpu(), cpu(b), act, st_b, slots.cpu(), info.cpu(), len(lens), want)
+    torch.testing.assert_close(got.float().cpu(), want.float(), **tol(dtype))
+    torch.testing.assert_close(st_a.cpu(), st_b, rtol=0, atol=0)
+
+
 @pytest.mark.parametrize("cuts", [[50], [1] * 50, [2, 3, 16, 17, 1, 11], [15, 1, 16, 2, 16]])
 def test_conv_act_cut_anywhere_is_the_whole(cuts):
     C, taps, T = 48, 4, 50
