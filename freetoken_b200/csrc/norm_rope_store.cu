@@ -24,6 +24,25 @@ constexpr int kMaxSections = 4;
 constexpr int kWarpsPerBlock = 4;
 constexpr int kMaxHeadDim = 256;
 
+// Two 32-bit operations in one instruction, each rounded as by itself.
+#define FTK_PAIR(v) (*reinterpret_cast<const unsigned long long*>(&(v)))
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<unsigned long long&>(d)) : "l"(FTK_PAIR(a)), "l"(FTK_PAIR(b)));
+  return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<unsigned long long&>(d)) : "l"(FTK_PAIR(a)), "l"(FTK_PAIR(b)));
+  return d;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(reinterpret_cast<unsigned long long&>(d)) : "l"(FTK_PAIR(a)), "l"(FTK_PAIR(b)), "l"(FTK_PAIR(c)));
+  return d;
+}
+#undef FTK_PAIR
+
 struct Sections {
   FtkSection s[kMaxSections];
   int n;
@@ -126,9 +145,10 @@ __global__ void norm_rope_store_kernel(const T* __restrict__ x, int n_tokens, in
 // The same for bfloat16 heads of 64, 128 or 256 elements with 16-byte accesses: a head is spread over
 // LPH = head_dim / 8 lanes (8 consecutive elements each), a warp takes 32 / LPH heads at once, and a
 // lane gets its rotation partners from the lane half a rotary span away (rotary_dim a multiple of 16).
-// (Measured at 2,048 tokens of 64 heads: 25.6 microseconds.  A block per token whose warps walk the token's
-// heads with eight loads in flight per lane and the token's table rows read once took 30 to 37; four
-// tokens per thread took 29.)
+// What bounds it: instructions (2.8 of 4 an SM cycle) and the latency of slot, position and table row, one behind the other
+// (the row itself no longer waits for them).  2,048 tokens of 64 heads: 27.5 us with the row asked for last and one sum or product an
+// instruction, 24.9 now, with the same bits.  (A block per token whose warps walk the token's heads with eight loads in flight per
+// lane and the token's table rows read once took 30 to 37; four tokens per thread took 29.)
 template <int LPH>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 norm_rope_store_vec_kernel(const __nv_bfloat16* __restrict__ x, int n_tokens, int row_elems, int rotary_dim,
@@ -149,15 +169,13 @@ norm_rope_store_vec_kernel(const __nv_bfloat16* __restrict__ x, int n_tokens, in
     ++si;
   }
   const FtkSection& S = sec.s[si];
-  long long slot = 0;
-  bool store = live;
-  if (S.slab) {
-    slot = S.slot_map[t];
-    if (slot < 0 || slot >= (long long)S.num_pages * S.page_size) store = false;  // not stored
-  }
-  const __nv_bfloat16* src = x + (size_t)t * row_elems + (size_t)(S.first_head + hl) * kHeadDim + l * 8;
-  // everything this thread reads is asked for before the first use: the row, the norm weight, and the
+  // everything this thread reads is asked for before the first use: the row, the slot, the norm weight, and the
   // two runs of eight table entries of its rotation (cos | sin halves of the position's row)
+  const __nv_bfloat16* src = x + (size_t)t * row_elems + (size_t)(S.first_head + hl) * kHeadDim + l * 8;
+  uint4 raw = make_uint4(0u, 0u, 0u, 0u);
+  if (live) raw = *reinterpret_cast<const uint4*>(src);
+  int slot = 0;
+  if (S.slab) slot = S.slot_map[t];
   const int half = rotary_dim >> 1;
   const bool rot = S.rotate && rotary_dim > 0;
   const bool low = l * 8 < half, in = l * 8 < rotary_dim;
@@ -192,8 +210,6 @@ norm_rope_store_vec_kernel(const __nv_bfloat16* __restrict__ x, int n_tokens, in
   }
   float v[8];
   {
-    uint4 raw = make_uint4(0u, 0u, 0u, 0u);
-    if (live) raw = *reinterpret_cast<const uint4*>(src);
     const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raw);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -222,7 +238,11 @@ norm_rope_store_vec_kernel(const __nv_bfloat16* __restrict__ x, int n_tokens, in
       const float inv = rsqrtf(ss / (float)kHeadDim + eps);
       const float one = gemma ? 1.f : 0.f;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) v[j] = v[j] * inv * (w[j] + one);
+      for (int j = 0; j < 8; j += 2) {
+        const float2 u = mul2(mul2(make_float2(v[j], v[j + 1]), make_float2(inv, inv)), add2(make_float2(w[j], w[j + 1]), make_float2(one, one)));
+        v[j] = u.x;
+        v[j + 1] = u.y;
+      }
     }
   }
   if (neighbours) {
@@ -250,15 +270,21 @@ norm_rope_store_vec_kernel(const __nv_bfloat16* __restrict__ x, int n_tokens, in
       }
     }
     if (rot && in) {
+      const float sign = low ? -1.f : 1.f;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) v[j] = low ? v[j] * ca[j] - partner[j] * cb[j] : v[j] * ca[j] + partner[j] * cb[j];
+      for (int j = 0; j < 8; j += 2) {
+        const float2 turned = mul2(make_float2(partner[j], partner[j + 1]), mul2(make_float2(cb[j], cb[j + 1]), make_float2(sign, sign)));
+        const float2 u = fma2(make_float2(v[j], v[j + 1]), make_float2(ca[j], ca[j + 1]), turned);
+        v[j] = u.x;
+        v[j + 1] = u.y;
+      }
     }
   }
   if (S.pos_scale) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) v[j] *= factor;
   }
-  if (!store) return;
+  if (!live || (S.slab && (slot < 0 || slot >= (long long)S.num_pages * S.page_size))) return;  // not stored
   __nv_bfloat16* dst;
   if (S.slab) {
     // (slots are 32-bit numbers: the 64-bit division costs several times the 32-bit one)
