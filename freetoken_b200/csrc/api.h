@@ -85,6 +85,9 @@ typedef struct {
   // with a window: queries also read the positions below keep_first (work items number the keys as build_plan does with
   // keep_first); not with block selection, a bias by distance or a soft cap.  0 = none
   int keep_first;
+  // the weight that the step reads next (or null): brought into L2 by the merge of split tiles while it waits for them
+  const void* ahead;
+  long long ahead_bytes;
 } FtkAttnExtras;
 
 // What ftk_stream_step does to the rows of the 32-bit stream (see gated_stream.cu).  x, passed, shared, gate, raw_out,

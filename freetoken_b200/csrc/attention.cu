@@ -69,6 +69,9 @@ struct AttnParams {
   // run over the first keep_span positions (keep_first rounded up to keep_quantum) and, right behind them, the tile's window
   // from the multiple of keep_quantum at or before its first key (see Item::jump).  keep_span 0: none
   int keep_first, keep_span, keep_quantum;
+  // the weight that the step reads next, or null (attention_merge_kernel)
+  const unsigned char* ahead;
+  long long ahead_bytes;
 };
 
 // Soft-capped scores of the bfloat16 kernels: raw products s become softcap * log2(e) * tanh(s * scale / softcap), scores
@@ -459,6 +462,11 @@ __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS) attention_f32_kernel(A
 template <typename T>
 __global__ void __launch_bounds__(512) attention_merge_kernel(AttnParams p) {
   const Item it = load_item(p, blockIdx.x);  // the work list was made on the host before the step
+  if (p.ahead) {  // (lines of 128 bytes, all asked for at once: a pause of 150 ns between a thread's gave the same, of 400 ns lost it)
+    const long long step = (long long)gridDim.x * gridDim.y * blockDim.x * 128;
+    for (long long at = ((long long)(blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x) * 128; at < p.ahead_bytes; at += step)
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(p.ahead + at));
+  }
   pdl_wait();
   pdl_trigger();
   if (!it.ok || it.nsplit <= 1) return;
@@ -1256,6 +1264,8 @@ static int paged_attention_tc_impl(const void* q, const void* k_slab, const void
   p.sink = extras ? extras->sink_logit : 0.f;
   p.sink_heads = extras ? extras->sink_heads : nullptr;
   p.softcap = extras ? extras->softcap : 0.f;
+  p.ahead = extras ? (const unsigned char*)extras->ahead : nullptr;
+  p.ahead_bytes = extras ? extras->ahead_bytes : 0;
   FTK_REQUIRE(!(p.softcap > 0.f) || (!p.dist_bias && scale > 0.f),
               "paged_attention_tc: a soft cap goes with a positive scale and no distance bias");
   FTK_REQUIRE(set_kept(p, extras, kTcKeys), "paged_attention_tc: kept first tokens go with a window, without bias or soft cap");
@@ -1370,6 +1380,8 @@ static int paged_attention_impl(const void* q, const void* k_slab, const void* v
   p.sink = extras ? extras->sink_logit : 0.f;
   p.sink_heads = extras ? extras->sink_heads : nullptr;
   p.softcap = extras ? extras->softcap : 0.f;
+  p.ahead = extras ? (const unsigned char*)extras->ahead : nullptr;
+  p.ahead_bytes = extras ? extras->ahead_bytes : 0;
   FTK_REQUIRE(!(p.softcap > 0.f) || (!sel && !p.dist_bias),
               "paged_attention: a soft cap cannot be combined with block selection or a distance bias");
   FTK_REQUIRE(set_kept(p, extras, kBN), "paged_attention: kept first tokens go with a window, without bias, soft cap or block selection");

@@ -7,11 +7,11 @@
 // so U = T X with X = beta (V - c K S), T = (I + L)^-1, L_ts = beta_t (c_t / c_s) (k_s . k_t), and O = c Q S + A T X.  T, A T and
 // the factors of a token depend on the chunks alone: delta_prep_kernel makes them for all chunks side by side (the decays in 64
 // bits: where a state lives for hundreds of tokens, their rounding is most of what a result is off), T from the inverses of
-// its two blocks of 32.  What is left to do in order (delta_chunk_kernel) is three products: [K; Q] S, [T; A T] X and K^T U.
+// its diagonal blocks of 16.  What is left to do in order (delta_chunk_kernel) is three products: [K; Q] S, [T; A T] X and K^T U.
 // Decays are running products, never differences of logarithms.  The state is rounded once in 64 tokens.
 //
 // The three products run on tcgen05, in 32 bits: K and Q are bfloat16 as they lie, and S, T, X and U are taken apart into three
-// bfloat16 numbers each, whose sum is exactly the 32-bit one (cut off, not rounded: 8 bits a piece).  Of T X the six products
+// bfloat16 numbers each, every piece rounded to the nearest, whose sum is exactly the 32-bit one.  Of T X the six products
 // that reach 2^-24 are taken.  The tensor core's accumulator cuts off instead of rounding (measured: a bias of half a unit a step of
 // 16; one step, and two, are as close to 64 bits as a chain of as many fmas), so the products of the leading pieces are chains of two
 // steps, added up in registers; the other pieces' are 2^-8 smaller.

@@ -84,7 +84,7 @@ class _StreamNorm(ctypes.Structure):
 
 class _AttnExtras(ctypes.Structure):
     _fields_ = [("dist_bias", _vp), ("dist_len", _i), ("kv_split", _i), ("has_sink", _i), ("sink_logit", _f),
-                ("sink_heads", _vp), ("softcap", _f), ("keep_first", _i)]
+                ("sink_heads", _vp), ("softcap", _f), ("keep_first", _i), ("ahead", _vp), ("ahead_bytes", ctypes.c_longlong)]
 
 
 class _StreamStep(ctypes.Structure):
@@ -482,7 +482,8 @@ def paged_attention(q: torch.Tensor, k_slab: torch.Tensor, v_slab: torch.Tensor,
                     part_ml: Optional[torch.Tensor], out: torch.Tensor, tile_rows: int, scale: float,
                     window: Optional[int], sel: Optional[torch.Tensor] = None, block_size: int = 0,
                     few_rows: bool = False, dist_bias: Optional[torch.Tensor] = None, kv_split: int = 1,
-                    sink: Any = None, softcap: Optional[float] = None, keep_first: int = 0) -> None:
+                    sink: Any = None, softcap: Optional[float] = None, keep_first: int = 0,
+                    ahead: Optional[torch.Tensor] = None) -> None:
     """Causal softmax attention of the step's queries over the paged keys and values.
 
     ``q, out [T, Hq, D]``; slabs ``[pages, Hkv, page_size, D]``; ``block_table [rows, width]``
@@ -522,6 +523,9 @@ def paged_attention(q: torch.Tensor, k_slab: torch.Tensor, v_slab: torch.Tensor,
     ``keep_first`` (with a window; the work list from ``build_plan(..., keep_first=...)``): positions below it stay visible
     however far back they are.  Of the tcgen05 kernels the one with 128-row tiles takes it; not with a bias by distance,
     block selection or a soft cap.
+
+    ``ahead``: the weight that the step reads next; with ``few_rows`` the merge of split tiles asks for it (into L2) before it waits
+    for the splits.  No result depends on it.
     """
     keep_first = int(keep_first or 0)
     if keep_first and (keep_first < 0 or not window or sel is not None or dist_bias is not None or softcap):
@@ -554,7 +558,7 @@ def paged_attention(q: torch.Tensor, k_slab: torch.Tensor, v_slab: torch.Tensor,
         # bfloat16 steps on the tcgen05 kernels: one query tile per CTA, a pair of them, or tiles of a few rows
         if sel is not None or q.dtype != torch.bfloat16:
             raise KernelError("paged_attention: the tcgen05 kernels take bfloat16 without block selection")
-        if window or sink is not None or dist_bias is not None or softcap or kv_split > 1:
+        if window or sink is not None or dist_bias is not None or softcap or kv_split > 1 or (ahead is not None and few_rows):
             # the form with one 128-row query tile a piece takes a window, a sink and a bias by distance (a bias not
             # together with a window); the form for tiles of at most 16 rows takes the bias alone
             if (window or sink is not None) and (tile_rows != 128 or few_rows):
@@ -564,8 +568,8 @@ def paged_attention(q: torch.Tensor, k_slab: torch.Tensor, v_slab: torch.Tensor,
                                   "distance bias [Hq, L] (no window)")
             ex = _AttnExtras(_dev(dist_bias, "dist_bias", torch.float32), dist_bias.shape[1] if dist_bias is not None else 0,
                              kv_split, 0 if sink is None else 1, 0.0 if sink is None else float(sink), sink_heads, softcap,
-                             keep_first)
-            what = "soft cap" if softcap else "distance bias" if dist_bias is not None else "window or sink"
+                             keep_first, _dev(ahead, "ahead"), 0 if ahead is None else ahead.numel() * ahead.element_size())
+            what = "soft cap" if softcap else "distance bias" if dist_bias is not None else "window, sink or decode step"
             _check(_lib().ftk_paged_attention_tc_ex(
                 _dev(q, "q"), _dev(k_slab, "k_slab"), _dev(v_slab, "v_slab"),
                 _dev(block_table, "block_table", torch.int32), block_table.shape[1],

@@ -53,6 +53,23 @@ def test_single_tokens_with_heads_of_64_in_the_form_for_few_rows(Hq, Hkv, P, spl
     assert ops.read_status() == 0
 
 
+@pytest.mark.parametrize("D,kv,splits,shape", [(128, 700, 5, (3, 40)), (64, 2000, 16, (1, 8)), (128, 5000, 8, (513, 1031)), (64, 100, 1, (64, 64))])
+def test_a_weight_asked_for_ahead_changes_no_bit(D, kv, splits, shape):
+    """Weights of less than a line, of no whole lines and of more than a line a thread; a step without split tiles."""
+    q, ks, vs, bt, seg = attention_problem(BF, 12, 2, D, 16, [(1, kv)])
+    plan = build_plan([(1, kv)], 6, 16, None, 2, fixed_splits=splits, sm_count=74, key_tile=128)
+    po = pm = None
+    if plan.n_slots:
+        po, pm = torch.empty(plan.n_slots, 2, 16, D, device=DEV), torch.empty(plan.n_slots, 2, 16, 2, device=DEV)
+    outs = []
+    for ahead in (None, torch.ones(shape, dtype=BF, device=DEV)):
+        outs.append(torch.full_like(q, float("nan")))
+        ops.paged_attention(q, ks, vs, bt, seg, 1, torch.from_numpy(plan.items).to(DEV), plan.n_items, po, pm, outs[-1], 16, 0.1, None,
+                            few_rows=True, ahead=ahead)
+    assert torch.equal(outs[0], outs[1]) and bool(plan.n_slots) == (splits > 1)
+    assert ops.read_status() == 0
+
+
 @pytest.mark.parametrize("D", [64, 128, 256])
 @pytest.mark.parametrize("Hq,Hkv,P,window,keep,split", [(6, 1, 16, 72, 0, 1), (48, 1, 16, None, 0, 3), (48, 1, 32, 200, 0, 3),
                                                         (256, 1, 16, 300, 0, 8), (8, 2, 48, 37, 5, 2), (128, 1, 16, 128, 129, 1)])
