@@ -35,6 +35,7 @@ int delta_scan_tokens(const void* q, long long q_stride, const void* k, long lon
 __device__ int g_delta_status[4];  // [0] first error code of a wait that ran out, [1] block; 0 = fine
 
 constexpr int kDcTokens = 64;  // tokens of the two chunks that go together
+constexpr float kDcMost = 3.38e38f;  // what bfloat16 reaches: larger numbers' first piece would be an infinity
 // Scratch of 64 tokens: a key head's [K; Q] as the tensor core reads it (per 64 channels 128 rows of 128 bytes, swizzled), then a
 // head's [T; A T] the same way (three pieces of 128 rows of 64 tokens), per token beta, beta c rk, c rq, (c_C / c) rk, and c_C.
 constexpr int kDcImage = 128 * 128;  // bytes of 128 rows
@@ -394,6 +395,84 @@ __device__ __forceinline__ void dc_bulk_load(uint32_t dst, const void* src, uint
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes),
                "r"(smem_addr(bar)) : "memory");
 }
+// Columns with an infinite or NaN number in the 64 tokens from token `first` on, once more, as delta.cu runs them (in pairs of tokens): an
+// infinity taken apart into pieces is a NaN, and so is what has infinities of both signs, which depends on where they meet.  A warp takes a
+// column: `state` [NV][D] holds them as the chunk finds them, and is left as it leaves them; outputs go out from a column's
+// first such token on.
+template <int D, int NV>
+__device__ __noinline__ void dc_by_token(const DeltaChunkArgs& a, float* state, const int* first_odd, int first, int nb, int h, int col0) {
+  constexpr int N = D / 32;
+  const int lane = threadIdx.x & 31, hqk = h / (a.H / a.G);
+  const float neg_rate = -expf(a.a_log[h]), bias = a.dt_bias[h];
+  for (int c = threadIdx.x >> 5; c < NV; c += blockDim.x >> 5) {
+    const int from = first_odd[c];
+    if (from >= kDcTokens || col0 + c >= a.Dv) continue;
+    float s[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) s[i] = state[c * D + lane + 32 * i];
+    for (int t = 0; t < nb; t += 2) {
+      const bool two = t + 1 < nb;  // (an odd last token's partner: zeros that decay nothing)
+      float k[2][N], q[2][N], g[2], beta[2], v[2], kq[2], dot[6] = {};
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const bool in = e == 0 || two;
+        const size_t tok = (size_t)(first + t + (in ? e : 0));
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+          k[e][i] = in ? __bfloat162float(a.k[tok * a.k_stride + (size_t)hqk * D + lane + 32 * i]) : 0.f;
+          q[e][i] = in ? __bfloat162float(a.q[tok * a.q_stride + (size_t)hqk * D + lane + 32 * i]) : 0.f;
+        }
+        const float z = __bfloat162float(a.a[tok * a.a_stride + h]) + bias;
+        g[e] = in ? expf(neg_rate * (z > 0.f ? z + log1pf(expf(-z)) : log1pf(expf(z)))) : 1.f;
+        beta[e] = in ? 1.f / (1.f + expf(-__bfloat162float(a.b[tok * a.b_stride + h]))) : 0.f;
+        v[e] = in ? __bfloat162float(a.v[tok * a.v_stride + (size_t)h * a.Dv + col0 + c]) : 0.f;
+      }
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          dot[e] = fmaf(k[e][i], k[e][i], dot[e]);
+          dot[2 + e] = fmaf(q[e][i], q[e][i], dot[2 + e]);
+          kq[e] = i ? fmaf(q[e][i], k[e][i], kq[e]) : q[e][i] * k[e][i];
+        }
+        dot[4] = fmaf(k[0][i], k[1][i], dot[4]);
+        dot[5] = fmaf(k[0][i], q[1][i], dot[5]);
+      }
+      float rk[2], rq[2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        rk[e] = e == 0 || two ? rsqrtf(warp_sum(dot[e]) + a.unit_eps) : 0.f;
+        rq[e] = e == 0 || two ? rsqrtf(warp_sum(dot[2 + e]) + a.unit_eps) * a.q_scale : 0.f;
+        kq[e] = warp_sum(kq[e]) * rq[e] * rk[e];
+      }
+      const float kk = warp_sum(dot[4]) * rk[0] * rk[1], kqab = warp_sum(dot[5]) * rk[0] * rq[1];
+      float r[2] = {0.f, 0.f}, p[2] = {0.f, 0.f};
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+          k[e][i] *= rk[e];
+          r[e] = fmaf(s[i], k[e][i], r[e]);
+          p[e] = fmaf(s[i], q[e][i] * rq[e], p[e]);
+        }
+        r[e] = warp_sum(r[e]);
+        p[e] = warp_sum(p[e]);
+      }
+      const float ua = beta[0] * (v[0] - g[0] * r[0]);
+      const float ub = two ? beta[1] * (v[1] - g[1] * fmaf(g[0], r[1], kk * ua)) : 0.f;
+      const float gab = g[0] * g[1], wa = g[1] * ua;
+#pragma unroll
+      for (int i = 0; i < N; ++i) s[i] = fmaf(gab, s[i], two ? fmaf(wa, k[0][i], ub * k[1][i]) : wa * k[0][i]);
+      if (lane < 2 && t + lane >= from && (lane == 0 || two)) {
+        const float o = lane == 0 ? fmaf(g[0], p[0], kq[0] * ua) : fmaf(g[1], fmaf(g[0], p[1], kqab * ua), kq[1] * ub);
+        a.out[((size_t)(first + t + lane) * a.H + h) * a.Dv + col0 + c] = o;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) state[c * D + lane + 32 * i] = s[i];
+  }
+}
+
 // A block owns NV value columns of one (request, head).  A thread has a row (a token of K, of Q; a key channel) and 8 or 16 of the
 // columns.  Products, by one thread (columns of NV in tensor memory; each is read before the next is issued, so all use the same):
 //   [K; Q] S      two 16-channel steps of the leading piece each in columns of their own (up to 4), the second and third piece (4, 5)
@@ -402,13 +481,13 @@ __device__ __forceinline__ void dc_bulk_load(uint32_t dst, const void* src, uint
 template <int NV>
 constexpr int dc_threads() { return NV == 64 ? 512 : 256; }
 template <int D, int NV>
-__global__ void __launch_bounds__(dc_threads<NV>()) delta_chunk_kernel(DeltaChunkArgs a) {
+__global__ void __launch_bounds__(dc_threads<NV>()) delta_chunk_kernel(const __grid_constant__ DeltaChunkArgs a) {
   constexpr int NH = NV * 128 / dc_threads<NV>(), NG = NH / 8;  // columns a thread, eights of them
   using At = DcPlace<NV>;
   extern __shared__ unsigned char dc_smem[];
   __shared__ uint64_t kq_full[2], t_full, mma_done;
   __shared__ uint32_t tmem_slot;
-  __shared__ int abort_flag, odd_flag[2], first_odd[NV];  // the first token whose X is no number, per column
+  __shared__ int abort_flag, odd_flag[2], first_odd[NV];  // the first token that has no number, per column
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, quad = warp & 3, share = warp >> 2;
   const uint32_t base = (smem_addr(dc_smem) + 1023u) & ~1023u;
   unsigned char* tiles = dc_smem + (base - smem_addr(dc_smem));
@@ -551,8 +630,8 @@ __global__ void __launch_bounds__(dc_threads<NV>()) delta_chunk_kernel(DeltaChun
       __syncwarp();
       tc_fence_after();
       float o[NH];  // Q's rows: what the state gives
-      // What a row of T and A T has behind its token is zero, but zero times an infinity or NaN is NaN: such an X goes into the product
-      // as zero, and its column is NaN from its token on.
+      // What a row of T and A T has behind its token is zero, but zero times an infinity or NaN is NaN: such an X (or one that bfloat16
+      // cannot reach) goes into the product as zero, and its column token by token from there on.
       bool odd = false;
 #pragma unroll
       for (int i = 0; i < NG; ++i) {
@@ -574,7 +653,7 @@ __global__ void __launch_bounds__(dc_threads<NV>()) delta_chunk_kernel(DeltaChun
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             y[j] = fmaf(f0, j & 1 ? bf2_high(w[j >> 1]) : bf2_low(w[j >> 1]), -f1 * y[j]);
-            if (!(fabsf(y[j]) < INFINITY)) {
+            if (!(fabsf(y[j]) < kDcMost)) {
               odd = true;
               atomicMin(&first_odd[share * NH + 8 * i + j], t);
               y[j] = 0.f;
@@ -590,7 +669,6 @@ __global__ void __launch_bounds__(dc_threads<NV>()) delta_chunk_kernel(DeltaChun
       fence_async_smem();
       tc_fence_before();
       if (__syncthreads_or(bad)) break;
-      const bool some_odd = odd_flag[ch & 1] != 0;
       if (warp == 0) {
         wait(&t_full, (uint32_t)ch & 1u, 503);
         ++t_seen;
@@ -625,11 +703,16 @@ __global__ void __launch_bounds__(dc_threads<NV>()) delta_chunk_kernel(DeltaChun
 #pragma unroll
         for (int j = 0; j < 8; ++j) u[8 * i + j] = (r[0][j] + r[1][j]) + (r[2][j] + r[3][j]);
       }
-      if (some_odd) {
+      odd = false;
 #pragma unroll
-        for (int j = 0; j < NH; ++j)
-          if (t >= first_odd[share * NH + j]) u[j] = NAN;
+      for (int j = 0; j < NH; ++j) {
+        if (!of_k) u[j] += o[j];
+        if (!(fabsf(u[j]) < kDcMost)) {
+          odd = true;
+          atomicMin(&first_odd[share * NH + j], t);
+        }
       }
+      if (odd) odd_flag[ch & 1] = 1;
       if (tid == 0 && ch + 1 < n_chunks && !bad) {
         load_t(ch + 1);
         ++t_issued;
@@ -643,7 +726,7 @@ __global__ void __launch_bounds__(dc_threads<NV>()) delta_chunk_kernel(DeltaChun
       fence_async_smem();
       tc_fence_before();
       if (__syncthreads_or(bad)) break;
-      if (some_odd && tid < NV) first_odd[tid] = kDcTokens;
+      const bool some_odd = odd_flag[ch & 1] != 0;
       if (warp == 0) {
         tc_fence_after();
         if (elect_one()) {
@@ -665,7 +748,7 @@ __global__ void __launch_bounds__(dc_threads<NV>()) delta_chunk_kernel(DeltaChun
           const int me = share * 64 + t, c = me % 16 * 4;
 #pragma unroll
           for (int j = 0; j < NH; j += 4)
-            *reinterpret_cast<float4*>(tiles + At::o + t * At::o_row + (share * NH + j) * 4) = make_float4(o[j] + u[j], o[j + 1] + u[j + 1], o[j + 2] + u[j + 2], o[j + 3] + u[j + 3]);
+            *reinterpret_cast<float4*>(tiles + At::o + t * At::o_row + (share * NH + j) * 4) = make_float4(u[j], u[j + 1], u[j + 2], u[j + 3]);
           asm volatile("bar.sync 1, %0;" ::"n"(dc_threads<NV>() / 2) : "memory");
           if ((int)blockIdx.z * NV + c < a.Dv) {
 #pragma unroll
@@ -676,7 +759,7 @@ __global__ void __launch_bounds__(dc_threads<NV>()) delta_chunk_kernel(DeltaChun
 #pragma unroll
           for (int j = 0; j < NH; j += 4)
             if (col0 + j < a.Dv)
-              *reinterpret_cast<float4*>(dst + t * stride + share * NH + j) = make_float4(o[j] + u[j], o[j + 1] + u[j + 1], o[j + 2] + u[j + 2], o[j + 3] + u[j + 3]);
+              *reinterpret_cast<float4*>(dst + t * stride + share * NH + j) = make_float4(u[j], u[j + 1], u[j + 2], u[j + 3]);
         }
       }
       wait(&mma_done, phase, 505);
@@ -686,6 +769,16 @@ __global__ void __launch_bounds__(dc_threads<NV>()) delta_chunk_kernel(DeltaChun
       if (tid == 0 && ch + 2 < n_chunks && !bad) {
         load_kq(ch + 2);
         ++kq_issued;
+      }
+      if (some_odd) {  // (the state as the chunk found it, where its pieces were)
+        float* found = reinterpret_cast<float*>(tiles + At::s);
+        if (channel) {
+#pragma unroll
+          for (int j = 0; j < NH; ++j) found[(share * NH + j) * D + row] = s[j];
+        }
+        __syncthreads();
+        dc_by_token<D, NV>(a, found, first_odd, q_start + ch * kDcTokens, min(kDcTokens, q_len - ch * kDcTokens), h, (int)blockIdx.z * NV);
+        __syncthreads();
       }
 #pragma unroll
       for (int i = 0; i < NG; ++i) {
@@ -697,6 +790,16 @@ __global__ void __launch_bounds__(dc_threads<NV>()) delta_chunk_kernel(DeltaChun
 #pragma unroll
           for (int j = 0; j < 8; ++j) s[8 * i + j] = fmaf(whole, s[8 * i + j], (r[0][j] + r[1][j]) + (r[2][j] + r[3][j]));
         }
+      }
+      if (some_odd) {
+        const float* found = reinterpret_cast<const float*>(tiles + At::s);
+        if (channel) {
+#pragma unroll
+          for (int j = 0; j < NH; ++j)
+            if (first_odd[share * NH + j] < kDcTokens) s[j] = found[(share * NH + j) * D + row];
+        }
+        __syncthreads();
+        if (tid < NV) first_odd[tid] = kDcTokens;
       }
     }
     if (tid == 0 && abort_flag) {  // copies still in flight
@@ -721,7 +824,7 @@ static int launch_delta_chunks_as(const DeltaChunkArgs& a, cudaStream_t s) {
   auto prep = delta_prep_kernel<D>;
   auto kern = delta_chunk_kernel<D, NV>;
   constexpr int prep_smem = (int)dc_prep_smem<D>(), smem = DcPlace<NV>::bytes + 1024;
-  static_assert(smem <= 227 * 1024, "shared memory");
+  static_assert(smem <= 227 * 1024 && NV * D * 4 <= (NV == 64 ? 3 : 1) * kDcImage, "shared memory, and room for the state where its pieces lie");
   FTK_REQUIRE(cudaFuncSetAttribute(prep, cudaFuncAttributeMaxDynamicSharedMemorySize, prep_smem) == cudaSuccess &&
                   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess,
               "delta_scan (chunks): cannot set up the kernels");
