@@ -169,6 +169,24 @@ __device__ __forceinline__ void gc_pairs(const float* k, const float* q, const f
   if (on && t < rows) *reinterpret_cast<float2*>(pout + t * prow + 2 * (place & 1)) = make_float2(sums[0], sums[1]);
 }
 
+// An element of a chunk's contribution that is no number as the tensor core has it, as 32-bit fmas: an infinity taken apart into pieces
+// is a NaN, and its product with another number's pieces of both signs is one.  (Such keys and values as they stand at the end of their 16
+// tokens: later decays change no infinity.)
+template <int D, int VT>
+__device__ __noinline__ float gc_contribution(const GcLocal<D, VT>& sh, int d, int j) {
+  const unsigned char* pieces = reinterpret_cast<const unsigned char*>(sh.q) + (d >> 6) * (kGcTokens * 128) + (d & 7) * 2;
+  const unsigned char* values = sh.v + (j >> 6) * (kGcTokens * 128) + (j & 7) * 2;
+  float y = 0.f;
+  for (int t = 0; t < kGcTokens; ++t) {
+    const int at = t * 128 + ((((d >> 3) & 7) ^ (t & 7)) << 4);
+    float k = 0.f;
+    for (int m = 2; m >= 0; --m) k += __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(pieces + m * GcLocal<D, VT>::piece + at));
+    const float v = __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(values + t * 128 + ((((j >> 3) & 7) ^ (t & 7)) << 4)));
+    y = fmaf(fabsf(k) < INFINITY && fabsf(v) < INFINITY ? k : sh.k[t][d], v, y);
+  }
+  return y;
+}
+
 // What bounds it: loads, decays and the pairs' sums on the fma pipe, one after the other between barriers, with two blocks an SM.  The
 // logits come through shared memory so that the decays are a loop of four instead of 32 copies of the code (a block's first pass
 // 38,000 -> 28,000 cycles).  The contribution, as L^T = V^T K, is on tcgen05, keys in three pieces (split3):
@@ -487,8 +505,13 @@ __global__ void __launch_bounds__(2 * D, 256 / D) gla_local_kernel(GlaArgs a) {
       tmem_ld8_start(my_tmem + D + i, r[1]);
       tmem_ld8_finish(r);
 #pragma unroll
-      for (int e = 0; e < 8; ++e)
-        if (j < a.Dv) dst[(size_t)(i + e) * a.Dv] = r[0][e] + r[1][e];
+      for (int e = 0; e < 8; ++e) {
+        if (j >= a.Dv) continue;
+        float y = r[0][e] + r[1][e];
+        if (!(fabsf(y) < INFINITY)) y = gc_contribution<D, VT>(sh, (warp >> 2) * 64 + i + e, j);
+        dst[(size_t)(i + e) * a.Dv] = y;
+      }
+      __syncwarp();
     }
   }
   tc_fence_before();
@@ -615,25 +638,28 @@ __global__ void __launch_bounds__(256, 2) gla_out_kernel(GlaArgs a) {
       }
     };
     const __nv_bfloat16* qb = (const __nv_bfloat16*)a.q + (size_t)(h / a.qk_div) * D;
+    auto load_q8 = [&](int t, int d, float (&y)[8]) {
+      if (!a.a_head) {
+        load8(a.z + ((x.row0 + t) * a.H + h) * D + d, t < n, y);
+      } else if (t < n) {  // one decay for all channels: the queries once more from their rows
+        if (a.rope) gc_rotated8(a, qb + (x.row0 + t) * a.q_stride, x.pos0 + t, d, y);
+        else gc_widen(*reinterpret_cast<const uint4*>(qb + (x.row0 + t) * a.q_stride + d), y);
+      } else {
+        load8(nullptr, false, y);
+      }
+    };
     auto load_q = [&](int st) {
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
-        const int i = tid + 256 * u, t = i >> 3, d = 64 * st + (i & 7) * 8;
-        if (!a.a_head) {
-          load8(a.z + ((x.row0 + t) * a.H + h) * D + d, t < n, qv[u]);
-        } else if (t < n) {  // one decay for all channels: the queries once more from their rows
-          if (a.rope) gc_rotated8(a, qb + (x.row0 + t) * a.q_stride, x.pos0 + t, d, qv[u]);
-          else gc_widen(*reinterpret_cast<const uint4*>(qb + (x.row0 + t) * a.q_stride + d), qv[u]);
-        } else {
-          load8(nullptr, false, qv[u]);
-        }
+        const int i = tid + 256 * u;
+        load_q8(i >> 3, 64 * st + (i & 7) * 8, qv[u]);
       }
     };
     load_s(0);
     load_q(0);
     {
       // The values.  A row of P holds zeros behind its own token, but zero times an infinity or NaN is NaN: such a value goes in as
-      // zero, and its column is NaN from its token on (as its column of the state is).
+      // zero, and its column is summed up once more from its token on.
       const __nv_bfloat16* vb = (const __nv_bfloat16*)a.v + (size_t)h * Dv;
       uint4 w[4];
 #pragma unroll
@@ -782,8 +808,9 @@ __global__ void __launch_bounds__(256, 2) gla_out_kernel(GlaArgs a) {
       __syncwarp();
     }
     wait();
-    const int j = quad * 32 + lane, odd = first_odd[j];
+    const int j = quad * 32 + lane, odd_from = j < Dv ? first_odd[j] : kGcTokens;
     float* o = a.out + (x.row0 * a.H + h) * Dv + j;
+    uint32_t odd = 0u;  // of this thread's 32 tokens those that have no number
 #pragma unroll
     for (int i = 0; i < 32; i += 8) {
       float r[4][8];
@@ -793,9 +820,34 @@ __global__ void __launch_bounds__(256, 2) gla_out_kernel(GlaArgs a) {
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         const int t = half * 32 + i + e;
-        const float y = acc[i + e] + ((r[0][e] + r[1][e]) + (r[2][e] + r[3][e]));
-        if (t < n && j < Dv) o[(size_t)t * row] = t >= odd ? NAN : y;
+        acc[i + e] += (r[0][e] + r[1][e]) + (r[2][e] + r[3][e]);
+        if (t < n && j < Dv && (t >= odd_from || !(fabsf(acc[i + e]) < INFINITY))) odd |= 1u << (i + e);
       }
+    }
+    // Such an output as 32-bit fmas, and up to its own token: an infinity taken apart into pieces is a NaN.  (All of them before one is
+    // stored: P lies where they go.)
+    if (__syncthreads_or(odd != 0u)) {
+      const __nv_bfloat16* vb = (const __nv_bfloat16*)a.v + (size_t)h * Dv + j;
+#pragma unroll 1
+      for (uint32_t rest = odd; rest; rest &= rest - 1) {
+        const int i = __ffs(rest) - 1, t = half * 32 + i;
+        float y = 0.f;
+        for (int d = 0; d < D; d += 8) {
+          float q[8];
+          load_q8(t, d, q);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) y = fmaf(a.a_head ? q[e] * (a.q_scale * dec[t]) : q[e], start[(size_t)(d + e) * Dv + j], y);
+        }
+        for (int s = 0; s <= t; ++s) y = fmaf(pin[(size_t)t * row + s], __bfloat162float(vb[(x.row0 + s) * a.v_stride]), y);
+#pragma unroll
+        for (int e = 0; e < 32; ++e) acc[e] = e == i ? y : acc[e];
+      }
+      __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      const int t = half * 32 + i;
+      if (t < n && j < Dv) o[(size_t)t * row] = acc[i];
     }
   }
   tc_fence_before();
