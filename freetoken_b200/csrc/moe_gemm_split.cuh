@@ -30,7 +30,7 @@ __global__ void __launch_bounds__(kSplitThreads) moe_gemm_split_kernel(const flo
                                                        int K, int N, int w_rows,
                                                        const int32_t* __restrict__ sorted_routes,
                                                        const float* __restrict__ route_weights, int n_routes,
-                                                       int act, float alpha, float limit, float* __restrict__ out) {
+                                                       int act, float alpha, float limit, float* __restrict__ out, bool fours) {
   extern __shared__ unsigned char split_smem[];
   __shared__ uint64_t done[2];
   __shared__ uint32_t tmem_slot;
@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(kSplitThreads) moe_gemm_split_kernel(const flo
 #pragma unroll
         for (int i = 0; i < 4; ++i) y[i] = finish<float, GATED>(acc[j + i], acc[(j + i + 16) & 31], weight, act, alpha, limit);
         const int n = n0 + column(0) + j;
-        if (N % 4 == 0 && n < N) {
+        if (fours && n < N) {
           Vec4<float>::store(o + j, y);
         } else {
 #pragma unroll
@@ -233,7 +233,8 @@ static int launch_moe_gemm_split(const float* x, const float* w, const int32_t* 
   if (grid.y > 65535u) return -1;
   FTK_REQUIRE(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmem) == cudaSuccess,
               "moe_gemm (32 bits): cannot set up the kernel");
-  FTK_LAUNCH(kern, grid, kSplitThreads, kSplitSmem, s, x, w, offsets, n_experts, K, N, w_rows, routes, weights, n_routes, act, alpha, limit, out);
+  const bool fours = N % 4 == 0 && ((uintptr_t)out & 15) == 0;  // (outputs may start anywhere: rows and weights alone decide on this kernel)
+  FTK_LAUNCH(kern, grid, kSplitThreads, kSplitSmem, s, x, w, offsets, n_experts, K, N, w_rows, routes, weights, n_routes, act, alpha, limit, out, fours);
   return 0;
 }
 

@@ -65,3 +65,15 @@ def test_what_three_pieces_do_not_hold(value):
     gu = torch.tensor([float(x[3, 7]) * float(w[0, 5, 7])] * 2)  # (its other products there are zeros)
     want = torch.nn.functional.silu(gu[0]) * gu[1]
     torch.testing.assert_close(got[3, 5].cpu(), want, rtol=1e-5, atol=0.0, equal_nan=True)
+
+
+def test_outputs_may_start_anywhere():
+    """Rows and weights on 16-byte boundaries, outputs one element off: the same numbers, and nothing beside them."""
+    x, w, w2, offsets, routes, weights = problem(128, 64, [70, 0, 6])
+    a, y = products(x, w, w2, offsets, routes, weights)
+    a1, y1 = (torch.full((t.numel() + 2,), 7.0, device=DEV) for t in (a, y))
+    ops.moe_gemm1_act(x, w, offsets, "silu", 1.702, 7.0, a1[1:-1].view(a.shape))
+    ops.moe_gemm2(a, w2, offsets, routes, weights, y1[1:-1].view(y.shape))
+    for got, want in ((a1, a), (y1, y)):
+        assert torch.equal(got[1:-1], want.view(-1)) and got[0] == got[-1] == 7.0
+    assert ops.read_status() == 0
