@@ -663,7 +663,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       const Item it = load_item(p, p.n_items - 1 - w / p.Hkv);
       const int n_tiles = tiles_of(it);
       if (n_tiles == 0) continue;
-      if (!mbar_wait(&q_full, (uint32_t)(qi & 1), abortp)) {
+      if (!all_of_warp(mbar_wait(&q_full, (uint32_t)(qi & 1), abortp))) {
         if (lane == 0) fail(203);
         ok = false;
         break;
@@ -672,7 +672,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         if (j < n_tiles) {
           const int g = g0 + j, st = g & 1, ks = g % kTcStages;  // score buffer, key stage
           const uint32_t par = (g >> 1) & 1;
-          if (!mbar_wait2(&k_full[ks], (uint32_t)(g / kTcStages) & 1u, &s_empty[st], par ^ 1, abortp)) {
+          if (!all_of_warp(mbar_wait2(&k_full[ks], (uint32_t)(g / kTcStages) & 1u, &s_empty[st], par ^ 1, abortp))) {
             if (lane == 0) fail(204);
             ok = false;
             break;
@@ -696,9 +696,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
           const int i = j - 1, g = g0 + i, st = g & 1, vs = g % kTcStages;  // probability buffer, value stage
           const uint32_t par = (g >> 1) & 1;
           // (tied values: the stage's keys have been waited for before the first product)
-          if (!(tied ? mbar_wait(&p_full[st], par, abortp)
-                     : mbar_wait2(&p_full[st], par, &v_full[vs], (uint32_t)(g / kTcStages) & 1u, abortp)) ||
-              (i == 0 && !mbar_wait(&o_free, (uint32_t)(qi & 1) ^ 1u, abortp))) {  // the piece before has read its output
+          if (!all_of_warp((tied ? mbar_wait(&p_full[st], par, abortp)
+                                 : mbar_wait2(&p_full[st], par, &v_full[vs], (uint32_t)(g / kTcStages) & 1u, abortp)) &&
+                           (i != 0 || mbar_wait(&o_free, (uint32_t)(qi & 1) ^ 1u, abortp)))) {  // the piece before has read its output
             if (lane == 0) fail(205);
             ok = false;
             break;

@@ -160,7 +160,7 @@ attention_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
       const int n_tiles = tiles_of(it);
       if (n_tiles == 0) continue;
       const int n_q = it.ntok > tpt ? 2 : 1;
-      if (!mbar_wait(&q_full, (uint32_t)(qi & 1), abortp)) {
+      if (!all_of_warp(mbar_wait(&q_full, (uint32_t)(qi & 1), abortp))) {
         if (lane == 0) fail(303);
         ok = false;
         break;
@@ -169,7 +169,7 @@ attention_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
       // the piece, the queries are given back
       auto scores = [&](int x, int j) -> bool {
         const int g = g0 + j, ks = g % kTc2Stages;
-        if (x == 0 && !mbar_wait(&k_full[ks], (uint32_t)(g / kTc2Stages) & 1u, abortp)) return false;
+        if (x == 0 && !all_of_warp(mbar_wait(&k_full[ks], (uint32_t)(g / kTc2Stages) & 1u, abortp))) return false;
         tc_fence_after();
         if (elect_one()) {
           const uint32_t d = tmem + (uint32_t)(x * kTcKeys);
@@ -191,9 +191,9 @@ attention_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
       // O_x += P_x(j) V(j); the first of a piece waits until the piece before has read its output
       auto product = [&](int x, int j) -> bool {
         const int g = g0 + j, vs = g % kTc2Stages;
-        if (!mbar_wait(&p_full[x], (uint32_t)((gx[x] + j) & 1), abortp)) return false;
+        if (!all_of_warp(mbar_wait(&p_full[x], (uint32_t)((gx[x] + j) & 1), abortp))) return false;
         if (x == 0) {
-          if (!mbar_wait(&v_full[vs], (uint32_t)(g / kTc2Stages) & 1u, abortp)) return false;
+          if (!all_of_warp(mbar_wait(&v_full[vs], (uint32_t)(g / kTc2Stages) & 1u, abortp))) return false;
           const int live = it.ke - (it.kb + j * kTcKeys);  // keys of the request in this tile
           if (live < kTcKeys) {
             // the value rows past the end of the request: zero, whatever the page holds there and
@@ -206,7 +206,7 @@ attention_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             fence_async_smem();
           }
         }
-        if (j == 0 && !mbar_wait(&o_free[x], (uint32_t)(px[x] & 1) ^ 1u, abortp)) return false;
+        if (j == 0 && !all_of_warp(mbar_wait(&o_free[x], (uint32_t)(px[x] & 1) ^ 1u, abortp))) return false;
         __syncwarp();
         tc_fence_after();
         if (elect_one()) {

@@ -156,7 +156,7 @@ attention_tc_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
       const Item it = load_item(p, p.n_items - 1 - w / p.Hkv);
       const int n_tiles = tiles_of(it);
       if (n_tiles == 0) continue;
-      if (!mbar_wait(&q_full, (uint32_t)(qi & 1), abortp)) {
+      if (!all_of_warp(mbar_wait(&q_full, (uint32_t)(qi & 1), abortp))) {
         if (lane == 0) fail(403);
         ok = false;
         break;
@@ -164,7 +164,7 @@ attention_tc_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
       for (int j = 0; j <= n_tiles && ok; ++j) {
         if (j < n_tiles) {
           const int g = g0 + j, s0 = (2 * g) % ring_k, s1 = (2 * g + 1) % ring_k;
-          if (!mbar_wait2(&k_full[s0], (uint32_t)((2 * g) / ring_k) & 1u, &k_full[s1], (uint32_t)((2 * g + 1) / ring_k) & 1u, abortp)) {
+          if (!all_of_warp(mbar_wait2(&k_full[s0], (uint32_t)((2 * g) / ring_k) & 1u, &k_full[s1], (uint32_t)((2 * g + 1) / ring_k) & 1u, abortp))) {
             if (lane == 0) fail(404);
             ok = false;
             break;
@@ -204,7 +204,7 @@ attention_tc_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
           if (there && !tied)
             there = mbar_wait2(&val_full[s0], (uint32_t)((2 * g) / ring_v) & 1u, &val_full[s1], (uint32_t)((2 * g + 1) / ring_v) & 1u, abortp);
           if (there && i == 0) there = mbar_wait(&o_free, (uint32_t)(qi & 1) ^ 1u, abortp);  // the piece before has read its output
-          if (!there) {
+          if (!all_of_warp(there)) {
             if (lane == 0) fail(405);
             ok = false;
             break;

@@ -1,0 +1,29 @@
+"""How the kernels' waits end that something never comes for, and the orders in their sources that no wait may depend on."""
+
+import os
+import re
+
+import pytest
+
+from freetoken_b200.kernels import library, ops
+
+
+def sources():
+    for name in sorted(os.listdir(library.CSRC)):
+        if name.endswith((".cu", ".cuh")):
+            with open(os.path.join(library.CSRC, name)) as f:
+                yield name, re.sub(r"//[^\n]*", "", f.read())
+
+
+def test_what_a_warp_does_together_follows_waits_that_end_alike_for_all_its_lanes():
+    """Lanes of a warp that give up singly would leave the others at elect.sync and tcgen05 instructions without end."""
+    seen = 0
+    for name, text in sources():
+        if not name.startswith("attention_tc"):
+            continue
+        for m in re.finditer(r"mbar_wait2?\(", text):
+            before = text[text.rindex(";", 0, m.start()):m.start()]
+            assert "all_of_warp(" in before or "__all_sync(" in before or "there =" in before, (name, text[m.start() - 80:m.end() + 60])
+            seen += 1
+        assert len(re.findall(r"there =", text)) == 0 or "if (!all_of_warp(there))" in text
+    assert seen > 25
