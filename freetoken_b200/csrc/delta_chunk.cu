@@ -100,8 +100,11 @@ __global__ void __launch_bounds__(256, 2) delta_prep_kernel(DeltaChunkArgs a) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) tmem_alloc(&tmem_slot, kParts * kDcTokens);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
   pdl_wait();
-  pdl_trigger();
+  pdl_trigger();  // (once the block has its columns: delta_chunk_kernel's may take what is left and hold it until this kernel has ended)
   if (warp == 0) {  // which segment's this is
     if (lane == 0) found[0] = -1;
     __syncwarp();
@@ -120,9 +123,7 @@ __global__ void __launch_bounds__(256, 2) delta_prep_kernel(DeltaChunkArgs a) {
       if (before > (int)blockIdx.x) break;
     }
   }
-  tc_fence_before();
   __syncthreads();
-  tc_fence_after();
   const uint32_t tmem = tmem_slot;
   const int seg = found[0];
   if (seg < 0) {

@@ -27,3 +27,16 @@ def test_what_a_warp_does_together_follows_waits_that_end_alike_for_all_its_lane
             seen += 1
         assert len(re.findall(r"there =", text)) == 0 or "if (!all_of_warp(there))" in text
     assert seen > 25
+
+
+def test_tensor_memory_is_allocated_before_the_next_kernel_may_start():
+    """A kernel that comes in early may hold columns until this one ends: this one must not still be waiting for its own."""
+    checked = 0
+    for name, text in sources():
+        for kernel in re.split(r"__global__", text)[1:]:
+            alloc, trigger = re.search(r"\btmem_alloc\(&", kernel), kernel.find("pdl_trigger();")
+            if not alloc or trigger < alloc.start():
+                continue
+            assert "__syncthreads();" in kernel[alloc.start():trigger], (name, kernel[:60])
+            checked += 1
+    assert checked >= 6
