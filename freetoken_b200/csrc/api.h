@@ -440,6 +440,9 @@ int ftk_read_status(int* out);
 // Writes `code` into a status word from the host (unit 0: grouped GEMM, 1: attention), so that a caller's
 // handling of a given-up wait can be tested without any wait running out on the device.
 int ftk_debug_set_status(int unit, int code);
+// A wait on a barrier that nothing arrives at (give_up: and another warp gives up meanwhile): out[0] = 1 if it ended well, out[1] =
+// the nanoseconds it took (out on the device).
+int ftk_debug_lost_wait(int give_up, long long* out, void* stream);
 // 0 sends bfloat16 grouped expert products to the CUDA-core kernels; default 1 (tcgen05).
 int ftk_set_moe_tensor_cores(int enabled);
 int ftk_set_moe_pairs(int enabled);

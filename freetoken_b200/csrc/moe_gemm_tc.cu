@@ -879,3 +879,40 @@ extern "C" int ftk_read_status(int* out) {
   }
   return 0;
 }
+
+namespace ftk {
+// A wait on a barrier that nothing arrives at: how it ends and after how many nanoseconds; with `give_up`, another warp gives up meanwhile.
+__global__ void lost_wait_kernel(int give_up, long long* out) {
+  __shared__ uint64_t bar;
+  __shared__ int abort_flag;
+  if (threadIdx.x == 0) {
+    mbar_init(&bar, 1);
+    abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  if (threadIdx.x >= 32) {
+    if (give_up) {
+      for (int i = 0; i < 100; ++i) __nanosleep(1000);
+      *(volatile int*)&abort_flag = 1;
+    }
+    return;
+  }
+  unsigned long long from, to;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(from));
+  const bool ok = mbar_wait(&bar, 0, &abort_flag);
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(to));
+  if (threadIdx.x == 0) {
+    out[0] = ok;
+    out[1] = (long long)(to - from);
+  }
+}
+}  // namespace ftk
+
+// out [2] on the device: 1 if the wait ended well, and the nanoseconds it took.
+extern "C" int ftk_debug_lost_wait(int give_up, long long* out, void* stream) {
+  FTK_REQUIRE(out, "debug_lost_wait: null pointer");
+  FTK_LAUNCH(lost_wait_kernel, 1, 64, 0, (cudaStream_t)stream, give_up, out);
+  FTK_LAUNCH_CHECK("debug_lost_wait");
+  return 0;
+}

@@ -29,20 +29,29 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
       : "=r"(ok) : "r"(smem_addr(bar)), "r"(parity) : "memory");
   return ok != 0;
 }
+// Asked once, for up to kTryNs: the barrier's unit wakes the thread when it flips.
+constexpr uint32_t kTryNs = 20000;
+__device__ __forceinline__ bool mbar_try(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok) : "r"(smem_addr(bar)), "r"(parity), "r"(kTryNs) : "memory");
+  return ok != 0;
+}
 // Bounded waits: false when the barrier did not flip within the limit (or another role gave up).  The first leaves the asking to the
 // barrier's unit: asked again and again by a tile's softmax threads, it is in the way of products that read shared memory at its full
-// rate (prompt attention 85 -> 81 us, a portion over 32k keys 557 -> 533, the chunks of the delta rule 183 -> 177).
+// rate (prompt attention 85 -> 81 us, a portion over 32k keys 557 -> 533, the chunks of the delta rule 183 -> 177).  Its limit is a time,
+// as a try may last anything up to its own: 2^31 cycles, 1.1 s at 1,965 MHz.
+constexpr uint32_t kWaitCycles = 1u << 31;
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-  for (uint32_t i = 0; i < kSpinLimit / 16; ++i) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(smem_addr(bar)), "r"(parity) : "memory");
-    if (ok) return true;
-    if ((i & 7) == 7 && *abort_flag) return false;
-  }
+  if (mbar_try(bar, parity)) return true;
+  const uint32_t from = (uint32_t)clock();
+  do {
+    if (mbar_try(bar, parity)) return true;
+    if (*abort_flag) return false;
+  } while ((uint32_t)clock() - from < kWaitCycles);
   return false;
 }
 __device__ __forceinline__ bool mbar_wait_spin(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {

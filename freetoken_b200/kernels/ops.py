@@ -47,7 +47,7 @@ long steps and decode steps), 256 (the same with two query tiles per CTA: very l
 from __future__ import annotations
 
 import ctypes
-from typing import Any, Optional, Sequence
+from typing import Any, Optional, Sequence, Tuple
 
 import torch
 
@@ -167,6 +167,7 @@ _SIGNATURES = {
     "ftk_set_moe_tensor_cores": [_i],
     "ftk_set_moe_pairs": [_i],
     "ftk_debug_set_status": [_i, _i],
+    "ftk_debug_lost_wait": [_i, _vp, _vp],
     "ftk_variant_counts": [ctypes.c_char_p, _i, _i],
     "ftk_softcap_f32": [_vp, ctypes.c_longlong, _f, _vp],
     "ftk_postnorm_add_norm": [_vp, _i, _vp, _i, _i, _vp, _vp, _f, _i, _vp, _vp, _f, _i, _vp, _vp, _vp, _i, _i, _vp],
@@ -294,6 +295,15 @@ def debug_set_status(unit: int, code: int) -> None:
     """Write ``code`` into a status word from the host (``unit`` 0: grouped GEMM, 1: attention), as a
     kernel whose bounded wait ran out would have.  For tests of the error path; nothing waits."""
     _check(_lib().ftk_debug_set_status(int(unit), int(code)), "debug_set_status", 0)
+
+
+def debug_lost_wait(give_up: bool) -> Tuple[bool, float]:
+    """A kernel's wait on a barrier that nothing arrives at (``give_up``: and another warp of its block gives up meanwhile): whether
+    it ended well, and the seconds it took.  For tests of the limit."""
+    out = torch.zeros(2, dtype=torch.int64, device="cuda")
+    _check(_lib().ftk_debug_lost_wait(int(give_up), out.data_ptr(), _stream()), "debug_lost_wait")
+    ok, ns = out.tolist()
+    return bool(ok), ns * 1e-9
 
 
 def set_moe_tensor_cores(enabled: bool) -> None:

@@ -40,3 +40,12 @@ def test_tensor_memory_is_allocated_before_the_next_kernel_may_start():
             assert "__syncthreads();" in kernel[alloc.start():trigger], (name, kernel[:60])
             checked += 1
     assert checked >= 6
+
+
+@pytest.mark.gpu
+def test_a_lost_wait_ends_within_its_limit():
+    ok, seconds = ops.debug_lost_wait(False)
+    # 2^31 cycles at 1,965 MHz are 1.09 s, at half of that clock 2.2 s; and one try more
+    assert not ok and 1.0 < seconds < 3.0, seconds
+    ok, seconds = ops.debug_lost_wait(True)
+    assert not ok and 1e-4 <= seconds < 0.01, seconds
