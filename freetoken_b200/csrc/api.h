@@ -437,8 +437,8 @@ int ftk_moe_combine(const void* y, int dtype, const int32_t* route_pos, int n_to
 // Kernel forms launched so far, as "name<TAB>count" lines (see ftk::note_variant); returns the bytes needed.
 int ftk_variant_counts(char* buf, int cap, int reset);
 int ftk_read_status(int* out);
-// Writes `code` into a status word from the host (unit 0: grouped GEMM, 1: attention), so that a caller's
-// handling of a given-up wait can be tested without any wait running out on the device.
+// Writes `code` into a status word from the host (unit 0: grouped GEMM, 1: attention, 2: the delta rule's chunks, 3: linear attention's,
+// 4: 32-bit products), so that a caller's handling of a given-up wait can be tested without any wait running out on the device.
 int ftk_debug_set_status(int unit, int code);
 // A wait on a barrier that nothing arrives at (give_up: and another warp gives up meanwhile): out[0] = 1 if it ended well, out[1] =
 // the nanoseconds it took (out on the device).

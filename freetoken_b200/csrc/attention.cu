@@ -1171,23 +1171,10 @@ static int launch_bf16(const AttnParams& p, cudaStream_t s) {
 
 using namespace ftk;
 
-// Status of the tensor-core attention kernel's bounded waits (merged into ftk_read_status).
-int ftk_attention_tc_status(int* out) {
-  int host[4] = {0, 0, 0, 0};
-  if (cudaMemcpyFromSymbol(host, g_attn_status, sizeof(host)) != cudaSuccess) return 2;
-  out[0] = host[0];
-  out[1] = host[1];
-  if (host[0]) {
-    int zero[4] = {0, 0, 0, 0};
-    cudaMemcpyToSymbol(g_attn_status, zero, sizeof(zero));
-  }
-  return 0;
-}
-
-int ftk_attention_tc_set_status(int code) {
-  int host[4] = {code, -1, 0, 0};
-  return cudaMemcpyToSymbol(g_attn_status, host, sizeof(host)) == cudaSuccess ? 0 : 2;
-}
+namespace ftk {
+int attention_tc_status(int* out) { return take_status(g_attn_status, out); }  // (merged into ftk_read_status)
+int attention_tc_set_status(int code) { return set_status(g_attn_status, code); }
+}  // namespace ftk
 
 extern "C" int ftk_attention_tc_fits(int head_dim, int page_size, int group) {
   return attention_tc_fits(head_dim, page_size, group) ? 1 : 0;

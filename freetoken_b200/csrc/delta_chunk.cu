@@ -845,18 +845,8 @@ static int launch_delta_chunks(const DeltaChunkArgs& a, cudaStream_t s) {
   return rounds(64) * (3 + 5 * pairs) < rounds(16) * 3 * pairs ? launch_delta_chunks_as<D, 64>(a, s) : launch_delta_chunks_as<D, 16>(a, s);
 }
 
-// What the bounded waits recorded (merged into ftk_read_status).
-int delta_chunk_status(int* out) {
-  int host[4] = {0, 0, 0, 0};
-  if (cudaMemcpyFromSymbol(host, g_delta_status, sizeof(host)) != cudaSuccess) return 2;
-  out[0] = host[0];
-  out[1] = host[1];
-  if (host[0]) {
-    int zero[4] = {0, 0, 0, 0};
-    cudaMemcpyToSymbol(g_delta_status, zero, sizeof(zero));
-  }
-  return 0;
-}
+int delta_chunk_status(int* out) { return take_status(g_delta_status, out); }  // (merged into ftk_read_status)
+int delta_chunk_set_status(int code) { return set_status(g_delta_status, code); }
 
 }  // namespace ftk
 

@@ -883,18 +883,8 @@ static int launch_gla_chunks_as(const GlaArgs& a, cudaStream_t s) {
   return 0;
 }
 
-// What the bounded waits recorded (merged into ftk_read_status).
-int gla_chunks_status(int* out) {
-  int host[4] = {0, 0, 0, 0};
-  if (cudaMemcpyFromSymbol(host, g_gla_status, sizeof(host)) != cudaSuccess) return 2;
-  out[0] = host[0];
-  out[1] = host[1];
-  if (host[0]) {
-    int zero[4] = {0, 0, 0, 0};
-    cudaMemcpyToSymbol(g_gla_status, zero, sizeof(zero));
-  }
-  return 0;
-}
+int gla_chunks_status(int* out) { return take_status(g_gla_status, out); }  // (merged into ftk_read_status)
+int gla_chunks_set_status(int code) { return set_status(g_gla_status, code); }
 
 inline int launch_gla_chunks(const GlaArgs& a, cudaStream_t s) {
   return a.D == 128 ? launch_gla_chunks_as<128, 2>(a, s) : a.Dv <= 64 ? launch_gla_chunks_as<64, 1>(a, s) : launch_gla_chunks_as<64, 2>(a, s);

@@ -238,17 +238,7 @@ static int launch_moe_gemm_split(const float* x, const float* w, const int32_t* 
   return 0;
 }
 
-// What the bounded waits recorded (merged into ftk_read_status).
-int moe_gemm_split_status(int* out) {
-  int host[4] = {0, 0, 0, 0};
-  if (cudaMemcpyFromSymbol(host, g_split_status, sizeof(host)) != cudaSuccess) return 2;
-  out[0] = host[0];
-  out[1] = host[1];
-  if (host[0]) {
-    int zero[4] = {0, 0, 0, 0};
-    cudaMemcpyToSymbol(g_split_status, zero, sizeof(zero));
-  }
-  return 0;
-}
+int moe_gemm_split_status(int* out) { return take_status(g_split_status, out); }  // (merged into ftk_read_status)
+int moe_gemm_split_set_status(int code) { return set_status(g_split_status, code); }
 
 }  // namespace ftk

@@ -819,63 +819,48 @@ int ftk_moe_gemm2_tc(const void* a, const void* w2, const int32_t* expert_offset
   return run_tc<false>(a, inter, w2, hidden, p, stream, "moe_gemm2 (tcgen05)");
 }
 
-// Status of the bounded waits: out[0] = first code recorded since the last call (0 = none),
-// out[1] = block, then cleared.  Synchronises with the device.
-int ftk_attention_tc_status(int* out);       // attention.cu
-int ftk_attention_tc_set_status(int code);  // attention.cu
+// The files' status words: attention's, the delta rule's chunks', linear attention's, the 32-bit products', and this file's (looked at in
+// this order).
 namespace ftk {
-int delta_chunk_status(int* out);  // delta_chunk.cu
-int gla_chunks_status(int* out);   // gla_chunks.cuh
+int attention_tc_status(int* out);    // attention.cu
+int delta_chunk_status(int* out);     // delta_chunk.cu
+int gla_chunks_status(int* out);      // gla_chunks.cuh
 int moe_gemm_split_status(int* out);  // moe_gemm_split.cuh
+int attention_tc_set_status(int code);
+int delta_chunk_set_status(int code);
+int gla_chunks_set_status(int code);
+int moe_gemm_split_set_status(int code);
+static int moe_gemm_tc_status(int* out) { return take_status(g_status, out); }
+static int moe_gemm_tc_set_status(int code) { return set_status(g_status, code); }
 }  // namespace ftk
 
 // Writes a code into a status word from the host, as a kernel whose wait ran out would: unit 0 = the
-// grouped GEMM's word, 1 = the attention kernel's.  It exists so that the path from a status word to the
-// caller's error can be exercised without making any wait on the device run out.
+// grouped GEMM's word, 1 = the attention kernel's, 2 = the delta rule's, 3 = linear attention's, 4 = the 32-bit products'.  It exists
+// so that the path from a status word to the caller's error can be exercised without making any wait on the device run out.
 extern "C" int ftk_debug_set_status(int unit, int code) {
-  if (unit == 1) {
-    if (ftk_attention_tc_set_status(code) != 0) {
-      set_error("debug_set_status: cannot write the attention status word");
-      return 2;
-    }
-    return 0;
-  }
-  if (unit != 0) {
-    set_error("debug_set_status: unit must be 0 (grouped GEMM) or 1 (attention), got %d", unit);
+  int (*const set[])(int) = {ftk::moe_gemm_tc_set_status, ftk::attention_tc_set_status, ftk::delta_chunk_set_status, ftk::gla_chunks_set_status,
+                             ftk::moe_gemm_split_set_status};
+  constexpr int n = sizeof(set) / sizeof(set[0]);
+  if (unit < 0 || unit >= n) {
+    set_error("debug_set_status: unit must be 0 to %d, got %d", n - 1, unit);
     return 1;
   }
-  int host[4] = {code, -1, 0, 0};
-  if (cudaMemcpyToSymbol(g_status, host, sizeof(host)) != cudaSuccess) {
-    set_error("debug_set_status: cannot write the status words");
+  if (set[unit](code) != 0) {
+    set_error("debug_set_status: cannot write the status word of unit %d", unit);
     return 2;
   }
   return 0;
 }
 
+// Status of the bounded waits: out[0] = first code recorded since the last call (0 = none),
+// out[1] = block, then cleared.  Synchronises with the device.
 extern "C" int ftk_read_status(int* out) {
-  int attn[2] = {0, 0};
-  if (ftk_attention_tc_status(attn) == 0 && attn[0]) {
-    out[0] = attn[0];
-    out[1] = attn[1];
-    return 0;
-  }
-  for (auto read : {ftk::delta_chunk_status, ftk::gla_chunks_status, ftk::moe_gemm_split_status}) {
-    if (read(attn) == 0 && attn[0]) {
-      out[0] = attn[0];
-      out[1] = attn[1];
-      return 0;
+  for (auto read : {ftk::attention_tc_status, ftk::delta_chunk_status, ftk::gla_chunks_status, ftk::moe_gemm_split_status, ftk::moe_gemm_tc_status}) {
+    if (read(out) != 0) {
+      set_error("read_status: cannot read the status words");
+      return 2;
     }
-  }
-  int host[4] = {0, 0, 0, 0};
-  if (cudaMemcpyFromSymbol(host, g_status, sizeof(host)) != cudaSuccess) {
-    set_error("read_status: cannot read the status words");
-    return 2;
-  }
-  out[0] = host[0];
-  out[1] = host[1];
-  if (host[0]) {
-    int zero[4] = {0, 0, 0, 0};
-    cudaMemcpyToSymbol(g_status, zero, sizeof(zero));
+    if (out[0]) return 0;
   }
   return 0;
 }

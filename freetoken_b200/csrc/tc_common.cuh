@@ -8,6 +8,25 @@ namespace ftk {
 
 constexpr uint32_t kSpinLimit = 1u << 22;
 
+// ---------------------------------------------------------------- status words
+// What a file's bounded waits record, in a __device__ int[4] of its own: [0] the first error code, [1] the block that left it; 0 = fine.
+// Read and cleared, or written as such a wait would; 0 or 2 (the word cannot be reached).
+template <typename Word>
+int take_status(Word& word, int* out) {
+  int host[4] = {0, 0, 0, 0};
+  if (cudaMemcpyFromSymbol(host, word, sizeof(host)) != cudaSuccess) return 2;
+  out[0] = host[0];
+  out[1] = host[1];
+  if (!host[0]) return 0;
+  const int zero[4] = {0, 0, 0, 0};
+  return cudaMemcpyToSymbol(word, zero, sizeof(zero)) == cudaSuccess ? 0 : 2;
+}
+template <typename Word>
+int set_status(Word& word, int code) {
+  const int host[4] = {code, -1, 0, 0};
+  return cudaMemcpyToSymbol(word, host, sizeof(host)) == cudaSuccess ? 0 : 2;
+}
+
 // ---------------------------------------------------------------- PTX wrappers
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 

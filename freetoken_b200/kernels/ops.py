@@ -292,8 +292,9 @@ def variant_counts(reset: bool = False) -> dict:
 
 
 def debug_set_status(unit: int, code: int) -> None:
-    """Write ``code`` into a status word from the host (``unit`` 0: grouped GEMM, 1: attention), as a
-    kernel whose bounded wait ran out would have.  For tests of the error path; nothing waits."""
+    """Write ``code`` into a status word from the host (``unit`` 0: grouped GEMM, 1: attention, 2: the delta rule's chunks, 3: gated
+    linear attention's, 4: 32-bit products), as a kernel whose bounded wait ran out would have.  For tests of the error path;
+    nothing waits."""
     _check(_lib().ftk_debug_set_status(int(unit), int(code)), "debug_set_status", 0)
 
 

@@ -49,3 +49,13 @@ def test_a_lost_wait_ends_within_its_limit():
     assert not ok and 1.0 < seconds < 3.0, seconds
     ok, seconds = ops.debug_lost_wait(True)
     assert not ok and 1e-4 <= seconds < 0.01, seconds
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("unit,code", [(0, 101), (1, 201), (2, 501), (3, 601), (4, 701)])
+def test_every_status_word_is_read_and_cleared(unit, code):
+    assert ops.read_status() == 0
+    ops.debug_set_status(unit, code)
+    with pytest.raises(ops.KernelError, match=f"status {code}"):
+        ops.check_status()
+    assert ops.read_status() == 0
