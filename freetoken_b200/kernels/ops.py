@@ -792,13 +792,26 @@ def linear_split(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
     _check(_lib().ftk_linear_split(_dev(x, "x", f32), _dev(w, "w", f32), _dev(out, "out", f32), T, N, K, _stream()), "linear_split")
 
 
+SPLIT_TILE = 128  # rows and columns of a tile of :func:`linear_split`
+SPLIT_MOST_ROWS = 65535 * SPLIT_TILE
+
+
+def split_pays(n_rows: int, n_out: int, k: int) -> bool:
+    """Whether :func:`linear_split` takes a product of these sizes, and sooner than the library's.
+
+    Its tiles of 128 x 128 run one on each of 148 SMs at a time.  A single round of them wins from 48 rows and 600,000 results on: 1,024 of k,
+    library and tiles, 512 x 1,536 50 and 39 us, 861 x 1,024 50 and 38, 64 x 8,192 42 and 34; 64 of k, 48 x 12,500 11 and 7.5.
+    Several rounds take 6.6 us each and 1.6 per 64 of k; the library's 33 TFLOP/s are the estimate of it, which narrow or short products
+    stay behind: 600,000 x 8 x 64 100 and 155, 75,000 x 32 x 128 24 and 28, 100,000 x 129 x 128 121 and 127, 8,192 x 1,024 x 16 21 and
+    32; with more of k or of columns 100,000 x 129 x 256 201 and 159, 8,192 x 8,192 x 64 228 and 221, 2,048 x 8,192 x 1,024 628 and 228."""
+    if n_rows < 48 or n_rows * n_out < 600000 or k % 4 or n_rows > SPLIT_MOST_ROWS:
+        return False
+    rounds = -(-(-(-n_rows // SPLIT_TILE) * -(-n_out // SPLIT_TILE)) // 148)
+    return rounds == 1 or 3.0 + rounds * (6.6 + 1.6 * -(-k // 64)) < 5.0 + 2.0 * n_rows * n_out * k / 33e6
+
+
 def _split_pays(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> bool:
-    """Whether :func:`linear_split` takes a product, and sooner than the library's: tiles of 128 x 128 take 2 us per 64 of k, one on
-    each SM at a time, and the library's 33 TFLOP/s are behind from about 600,000 results on.  Library and tiles, 1,024 of k: 256 x
-    1,536 36 and 39 us, 512 x 1,536 50 and 39, 861 x 1,536 81 and 39, 861 x 1,024 50 and 38, 64 x 8,192 42 and 34, 2,048 x 8,192 628
-    and 228; 6,144 of k, 192 x 3,072 179 and 164; 256 of k, 2,048 x 256 15 and 18."""
-    T, K = x.shape
-    return (T >= 48 and T * w.shape[0] >= 600000 and K % 4 == 0 and x.dtype == w.dtype == out.dtype == torch.float32
+    return (x.dtype == w.dtype == out.dtype == torch.float32 and split_pays(x.shape[0], w.shape[0], x.shape[1])
             and x.is_cuda and x.is_contiguous() and w.is_contiguous() and out.is_contiguous()
             and (x.data_ptr() | w.data_ptr() | out.data_ptr()) % 16 == 0)
 
