@@ -280,12 +280,15 @@ int ftk_delta_scan(const void* q, long long q_stride, const void* k, long long k
 // The same for portions of bfloat16 prompts in chunks of 32 tokens, two at a time (one decay a head, keys of 64 or 128 channels, value channels in
 // multiples of 16): of the n_segs requests the n_long that bring long_from tokens and more; the others go token by token, in a
 // launch before.  ftk_delta_chunk_scratch says how many bytes of scratch n_long requests take, 0 where the sizes are not taken.
+// passes (host memory, or null for one over everything): with less scratch, what is worked on one after the other, five numbers each:
+// the first of the long requests and how many, rows of 64 tokens from .. to of each of them, and how many rows that is together.
 long long ftk_delta_chunk_scratch(int dtype, int n_tokens, int n_long, int n_heads, int n_kv_heads, int dim, int vdim);
 int ftk_delta_scan_chunks(const void* q, long long q_stride, const void* k, long long k_stride, const void* v, long long v_stride,
                           const void* b, long long b_stride, const void* a, long long a_stride, int dtype, const float* a_log,
                           const float* dt_bias, float q_scale, float unit_eps, float* state, int n_slots, const int32_t* state_slots,
                           const int32_t* seg_info, int n_segs, float* out, int n_tokens, int n_heads, int n_kv_heads, int dim,
-                          int vdim, int long_from, int n_long, void* scratch, long long scratch_bytes, void* stream);
+                          int vdim, int long_from, int n_long, const int32_t* passes, int n_passes, void* scratch,
+                          long long scratch_bytes, void* stream);
 // (z [n_tokens, n_heads * dim] float32 instead of a: logits of one decay per head and key channel; dt_bias is then
 // [n_heads * dim].  When a segment has several tokens z is overwritten with the decays.)
 // Short causal convolution over time with a residual (shortconv.cu): out[t, c] = x[t, c] + sum_j w[c, j] *

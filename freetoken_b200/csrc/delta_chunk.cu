@@ -51,14 +51,20 @@ struct DeltaChunkArgs {
   const int32_t* state_slots; const int32_t* seg_info; int n_segs;
   float* out; int n_tokens, H, G, D, Dv;
   unsigned char* scratch; long long row_bytes;
-  int long_from, n_long, n_chunks;  // requests of long_from tokens and more go in chunks: n_long of them; the rows (of 64 tokens) that scratch holds
+  int long_from, n_chunks;  // requests of long_from tokens and more go in chunks; the rows (of 64 tokens) that scratch holds
+  int first_req, n_req, row0, row1;  // of those requests this pass's, and which rows of each
 };
 
-// rows of 64 tokens of a segment; 0 for one that the kernels leave alone
+// rows of 64 tokens of a segment; 0 for one that no pass takes
 __device__ __forceinline__ int dc_chunks(const DeltaChunkArgs& a, int seg) {
   const int q_start = a.seg_info[seg * 4], q_len = a.seg_info[seg * 4 + 1], kv_len = a.seg_info[seg * 4 + 2];
   if (q_len < a.long_from || q_start < 0 || q_start + q_len > a.n_tokens || kv_len < q_len) return 0;
   return (q_len + kDcTokens - 1) / kDcTokens;
+}
+
+// Of those the pass's: `rows` of the `index`-th request that goes in chunks.
+__device__ __forceinline__ int dc_pass_rows(const DeltaChunkArgs& a, int rows, int index) {
+  return rows > 0 && index >= a.first_req && index < a.first_req + a.n_req ? max(0, min(rows, a.row1) - a.row0) : 0;
 }
 
 // Four warps a head, two heads a block: shared memory of one
@@ -108,9 +114,12 @@ __global__ void __launch_bounds__(256, 2) delta_prep_kernel(DeltaChunkArgs a) {
   if (warp == 0) {  // which segment's this is
     if (lane == 0) found[0] = -1;
     __syncwarp();
-    int before = 0;
+    int before = 0, requests = 0;
     for (int i0 = 0; i0 < a.n_segs; i0 += 32) {
-      const int n = i0 + lane < a.n_segs ? dc_chunks(a, i0 + lane) : 0;
+      const int all = i0 + lane < a.n_segs ? dc_chunks(a, i0 + lane) : 0;
+      const unsigned some = __ballot_sync(0xffffffffu, all > 0);
+      const int n = dc_pass_rows(a, all, requests + __popc(some & ((1u << lane) - 1u)));
+      requests += __popc(some);
       int upto = n;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -118,7 +127,7 @@ __global__ void __launch_bounds__(256, 2) delta_prep_kernel(DeltaChunkArgs a) {
         if (lane >= o) upto += v;
       }
       const int t = (int)blockIdx.x - before - (upto - n);
-      if (t >= 0 && t < n) { found[0] = i0 + lane; found[1] = t; }
+      if (t >= 0 && t < n) { found[0] = i0 + lane; found[1] = a.row0 + t; }
       before += __shfl_sync(0xffffffffu, upto, 31);
       if (before > (int)blockIdx.x) break;
     }
@@ -509,13 +518,15 @@ __global__ void __launch_bounds__(dc_threads<NV>()) delta_chunk_kernel(const __g
   pdl_trigger();
   const uint32_t tmem = tmem_slot, my_tmem = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(share * NH);
   const int h = blockIdx.y, col0 = blockIdx.z * NV + share * NH;
-  // the block's request: the blockIdx.x-th of those that go in chunks (every warp looks for it)
-  int seg = -1, n_chunks = 0, before = 0, left = blockIdx.x;  // before: rows of the requests in front of it
+  // the block's request: the blockIdx.x-th of the pass's (every warp looks for it)
+  int seg = -1, n_chunks = 0, before = 0, left = a.first_req + blockIdx.x, requests = 0;  // before: rows of the requests in front of it
   for (int i0 = 0; i0 < a.n_segs && seg < 0; i0 += 32) {
-    const int n = i0 + lane < a.n_segs ? dc_chunks(a, i0 + lane) : 0;
-    const unsigned some = __ballot_sync(0xffffffffu, n > 0);
+    const int all = i0 + lane < a.n_segs ? dc_chunks(a, i0 + lane) : 0;
+    const unsigned some = __ballot_sync(0xffffffffu, all > 0);
+    const int n = dc_pass_rows(a, all, requests + __popc(some & ((1u << lane) - 1u)));
     const int at = left < __popc(some) ? (int)__fns(some, 0, left + 1) : 32;  // its lane
     left -= __popc(some);
+    requests += __popc(some);
     int sum = lane < at ? n : 0;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
@@ -530,7 +541,9 @@ __global__ void __launch_bounds__(dc_threads<NV>()) delta_chunk_kernel(const __g
   const int slot = n_chunks ? a.state_slots[seg] : -1;
   if (slot < 0 || slot >= a.n_slots) n_chunks = 0;
   if (n_chunks) {
-    const int q_start = a.seg_info[seg * 4], q_len = a.seg_info[seg * 4 + 1], kv_len = a.seg_info[seg * 4 + 2];
+    // (of the request's tokens those that no pass before has taken; what they left in the slot goes on)
+    const int q_start = a.seg_info[seg * 4] + a.row0 * kDcTokens, q_len = a.seg_info[seg * 4 + 1] - a.row0 * kDcTokens;
+    const bool fresh = a.row0 == 0 && a.seg_info[seg * 4 + 2] == a.seg_info[seg * 4 + 1];
     const unsigned char* rows = a.scratch + (size_t)before * a.row_bytes;
     const unsigned char* kq_src = rows + (size_t)(h / (a.H / a.G)) * (D / 64) * kDcImage;
     const unsigned char* head_src = rows + (size_t)a.G * (D / 64) * kDcImage + (size_t)h * kDcHeadBytes;
@@ -570,7 +583,7 @@ __global__ void __launch_bounds__(dc_threads<NV>()) delta_chunk_kernel(const __g
     float* sta = a.state + (((size_t)slot * a.H + h) * a.Dv + col0) * D + row;
     float s[NH];
 #pragma unroll
-    for (int j = 0; j < NH; ++j) s[j] = channel && kv_len != q_len && col0 + j < a.Dv ? sta[(size_t)j * D] : 0.f;
+    for (int j = 0; j < NH; ++j) s[j] = channel && !fresh && col0 + j < a.Dv ? sta[(size_t)j * D] : 0.f;
     // eight columns as three pieces into row `r` of an operand
     auto put = [&](int at, int piece, int r, int i, const float (&x)[8]) {
       uint4 w[3];
@@ -831,7 +844,7 @@ static int launch_delta_chunks_as(const DeltaChunkArgs& a, cudaStream_t s) {
               "delta_scan (chunks): cannot set up the kernels");
   FTK_LAUNCH(prep, dim3(a.n_chunks, a.G, (a.H / a.G + 1) / 2), 256, prep_smem, s, a);
   FTK_LAUNCH_CHECK("delta_scan (chunks, triangles)");
-  FTK_LAUNCH(kern, dim3(a.n_long, a.H, (a.Dv + NV - 1) / NV), dc_threads<NV>(), smem, s, a);
+  FTK_LAUNCH(kern, dim3(a.n_req, a.H, (a.Dv + NV - 1) / NV), dc_threads<NV>(), smem, s, a);
   FTK_LAUNCH_CHECK("delta_scan (chunks)");
   return 0;
 }
@@ -839,9 +852,9 @@ static int launch_delta_chunks_as(const DeltaChunkArgs& a, cudaStream_t s) {
 // Columns a block: by the rounds of blocks over the SMs and what a pair of chunks takes, 3.0 us with 16 columns, 5.0 with 64 (and 3 more
 // a block).  16 heads of 128 columns, 2,048 tokens: 123 us with 16 (128 blocks); 48 heads 228 with 64 (96 blocks), three rounds with 16.
 template <int D>
-static int launch_delta_chunks(const DeltaChunkArgs& a, cudaStream_t s) {
-  const long long pairs = max(1, a.n_tokens / kDcTokens / a.n_long);  // (of a request, about)
-  auto rounds = [&](int cols) { return ((long long)a.n_long * a.H * ((a.Dv + cols - 1) / cols) + 147) / 148; };
+static int launch_delta_chunks(const DeltaChunkArgs& a, int tokens, cudaStream_t s) {  // tokens: of the pass, about
+  const long long pairs = max(1, tokens / kDcTokens / a.n_req);  // (of a request, about)
+  auto rounds = [&](int cols) { return ((long long)a.n_req * a.H * ((a.Dv + cols - 1) / cols) + 147) / 148; };
   return rounds(64) * (3 + 5 * pairs) < rounds(16) * 3 * pairs ? launch_delta_chunks_as<D, 64>(a, s) : launch_delta_chunks_as<D, 16>(a, s);
 }
 
@@ -864,15 +877,25 @@ extern "C" int ftk_delta_scan_chunks(const void* q, long long q_stride, const vo
                                      long long v_stride, const void* b, long long b_stride, const void* a, long long a_stride,
                                      int dtype, const float* a_log, const float* dt_bias, float q_scale, float unit_eps, float* state,
                                      int n_slots, const int32_t* state_slots, const int32_t* seg_info, int n_segs, float* out,
-                                     int n_tokens, int n_heads, int n_kv_heads, int dim, int vdim, int long_from, int n_long, void* scratch,
-                                     long long scratch_bytes, void* stream) {
+                                     int n_tokens, int n_heads, int n_kv_heads, int dim, int vdim, int long_from, int n_long,
+                                     const int32_t* passes, int n_passes, void* scratch, long long scratch_bytes, void* stream) {
   FTK_REQUIRE(long_from >= 1 && n_long >= 1 && n_long <= n_segs, "delta_scan (chunks): %d of %d requests of %d tokens and more", n_long,
               n_segs, long_from);
   const long long need = ftk_delta_chunk_scratch(dtype, n_tokens, n_long, n_heads, n_kv_heads, dim, vdim);
   FTK_REQUIRE(need > 0, "delta_scan (chunks): type %d, heads of %d x %d, %d tokens are not taken", dtype, dim, vdim, n_tokens);
   FTK_REQUIRE(q && k && v && b && a && a_log && dt_bias && state && state_slots && seg_info && out && scratch,
               "delta_scan (chunks): null pointer");
-  FTK_REQUIRE(scratch_bytes >= need, "delta_scan (chunks): %lld bytes of scratch, %lld needed", scratch_bytes, need);
+  const long long row_bytes = dc_row_bytes(n_heads, n_kv_heads, dim);
+  if (!passes) {  // one, of all rows
+    n_passes = 1;
+    FTK_REQUIRE(scratch_bytes >= need, "delta_scan (chunks): %lld bytes of scratch, %lld needed", scratch_bytes, need);
+  }
+  FTK_REQUIRE(n_passes >= 1, "delta_scan (chunks): no pass");
+  for (int i = 0; passes && i < n_passes; ++i) {
+    const int32_t* p = passes + 5 * i;
+    FTK_REQUIRE(p[0] >= 0 && p[1] >= 1 && p[1] <= n_long - p[0] && p[2] >= 0 && p[3] > p[2] && p[4] >= 1 && p[4] * row_bytes <= scratch_bytes,
+                "delta_scan (chunks): a pass of %d rows (%d to %d of %d requests from the %d-th on)", p[4], p[2], p[3], p[1], p[0]);
+  }
   FTK_REQUIRE((q_stride | k_stride | v_stride) % 8 == 0 &&
                   (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)scratch | (uintptr_t)out) & 15) == 0,
               "delta_scan (chunks): rows, outputs and scratch on 16-byte boundaries");
@@ -883,8 +906,8 @@ extern "C" int ftk_delta_scan_chunks(const void* q, long long q_stride, const vo
   d.a_log = a_log; d.dt_bias = dt_bias; d.q_scale = q_scale; d.unit_eps = unit_eps;
   d.state = state; d.n_slots = n_slots; d.state_slots = state_slots; d.seg_info = seg_info; d.n_segs = n_segs;
   d.out = out; d.n_tokens = n_tokens; d.H = n_heads; d.G = n_kv_heads; d.D = dim; d.Dv = vdim;
-  d.scratch = (unsigned char*)scratch; d.row_bytes = dc_row_bytes(n_heads, n_kv_heads, dim);
-  d.long_from = long_from; d.n_long = n_long; d.n_chunks = n_tokens / kDcTokens + n_long;
+  d.scratch = (unsigned char*)scratch; d.row_bytes = row_bytes;
+  d.long_from = long_from;
   if (n_long < n_segs) {
     const int rc = delta_scan_tokens(q, q_stride, k, k_stride, v, v_stride, b, b_stride, a, a_stride, nullptr, dtype, a_log, dt_bias, q_scale,
                                      unit_eps, state, n_slots, state_slots, seg_info, n_segs, out, n_tokens, n_heads, n_kv_heads, dim, vdim,
@@ -892,5 +915,13 @@ extern "C" int ftk_delta_scan_chunks(const void* q, long long q_stride, const vo
     if (rc) return rc;
   }
   note_variant("delta rule: chunks of 32 tokens");
-  return dim == 64 ? launch_delta_chunks<64>(d, (cudaStream_t)stream) : launch_delta_chunks<128>(d, (cudaStream_t)stream);
+  for (int i = 0; i < n_passes; ++i) {
+    const int32_t whole[5] = {0, n_long, 0, 0x7fffffff, n_tokens / kDcTokens + n_long};
+    const int32_t* p = passes ? passes + 5 * i : whole;
+    const int tokens = passes ? p[4] * kDcTokens : n_tokens;
+    d.first_req = p[0]; d.n_req = p[1]; d.row0 = p[2]; d.row1 = p[3]; d.n_chunks = p[4];
+    const int rc = dim == 64 ? launch_delta_chunks<64>(d, tokens, (cudaStream_t)stream) : launch_delta_chunks<128>(d, tokens, (cudaStream_t)stream);
+    if (rc) return rc;
+  }
+  return 0;
 }

@@ -187,7 +187,7 @@ _SIGNATURES = {
     "ftk_hyper_step": [_vp, ctypes.c_longlong, _i, _i, _i, _vp, _vp, _i, _vp, _vp, _vp, _vp, _f, _vp, _i, _vp, _vp],
     "ftk_conv_act": [_vp, ctypes.c_longlong, _i, _vp, _vp, _i, _i, _vp, _i, _vp, _vp, _i, _vp, _i, _i, _vp],
     "ftk_delta_scan_chunks": [_vp, ctypes.c_longlong, _vp, ctypes.c_longlong, _vp, ctypes.c_longlong, _vp, ctypes.c_longlong,
-                              _vp, ctypes.c_longlong, _i, _vp, _vp, _f, _f, _vp, _i, _vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _i, _vp,
+                              _vp, ctypes.c_longlong, _i, _vp, _vp, _f, _f, _vp, _i, _vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _i, _vp, _i, _vp,
                               ctypes.c_longlong, _vp],
     "ftk_delta_scan": [_vp, ctypes.c_longlong, _vp, ctypes.c_longlong, _vp, ctypes.c_longlong, _vp, ctypes.c_longlong,
                        _vp, ctypes.c_longlong, _vp, _i, _vp, _vp, _f, _f, _vp, _i, _vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _vp],
@@ -1691,7 +1691,7 @@ def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, b_raw: torch.T
                a_log: torch.Tensor, dt_bias: torch.Tensor, q_scale: float, unit_eps: float, state: torch.Tensor,
                state_slots: torch.Tensor, seg_info: torch.Tensor, n_segs: int, out: torch.Tensor,
                z: Optional[torch.Tensor] = None, scratch: Optional[torch.Tensor] = None, long_from: int = 1,
-               n_long: Optional[int] = None) -> None:
+               n_long: Optional[int] = None, passes: Optional[Sequence[Sequence[int]]] = None) -> None:
     """The gated delta rule over the step's tokens, per (request, head), a request's tokens in order:
     ``S <- g S``, ``u = beta (v - S^T k)``, ``S <- S + k u^T``, ``o = S^T q``, with ``beta = sigmoid(b_raw)``,
     ``g = exp(-exp(a_log) softplus(a_raw + dt_bias))``, and ``q``, ``k`` first made unit vectors per head
@@ -1708,7 +1708,9 @@ def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, b_raw: torch.T
 
     ``scratch`` (bytes on the device, :func:`delta_chunk_scratch` of them): where the sizes and alignments allow it, the
     ``n_long`` requests (None: all) that bring ``long_from`` tokens and more go in chunks (of 32 tokens, two at a time), and the others token by
-    token beside them (``csrc/delta_chunk.cu``)."""
+    token beside them (``csrc/delta_chunk.cu``).  ``passes``: with less scratch, what is worked on one after the other, per pass the
+    first of the long requests and how many, rows of :data:`DELTA_CHUNK` tokens from .. to of each, and how many rows that is together
+    (as many must fit in ``scratch``); every row of every long request in one of them, a request's in order."""
     T, H, Dv = out.shape
     D = state.shape[3]
     if (a_raw is None) == (z is None) or (z is not None and z.shape != (T, H * D)):
@@ -1723,15 +1725,19 @@ def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, b_raw: torch.T
     if a_log.shape != (H,) or dt_bias.shape != ((H,) if z is None else (H * D,)):
         raise KernelError("delta_scan: a_log must be [H], dt_bias [H] (or [H * D] with a decay per channel)")
     n_long = n_segs if n_long is None else int(n_long)
-    if scratch is not None and z is None and 0 < delta_chunk_scratch(q.dtype, T, n_long, H, G, D, Dv) <= scratch.numel() \
+    need = delta_chunk_scratch(q.dtype, T, n_long, H, G, D, Dv)
+    if passes is not None and need:
+        need = need // (T // DELTA_CHUNK + n_long) * max(p[4] for p in passes)
+    if scratch is not None and z is None and 0 < need <= scratch.numel() \
             and (qs | ks | vs) % 8 == 0 and (q.data_ptr() | k.data_ptr() | v.data_ptr() | out.data_ptr() | scratch.data_ptr()) % 16 == 0:
         _check(_lib().ftk_delta_scan_chunks(
             q.data_ptr(), qs, k.data_ptr(), ks, v.data_ptr(), vs, b_raw.data_ptr(), bs, a_raw.data_ptr(), as_, _code(q, "q"),
             _dev(a_log, "a_log", torch.float32), _dev(dt_bias, "dt_bias", torch.float32), float(q_scale), float(unit_eps),
             _dev(state, "state", torch.float32), state.shape[0], _dev(state_slots, "state_slots", torch.int32),
             _dev(seg_info, "seg_info", torch.int32), n_segs, _dev(out, "out", torch.float32), T, H, G, D, Dv,
-            int(long_from), n_long, _dev(scratch, "scratch", torch.uint8), scratch.numel(), _stream()), "delta_scan (chunks)",
-            2 + (n_long < n_segs))
+            int(long_from), n_long, (ctypes.c_int32 * (5 * len(passes)))(*[x for p in passes for x in p]) if passes else None,
+            len(passes or ()), _dev(scratch, "scratch", torch.uint8), scratch.numel(), _stream()), "delta_scan (chunks)",
+            2 * len(passes or (0,)) + (n_long < n_segs))
         return
     _check(_lib().ftk_delta_scan(
         q.data_ptr(), qs, k.data_ptr(), ks, v.data_ptr(), vs, b_raw.data_ptr(), bs,

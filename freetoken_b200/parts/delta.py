@@ -26,7 +26,7 @@ slot of the cache manager's state pool; both start from zero.  The reference has
 from __future__ import annotations
 
 import math
-from typing import Any, Dict, Sequence
+from typing import Any, Dict, List, Sequence, Tuple
 
 import torch
 
@@ -96,6 +96,20 @@ def pairs_pay(lens: Sequence[int], beside: bool, n_heads: int, n_kv_heads: int, 
     blocks = sum(lens) / longest * pairs * n_kv_heads * -(-(n_heads // n_kv_heads) // 2)  # (that prepare)
     in_chunks += 16.0 * max(0.0, blocks / (2 * SMS) - 0.3)
     return in_chunks < 8.0 + longest * token_time(states, wide, v_dim)
+
+
+def chunk_passes(lens: Sequence[int], most: int) -> List[Tuple[int, int, int, int, int]]:
+    """Requests of ``lens`` tokens in passes of at most ``most`` rows (of 64 tokens): first request and how many, rows from .. to of each of
+    them, and how many rows that is.  Requests go side by side, as many as there are rows for, each as far as all of them can."""
+    out = []
+    for first in range(0, len(lens), most):
+        left = [-(-n // ops.DELTA_CHUNK) for n in lens[first:first + most]]
+        count, done = len(left), 0
+        while max(left) > 0:
+            far = max(m for m in range(1, max(left) + 1) if sum(min(r, m) for r in left) <= most)
+            out.append((first, count, done, done + far, sum(min(r, far) for r in left)))
+            left, done = [max(r - far, 0) for r in left], done + far
+    return out
 
 
 @MIXERS.register("gated_delta")
@@ -168,11 +182,17 @@ class GatedDelta(Mixer):
         return n_tokens * (own + (H * Dv + (H * D if self.decay_rank else 0)) * 4) + self.chunk_scratch(n_tokens, n_tokens // CHUNK_MIN_TOKENS)[1]
 
     def chunk_scratch(self, n_tokens: int, n_long: int):
-        """``(chunks, bytes)`` of what ``n_long`` requests of a step of so many tokens need to go in chunks (0 bytes: they do not)."""
+        """``(rows, bytes)`` of scratch for ``n_long`` requests of a step of so many tokens to go in chunks (0 bytes: they do not).
+
+        A row of 64 tokens takes 50 KB a head and 16 or 32 a key head, 2.67 MB for 48 heads on 8 of 128.  All rows of the longest step
+        would be 614 MB at 8,192 tokens, so larger steps than 32 rows get half of them (:func:`chunk_passes`): 171 MB, 342 MB at
+        16,384 tokens, 85 MB below 4,096.  A pass more costs two launches."""
         if self.decay_rank:
             return 0, 0
-        return n_tokens // ops.DELTA_CHUNK + n_long, ops.delta_chunk_scratch(self.env.dtype, n_tokens, n_long, self.n_heads, self.n_kv_heads,
-                                                               self.head_dim, self.v_dim)
+        rows = n_tokens // ops.DELTA_CHUNK + n_long
+        size = ops.delta_chunk_scratch(self.env.dtype, n_tokens, n_long, self.n_heads, self.n_kv_heads, self.head_dim, self.v_dim)
+        most = min(rows, max(32, self.env.max_step_tokens // (2 * ops.DELTA_CHUNK)))
+        return most, size // max(rows, 1) * most
 
     def forward(self, h: torch.Tensor, step: StepState, cache: Any, writes_cache: bool) -> torch.Tensor:
         if not writes_cache:
@@ -196,10 +216,12 @@ class GatedDelta(Mixer):
         long = [seg.q_len for seg in step.segments if seg.q_len >= CHUNK_MIN_TOKENS] if z is None and h.is_cuda else []
         n_long = len(long)
         if long and (chunks_pay(long, n_long < n_segs, H, D, Dv) or pairs_pay(long, n_long < n_segs, H, self.n_kv_heads, D, Dv)):
-            chunks, n = self.chunk_scratch(T, n_long)
-            if n:  # (a row a chunk: layers of other sizes have a buffer of their own, and no step asks for more rows)
-                row, most = n // chunks, self.chunk_scratch(cap, cap // CHUNK_MIN_TOKENS)[0]
-                args = dict(scratch=ws.get("delta.chunks", (chunks, row), torch.uint8, (most, row)), long_from=CHUNK_MIN_TOKENS, n_long=n_long)
+            rows, n = self.chunk_scratch(T, n_long)
+            if n:  # (by rows: layers of other sizes have a buffer of their own, and no step asks for more rows)
+                row, most = n // rows, self.chunk_scratch(cap, cap // CHUNK_MIN_TOKENS)[0]
+                args = dict(scratch=ws.get("delta.chunks", (rows, row), torch.uint8, (most, row)), long_from=CHUNK_MIN_TOKENS, n_long=n_long)
+                if rows < T // ops.DELTA_CHUNK + n_long:
+                    args["passes"] = chunk_passes(long, rows)
         ops.delta_scan(qkv[:, : self.k_col], qkv[:, self.k_col: self.v_col], qkv[:, self.v_col:],
                        proj[:, self.b_col: self.a_col], a, self.params["A_log"], self.params["dt_bias"],
                        D ** -0.5, UNIT_EPS, cache.tensors["s"], step.state_slots, step.seg_info, n_segs, o32, **args)
