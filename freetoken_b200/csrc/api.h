@@ -277,7 +277,7 @@ int ftk_delta_scan(const void* q, long long q_stride, const void* k, long long k
                    const float* dt_bias, float q_scale, float unit_eps, float* state, int n_slots,
                    const int32_t* state_slots, const int32_t* seg_info, int n_segs, float* out, int n_tokens,
                    int n_heads, int n_kv_heads, int dim, int vdim, void* stream);
-// The same for portions of bfloat16 prompts in chunks of 32 tokens, two at a time (one decay a head, keys of 64 or 128 channels, value channels in
+// The same for portions of bfloat16 prompts in chunks of 64 tokens (one decay a head, keys of 64 or 128 channels, value channels in
 // multiples of 16): of the n_segs requests the n_long that bring long_from tokens and more; the others go token by token, in a
 // launch before.  ftk_delta_chunk_scratch says how many bytes of scratch n_long requests take, 0 where the sizes are not taken.
 // passes (host memory, or null for one over everything): with less scratch, what is worked on one after the other, five numbers each:

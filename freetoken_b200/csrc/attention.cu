@@ -1395,11 +1395,11 @@ static int paged_attention_impl(const void* q, const void* k_slab, const void* v
                 kF32Rows, tile_rows);
     FTK_REQUIRE(p.G <= kF32Rows, "paged_attention: %d query heads per KV head exceed the %d-row tile", p.G, kF32Rows);
     const size_t smem = ((size_t)kF32Rows * head_dim + (size_t)kF32Chunk * 2 * (head_dim + 4)) * sizeof(float);
-    note_variant(sel ? "attention: float32, block-sparse" : "attention: float32, warp per row");
     // Four rows a warp for heads of 64, two above: with four rows a head of 128 takes twice the registers for its chunk's words (300
     // tokens each of four requests 254 us against 177, decode steps 57 against 32).  Two for heads of 64 as well where blocks leave SMs idle
     // (with four: one request of 500 keys, 16 heads on 2 79 us and 42, on 4 41 and 37; 40 tokens on 8 12.9 and 10.1).
     const bool four = head_dim <= 64 && (long long)grid.x * grid.y > 148;
+    note_variant(sel ? "attention: float32, block-sparse" : four ? "attention: float32, up to four rows a warp" : "attention: float32, up to two rows a warp");
     const int warps = four ? 4 : 8;
     auto kern = four ? attention_f32_kernel<2, 4> : head_dim <= 64 ? attention_f32_kernel<2, 8> : head_dim <= 128 ? attention_f32_kernel<4, 8> : attention_f32_kernel<8, 8>;
     if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

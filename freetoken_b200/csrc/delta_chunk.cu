@@ -1,5 +1,5 @@
-// The gated delta rule in chunks, for portions of bfloat16 prompts with one decay a head (delta.cu runs everything else token
-// by token).  Chunks of 32 tokens go two at a time.
+// The gated delta rule in chunks of 64 tokens, for portions of bfloat16 prompts with one decay a head (delta.cu runs everything else token
+// by token).
 //
 // With S the state as 64 tokens find it, c_t = g_1 ... g_t and c_t / c_s the decays behind token s,
 //   u_t = beta_t (v_t - c_t S^T k_t - sum_(s < t) (c_t / c_s) (k_s . k_t) u_s)
@@ -16,8 +16,8 @@
 // 16; one step, and two, are as close to 64 bits as a chain of as many fmas), so the products of the leading pieces are chains of two
 // steps, added up in registers; the other pieces' are 2^-8 smaller.
 //
-// What bounds it: the chain of a chunk pair, product, registers, shared memory, product, which no other block can hide: the
-// tensor pipe is at work about half of the time.  With 64 columns a block, 48 heads of 128 x 128: 5.0 us a pair (product 0.8, registers 1.1, product 0.8, registers
+// What bounds it: the chain of a chunk, product, registers, shared memory, product, which no other block can hide: the
+// tensor pipe is at work about half of the time.  With 64 columns a block, 48 heads of 128 x 128: 5.0 us a chunk (product 0.8, registers 1.1, product 0.8, registers
 // 0.7, product 0.5, registers 1.0); 16 columns a block, 16 heads: 2.9.
 // 2,048 tokens of one request, prep and chunks together (token by token, 32-bit fmas on the CUDA cores in chunks of 32, now): 48 heads of
 // 128 x 128 869, 431 and 228 us, 16 heads 563, 282 and 123; 16 heads of 64 x 64 535, 292 and 110.  Distance from 64 bits, token by token
@@ -34,7 +34,7 @@ int delta_scan_tokens(const void* q, long long q_stride, const void* k, long lon
 
 __device__ int g_delta_status[4];  // [0] first error code of a wait that ran out, [1] block; 0 = fine
 
-constexpr int kDcTokens = 64;  // tokens of the two chunks that go together
+constexpr int kDcTokens = 64;  // tokens of a chunk
 constexpr float kDcMost = 3.38e38f;  // what bfloat16 reaches: larger numbers' first piece would be an infinity
 // Scratch of 64 tokens: a key head's [K; Q] as the tensor core reads it (per 64 channels 128 rows of 128 bytes, swizzled), then a
 // head's [T; A T] the same way (three pieces of 128 rows of 64 tokens), per token beta, beta c rk, c rq, (c_C / c) rk, and c_C.
@@ -849,7 +849,7 @@ static int launch_delta_chunks_as(const DeltaChunkArgs& a, cudaStream_t s) {
   return 0;
 }
 
-// Columns a block: by the rounds of blocks over the SMs and what a pair of chunks takes, 3.0 us with 16 columns, 5.0 with 64 (and 3 more
+// Columns a block: by the rounds of blocks over the SMs and what a chunk takes, 3.0 us with 16 columns, 5.0 with 64 (and 3 more
 // a block).  16 heads of 128 columns, 2,048 tokens: 123 us with 16 (128 blocks); 48 heads 228 with 64 (96 blocks), three rounds with 16.
 template <int D>
 static int launch_delta_chunks(const DeltaChunkArgs& a, int tokens, cudaStream_t s) {  // tokens: of the pass, about
@@ -914,7 +914,7 @@ extern "C" int ftk_delta_scan_chunks(const void* q, long long q_stride, const vo
                                      long_from, stream);
     if (rc) return rc;
   }
-  note_variant("delta rule: chunks of 32 tokens");
+  note_variant("delta rule: chunks of 64 tokens, tcgen05");
   for (int i = 0; i < n_passes; ++i) {
     const int32_t whole[5] = {0, n_long, 0, 0x7fffffff, n_tokens / kDcTokens + n_long};
     const int32_t* p = passes ? passes + 5 * i : whole;

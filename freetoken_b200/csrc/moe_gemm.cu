@@ -263,12 +263,22 @@ static int launch_moe_gemm(const void* x, const void* w, const int32_t* offsets,
     return 0; \
   } while (0)
   constexpr int cols = GATED ? kTiledCols / 2 : kTiledCols;
+  constexpr bool f32 = sizeof(T) == 4;
+  auto note = [](const char* gate_up, const char* down) { note_variant(GATED ? gate_up : down); };
   // (tiles of a few rows are the most: with so many experts that a grid cannot hold them, larger ones)
-  if (wide && n_routes <= 4 * n_experts && grid_of(kFewRows, 1).y <= 65535u)
+  if (wide && n_routes <= 4 * n_experts && grid_of(kFewRows, 1).y <= 65535u) {
+    if (f32) note("expert gate/up product: float32, few rows an expert", "expert down product: float32, few rows an expert");
+    else note("expert gate/up product: bfloat16, few rows an expert", "expert down product: bfloat16, few rows an expert");
     FTK_MOE_GEMM((moe_gemm_few_kernel<T, GATED>), kFewRows, (GATED ? 1 : 2) * kFewPairs * kFewWarps, 32 * kFewWarps);
-  if constexpr (sizeof(T) == 4) {
-    if (wide) return launch_moe_gemm_split<GATED>((const float*)x, (const float*)w, offsets, n_experts, K, N, w_rows, routes, weights, n_routes, act, alpha, limit, (float*)out, s);
+  }
+  if constexpr (f32) {
+    if (wide) {
+      note("expert gate/up product: float32 on the tensor cores", "expert down product: float32 on the tensor cores");
+      return launch_moe_gemm_split<GATED>((const float*)x, (const float*)w, offsets, n_experts, K, N, w_rows, routes, weights, n_routes, act, alpha, limit, (float*)out, s);
+    }
+    note("expert gate/up product: float32 on CUDA cores", "expert down product: float32 on CUDA cores");
   } else {
+    note("expert gate/up product: bfloat16 on CUDA cores", "expert down product: bfloat16 on CUDA cores");
     if (wide && n_routes <= 32 * n_experts) FTK_MOE_GEMM((moe_gemm_kernel<T, GATED, 32, true>), 32, cols, kTiledThreads);
     if (wide) FTK_MOE_GEMM((moe_gemm_kernel<T, GATED, 64, true>), 64, cols, kTiledThreads);
   }
@@ -303,7 +313,6 @@ extern "C" int ftk_moe_gemm1_act(const void* x_sorted, const void* w1, int dtype
                                         limit, out, nullptr, 0, 0, s);
     if (rc >= 0) return rc;
   }
-  note_variant(dtype == FTK_F32 ? "expert gate/up product: float32 on CUDA cores" : "expert gate/up product: bfloat16 on CUDA cores");
   const int rc = dtype == FTK_F32
       ? launch_moe_gemm<float, true>(x_sorted, w1, expert_offsets, n_experts, hidden, inter, 2 * inter, nullptr, nullptr, n_routes, act,
                                      alpha, limit, out, s)
@@ -345,7 +354,6 @@ extern "C" int ftk_moe_gemm2(const void* a, const void* w2, int dtype, const int
                                     inter, out, s);
     if (rc >= 0) return rc;
   }
-  note_variant(dtype == FTK_F32 ? "expert down product: float32 on CUDA cores" : "expert down product: bfloat16 on CUDA cores");
   const int rc = dtype == FTK_F32
       ? launch_moe_gemm<float, false>(a, w2, expert_offsets, n_experts, inter, hidden, hidden, sorted_routes, topk_weights, n_routes, 0,
                                       0.f, 0.f, out, s)

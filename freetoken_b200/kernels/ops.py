@@ -1673,7 +1673,7 @@ def ssm_output(o32: torch.Tensor, x: torch.Tensor, d_skip: torch.Tensor, z: torc
                                  int(norm_groups), float(eps), _dev(out, "out"), T, H, P, _stream()), "ssm_output")
 
 
-DELTA_CHUNK = 64  # tokens of the two chunks that go together
+DELTA_CHUNK = 64  # tokens of a chunk
 DELTA_ROW_BYTES = 128 * 128  # 128 rows of 64 channels or tokens as the tensor core reads them (csrc/delta_chunk.cu: kDcImage)
 # of a head: three pieces of T and A T, four factors a token, the decay of all (csrc/delta_chunk.cu: kDcHeadBytes)
 DELTA_HEAD_BYTES = 3 * DELTA_ROW_BYTES + 4 * DELTA_CHUNK * 4 + 16
@@ -1707,7 +1707,7 @@ def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, b_raw: torch.T
     has several tokens, ``z`` is overwritten with the decays.
 
     ``scratch`` (bytes on the device, :func:`delta_chunk_scratch` of them): where the sizes and alignments allow it, the
-    ``n_long`` requests (None: all) that bring ``long_from`` tokens and more go in chunks (of 32 tokens, two at a time), and the others token by
+    ``n_long`` requests (None: all) that bring ``long_from`` tokens and more go in chunks of 64 tokens, and the others token by
     token beside them (``csrc/delta_chunk.cu``).  ``passes``: with less scratch, what is worked on one after the other, per pass the
     first of the long requests and how many, rows of :data:`DELTA_CHUNK` tokens from .. to of each, and how many rows that is together
     (as many must fit in ``scratch``); every row of every long request in one of them, a request's in order."""

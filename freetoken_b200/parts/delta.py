@@ -77,10 +77,10 @@ def chunks_pay(lens: Sequence[int], beside: bool, n_heads: int, head_dim: int, v
 
 
 def pairs_pay(lens: Sequence[int], beside: bool, n_heads: int, n_kv_heads: int, head_dim: int, v_dim: int) -> bool:
-    """Whether requests of ``lens`` tokens are through sooner in chunks on tcgen05 (two at a time) than token by token;
+    """Whether requests of ``lens`` tokens are through sooner in chunks on tcgen05 than token by token;
     arguments as :func:`chunks_pay`.
 
-    Both kernels are chains (of pairs of chunks, of tokens) until a step has more blocks than the GPU holds at once, then waves or a
+    Both kernels are chains (of chunks, of tokens) until a step has more blocks than the GPU holds at once, then waves or a
     rate; the chunks also have a launch that prepares them, two blocks an SM.  Fitted to timings of both (heads of 64 and 128, 4 to 48
     of them, 1 to 16 requests of 32 to 2,048 tokens, 16 to 256 value columns; 5 % off on average).  One request, 48 heads of 128, token
     by token against chunks: 43 and 40 us for 80 tokens, 50 and 36 for 96, 64 and 38 for 128, 224 and 72 for 512; 16 heads of 64: 29

@@ -17,8 +17,11 @@ def run(q, ks, vs, bt, seg, lens, Hkv, **kw):
     plan = build_plan(lens, G, 16, None, Hkv, fixed_splits=1, sm_count=148)
     assert not plan.n_slots
     out = torch.full_like(q, float("nan"))
+    ops.variant_counts(reset=True)
     ops.paged_attention(q, ks, vs, bt, seg, len(lens), torch.from_numpy(plan.items).to(DEV), plan.n_items, None, None, out, 16, 0.3 * D ** -0.5,
                         None, **kw)
+    form = "up to %s rows a warp" % ("four" if D <= 64 and plan.n_items * Hkv > 148 else "two")
+    assert [k for k in ops.variant_counts() if k.startswith("attention: float32")] == ["attention: float32, " + form]
     return out
 
 

@@ -39,7 +39,7 @@ def run(p, chunks):
     ops.variant_counts(reset=True)
     ops.delta_scan(p["q"], p["k"], p["v"], p["b"], p["a"], p["a_log"], p["dt_bias"], D ** -0.5, EPS, state, p["slots"], p["info"],
                    len(p["info"]), out, scratch=scratch)
-    assert bool(ops.variant_counts().get("delta rule: chunks of 32 tokens")) == chunks
+    assert bool(ops.variant_counts().get("delta rule: chunks of 64 tokens, tcgen05")) == chunks
     return out, state
 
 
@@ -132,7 +132,7 @@ def test_what_is_not_taken_goes_token_by_token():
     ops.variant_counts(reset=True)
     ops.delta_scan(p["q"], p["k"], p["v"], p["b"], p["a"], p["a_log"], p["dt_bias"], 128 ** -0.5, EPS, state, p["slots"], p["info"], 1, got,
                    scratch=scratch)
-    assert not ops.variant_counts().get("delta rule: chunks of 32 tokens")
+    assert not ops.variant_counts().get("delta rule: chunks of 64 tokens, tcgen05")
     torch.testing.assert_close(got, out, rtol=1e-4, atol=2e-5)
 
 
@@ -158,7 +158,7 @@ def test_only_the_long_requests_of_a_step_go_in_chunks(H, G, D, Dv, lens):
     p = problem(lens, H, G, D, Dv, seed=D + len(lens))
     is_long = [n >= 64 for n, _ in lens]
     out, state = scan(p, long_from=64, n_long=sum(is_long))
-    assert ops.variant_counts().get("delta rule: chunks of 32 tokens")
+    assert ops.variant_counts().get("delta rule: chunks of 64 tokens, tcgen05")
     (chunks, chunk_state), (tokens, token_state) = run(p, True), run(p, False)
     for i, (q0, n, _, _) in enumerate(p["info"].tolist()):
         slot, rows = int(p["slots"][i]), slice(q0, q0 + n)

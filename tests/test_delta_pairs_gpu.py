@@ -1,4 +1,4 @@
-"""The gated delta rule in pairs of chunks at the borders of its 64 tokens and of a block's 64 value columns."""
+"""The gated delta rule in chunks at the borders of their 64 tokens and of a block's 64 value columns."""
 
 import pytest
 import torch

@@ -22,8 +22,10 @@ def problem(hidden, inter, rows, seed=0):
 
 def products(x, w, w2, offsets, routes, weights):
     a, y = torch.full((len(x), w2.shape[2]), float("nan"), device=DEV), torch.full_like(x, float("nan"))
+    ops.variant_counts(reset=True)
     ops.moe_gemm1_act(x, w, offsets, "silu", 1.702, 7.0, a)
     ops.moe_gemm2(a, w2, offsets, routes, weights, y)
+    assert ops.variant_counts() == {f"expert {which} product: float32 on the tensor cores": 1 for which in ("gate/up", "down")}
     assert ops.read_status() == 0
     return a, y
 

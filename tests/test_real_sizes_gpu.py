@@ -104,7 +104,7 @@ def test_float32_engine_equals_plain_at_real_sizes(real):
     torch.testing.assert_close(cut, ref, **F32_TOL)
     ran = ops.variant_counts()
     assert ran.get("routing: expert choice from given logits") and ran.get("routing: product, choice and sort in one launch")
-    assert ran.get("expert gate/up product: float32 on CUDA cores") and ran.get("attention: float32, warp per row")
+    assert ran.get("expert gate/up product: float32, few rows an expert") and ran.get("attention: float32, up to two rows a warp")
     print("\nkernel forms, float32, 128 tokens whole and cut:", sorted(ran.items()))
 
 
