@@ -24,25 +24,6 @@ constexpr int kMaxSections = 4;
 constexpr int kWarpsPerBlock = 4;
 constexpr int kMaxHeadDim = 256;
 
-// Two 32-bit operations in one instruction, each rounded as by itself.
-#define FTK_PAIR(v) (*reinterpret_cast<const unsigned long long*>(&(v)))
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-  float2 d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<unsigned long long&>(d)) : "l"(FTK_PAIR(a)), "l"(FTK_PAIR(b)));
-  return d;
-}
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-  float2 d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<unsigned long long&>(d)) : "l"(FTK_PAIR(a)), "l"(FTK_PAIR(b)));
-  return d;
-}
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-  float2 d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(reinterpret_cast<unsigned long long&>(d)) : "l"(FTK_PAIR(a)), "l"(FTK_PAIR(b)), "l"(FTK_PAIR(c)));
-  return d;
-}
-#undef FTK_PAIR
-
 struct Sections {
   FtkSection s[kMaxSections];
   int n;
@@ -239,9 +220,7 @@ norm_rope_store_vec_kernel(const __nv_bfloat16* __restrict__ x, int n_tokens, in
       const float one = gemma ? 1.f : 0.f;
 #pragma unroll
       for (int j = 0; j < 8; j += 2) {
-        const float2 u = mul2(mul2(make_float2(v[j], v[j + 1]), make_float2(inv, inv)), add2(make_float2(w[j], w[j + 1]), make_float2(one, one)));
-        v[j] = u.x;
-        v[j + 1] = u.y;
+        f2_unpair(f2_mul(f2_mul(f2_pair(v[j], v[j + 1]), f2_pair(inv, inv)), f2_add(f2_pair(w[j], w[j + 1]), f2_pair(one, one))), v[j], v[j + 1]);
       }
     }
   }
@@ -273,10 +252,9 @@ norm_rope_store_vec_kernel(const __nv_bfloat16* __restrict__ x, int n_tokens, in
       const float sign = low ? -1.f : 1.f;
 #pragma unroll
       for (int j = 0; j < 8; j += 2) {
-        const float2 turned = mul2(make_float2(partner[j], partner[j + 1]), mul2(make_float2(cb[j], cb[j + 1]), make_float2(sign, sign)));
-        const float2 u = fma2(make_float2(v[j], v[j + 1]), make_float2(ca[j], ca[j + 1]), turned);
-        v[j] = u.x;
-        v[j + 1] = u.y;
+        uint64_t turned = f2_mul(f2_pair(partner[j], partner[j + 1]), f2_mul(f2_pair(cb[j], cb[j + 1]), f2_pair(sign, sign)));
+        f2_fma(turned, f2_pair(v[j], v[j + 1]), f2_pair(ca[j], ca[j + 1]));
+        f2_unpair(turned, v[j], v[j + 1]);
       }
     }
   }

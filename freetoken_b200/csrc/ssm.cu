@@ -23,7 +23,7 @@ __device__ __forceinline__ float silu_f(float z) { return z / (1.f + expf(-z)); 
 
 // What bounds it: instructions, half of them the activation's exponential and division (2.8 of 4 an SM cycle), behind the latency
 // of the rows.  2,048 tokens of 8,192 channels, 4 taps, with silu: 43 us with the rows' loads between the divisions, 30 now (67 MB to and
-// from memory: 10); 1,024 tokens of 1,536 channels 13.6 and 9.1.
+// from memory: 10); 1,024 tokens of 1,536 channels 13.6 and 9.1.  Rows that are not aligned, one number off: 41 and 34, 14.4 and 13.3.
 template <typename T, int TAPS>
 __global__ void __launch_bounds__(kCaThreads)
 conv_act_kernel(const T* __restrict__ x, long long x_stride, const float* __restrict__ w, const float* __restrict__ bias,
