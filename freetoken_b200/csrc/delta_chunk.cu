@@ -37,9 +37,10 @@ __device__ int g_delta_status[4];  // [0] first error code of a wait that ran ou
 constexpr int kDcTokens = 64;  // tokens of a chunk
 constexpr float kDcMost = 3.38e38f;  // what bfloat16 reaches: larger numbers' first piece would be an infinity
 // Scratch of 64 tokens: a key head's [K; Q] as the tensor core reads it (per 64 channels 128 rows of 128 bytes, swizzled), then a
-// head's [T; A T] the same way (three pieces of 128 rows of 64 tokens), per token beta, beta c rk, c rq, (c_C / c) rk, and c_C.
+// head's [T; A T] without their diagonals the same way (three pieces of 128 rows of 64 tokens), per token beta, beta c rk, c rq,
+// (c_C / c) rk and A's diagonal, and c_C.
 constexpr int kDcImage = 128 * 128;  // bytes of 128 rows
-constexpr int kDcHeadBytes = 3 * kDcImage + 4 * kDcTokens * 4 + 16;
+constexpr int kDcHeadBytes = 3 * kDcImage + 5 * kDcTokens * 4 + 16;
 __host__ __device__ constexpr long long dc_row_bytes(int H, int G, int D) { return (long long)G * (D / 64) * kDcImage + (long long)H * kDcHeadBytes; }
 
 struct DeltaChunkArgs {
@@ -254,7 +255,7 @@ __global__ void __launch_bounds__(256, 2) delta_prep_kernel(DeltaChunkArgs a) {
       vec[kDcTokens + tt] = (float)(sh.beta[tt] * upto * srk[tt]);
       vec[2 * kDcTokens + tt] = (float)(upto * srq[tt]);
       vec[3 * kDcTokens + tt] = (float)(rest * srk[tt]);
-      if (tt == 0) vec[4 * kDcTokens] = (float)((sh.total[0] * sh.total[1]) * (sh.total[2] * sh.total[3]));
+      if (tt == 0) vec[5 * kDcTokens] = (float)((sh.total[0] * sh.total[1]) * (sh.total[2] * sh.total[3]));
     }
     // L or A, 16 entries of a row a thread and turn
     auto fill = [&](bool of_a) {
@@ -379,6 +380,16 @@ __global__ void __launch_bounds__(256, 2) delta_prep_kernel(DeltaChunkArgs a) {
         float v[8];
         Vec4<float>::load(src, reinterpret_cast<float (&)[4]>(v[0]));
         Vec4<float>::load(src + 4, reinterpret_cast<float (&)[4]>(v[4]));
+        if (c == (t & ~7)) {  // the diagonals (T's are ones) go through registers
+          float own = 0.f;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            if (c + i != t) continue;
+            own = v[i];
+            v[i] = 0.f;
+          }
+          if (r != t) reinterpret_cast<float*>(image + 3 * kDcImage)[4 * kDcTokens + t] = own;
+        }
         split3(v, w);
       }
 #pragma unroll
@@ -396,15 +407,26 @@ struct DcPlace {
   static constexpr int s_piece = NV == 64 ? kDcImage : 2 * NV;       // (64 columns fill the 128 bytes of a row, 16 columns' three pieces lie in one)
   static constexpr int x = s + (NV == 64 ? 3 : 1) * kDcImage;        // X's, then U's: rows of tokens
   static constexpr int x_piece = NV == 64 ? kDcImage / 2 : 2 * NV;
-  static constexpr int o = x + (NV == 64 ? 3 : 1) * kDcImage / 2;    // outputs on their way: rows of tokens, in different banks
+  static constexpr int o = x + (NV == 64 ? 3 : 1) * kDcImage / 2;    // X from K's rows to Q's, then outputs on their way: rows of tokens, in different banks
   static constexpr int o_row = NV * 4 + 16;
-  static constexpr int bytes = o + (NV == 64 ? kDcTokens * o_row : 0);
+  static constexpr int bytes = o + kDcTokens * o_row;
 };
 __device__ __forceinline__ void dc_bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint64_t* bar) {
   mbar_expect_tx(bar, bytes);
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes),
                "r"(smem_addr(bar)) : "memory");
 }
+// Whether one of them may be no number, or one that bfloat16 cannot reach (kDcMost, or a little less).
+template <int N>
+__device__ __forceinline__ bool dc_none(const float (&y)[N]) {
+  uint64_t z = 0;
+#pragma unroll
+  for (int j = 0; j < N; j += 2) f2_fma(z, f2_mul(f2_pair(y[j], y[j + 1]), f2_pair(1.0079f, 1.0079f)), 0);  // (an infinity times zero is a NaN)
+  float a, b;
+  f2_unpair(z, a, b);
+  return !(a + b == 0.f);
+}
+
 // Columns with an infinite or NaN number in the 64 tokens from token `first` on, once more, as delta.cu runs them (in pairs of tokens): an
 // infinity taken apart into pieces is a NaN, and so is what has infinities of both signs, which depends on where they meet.  A warp takes a
 // column: `state` [NV][D] holds them as the chunk finds them, and is left as it leaves them; outputs go out from a column's
@@ -497,6 +519,7 @@ __global__ void __launch_bounds__(dc_threads<NV>()) delta_chunk_kernel(const __g
   extern __shared__ unsigned char dc_smem[];
   __shared__ uint64_t kq_full[2], t_full, mma_done;
   __shared__ uint32_t tmem_slot;
+  __shared__ float newest[NV];
   __shared__ int abort_flag, odd_flag[2], first_odd[NV];  // the first token that has no number, per column
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, quad = warp & 3, share = warp >> 2;
   const uint32_t base = (smem_addr(dc_smem) + 1023u) & ~1023u;
@@ -565,7 +588,7 @@ __global__ void __launch_bounds__(dc_threads<NV>()) delta_chunk_kernel(const __g
     float f_next[3], whole_next;
     auto fetch = [&](int ch) {
       const float* vec = reinterpret_cast<const float*>(head_src + (size_t)ch * a.row_bytes + 3 * kDcImage);
-      whole_next = vec[4 * kDcTokens];
+      whole_next = vec[5 * kDcTokens];
       if (of_k) {
         const bool in = ch * kDcTokens + t < q_len;
         const __nv_bfloat16* src = a.v + (size_t)(q_start + (in ? ch * kDcTokens + t : 0)) * a.v_stride + (size_t)h * a.Dv;
@@ -577,6 +600,7 @@ __global__ void __launch_bounds__(dc_threads<NV>()) delta_chunk_kernel(const __g
         f_next[2] = vec[3 * kDcTokens + t];
       } else {
         f_next[0] = vec[2 * kDcTokens + t];
+        f_next[1] = vec[4 * kDcTokens + t];
       }
     };
     fetch(0);
@@ -643,10 +667,9 @@ __global__ void __launch_bounds__(dc_threads<NV>()) delta_chunk_kernel(const __g
       phase ^= 1;
       __syncwarp();
       tc_fence_after();
-      float o[NH];  // Q's rows: what the state gives
+      float o[NH];  // K's rows: X, which T's ones on the diagonal pass on; Q's: what the state gives, and X times A's diagonal
       // What a row of T and A T has behind its token is zero, but zero times an infinity or NaN is NaN: such an X (or one that bfloat16
       // cannot reach) goes into the product as zero, and its column token by token from there on.
-      bool odd = false;
 #pragma unroll
       for (int i = 0; i < NG; ++i) {
         constexpr int kParts = D / 32;
@@ -665,21 +688,27 @@ __global__ void __launch_bounds__(dc_threads<NV>()) delta_chunk_kernel(const __g
         if (of_k) {
           const uint32_t w[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            y[j] = fmaf(f0, j & 1 ? bf2_high(w[j >> 1]) : bf2_low(w[j >> 1]), -f1 * y[j]);
-            if (!(fabsf(y[j]) < kDcMost)) {
-              odd = true;
+          for (int j = 0; j < 8; ++j) y[j] = fmaf(f0, j & 1 ? bf2_high(w[j >> 1]) : bf2_low(w[j >> 1]), -f1 * y[j]);
+          if (dc_none<8>(y)) {
+            odd_flag[ch & 1] = 1;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              if (fabsf(y[j]) < kDcMost) continue;
               atomicMin(&first_odd[share * NH + 8 * i + j], t);
               y[j] = 0.f;
             }
           }
           put(At::x, At::x_piece, row, i, y);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) o[8 * i + j] = y[j];
+#pragma unroll
+          for (int j = 0; j < 8; j += 4)
+            *reinterpret_cast<float4*>(tiles + At::o + t * At::o_row + (share * NH + 8 * i + j) * 4) = make_float4(y[j], y[j + 1], y[j + 2], y[j + 3]);
         } else {
 #pragma unroll
           for (int j = 0; j < 8; ++j) o[8 * i + j] = f0 * y[j];
         }
       }
-      if (odd) odd_flag[ch & 1] = 1;
       fence_async_smem();
       tc_fence_before();
       if (__syncthreads_or(bad)) break;
@@ -703,6 +732,13 @@ __global__ void __launch_bounds__(dc_threads<NV>()) delta_chunk_kernel(const __g
         }
         __syncwarp();
       }
+      if (!of_k) {
+#pragma unroll
+        for (int j = 0; j < NH; j += 4) {
+          const float4 x = *reinterpret_cast<const float4*>(tiles + At::o + t * At::o_row + (share * NH + j) * 4);
+          o[j] = fmaf(f1, x.x, o[j]); o[j + 1] = fmaf(f1, x.y, o[j + 1]); o[j + 2] = fmaf(f1, x.z, o[j + 2]); o[j + 3] = fmaf(f1, x.w, o[j + 3]);
+        }
+      }
       float u[NH];
       wait(&mma_done, phase, 504);
       phase ^= 1;
@@ -717,23 +753,30 @@ __global__ void __launch_bounds__(dc_threads<NV>()) delta_chunk_kernel(const __g
 #pragma unroll
         for (int j = 0; j < 8; ++j) u[8 * i + j] = (r[0][j] + r[1][j]) + (r[2][j] + r[3][j]);
       }
-      odd = false;
 #pragma unroll
-      for (int j = 0; j < NH; ++j) {
-        if (!of_k) u[j] += o[j];
-        if (!(fabsf(u[j]) < kDcMost)) {
-          odd = true;
-          atomicMin(&first_odd[share * NH + j], t);
-        }
+      for (int j = 0; j < NH; ++j) u[j] += o[j];
+      if (dc_none<NH>(u)) {
+        odd_flag[ch & 1] = 1;
+#pragma unroll
+        for (int j = 0; j < NH; ++j)
+          if (!(fabsf(u[j]) < kDcMost)) atomicMin(&first_odd[share * NH + j], t);
       }
-      if (odd) odd_flag[ch & 1] = 1;
       if (tid == 0 && ch + 1 < n_chunks && !bad) {
         load_t(ch + 1);
         ++t_issued;
       }
+      const int last = min(kDcTokens, q_len - ch * kDcTokens) - 1;  // the newest token: the largest share of the state where decays are strong
+      const float k_last = channel ? __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(
+          tiles + At::kq + (ch & 1) * 2 * kDcImage + (row >> 6) * kDcImage + last * 128 + ((((row >> 3) & 7) ^ (last & 7)) << 4) + (row & 7) * 2)) : 0.f;
       if (of_k) {
 #pragma unroll
-        for (int j = 0; j < NH; ++j) u[j] *= f2;
+        for (int j = 0; j < NH; ++j) {
+          u[j] *= f2;
+          if (t == last) {
+            newest[share * NH + j] = u[j];
+            u[j] = 0.f;
+          }
+        }
 #pragma unroll
         for (int i = 0; i < NG; ++i) put(At::x, At::x_piece, row, i, reinterpret_cast<const float (&)[8]>(u[8 * i]));
       }
@@ -802,7 +845,7 @@ __global__ void __launch_bounds__(dc_threads<NV>()) delta_chunk_kernel(const __g
         tmem_ld8_finish(r);
         if (channel) {
 #pragma unroll
-          for (int j = 0; j < 8; ++j) s[8 * i + j] = fmaf(whole, s[8 * i + j], (r[0][j] + r[1][j]) + (r[2][j] + r[3][j]));
+          for (int j = 0; j < 8; ++j) s[8 * i + j] = fmaf(k_last, newest[share * NH + 8 * i + j], fmaf(whole, s[8 * i + j], (r[0][j] + r[1][j]) + (r[2][j] + r[3][j])));
         }
       }
       if (some_odd) {

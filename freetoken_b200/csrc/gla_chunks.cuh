@@ -169,20 +169,30 @@ __device__ __forceinline__ void gc_pairs(const float* k, const float* q, const f
   if (on && t < rows) *reinterpret_cast<float2*>(pout + t * prow + 2 * (place & 1)) = make_float2(sums[0], sums[1]);
 }
 
+// Whether one of eight is no number.
+__device__ __forceinline__ bool gc_none(const float (&y)[8]) {
+  uint64_t z = 0;
+#pragma unroll
+  for (int j = 0; j < 8; j += 2) f2_fma(z, f2_pair(y[j], y[j + 1]), 0);  // (an infinity times zero is a NaN)
+  float a, b;
+  f2_unpair(z, a, b);
+  return !(a + b == 0.f);
+}
+
 // An element of a chunk's contribution that is no number as the tensor core has it, as 32-bit fmas: an infinity taken apart into pieces
 // is a NaN, and its product with another number's pieces of both signs is one.  (Such keys and values as they stand at the end of their 16
-// tokens: later decays change no infinity.)
+// tokens: later decays change no infinity.  From `newest` on keys have no pieces.)
 template <int D, int VT>
-__device__ __noinline__ float gc_contribution(const GcLocal<D, VT>& sh, int d, int j) {
+__device__ __noinline__ float gc_contribution(const GcLocal<D, VT>& sh, int d, int j, int newest) {
   const unsigned char* pieces = reinterpret_cast<const unsigned char*>(sh.q) + (d >> 6) * (kGcTokens * 128) + (d & 7) * 2;
   const unsigned char* values = sh.v + (j >> 6) * (kGcTokens * 128) + (j & 7) * 2;
   float y = 0.f;
   for (int t = 0; t < kGcTokens; ++t) {
     const int at = t * 128 + ((((d >> 3) & 7) ^ (t & 7)) << 4);
     float k = 0.f;
-    for (int m = 2; m >= 0; --m) k += __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(pieces + m * GcLocal<D, VT>::piece + at));
+    for (int m = 2; m >= 0 && t < newest; --m) k += __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(pieces + m * GcLocal<D, VT>::piece + at));
     const float v = __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(values + t * 128 + ((((j >> 3) & 7) ^ (t & 7)) << 4)));
-    y = fmaf(fabsf(k) < INFINITY && fabsf(v) < INFINITY ? k : sh.k[t][d], v, y);
+    y = fmaf(fabsf(k) < INFINITY && fabsf(v) < INFINITY && t < newest ? k : sh.k[t][d], v, y);
   }
   return y;
 }
@@ -439,6 +449,7 @@ __global__ void __launch_bounds__(2 * D, 256 / D) gla_local_kernel(GlaArgs a) {
     }
     a.decay_prod[((size_t)c * a.H + h) * D + tid] = hi;
   }
+  const int two = (n - 1) % kGcBlock != 0;
   // the chunk's contribution: keys decayed to its end, in three pieces; a thread has eight channels of a token of every 16
   {
     constexpr int kPass = kThreads / kLanes;  // tokens at a time
@@ -455,6 +466,12 @@ __global__ void __launch_bounds__(2 * D, 256 / D) gla_local_kernel(GlaArgs a) {
     for (int b = 0; b < kGcBlocks; ++b) {
       const int t = b * kGcBlock + t0;
       float y[8];
+      if (t >= n - 1 - two && t < n) {  // (the newest tokens': added in registers)
+        *reinterpret_cast<uint4*>(pieces + (d >> 6) * (kGcTokens * 128) + t * 128 + ((((d >> 3) & 7) ^ (t & 7)) << 4)) = make_uint4(0u, 0u, 0u, 0u);
+        *reinterpret_cast<uint4*>(pieces + sh.piece + (d >> 6) * (kGcTokens * 128) + t * 128 + ((((d >> 3) & 7) ^ (t & 7)) << 4)) = make_uint4(0u, 0u, 0u, 0u);
+        *reinterpret_cast<uint4*>(pieces + 2 * sh.piece + (d >> 6) * (kGcTokens * 128) + t * 128 + ((((d >> 3) & 7) ^ (t & 7)) << 4)) = make_uint4(0u, 0u, 0u, 0u);
+        continue;
+      }
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         uint64_t kv = *reinterpret_cast<const uint64_t*>(&sh.k[t][d + 2 * j]);
@@ -472,46 +489,82 @@ __global__ void __launch_bounds__(2 * D, 256 / D) gla_local_kernel(GlaArgs a) {
   fence_async_smem();
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) {
-    tc_fence_after();
-    if (elect_one()) {
-      constexpr uint32_t id = instr_desc(D) | kMnMajorA | kMnMajorB;
-      const uint32_t v0 = smem_addr(sh.v), k0 = smem_addr(sh.q);
+  // Products, two sums of them at a time (2 D columns): the second and third pieces' and the first's of 32 tokens, then the first's of the
+  // other 32.  They are added up in registers, and the two newest tokens', the largest where decays are strong, last and by themselves:
+  // the accumulator cuts off instead of rounding.  (Two, where they lie in the same 16; else the newest.)
+  const int j = (warp & 3) * 32 + lane;  // a value column; 64 channels of it
+  const uint32_t my_tmem = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)((warp >> 2) * 64);
+  const float* k_last = &sh.k[n - 1][(warp >> 2) * 64];  // (no token after it decays it; the one before lies, decayed by it, a row in front)
+  auto value = [&](int t) {
+    return __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(sh.v + (j >> 6) * (kGcTokens * 128) + t * 128 + ((((j >> 3) & 7) ^ (t & 7)) << 4) + (j & 7) * 2));
+  };
+  const float v_last = j < 64 * VT ? value(n - 1) : 0.f, v_before = j < 64 * VT && two ? value(n - 2) : 0.f;
+  float* dst = a.carry + (((size_t)c * a.H + h) * D + (warp >> 2) * 64) * a.Dv + j;
+  float acc[64];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const uint64_t v = smem_desc_mn(v0 + k * 2048, kGcTokens * 128);
-        tc_mma(tmem, v, smem_desc_mn(k0 + k * 2048, kGcTokens * 128), id, k != 0);
-        tc_mma(tmem + D, v, smem_desc_mn(k0 + GcLocal<D, VT>::piece + k * 2048, kGcTokens * 128), id, k != 0);
-        tc_mma(tmem + D, v, smem_desc_mn(k0 + 2 * GcLocal<D, VT>::piece + k * 2048, kGcTokens * 128), id, 1);
+  for (int round = 0; round < 2; ++round) {
+    if (warp == 0) {
+      tc_fence_after();
+      if (elect_one()) {
+        constexpr uint32_t id = instr_desc(D) | kMnMajorA | kMnMajorB;
+        const uint32_t v0 = smem_addr(sh.v), k0 = smem_addr(sh.q);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const uint64_t v = smem_desc_mn(v0 + k * 2048, kGcTokens * 128);
+          if (round == 0) {
+            tc_mma(tmem, v, smem_desc_mn(k0 + GcLocal<D, VT>::piece + k * 2048, kGcTokens * 128), id, k != 0);
+            tc_mma(tmem, v, smem_desc_mn(k0 + 2 * GcLocal<D, VT>::piece + k * 2048, kGcTokens * 128), id, 1);
+          }
+          if (k / 2 == round) tc_mma(tmem + (1 - round) * D, v, smem_desc_mn(k0 + k * 2048, kGcTokens * 128), id, k % 2);
+        }
+        tc_commit(&mma_done);
       }
-      tc_commit(&mma_done);
+      __syncwarp();
+    }
+    if (!mbar_wait(&mma_done, round, &abort_flag)) {
+      if (atomicCAS(&g_gla_status[0], 0, 602) == 0) g_gla_status[1] = blockIdx.x;
+      abort_flag = 1;
     }
     __syncwarp();
-  }
-  if (!mbar_wait(&mma_done, 0, &abort_flag)) {
-    if (atomicCAS(&g_gla_status[0], 0, 602) == 0) g_gla_status[1] = blockIdx.x;
-    abort_flag = 1;
-  }
-  __syncwarp();
-  tc_fence_after();
-  {
-    const int j = (warp & 3) * 32 + lane;  // a value column; 64 channels of it
-    const uint32_t my_tmem = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)((warp >> 2) * 64);
-    float* dst = a.carry + (((size_t)c * a.H + h) * D + (warp >> 2) * 64) * a.Dv + j;
-#pragma unroll 2
+    tc_fence_after();
+#pragma unroll
     for (int i = 0; i < 64; i += 8) {
       float r[2][8];
       tmem_ld8_start(my_tmem + i, r[0]);
-      tmem_ld8_start(my_tmem + D + i, r[1]);
+      if (round == 0) tmem_ld8_start(my_tmem + D + i, r[1]);
       tmem_ld8_finish(r);
+      if (round == 0) {
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        if (j >= a.Dv) continue;
-        float y = r[0][e] + r[1][e];
-        if (!(fabsf(y) < INFINITY)) y = gc_contribution<D, VT>(sh, (warp >> 2) * 64 + i + e, j);
-        dst[(size_t)(i + e) * a.Dv] = y;
+        for (int e = 0; e < 8; ++e) acc[i + e] = r[0][e] + r[1][e];
+        continue;
+      }
+      float y[8], k[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) y[e] = acc[i + e] + r[0][e];
+      if (two) {
+        Vec4<float>::load(k_last - LD + i, reinterpret_cast<float (&)[4]>(k[0]));
+        Vec4<float>::load(k_last - LD + i + 4, reinterpret_cast<float (&)[4]>(k[4]));
+#pragma unroll
+        for (int e = 0; e < 8; ++e) y[e] = fmaf(k[e], v_before, y[e]);
+      }
+      Vec4<float>::load(k_last + i, reinterpret_cast<float (&)[4]>(k[0]));
+      Vec4<float>::load(k_last + i + 4, reinterpret_cast<float (&)[4]>(k[4]));
+#pragma unroll
+      for (int e = 0; e < 8; ++e) y[e] = fmaf(k[e], v_last, y[e]);
+      if (j < a.Dv) {
+        if (gc_none(y)) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e)
+            if (!(fabsf(y[e]) < INFINITY)) y[e] = gc_contribution<D, VT>(sh, (warp >> 2) * 64 + i + e, j, n - 1 - two);
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) dst[(size_t)(i + e) * a.Dv] = y[e];
       }
       __syncwarp();
+    }
+    if (round == 0) {
+      tc_fence_before();
+      __syncthreads();
     }
   }
   tc_fence_before();
@@ -588,7 +641,7 @@ __global__ void __launch_bounds__(256, 2) gla_out_kernel(GlaArgs a) {
   __shared__ uint64_t mma_done;
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag, first_odd[128];  // the first token whose value is no number, per column
-  __shared__ float dec[kGcTokens];
+  __shared__ float dec[kGcTokens], own[kGcTokens];  // own: P's diagonal
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, quad = warp & 3, half = warp >> 2;
   const uint32_t base = (smem_addr(go_smem) + 1023u) & ~1023u;
   unsigned char* tiles = go_smem + (base - smem_addr(go_smem));
@@ -741,7 +794,7 @@ __global__ void __launch_bounds__(256, 2) gla_out_kernel(GlaArgs a) {
         tmem_ld8_start(my_tmem + 64 + i, r[1]);
         tmem_ld8_finish(r);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i + j] += r[0][j] + r[1][j];
+        for (int j = 0; j < 8; ++j) acc[i + j] = (acc[i + j] + r[0][j]) + r[1][j];
       }
     };
 #pragma unroll 1
@@ -788,29 +841,42 @@ __global__ void __launch_bounds__(256, 2) gla_out_kernel(GlaArgs a) {
     }
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
-      const int i = tid + 256 * u;
+      const int i = tid + 256 * u, t = i >> 3, s0 = (i & 7) * 8;
+      if (s0 == (t & ~7)) {  // (a token's own value, the largest share where decays are strong: added in registers)
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (s0 + j == t) {
+            own[t] = qv[u][j];
+            qv[u][j] = 0.f;
+          }
+      }
       put8(GoPlace::q, GoPlace::tile, i >> 3, i & 7, qv[u]);
     }
     fence_async_smem();
-    tc_fence_before();
-    __syncthreads();
-    if (warp == 0) {
-      tc_fence_after();
-      if (elect_one()) {
+#pragma unroll 1
+    for (int pair = 0; pair < 2; ++pair) {  // sums of 16 tokens
+      tc_fence_before();
+      __syncthreads();
+      if (warp == 0) {
+        tc_fence_after();
+        if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const uint64_t v = smem_desc_mn(base + GoPlace::v + k * 2048, GoPlace::tile);
-          tc_mma(tmem + (k >> 1) * 64, v, smem_desc(base + GoPlace::q) + 2 * k, id1, k & 1);
-          tc_mma(tmem + 128, v, smem_desc(base + GoPlace::q + GoPlace::tile) + 2 * k, id2, 1);
+          for (int x = 0; x < 2; ++x) {
+            const int k = 2 * pair + x;
+            const uint64_t v = smem_desc_mn(base + GoPlace::v + k * 2048, GoPlace::tile);
+            tc_mma(tmem + x * 64, v, smem_desc(base + GoPlace::q) + 2 * k, id1, 0);
+            tc_mma(tmem + 128, v, smem_desc(base + GoPlace::q + GoPlace::tile) + 2 * k, id2, 1);
+          }
+          tc_commit(&mma_done);
         }
-        tc_commit(&mma_done);
+        __syncwarp();
       }
-      __syncwarp();
+      wait();
+      if (pair == 0) add_chains();
     }
-    wait();
     const int j = quad * 32 + lane, odd_from = j < Dv ? first_odd[j] : kGcTokens;
     float* o = a.out + (x.row0 * a.H + h) * Dv + j;
-    uint32_t odd = 0u;  // of this thread's 32 tokens those that have no number
+    bool odd = j < Dv && odd_from < n;
 #pragma unroll
     for (int i = 0; i < 32; i += 8) {
       float r[4][8];
@@ -820,18 +886,24 @@ __global__ void __launch_bounds__(256, 2) gla_out_kernel(GlaArgs a) {
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         const int t = half * 32 + i + e;
-        acc[i + e] += (r[0][e] + r[1][e]) + (r[2][e] + r[3][e]);
-        if (t < n && j < Dv && (t >= odd_from || !(fabsf(acc[i + e]) < INFINITY))) odd |= 1u << (i + e);
+        const float v = __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(
+            tiles + GoPlace::v + (j >> 6) * GoPlace::tile + t * 128 + ((((j >> 3) & 7) ^ (t & 7)) << 4) + (j & 7) * 2));
+        acc[i + e] = fmaf(t < n ? own[t] : 0.f, v, ((acc[i + e] + (r[2][e] + r[3][e])) + r[0][e]) + r[1][e]);
       }
+      if (j < Dv) odd |= gc_none(reinterpret_cast<const float (&)[8]>(acc[i]));
     }
     // Such an output as 32-bit fmas, and up to its own token: an infinity taken apart into pieces is a NaN.  (All of them before one is
     // stored: P lies where they go.)
-    if (__syncthreads_or(odd != 0u)) {
+    if (__syncthreads_or(odd)) {
       const __nv_bfloat16* vb = (const __nv_bfloat16*)a.v + (size_t)h * Dv + j;
 #pragma unroll 1
-      for (uint32_t rest = odd; rest; rest &= rest - 1) {
-        const int i = __ffs(rest) - 1, t = half * 32 + i;
+      for (int i = 0; i < (odd ? 32 : 0); ++i) {
+        const int t = half * 32 + i;
         float y = 0.f;
+#pragma unroll
+        for (int e = 0; e < 32; ++e) y = e == i ? acc[e] : y;
+        if (t >= n || (t < odd_from && fabsf(y) < INFINITY)) continue;
+        y = 0.f;
         for (int d = 0; d < D; d += 8) {
           float q[8];
           load_q8(t, d, q);

@@ -1675,8 +1675,8 @@ def ssm_output(o32: torch.Tensor, x: torch.Tensor, d_skip: torch.Tensor, z: torc
 
 DELTA_CHUNK = 64  # tokens of a chunk
 DELTA_ROW_BYTES = 128 * 128  # 128 rows of 64 channels or tokens as the tensor core reads them (csrc/delta_chunk.cu: kDcImage)
-# of a head: three pieces of T and A T, four factors a token, the decay of all (csrc/delta_chunk.cu: kDcHeadBytes)
-DELTA_HEAD_BYTES = 3 * DELTA_ROW_BYTES + 4 * DELTA_CHUNK * 4 + 16
+# of a head: three pieces of T and A T, five factors a token, the decay of all (csrc/delta_chunk.cu: kDcHeadBytes)
+DELTA_HEAD_BYTES = 3 * DELTA_ROW_BYTES + 5 * DELTA_CHUNK * 4 + 16
 
 
 def delta_chunk_scratch(dtype: torch.dtype, n_tokens: int, n_long: int, n_heads: int, n_kv_heads: int, dim: int, vdim: int) -> int:

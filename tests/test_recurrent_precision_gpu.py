@@ -1,0 +1,37 @@
+"""The chunked recurrences against 64 bits where decays are strong: one token's product is then most of a result, and sums that cut off
+instead of rounding would show."""
+
+import pytest
+import torch
+
+import test_delta_chunks_gpu as delta
+import test_gla_chunks_gpu as gla
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("kw", [dict(D=128, Dv=128), dict(D=64, Dv=64), dict(D=128, Dv=128, decay="head"), dict(D=128, Dv=128, decay="fixed")], ids=str)
+@pytest.mark.parametrize("bias", [-6.0, -2.0, 0.0])
+def test_linear_attention_loses_nothing_where_decays_are_strong(kw, bias):
+    """Lengths whose last chunk ends in the middle and at the start of 16 tokens too."""
+    for lens in ([(1024, 1024)], [(1000, 1100), (209, 209)]):
+        p = gla.problem(lens, H=4, chunk=64, bias=bias, seed=len(lens), **kw)
+        want, want_state = gla.exact(p)
+        (out, state, taken), (plain, plain_state, _) = gla.run(p, 64), gla.run(p, 0)
+        used = p["slots"].long()
+        assert taken
+        # token by token a result is rounded a few times; the chunks measure 0.97 to 1.1 times that (with cut-off sums 1.2, states 2.0)
+        assert gla.rel(out, want) <= 1.12 * gla.rel(plain, want)
+        assert gla.rel(state[used], want_state[used]) <= 1.12 * gla.rel(plain_state[used], want_state[used])
+
+
+@pytest.mark.parametrize("D,Dv", [(128, 128), (64, 64)])
+@pytest.mark.parametrize("a_log", [2.5, 0.0, -1.0])
+def test_the_delta_rule_loses_nothing_where_decays_are_strong(D, Dv, a_log):
+    for lens in ([(512, 600)], [(450, 450), (65, 65)]):
+        p = delta.problem(lens, 4, 2, D, Dv, seed=len(lens), a_log=a_log)
+        want, want_state = delta.exact(p)
+        (out, state), (plain, plain_state) = delta.run(p, True), delta.run(p, False)
+        used = p["slots"].long()
+        assert delta.off(out, want) <= 1.02 * delta.off(plain, want)
+        assert delta.off(state[used], want_state[used]) <= 1.02 * delta.off(plain_state[used], want_state[used])
