@@ -169,9 +169,9 @@ attention_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
       // the piece, the queries are given back
       auto scores = [&](int x, int j) -> bool {
         const int g = g0 + j, ks = g % kTc2Stages;
-        if (x == 0 && !all_of_warp(mbar_wait(&k_full[ks], (uint32_t)(g / kTc2Stages) & 1u, abortp))) return false;
+        const bool there = x != 0 || mbar_wait(&k_full[ks], (uint32_t)(g / kTc2Stages) & 1u, abortp);
         tc_fence_after();
-        if (elect_one()) {
+        if (elect_one()) if (there) {
           const uint32_t d = tmem + (uint32_t)(x * kTcKeys);
 #pragma unroll
           for (int kk = 0; kk < 4 * kHalves; ++kk) {  // 16 elements of the head dimension per MMA
@@ -185,15 +185,14 @@ attention_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             if (j == n_tiles - 1) tc_commit(&q_empty);
           }
         }
-        __syncwarp();
-        return true;
+        return all_of_warp(there);
       };
       // O_x += P_x(j) V(j); the first of a piece waits until the piece before has read its output
       auto product = [&](int x, int j) -> bool {
         const int g = g0 + j, vs = g % kTc2Stages;
-        if (!all_of_warp(mbar_wait(&p_full[x], (uint32_t)((gx[x] + j) & 1), abortp))) return false;
+        bool there = mbar_wait(&p_full[x], (uint32_t)((gx[x] + j) & 1), abortp);
         if (x == 0) {
-          if (!all_of_warp(mbar_wait(&v_full[vs], (uint32_t)(g / kTc2Stages) & 1u, abortp))) return false;
+          there = there && mbar_wait(&v_full[vs], (uint32_t)(g / kTc2Stages) & 1u, abortp);
           const int live = it.ke - (it.kb + j * kTcKeys);  // keys of the request in this tile
           if (live < kTcKeys) {
             // the value rows past the end of the request: zero, whatever the page holds there and
@@ -206,10 +205,10 @@ attention_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             fence_async_smem();
           }
         }
-        if (j == 0 && !all_of_warp(mbar_wait(&o_free[x], (uint32_t)(px[x] & 1) ^ 1u, abortp))) return false;
+        there = there && (j != 0 || mbar_wait(&o_free[x], (uint32_t)(px[x] & 1) ^ 1u, abortp));
         __syncwarp();
         tc_fence_after();
-        if (elect_one()) {
+        if (elect_one()) if (there) {
           const uint32_t d = tmem + (uint32_t)((2 + x) * kTcKeys);
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk) {  // 16 keys per MMA
@@ -220,8 +219,7 @@ attention_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
           tc_commit(&pv_done[x]);
           if (x == n_q - 1) tc_commit(&v_empty[vs]);
         }
-        __syncwarp();
-        return true;
+        return all_of_warp(there);
       };
       for (int x = 0; x < n_q && ok; ++x) ok = scores(x, 0);
       for (int j = 0; j < n_tiles && ok; ++j)
