@@ -48,27 +48,28 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
       : "=r"(ok) : "r"(smem_addr(bar)), "r"(parity) : "memory");
   return ok != 0;
 }
-// Asked once, for up to kTryNs: the barrier's unit wakes the thread when it flips.
-constexpr uint32_t kTryNs = 20000;
+// Asked once: the barrier's unit wakes the thread when it flips, or after a while of its own.
 __device__ __forceinline__ bool mbar_try(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok) : "r"(smem_addr(bar)), "r"(parity), "r"(kTryNs) : "memory");
+      : "=r"(ok) : "r"(smem_addr(bar)), "r"(parity) : "memory");
   return ok != 0;
 }
 // Bounded waits: false when the barrier did not flip within the limit (or another role gave up).  The first leaves the asking to the
 // barrier's unit: asked again and again by a tile's softmax threads, it is in the way of products that read shared memory at its full
 // rate (prompt attention 85 -> 81 us, a portion over 32k keys 557 -> 533, the chunks of the delta rule 183 -> 177).  Its limit is a time,
-// as a try may last anything up to its own: 2^31 cycles, 1.1 s at 1,965 MHz.
+// as a try lasts as long as the hardware sees fit: 2^31 cycles, 1.1 s at 1,965 MHz, and eight tries more.
 constexpr uint32_t kWaitCycles = 1u << 31;
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
   if (mbar_try(bar, parity)) return true;
   const uint32_t from = (uint32_t)clock();
   do {
-    if (mbar_try(bar, parity)) return true;
+#pragma unroll 1
+    for (int i = 0; i < 8; ++i)
+      if (mbar_try(bar, parity)) return true;
     if (*abort_flag) return false;
   } while ((uint32_t)clock() - from < kWaitCycles);
   return false;
