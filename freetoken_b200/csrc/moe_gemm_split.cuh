@@ -1,7 +1,7 @@
 // Grouped expert products in 32 bits on the tensor cores.  Included by moe_gemm.cu after find_tile and finish.
 //
 // A tile is 128 of an expert's rows x 128 weight rows (64 gate and 64 up rows), k in steps of 64.  Every operand is taken apart into
-// three bfloat16 numbers whose sum it is (split3), and the six products that reach 2^-24 are taken:
+// three bfloat16 numbers whose sum it is (split3; from 2^-110 up exactly), and the six products that reach 2^-24 are taken:
 //   a1 b1                    the leading product: a chain of four steps of 16 in one of two places in tensor memory, read and added up in
 //                            registers while the next step fills the other (the tensor core's accumulator cuts off instead of rounding)
 //   a1 b2 + a2 b1            second order, 2^-9 smaller, and

@@ -289,7 +289,7 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
 }
 
 // Two 32-bit numbers in three words of two bfloat16, whose sums they are: rounded to nearest, so that the pieces shrink by 2^-9 and what
-// is left after the second fits the third.  (An infinity leaves a NaN in the second.)
+// is left after the second fits the third.  (An infinity leaves a NaN in the second; below 2^-110 the third loses what lies under 2^-133.)
 struct Pieces { uint32_t w[3]; };
 __device__ __forceinline__ Pieces split3(float x, float y) {
   Pieces p;

@@ -31,3 +31,15 @@ def test_where_the_library_hands_over():
     ops.variant_counts(reset=True)
     ops.linear(wide[:, :64], torch.randn(600, 64, device=DEV), torch.empty(1000, 600, device=DEV))
     assert not ops.variant_counts().get("linear: float32 on the tensor cores")
+
+
+@pytest.mark.parametrize("small,large", [(2.0 ** -100, 2.0 ** 60), (2.0 ** -112, 2.0 ** 80), (2.0 ** -124, 2.0 ** 100)])
+def test_numbers_that_the_third_piece_does_not_reach(small, large):
+    """Three bfloat16 numbers hold a 32-bit one down to 2^-110; of smaller ones they leave out what lies under 2^-133."""
+    g = torch.Generator(device=DEV).manual_seed(7)
+    x, w = torch.randn(130, 256, device=DEV, generator=g) * small, torch.randn(130, 256, device=DEV, generator=g) * large
+    out = torch.empty(130, 130, device=DEV)
+    ops.linear_split(x, w, out)
+    want, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    left_out = 2.0 ** -134 * w.double().abs().sum(1)
+    assert ((out - want).abs() <= (2.0 ** -21 + 8 * 2.0 ** -24) * size + left_out).all()
