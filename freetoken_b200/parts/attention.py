@@ -42,6 +42,7 @@ TC_MIN_TOKENS = 128      # shortest step that goes to the tcgen05 attention kern
 TC_PAIR_MIN_TOKENS = 1024  # from this many tokens on, a step goes to the kernel with two query tiles per CTA
 TC_PAIR_MIN_TOKENS_LONG = 256  # ... and from this many on when its longest request has TC_PAIR_MIN_SPAN keys and more
 TC_PAIR_MIN_SPAN = 16384       # (rounded up to 2^n): such tiles are cut along the keys into enough pieces for every SM
+AHEAD_MOST_BYTES = 40_000_000  # largest weight that a single token's attention brings into L2 (see GQAttention._weight_ahead)
 TC_MIN_DECODE_SPAN = 0   # decode steps go there from this length of the longest request (rounded up to 2^n) on
 
 
@@ -319,11 +320,15 @@ class GQAttention(Mixer):
 
     def _weight_ahead(self, n_tokens: int, weight: torch.Tensor) -> Dict[str, torch.Tensor]:
         """A single token's attention leaves memory idle while its splits' few tiles come in: the output projection's weight is then
-        brought into L2 meanwhile, as long as the keys and values are not more than it.  48 heads on 8 of 128, weight 37.7 MB, a
-        layer's attention: 1,024 tokens 31.2 -> 29.3 us, 4,096 33.9 -> 31.6, 8,192 37.8 -> 35.5, but 16,384 42.3 -> 44.2 and 32,768
-        57.4 -> 60.5; two tokens of 2,048 35.5 -> 37.2, of 1,024 33.4 and 33.4; 16 heads on 4: the same within 2 %."""
+        brought into L2 meanwhile, where it and the keys and values stay well inside: a weight of at most 40 MB, cached rows of at most a
+        quarter of it.  48 heads on 8 of 128, weight 37.7 MB, a layer's attention with layers of other weights in turn: 1,024 tokens 31.2
+        -> 29.3 us, 2,048 33.1 -> 30.9; with all of L2 read by others before each: 100 tokens 34.9 -> 33.2, 500 36.2 -> 35.7, 2,048 37.1
+        -> 37.5, but 4,096 37.3 -> 39.4 and 8,192 41.3 -> 43.3; a weight of 52 MB 2,048 45.3 -> 46.1, 4,096 46.5 -> 49.7, one of
+        134 MB (past L2) 100 64 -> 72.  16 heads on 4 within 2 % either way.  Layers with a bias by distance lose up to 1 us and those
+        with a gate gain or lose 1.5: they do not ask."""
+        size = weight.numel() * weight.element_size()
         cached = 2 * self._step_span * self.n_kv_heads * self.pad_dim * weight.element_size()
-        if n_tokens == 1 and self._step_plan[6] and weight.is_contiguous() and cached <= weight.numel() * weight.element_size():
+        if n_tokens == 1 and self._step_plan[6] and weight.is_contiguous() and size <= AHEAD_MOST_BYTES and 4 * cached <= size:
             return {"ahead": weight}
         return {}
 
@@ -361,8 +366,7 @@ class GQAttention(Mixer):
                             len(step.segments), plan.items_dev, plan.n_items, plan.part_o, plan.part_ml,
                             o, self._step_plan[2], self.scale, self.window, few_rows=self._step_plan[6],
                             kv_split=self.kv_split, sink=self.params["sink"] if self.learned_sink else self.sink,
-                            dist_bias=self.dist_table(), keep_first=self.keep_first,
-                            **self._weight_ahead(T, self._o_weight))
+                            dist_bias=self.dist_table(), keep_first=self.keep_first)
         if self.out_gate:
             ops.gated_heads(o, proj[:, self.g_row:], o, Dv, self.out_gate)
         out = ws.get("attn.out", (T, self.hidden), dt, (cap, self.hidden))
