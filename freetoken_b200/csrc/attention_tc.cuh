@@ -668,13 +668,14 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         ok = false;
         break;
       }
+      bool fine = true;  // this lane's waits; the warp votes on them once a key tile
       for (int j = 0; j <= n_tiles && ok; ++j) {
         if (j < n_tiles) {
           const int g = g0 + j, st = g & 1, ks = g % kTcStages;  // score buffer, key stage
           const uint32_t par = (g >> 1) & 1;
-          const bool there = mbar_wait2(&k_full[ks], (uint32_t)(g / kTcStages) & 1u, &s_empty[st], par ^ 1, abortp);
+          if (!mbar_wait2(&k_full[ks], (uint32_t)(g / kTcStages) & 1u, &s_empty[st], par ^ 1, abortp)) { fail(204); fine = false; }
           tc_fence_after();
-          if (elect_one()) if (there) {
+          if (elect_one()) if (fine) {
             const uint32_t d = tmem + (uint32_t)(st * kTcKeys);
 #pragma unroll
             for (int kk = 0; kk < 4 * kHalves; ++kk) {  // 16 elements of the head dimension per MMA
@@ -686,19 +687,18 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             tc_commit(&s_full[st]);
             if (j == n_tiles - 1) tc_commit(&q_empty);  // the next piece's queries may come
           }
-          if (!all_of_warp(there)) {
-            if (lane == 0) fail(204);
-            ok = false;
-            break;
-          }
+          __syncwarp();
         }
         if (j >= 1) {
           const int i = j - 1, g = g0 + i, st = g & 1, vs = g % kTcStages;  // probability buffer, value stage
           const uint32_t par = (g >> 1) & 1;
           // (tied values: the stage's keys have been waited for before the first product)
-          const bool there = (tied ? mbar_wait(&p_full[st], par, abortp)
-                                   : mbar_wait2(&p_full[st], par, &v_full[vs], (uint32_t)(g / kTcStages) & 1u, abortp)) &&
-                             (i != 0 || mbar_wait(&o_free, (uint32_t)(qi & 1) ^ 1u, abortp));  // the piece before has read its output
+          if (!(tied ? mbar_wait(&p_full[st], par, abortp)
+                     : mbar_wait2(&p_full[st], par, &v_full[vs], (uint32_t)(g / kTcStages) & 1u, abortp)) ||
+              (i == 0 && !mbar_wait(&o_free, (uint32_t)(qi & 1) ^ 1u, abortp))) {  // the piece before has read its output
+            fail(205);
+            fine = false;
+          }
           const int key0 = it.kb + i * kTcKeys;
           const int live = it.ke - key0;  // keys of the request in this tile
           if (p.window > 0) {
@@ -728,7 +728,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
           }
           __syncwarp();
           tc_fence_after();
-          if (elect_one()) if (there) {
+          if (elect_one()) if (fine) {
             const uint32_t d = tmem + 2 * kTcKeys;
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk) {  // 16 keys per MMA
@@ -739,12 +739,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             tc_commit(tied ? &k_empty[vs] : &v_empty[vs]);
             tc_commit(&pv_done[st]);
           }
-          if (!all_of_warp(there)) {
-            if (lane == 0) fail(205);
-            ok = false;
-            break;
-          }
+          __syncwarp();
         }
+        ok = all_of_warp(fine);
       }
       g0 += n_tiles;
       ++qi;

@@ -165,13 +165,14 @@ attention_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         ok = false;
         break;
       }
+      bool fine = true;  // this lane's waits; the warp votes on them once a key tile
       // S_x(j) = Q_x K(j)^T; after the last tile's scores of the last query tile the key stage and, at the end of
       // the piece, the queries are given back
-      auto scores = [&](int x, int j) -> bool {
+      auto scores = [&](int x, int j) {
         const int g = g0 + j, ks = g % kTc2Stages;
-        const bool there = x != 0 || mbar_wait(&k_full[ks], (uint32_t)(g / kTc2Stages) & 1u, abortp);
+        if (x == 0 && !mbar_wait(&k_full[ks], (uint32_t)(g / kTc2Stages) & 1u, abortp)) { fail(304); fine = false; }
         tc_fence_after();
-        if (elect_one()) if (there) {
+        if (elect_one()) if (fine) {
           const uint32_t d = tmem + (uint32_t)(x * kTcKeys);
 #pragma unroll
           for (int kk = 0; kk < 4 * kHalves; ++kk) {  // 16 elements of the head dimension per MMA
@@ -185,14 +186,14 @@ attention_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             if (j == n_tiles - 1) tc_commit(&q_empty);
           }
         }
-        return all_of_warp(there);
+        __syncwarp();
       };
       // O_x += P_x(j) V(j); the first of a piece waits until the piece before has read its output
-      auto product = [&](int x, int j) -> bool {
+      auto product = [&](int x, int j) {
         const int g = g0 + j, vs = g % kTc2Stages;
-        bool there = mbar_wait(&p_full[x], (uint32_t)((gx[x] + j) & 1), abortp);
+        if (!mbar_wait(&p_full[x], (uint32_t)((gx[x] + j) & 1), abortp)) { fail(304); fine = false; }
         if (x == 0) {
-          there = there && mbar_wait(&v_full[vs], (uint32_t)(g / kTc2Stages) & 1u, abortp);
+          if (!mbar_wait(&v_full[vs], (uint32_t)(g / kTc2Stages) & 1u, abortp)) { fail(304); fine = false; }
           const int live = it.ke - (it.kb + j * kTcKeys);  // keys of the request in this tile
           if (live < kTcKeys) {
             // the value rows past the end of the request: zero, whatever the page holds there and
@@ -205,10 +206,10 @@ attention_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             fence_async_smem();
           }
         }
-        there = there && (j != 0 || mbar_wait(&o_free[x], (uint32_t)(px[x] & 1) ^ 1u, abortp));
+        if (j == 0 && !mbar_wait(&o_free[x], (uint32_t)(px[x] & 1) ^ 1u, abortp)) { fail(304); fine = false; }
         __syncwarp();
         tc_fence_after();
-        if (elect_one()) if (there) {
+        if (elect_one()) if (fine) {
           const uint32_t d = tmem + (uint32_t)((2 + x) * kTcKeys);
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk) {  // 16 keys per MMA
@@ -219,18 +220,17 @@ attention_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
           tc_commit(&pv_done[x]);
           if (x == n_q - 1) tc_commit(&v_empty[vs]);
         }
-        return all_of_warp(there);
+        __syncwarp();
       };
-      for (int x = 0; x < n_q && ok; ++x) ok = scores(x, 0);
-      for (int j = 0; j < n_tiles && ok; ++j)
-        for (int x = 0; x < n_q && ok; ++x) {
-          ok = product(x, j);
-          if (ok && j + 1 < n_tiles) ok = scores(x, j + 1);
+      for (int x = 0; x < n_q; ++x) scores(x, 0);
+      for (int j = 0; j < n_tiles && ok; ++j) {
+        for (int x = 0; x < n_q; ++x) {
+          product(x, j);
+          if (j + 1 < n_tiles) scores(x, j + 1);
         }
-      if (!ok) {
-        if (lane == 0) fail(304);
-        break;
+        ok = all_of_warp(fine);
       }
+      if (!ok) break;
       g0 += n_tiles;
       ++qi;
       for (int x = 0; x < n_q; ++x) {

@@ -161,12 +161,13 @@ attention_tc_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         ok = false;
         break;
       }
+      bool fine = true;  // this lane's waits; the warp votes on them once a key tile
       for (int j = 0; j <= n_tiles && ok; ++j) {
         if (j < n_tiles) {
           const int g = g0 + j, s0 = (2 * g) % ring_k, s1 = (2 * g + 1) % ring_k;
-          const bool there = mbar_wait2(&k_full[s0], (uint32_t)((2 * g) / ring_k) & 1u, &k_full[s1], (uint32_t)((2 * g + 1) / ring_k) & 1u, abortp);
+          if (!mbar_wait2(&k_full[s0], (uint32_t)((2 * g) / ring_k) & 1u, &k_full[s1], (uint32_t)((2 * g + 1) / ring_k) & 1u, abortp)) { fail(404); fine = false; }
           tc_fence_after();
-          if (elect_one()) if (there) {
+          if (elect_one()) if (fine) {
             const uint32_t d = tmem + (uint32_t)((g & 1) * kTcKeys);
             if (s1 > s0) {  // the tile's two steps lie one behind the other
 #pragma unroll
@@ -191,19 +192,16 @@ attention_tc_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             tc_commit(&s_full[g & 1]);
             if (j == n_tiles - 1) tc_commit(&q_empty);  // the next piece's queries may come
           }
-          if (!all_of_warp(there)) {
-            if (lane == 0) fail(404);
-            ok = false;
-            break;
-          }
+          __syncwarp();
         }
         if (j >= 1) {
           const int i = j - 1, g = g0 + i, s0 = (2 * g) % ring_v, s1 = (2 * g + 1) % ring_v;
-          bool there = mbar_wait(&p_full[g & 1], (uint32_t)(g >> 1) & 1u, abortp);
+          bool here = mbar_wait(&p_full[g & 1], (uint32_t)(g >> 1) & 1u, abortp);
           // (one slab: the steps have been waited for before the first product)
-          if (there && !tied)
-            there = mbar_wait2(&val_full[s0], (uint32_t)((2 * g) / ring_v) & 1u, &val_full[s1], (uint32_t)((2 * g + 1) / ring_v) & 1u, abortp);
-          if (there && i == 0) there = mbar_wait(&o_free, (uint32_t)(qi & 1) ^ 1u, abortp);  // the piece before has read its output
+          if (here && !tied)
+            here = mbar_wait2(&val_full[s0], (uint32_t)((2 * g) / ring_v) & 1u, &val_full[s1], (uint32_t)((2 * g + 1) / ring_v) & 1u, abortp);
+          if (here && i == 0) here = mbar_wait(&o_free, (uint32_t)(qi & 1) ^ 1u, abortp);  // the piece before has read its output
+          if (!here) { fail(405); fine = false; }
           // value rows that no row of the tile reads are zeroed, whatever lies there: in front of a window's first key
           // (but for the kept first tokens), and past the request's end
           const int key0 = it.kb + i * kTcKeys;
@@ -223,7 +221,7 @@ attention_tc_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
           if (it.ke - key0 < kTcKeys) clear(it.ke - key0, kTcKeys);
           __syncwarp();
           tc_fence_after();
-          if (elect_one()) if (there) {
+          if (elect_one()) if (fine) {
             const uint32_t d = tmem + 2 * kTcKeys;
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk) {  // 16 keys per MMA
@@ -235,12 +233,9 @@ attention_tc_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             tc_commit(&val_empty[s1]);
             tc_commit(&pv_done[g & 1]);
           }
-          if (!all_of_warp(there)) {
-            if (lane == 0) fail(405);
-            ok = false;
-            break;
-          }
+          __syncwarp();
         }
+        ok = all_of_warp(fine);
       }
       g0 += n_tiles;
       ++qi;

@@ -206,8 +206,8 @@ __device__ __forceinline__ void tc_mma_pair(uint32_t d_tmem, uint64_t a_desc, ui
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
 // Whether a wait ended well for every lane of a warp.  A lane may give up where another still saw its barrier flip; what the warp does
-// together next (elect.sync, tcgen05) would wait for that lane without end.  (Asked behind the products that were waited for: in front of
-// them it costs a portion over 32k keys 15 of 625 us.)
+// together next (elect.sync, tcgen05) would wait for that lane without end.  (Asked once a key tile, behind the products: in front of
+// each of them it costs a portion over 32k keys 15 of 625 us, behind each 10.)
 __device__ __forceinline__ bool all_of_warp(bool ok) { return __all_sync(0xffffffffu, ok); }
 // One lane of a warp that is together, the same one each time.  (Products issued behind it, instead of behind a comparison of the
 // lane's number, leave their thread every 31 instead of every 51 cycles: the compiler sees that their operands are the warp's.  A

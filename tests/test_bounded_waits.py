@@ -16,18 +16,21 @@ def sources():
 
 
 def test_what_a_warp_does_together_follows_waits_that_end_alike_for_all_its_lanes():
-    """Lanes of a warp that give up singly would leave the others at elect.sync and tcgen05 instructions without end."""
+    """Lanes of a warp that give up singly would leave the others at elect.sync and tcgen05 instructions without end: every wait is voted
+    on, at once or (issuing warps) at the end of the key tile, with no way out before that."""
     seen = 0
     for name, text in sources():
         if not name.startswith("attention_tc"):
             continue
         for m in re.finditer(r"mbar_wait2?\(", text):
-            before = text[text.rindex(";", 0, m.start()):m.start()]
-            assert "all_of_warp(" in before or "__all_sync(" in before or "there =" in before, (name, text[m.start() - 80:m.end() + 60])
-            if "there =" in before:  # (kept until the warp has voted, with no way out before it)
-                issue = re.sub(r"return\s*$", "", text[m.end():text.index("all_of_warp(there)", m.end())])
-                assert "if (elect_one()) if (there)" in issue and not re.search(r"\b(break|return|continue)\b", issue)
+            before = text[max(text.rindex(";", 0, m.start()), text.rindex("{", 0, m.start())):m.start()]
             seen += 1
+            if "all_of_warp(" in before or "__all_sync(" in before:
+                continue
+            rest = text[m.end():text.index("ok = all_of_warp(fine)", m.end())]
+            assert "fine = false;" in rest[:600] and not re.search(r"\b(break|return|continue)\b", rest), (name, text[m.start() - 80:m.end() + 60])
+        for issue in re.finditer(r"elect_one\(\)\) ([^\n]*)", text):
+            assert issue.group(1).startswith("if (fine)")
     assert seen > 25
 
 
