@@ -449,7 +449,7 @@ __global__ void __launch_bounds__(2 * D, 256 / D) gla_local_kernel(GlaArgs a) {
     }
     a.decay_prod[((size_t)c * a.H + h) * D + tid] = hi;
   }
-  const int two = (n - 1) % kGcBlock != 0;
+  const bool two = n >= 2;
   // the chunk's contribution: keys decayed to its end, in three pieces; a thread has eight channels of a token of every 16
   {
     constexpr int kPass = kThreads / kLanes;  // tokens at a time
@@ -466,18 +466,18 @@ __global__ void __launch_bounds__(2 * D, 256 / D) gla_local_kernel(GlaArgs a) {
     for (int b = 0; b < kGcBlocks; ++b) {
       const int t = b * kGcBlock + t0;
       float y[8];
-      if (t >= n - 1 - two && t < n) {  // (the newest tokens': added in registers)
-        *reinterpret_cast<uint4*>(pieces + (d >> 6) * (kGcTokens * 128) + t * 128 + ((((d >> 3) & 7) ^ (t & 7)) << 4)) = make_uint4(0u, 0u, 0u, 0u);
-        *reinterpret_cast<uint4*>(pieces + sh.piece + (d >> 6) * (kGcTokens * 128) + t * 128 + ((((d >> 3) & 7) ^ (t & 7)) << 4)) = make_uint4(0u, 0u, 0u, 0u);
-        *reinterpret_cast<uint4*>(pieces + 2 * sh.piece + (d >> 6) * (kGcTokens * 128) + t * 128 + ((((d >> 3) & 7) ^ (t & 7)) << 4)) = make_uint4(0u, 0u, 0u, 0u);
-        continue;
-      }
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         uint64_t kv = *reinterpret_cast<const uint64_t*>(&sh.k[t][d + 2 * j]);
 #pragma unroll
         for (int m = b + 1; m < kGcBlocks; ++m) kv = f2_mul(kv, lam[m - 1][j]);
         f2_unpair(kv, y[2 * j], y[2 * j + 1]);
+      }
+      if (t >= n - 2 && t < n) {  // (the newest tokens' are added in registers, from here)
+        Vec4<float>::store(&sh.k[t][d], reinterpret_cast<float (&)[4]>(y[0]));
+        Vec4<float>::store(&sh.k[t][d + 4], reinterpret_cast<float (&)[4]>(y[4]));
+#pragma unroll
+        for (int j = 0; j < 8; ++j) y[j] = 0.f;
       }
       uint4 w[3];
       split3(y, w);
@@ -491,10 +491,10 @@ __global__ void __launch_bounds__(2 * D, 256 / D) gla_local_kernel(GlaArgs a) {
   __syncthreads();
   // Products, two sums of them at a time (2 D columns): the second and third pieces' and the first's of 32 tokens, then the first's of the
   // other 32.  They are added up in registers, and the two newest tokens', the largest where decays are strong, last and by themselves:
-  // the accumulator cuts off instead of rounding.  (Two, where they lie in the same 16; else the newest.)
+  // the accumulator cuts off instead of rounding.
   const int j = (warp & 3) * 32 + lane;  // a value column; 64 channels of it
   const uint32_t my_tmem = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)((warp >> 2) * 64);
-  const float* k_last = &sh.k[n - 1][(warp >> 2) * 64];  // (no token after it decays it; the one before lies, decayed by it, a row in front)
+  const float* k_last = &sh.k[n - 1][(warp >> 2) * 64];
   auto value = [&](int t) {
     return __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(sh.v + (j >> 6) * (kGcTokens * 128) + t * 128 + ((((j >> 3) & 7) ^ (t & 7)) << 4) + (j & 7) * 2));
   };
@@ -555,7 +555,7 @@ __global__ void __launch_bounds__(2 * D, 256 / D) gla_local_kernel(GlaArgs a) {
         if (gc_none(y)) {
 #pragma unroll
           for (int e = 0; e < 8; ++e)
-            if (!(fabsf(y[e]) < INFINITY)) y[e] = gc_contribution<D, VT>(sh, (warp >> 2) * 64 + i + e, j, n - 1 - two);
+            if (!(fabsf(y[e]) < INFINITY)) y[e] = gc_contribution<D, VT>(sh, (warp >> 2) * 64 + i + e, j, n - 2);
         }
 #pragma unroll
         for (int e = 0; e < 8; ++e) dst[(size_t)(i + e) * a.Dv] = y[e];
