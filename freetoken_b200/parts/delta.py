@@ -51,38 +51,14 @@ def token_time(states: float, wide: bool, v_dim: int) -> float:
     return 0.26 if rounds(16) <= 2 else max(0.36, 0.086 * rounds(16))
 
 
-def chunks_pay(lens: Sequence[int], beside: bool, n_heads: int, head_dim: int, v_dim: int) -> bool:
+def chunks_pay(lens: Sequence[int], beside: bool, n_heads: int, n_kv_heads: int, head_dim: int, v_dim: int) -> bool:
     """Whether requests of ``lens`` tokens are through sooner in chunks (``csrc/delta_chunk.cu``) than token by token
-    (``csrc/delta.cu``); ``beside``: the step has others, which then take a launch of their own.  A rule on the safe side: it was fitted
-    to chunks as 32-bit fmas on the CUDA cores, and is kept for what it names (the products on tcgen05 are faster at all of that);
-    :func:`pairs_pay` adds what only they make worth while.
-
-    Both kernels are chains (of chunks, of tokens) until a step has more blocks than the GPU holds at once, then waves or a rate.
-    Fitted to timings of both (heads of 64 and 128, 4 to 48 of them, 1 to 32 requests of 32 to 2,048 tokens, 16 to 256 value
-    channels).  One request, 48 heads of 128, token by token against chunks: 37 and 40 us for 64 tokens, 43 and 44 for 80, 51 and
-    46 for 96, 63 and 50 for 128, 227 and 120 for 512; 16 heads of 64: 23 and 26, 29 and 28, 32 and 28, 41 and 30, 139 and 54.
-    Many requests fill the GPU token by token as well: 32 heads of 128, four of 256 tokens 162 and 177, eight of 512 612 and 644;
-    48 heads, eight of 128 tokens 248 and 247, two of 512 311 and 220."""
-    longest = max(lens)
-    states = sum(lens) / longest * n_heads  # (request, head) pairs at work, on average
-    wide = head_dim > 64
-    rounds = lambda cols: math.ceil(states * -(-v_dim // cols) / SMS)  # noqa: E731  (blocks of so many value columns an SM)
-    chunks = -(-longest // 32)
-    if states * -(-v_dim // 16) <= 2 * SMS:  # (blocks of 16 or 48 columns)
-        in_chunks = 22.5 + chunks * (2.6 if wide else 1.7) * (1.0 if rounds(16) == 1 else 1.5 if wide else 2.1)
-    else:
-        in_chunks = (22.0 + rounds(48) * (4.5 + 5.2 * chunks)) if wide else (17.0 + rounds(48) * (3.0 + 3.5 * chunks))
-    in_chunks += 0.014 * states * chunks + (6.0 if beside else 0.0)
-    return in_chunks < 8.0 + longest * token_time(states, wide, v_dim)
-
-
-def pairs_pay(lens: Sequence[int], beside: bool, n_heads: int, n_kv_heads: int, head_dim: int, v_dim: int) -> bool:
-    """Whether requests of ``lens`` tokens are through sooner in chunks on tcgen05 than token by token;
-    arguments as :func:`chunks_pay`.
+    (``csrc/delta.cu``); ``beside``: the step has others, which then take a launch of their own.
 
     Both kernels are chains (of chunks, of tokens) until a step has more blocks than the GPU holds at once, then waves or a
-    rate; the chunks also have a launch that prepares them, two blocks an SM.  Fitted to timings of both (heads of 64 and 128, 4 to 48
-    of them, 1 to 16 requests of 32 to 2,048 tokens, 16 to 256 value columns; 5 % off on average).  One request, 48 heads of 128, token
+    rate; the chunks also have a launch that prepares them, two blocks an SM.  Fitted to 620 timings of both (heads of 64 and 128, 4 to 48 of
+    them, 1 to 32 requests of 80 to 2,048 tokens, most of at most 192, 16 to 256 value columns): the slower one is named in 27, 0.4 % lost on
+    average, a third at most (16 requests of 112 tokens, 48 heads of 64 on 24, 48 columns: 149 and 201).  One request, 48 heads of 128, token
     by token against chunks: 43 and 40 us for 80 tokens, 50 and 36 for 96, 64 and 38 for 128, 224 and 72 for 512; 16 heads of 64: 29
     and 29, 33 and 29, 41 and 30, 139 and 44.  Many requests: 48 heads, 16 of 80 tokens 311 and 222, four of 512 604 and 199; 48 heads
     of 64 columns that share no keys, 16 of 80 160 and 188, of 128 244 and 198."""
@@ -90,11 +66,12 @@ def pairs_pay(lens: Sequence[int], beside: bool, n_heads: int, n_kv_heads: int, 
     states = sum(lens) / longest * n_heads  # (request, head) pairs at work, on average
     wide = head_dim > 64
     rounds = lambda cols: math.ceil(states * -(-v_dim // cols) / SMS)  # noqa: E731  (blocks of so many value columns an SM)
-    pairs = -(-longest // ops.DELTA_CHUNK)
-    chain = min(rounds(64) * (3.0 + 5.0 * pairs), rounds(16) * 3.0 * pairs)  # (as csrc/delta_chunk.cu: launch_delta_chunks)
-    in_chunks = 24.0 + chain * (1.0 if wide else 0.88) + (6.0 if beside else 0.0)
-    blocks = sum(lens) / longest * pairs * n_kv_heads * -(-(n_heads // n_kv_heads) // 2)  # (that prepare)
-    in_chunks += 16.0 * max(0.0, blocks / (2 * SMS) - 0.3)
+    chunks = -(-longest // ops.DELTA_CHUNK)
+    large = rounds(64) * (3 + 5 * chunks) < rounds(16) * 3 * chunks  # (blocks of 64 columns: csrc/delta_chunk.cu: launch_delta_chunks)
+    chain = rounds(64) * (4.3 + 6.4 * chunks) if large else rounds(16) * 4.2 * chunks
+    in_chunks = 22.4 + chain * (1.0 if wide else 0.88) + (6.0 if beside else 0.0)
+    blocks = sum(lens) / longest * chunks * n_kv_heads * -(-(n_heads // n_kv_heads) // 2)  # (that prepare)
+    in_chunks += 13.7 * max(0.0, blocks / (2 * SMS) - 0.35)
     return in_chunks < 8.0 + longest * token_time(states, wide, v_dim)
 
 
@@ -215,7 +192,7 @@ class GatedDelta(Mixer):
         args = dict(z=z)
         long = [seg.q_len for seg in step.segments if seg.q_len >= CHUNK_MIN_TOKENS] if z is None and h.is_cuda else []
         n_long = len(long)
-        if long and (chunks_pay(long, n_long < n_segs, H, D, Dv) or pairs_pay(long, n_long < n_segs, H, self.n_kv_heads, D, Dv)):
+        if long and chunks_pay(long, n_long < n_segs, H, self.n_kv_heads, D, Dv):
             rows, n = self.chunk_scratch(T, n_long)
             if n:  # (by rows: layers of other sizes have a buffer of their own, and no step asks for more rows)
                 row, most = n // rows, self.chunk_scratch(cap, cap // CHUNK_MIN_TOKENS)[0]

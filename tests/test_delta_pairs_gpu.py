@@ -6,7 +6,7 @@ import torch
 from test_delta_chunks_gpu import exact, off, problem, run
 
 from freetoken_b200.kernels import ops
-from freetoken_b200.parts.delta import pairs_pay
+from freetoken_b200.parts.delta import chunks_pay
 
 gpu = pytest.mark.gpu
 EDGES = [(63, 63), (64, 80), (65, 65), (127, 300), (128, 128), (129, 129)]
@@ -39,8 +39,8 @@ def test_no_number_reaches_no_earlier_token_in_blocks_of_64(what, at, value):
     assert ops.read_status() == 0
 
 
-@pytest.mark.parametrize("lens,heads,kv,dim,vdim,tokens_us,pairs_us", [
+@pytest.mark.parametrize("lens,heads,kv,dim,vdim,tokens_us,chunks_us", [
     ([80], 48, 8, 128, 128, 43, 40), ([96], 16, 4, 64, 64, 33, 29), ([128] * 8, 16, 4, 128, 128, 86, 56), ([256] * 4, 32, 4, 128, 128, 162, 75),
     ([512] * 8, 32, 8, 64, 64, 299, 161), ([128] * 16, 48, 48, 128, 64, 244, 198), ([80], 16, 4, 128, 32, 29, 32), ([128] * 16, 24, 3, 64, 16, 49, 77)])
-def test_the_faster_kernel_is_named(lens, heads, kv, dim, vdim, tokens_us, pairs_us):
-    assert pairs_pay(lens, False, heads, kv, dim, vdim) == (pairs_us < tokens_us)
+def test_the_faster_kernel_is_named(lens, heads, kv, dim, vdim, tokens_us, chunks_us):
+    assert chunks_pay(lens, False, heads, kv, dim, vdim) == (chunks_us < tokens_us)

@@ -7,14 +7,15 @@ from freetoken_b200.kernels import ops
 from freetoken_b200.parts.delta import chunks_pay
 
 
-@pytest.mark.parametrize("lens,heads,dim,vdim,tokens_us,chunks_us", [
-    ([80], 48, 128, 128, 43, 44), ([96], 48, 128, 128, 51, 46), ([512], 48, 128, 128, 227, 120), ([80], 16, 128, 128, 29, 32),
-    ([96], 16, 128, 128, 35, 32), ([96], 16, 64, 64, 32, 28), ([128] * 2, 48, 128, 128, 88, 79), ([128] * 8, 16, 128, 128, 88, 107),
-    ([256] * 4, 32, 128, 128, 162, 177), ([256] * 4, 48, 128, 64, 162, 175), ([512] * 4, 48, 128, 128, 608, 427),
-    ([128] * 32, 48, 128, 128, 880, 949), ([256] * 16, 16, 64, 64, 156, 177), ([512] * 8, 16, 64, 64, 195, 173),
-    ([256] * 8, 48, 128, 80, 463, 345), ([2048], 48, 128, 16, 563, 316)])
-def test_the_faster_kernel_is_named(lens, heads, dim, vdim, tokens_us, chunks_us):
-    assert chunks_pay(lens, False, heads, dim, vdim) == (chunks_us < tokens_us)
+@pytest.mark.parametrize("lens,heads,kv,dim,vdim,tokens_us,chunks_us", [
+    ([80], 24, 12, 64, 64, 26.7, 29.9), ([80], 4, 1, 64, 64, 25.9, 28.9), ([80], 16, 4, 64, 64, 26.2, 27.4), ([80] * 8, 32, 16, 64, 32, 39.7, 55.1),
+    ([96] * 16, 48, 48, 64, 48, 129, 228), ([96] * 32, 24, 24, 64, 80, 207, 313), ([96] * 32, 32, 32, 128, 32, 237, 256),
+    ([192] * 16, 48, 24, 64, 32, 179, 205), ([192] * 8, 32, 32, 128, 16, 72.6, 79.6), ([80] * 32, 16, 8, 64, 80, 123, 183),
+    ([96], 48, 8, 128, 128, 50, 36), ([512], 48, 8, 128, 128, 224, 72), ([96], 24, 6, 128, 64, 31.9, 28.5), ([192] * 32, 16, 4, 64, 80, 281, 183),
+    ([256] * 8, 48, 48, 128, 64, 310, 182), ([2048] * 8, 16, 2, 128, 16, 533, 240), ([80] * 16, 32, 4, 128, 256, 361, 241),
+    ([96] * 32, 32, 32, 64, 128, 419, 295), ([128] * 32, 32, 16, 64, 48, 216, 176), ([2048] * 2, 32, 32, 64, 48, 568, 250)])
+def test_the_faster_kernel_is_named(lens, heads, kv, dim, vdim, tokens_us, chunks_us):
+    assert chunks_pay(lens, False, heads, kv, dim, vdim) == (chunks_us < tokens_us)
 
 
 @pytest.mark.parametrize("sizes", [(64, 1, 4, 2, 128, 64), (1, 1, 4, 2, 64, 16), (33, 2, 48, 8, 128, 128), (65536, 800, 65535, 5, 64, 4096),
