@@ -26,7 +26,7 @@ slot of the cache manager's state pool; both start from zero.  The reference has
 from __future__ import annotations
 
 import math
-from typing import Any, Dict, List, Sequence, Tuple
+from typing import Any, Dict, List, Optional, Sequence, Tuple
 
 import torch
 
@@ -51,42 +51,57 @@ def token_time(states: float, wide: bool, v_dim: int) -> float:
     return 0.26 if rounds(16) <= 2 else max(0.36, 0.086 * rounds(16))
 
 
-def chunks_pay(lens: Sequence[int], beside: bool, n_heads: int, n_kv_heads: int, head_dim: int, v_dim: int) -> bool:
+def chunk_time(lens: Sequence[int], n_heads: int, n_kv_heads: int, head_dim: int, v_dim: int) -> float:
+    """Microseconds of requests of ``lens`` tokens in chunks (``csrc/delta_chunk.cu``), in one pass."""
+    longest = max(lens)
+    states = sum(lens) / longest * n_heads  # (request, head) pairs at work, on average
+    rounds = lambda cols: math.ceil(states * -(-v_dim // cols) / SMS)  # noqa: E731  (blocks of so many value columns an SM)
+    chunks = -(-longest // ops.DELTA_CHUNK)
+    large = rounds(64) * (3 + 5 * chunks) < rounds(16) * 3 * chunks  # (blocks of 64 columns: csrc/delta_chunk.cu: launch_delta_chunks)
+    chain = rounds(64) * (4.3 + 6.4 * chunks) if large else rounds(16) * 4.2 * chunks
+    blocks = sum(lens) / longest * chunks * n_kv_heads * -(-(n_heads // n_kv_heads) // 2)  # (that prepare)
+    return 22.4 + chain * (1.0 if head_dim > 64 else 0.88) + 13.7 * max(0.0, blocks / (2 * SMS) - 0.35)
+
+
+def chunk_passes(lens: Sequence[int], most: int) -> List[Tuple[int, int, int, int, int]]:
+    """Requests of ``lens`` tokens in passes of at most ``most`` rows (of 64 tokens): first request and how many, rows from .. to of each of
+    them, and how many rows that is.  Whole requests side by side, as many as there are rows for (a state is read and written once); a
+    longer one by itself, in pieces."""
+    out, first, total, longest = [], 0, 0, 0
+    for i, n in enumerate(lens):
+        rows = -(-n // ops.DELTA_CHUNK)
+        if total and total + rows > most:
+            out.append((first, i - first, 0, longest, total))
+            total = longest = 0
+        if not total:
+            first = i
+        if rows > most:
+            out.extend((i, 1, r, min(r + most, rows), min(most, rows - r)) for r in range(0, rows, most))
+        else:
+            total, longest = total + rows, max(longest, rows)
+    if total:
+        out.append((first, len(lens) - first, 0, longest, total))
+    return out
+
+
+def chunks_pay(lens: Sequence[int], beside: bool, n_heads: int, n_kv_heads: int, head_dim: int, v_dim: int, most: Optional[int] = None) -> bool:
     """Whether requests of ``lens`` tokens are through sooner in chunks (``csrc/delta_chunk.cu``) than token by token
-    (``csrc/delta.cu``); ``beside``: the step has others, which then take a launch of their own.
+    (``csrc/delta.cu``); ``beside``: the step has others, which then take a launch of their own; ``most``: rows of scratch.
 
     Both kernels are chains (of chunks, of tokens) until a step has more blocks than the GPU holds at once, then waves or a
     rate; the chunks also have a launch that prepares them, two blocks an SM.  Fitted to 620 timings of both (heads of 64 and 128, 4 to 48 of
     them, 1 to 32 requests of 80 to 2,048 tokens, most of at most 192, 16 to 256 value columns): the slower one is named in 27, 0.4 % lost on
     average, a third at most (16 requests of 112 tokens, 48 heads of 64 on 24, 48 columns: 149 and 201).  One request, 48 heads of 128, token
-    by token against chunks: 43 and 40 us for 80 tokens, 50 and 36 for 96, 64 and 38 for 128, 224 and 72 for 512; 16 heads of 64: 29
-    and 29, 33 and 29, 41 and 30, 139 and 44.  Many requests: 48 heads, 16 of 80 tokens 311 and 222, four of 512 604 and 199; 48 heads
+    by token against chunks: 39 and 38 us for 80 tokens, 46 and 32 for 96, 59 and 37 for 128, 213 and 69 for 512; 16 heads of 64: 23
+    and 26, 27 and 26, 35 and 31, 127 and 40.  Many requests: 48 heads, 16 of 80 tokens 311 and 222, four of 512 604 and 199; 48 heads
     of 64 columns that share no keys, 16 of 80 160 and 188, of 128 244 and 198."""
+    parts = [lens]
+    if most is not None:
+        parts = [[min(n, row1 * ops.DELTA_CHUNK) - row0 * ops.DELTA_CHUNK for n in lens[first:first + count]]
+                 for first, count, row0, row1, _ in chunk_passes(lens, most)]
+    in_chunks = sum(chunk_time(p, n_heads, n_kv_heads, head_dim, v_dim) for p in parts) + (6.0 if beside else 0.0)
     longest = max(lens)
-    states = sum(lens) / longest * n_heads  # (request, head) pairs at work, on average
-    wide = head_dim > 64
-    rounds = lambda cols: math.ceil(states * -(-v_dim // cols) / SMS)  # noqa: E731  (blocks of so many value columns an SM)
-    chunks = -(-longest // ops.DELTA_CHUNK)
-    large = rounds(64) * (3 + 5 * chunks) < rounds(16) * 3 * chunks  # (blocks of 64 columns: csrc/delta_chunk.cu: launch_delta_chunks)
-    chain = rounds(64) * (4.3 + 6.4 * chunks) if large else rounds(16) * 4.2 * chunks
-    in_chunks = 22.4 + chain * (1.0 if wide else 0.88) + (6.0 if beside else 0.0)
-    blocks = sum(lens) / longest * chunks * n_kv_heads * -(-(n_heads // n_kv_heads) // 2)  # (that prepare)
-    in_chunks += 13.7 * max(0.0, blocks / (2 * SMS) - 0.35)
-    return in_chunks < 8.0 + longest * token_time(states, wide, v_dim)
-
-
-def chunk_passes(lens: Sequence[int], most: int) -> List[Tuple[int, int, int, int, int]]:
-    """Requests of ``lens`` tokens in passes of at most ``most`` rows (of 64 tokens): first request and how many, rows from .. to of each of
-    them, and how many rows that is.  Requests go side by side, as many as there are rows for, each as far as all of them can."""
-    out = []
-    for first in range(0, len(lens), most):
-        left = [-(-n // ops.DELTA_CHUNK) for n in lens[first:first + most]]
-        count, done = len(left), 0
-        while max(left) > 0:
-            far = max(m for m in range(1, max(left) + 1) if sum(min(r, m) for r in left) <= most)
-            out.append((first, count, done, done + far, sum(min(r, far) for r in left)))
-            left, done = [max(r - far, 0) for r in left], done + far
-    return out
+    return in_chunks < 8.0 + longest * token_time(sum(lens) / longest * n_heads, head_dim > 64, v_dim)
 
 
 @MIXERS.register("gated_delta")
@@ -192,9 +207,9 @@ class GatedDelta(Mixer):
         args = dict(z=z)
         long = [seg.q_len for seg in step.segments if seg.q_len >= CHUNK_MIN_TOKENS] if z is None and h.is_cuda else []
         n_long = len(long)
-        if long and chunks_pay(long, n_long < n_segs, H, self.n_kv_heads, D, Dv):
+        if long:
             rows, n = self.chunk_scratch(T, n_long)
-            if n:  # (by rows: layers of other sizes have a buffer of their own, and no step asks for more rows)
+            if n and chunks_pay(long, n_long < n_segs, H, self.n_kv_heads, D, Dv, rows):  # (by rows: layers of other sizes have a buffer of their own, and no step asks for more rows)
                 row, most = n // rows, self.chunk_scratch(cap, cap // CHUNK_MIN_TOKENS)[0]
                 args = dict(scratch=ws.get("delta.chunks", (rows, row), torch.uint8, (most, row)), long_from=CHUNK_MIN_TOKENS, n_long=n_long)
                 if rows < T // ops.DELTA_CHUNK + n_long:
