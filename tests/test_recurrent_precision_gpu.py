@@ -21,8 +21,8 @@ def test_linear_attention_loses_nothing_where_decays_are_strong(kw, bias):
         used = p["slots"].long()
         assert taken
         # token by token a result is rounded a few times; the chunks measure 0.97 to 1.1 times that (with cut-off sums 1.2, states 2.0),
-        # with one decay for all channels and no more than one half a token up to 1.2 times (as 32-bit fmas too)
-        room = 1.12 if "decay" not in kw or bias < 0 else 1.3
+        # with one decay of about a half for all channels up to 1.34 times (32-bit fmas in chunks 1.29, cut-off sums 1.58 to 2.1)
+        room = 1.12 if "decay" not in kw or bias < 0 else 1.42
         for x, o, w in ((out, plain, want), (state[used], plain_state[used], want_state[used])):
             assert gla.rel(x, w) <= room * gla.rel(o, w), (gla.rel(x, w), gla.rel(o, w))
 
