@@ -11,17 +11,18 @@
 // Decays are running products, never differences of logarithms.  The state is rounded once in 64 tokens.
 //
 // The three products run on tcgen05, in 32 bits: K and Q are bfloat16 as they lie, and S, T, X and U are taken apart into three
-// bfloat16 numbers each, every piece rounded to the nearest, whose sum is exactly the 32-bit one.  Of T X the six products
-// that reach 2^-24 are taken.  The tensor core's accumulator cuts off instead of rounding (measured: a bias of half a unit a step of
-// 16; one step, and two, are as close to 64 bits as a chain of as many fmas), so the products of the leading pieces are chains of two
-// steps, added up in registers; the other pieces' are 2^-8 smaller.
+// bfloat16 numbers each, every piece rounded to the nearest, whose sum is the 32-bit one (exactly from 2^-110 up).  Of T X the six products
+// that reach 2^-24 are taken.  The tensor core's accumulator cuts off instead of rounding, so the products of the leading pieces are
+// chains of two steps, added up in registers; the other pieces' are 2^-8 smaller.  What is most of a sum where decays are strong goes
+// through registers by itself: the diagonals of T and A T, and the newest token's share of the state.
 //
-// What bounds it: the chain of a chunk, product, registers, shared memory, product, which no other block can hide: the
-// tensor pipe is at work about half of the time.  With 64 columns a block, 48 heads of 128 x 128: 5.0 us a chunk (product 0.8, registers 1.1, product 0.8, registers
-// 0.7, product 0.5, registers 1.0); 16 columns a block, 16 heads: 2.9.
+// What bounds it: the chain of a chunk, product, registers, shared memory, product, which no other block can hide: an SM's
+// tensor pipe is at work about a third of the time.  With 64 columns a block, 48 heads of 128 x 128: 5.2 us a chunk (product 0.8, registers 1.1,
+// product 0.8, registers 0.7, product 0.5, registers 1.0, and what has gone through registers since); 16 columns a block, 16 heads: 2.9.
 // 2,048 tokens of one request, prep and chunks together (token by token, 32-bit fmas on the CUDA cores in chunks of 32, now): 48 heads of
-// 128 x 128 869, 431 and 228 us, 16 heads 563, 282 and 123; 16 heads of 64 x 64 535, 292 and 110.  Distance from 64 bits, token by token
-// and now: 2.5e-7 and 1.5e-7, with decays near one 2.4e-6 and 1.8e-7, with decays of e^-12 1.2e-7 and 1.1e-7.
+// 128 x 128 857, 431 and 234 us, 16 heads 529, 282 and 122; 16 heads of 64 x 64 493, 292 and 109.  Distance of outputs and states from 64
+// bits (512 tokens, heads of 128; token by token, as fmas, now): 1.5e-7 and 1.3e-7, 1.3 and 0.95, 1.2 and 0.85; with decays near one 16
+// and 21, 2.2 and 1.7, 1.6 and 1.3; of e^-12 1.1 and 0.91, 1.1 and 0.86, 1.0 and 0.80.
 #include "tc_common.cuh"
 
 namespace ftk {

@@ -15,14 +15,15 @@
 //                      contributions lay, the final state to the slot
 //   gla_out_kernel     a block a (chunk, head): [decayed q | P] [S; V]
 // P's sums are 32-bit fmas on the CUDA cores (two at a time, fma.rn.f32x2); the contributions and the outputs run on tcgen05 with
-// 32-bit operands taken apart into three bfloat16 numbers each (split3).  The decays are products of at most 9 factors instead of a
+// 32-bit operands taken apart into three bfloat16 numbers each (split3).  What is most of a sum where decays are strong goes through
+// registers: the two newest tokens of a contribution, an output's own token.  The decays are products of at most 9 factors instead of a
 // running product.
 //
-// 48 heads of 128 x 128, 2,048 tokens, a decay per channel, each kernel with its wait for the one before: decays 53 us,
-// contributions 226, carry 99 and outputs 359 token by token; 207, 84 and 137 with all products as 32-bit fmas; 163, 73 and 105 now.  The
-// layer 973 -> 690 -> 600 us, with one decay a head 949 -> 653 -> 589; 16 heads 371 -> 231 -> 205.  Against 64 bits, fmas and now: outputs
-// 1.4e-7 and 1.3e-7, where the decays are close to 1 3.0e-7 and 2.0e-7 (2.3e-7 and 1.5e-7 at the layer's own), states 2.5e-7 and
-// 1.9e-7; with decays of e^-6 a token, where a result is one token's product, 0.9e-7 and 1.0e-7 (the tensor core cuts off).
+// 48 heads of 128 x 128, 2,048 tokens, a decay per channel, cold caches: contributions 212 us, carry 48 and outputs 130 with all products
+// as 32-bit fmas, 179, 50 and 94 now, 328 in a row (one decay a head 294; 16 heads 124 and 98; token by token 226, 99 and 359 with their
+// waits).  The layer 973 -> 690 -> 632 us.  Outputs and states against 64 bits (1,024 tokens; as fmas, now): 1.4e-7 and 0.98e-7, 1.2 and
+// 0.83; where the decays are close to 1 2.8 and 2.0, 1.8 and 1.5; with decays of e^-6 a token, where a result is one token's product,
+// 0.89 and 0.25, 0.86 and 0.25; with one decay of 0.88 for all channels 1.05 and 0.60, 1.02 and 0.62.
 #pragma once
 #include "tc_common.cuh"
 
@@ -200,7 +201,7 @@ __device__ __noinline__ float gc_contribution(const GcLocal<D, VT>& sh, int d, i
 // What bounds it: loads, decays and the pairs' sums on the fma pipe, one after the other between barriers, with two blocks an SM.  The
 // logits come through shared memory so that the decays are a loop of four instead of 32 copies of the code (a block's first pass
 // 38,000 -> 28,000 cycles).  The contribution, as L^T = V^T K, is on tcgen05, keys in three pieces (split3):
-// 207 -> 163 us against fmas.
+// 212 -> 179 us against fmas (cold caches).
 template <int D, int VT>
 __global__ void __launch_bounds__(2 * D, 256 / D) gla_local_kernel(GlaArgs a) {
   constexpr int kThreads = 2 * D, LD = D + 4, kLanes = D / 8;  // lanes a token
@@ -632,8 +633,8 @@ struct GoPlace {
 // Outputs of a chunk: o^T = S^T q^T + V^T P^T, 128 value columns (rows of the tensor core's tile) x 64 tokens.  Two threads a value column.  S,
 // q and P are taken apart into three bfloat16 numbers each (split3) and the six products that reach 2^-24 are taken (with V, which is
 // bfloat16, three); the leading pieces' products are chains of two steps of 16, added up in registers.  Two blocks an SM; what bounds them is
-// memory's latency (2.7 TB/s: loads, taking apart, products and stores of a block follow one another; the tensor pipe is 13 % busy).
-// 137 -> 105 us against fmas.
+// memory's latency (2.4 TB/s: loads, taking apart, products and stores of a block follow one another; the tensor pipe is 13 % busy).
+// 130 -> 94 us against fmas (cold caches).
 template <int D>
 __global__ void __launch_bounds__(256, 2) gla_out_kernel(GlaArgs a) {
   constexpr int kStages = D / 64;

@@ -9,7 +9,8 @@
 // 512 threads fetch the next step's rows, take them apart into the other buffer and add up; one of them issues.  An infinity or NaN (or
 // a number that bfloat16 cannot reach) makes its row or column of the tile NaN: such a result is summed once more as 32-bit fmas.
 //
-// What bounds it: the tensor pipe (24 products of 128 x 128 x 16 a step, 0.8 us), then the taking apart beside it.  16
+// What bounds it: a step's chain, rows fetched and taken apart into shared memory (busy 63 % of the time), a barrier, 24 products of
+// 128 x 128 x 16 (0.8 us; the tensor pipe is busy 46 %).  16
 // experts of 1,024 x 1,408, gate/up and down (32-bit fmas on the CUDA cores, now): 8 rows each 111 + 86 and 90 + 43 us, 108 rows 287 + 176
 // and 101 + 51, 300 rows 651 + 397 and 238 + 127 (180 TFLOP/s of 32-bit products).  Off from 64 bits by 8.7e-7 and 6.7e-7 with fmas
 // in order, by 1.8e-7 and 1.3e-7 here.

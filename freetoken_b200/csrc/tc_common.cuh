@@ -211,8 +211,7 @@ __device__ __forceinline__ void tc_mma_pair(uint32_t d_tmem, uint64_t a_desc, ui
 __device__ __forceinline__ bool all_of_warp(bool ok) { return __all_sync(0xffffffffu, ok); }
 // One lane of a warp that is together, the same one each time.  (Products issued behind it, instead of behind a comparison of the
 // lane's number, leave their thread every 31 instead of every 51 cycles: the compiler sees that their operands are the warp's.  A
-// portion over 32k keys 530 -> 496 us, prompt attention 81 -> 78, decode attention of 64 requests 122 -> 116, of eight experts' weights
-// 250 -> 244.)
+// portion over 32k keys 530 -> 496 us, prompt attention 81 -> 78, decode attention of 64 requests 122 -> 116.)
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(p));
