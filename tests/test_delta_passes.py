@@ -26,7 +26,8 @@ def test_passes_take_every_row_once_and_in_order(most):
     assert chunk_passes([2048] * 4, 128) == [(0, 4, 0, 32, 128)]
     assert chunk_passes([2048] * 4, 64) == [(0, 4, 0, 16, 64), (0, 4, 16, 32, 64)]  # side by side
     assert chunk_passes([8192], 64) == [(0, 1, 0, 64, 64), (0, 1, 64, 128, 64)]
-    assert chunk_passes([80, 8192, 65, 64], 64) == [(0, 1, 0, 2, 2), (1, 1, 0, 64, 64), (1, 1, 64, 128, 64), (2, 2, 0, 2, 3)]
+    assert chunk_passes([80, 8192, 65, 64], 64) == [(0, 4, 0, 59, 64), (0, 4, 59, 123, 64), (0, 4, 123, 128, 5)]
+    assert chunk_passes([4096] + [80] * 51, 63) == [(0, 1, 0, 63, 63), (0, 1, 63, 64, 1), (1, 31, 0, 2, 62), (32, 20, 0, 2, 40)]
     assert [p[1] for p in chunk_passes([80] * 102, 64)] == [32, 32, 32, 6]  # whole: a state is read and written once
 
 
