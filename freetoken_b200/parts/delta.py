@@ -25,6 +25,7 @@ slot of the cache manager's state pool; both start from zero.  The reference has
 
 from __future__ import annotations
 
+import functools
 import math
 from typing import Any, Dict, List, Optional, Sequence, Tuple
 
@@ -75,7 +76,11 @@ def chunk_passes(lens: Sequence[int], most: int) -> List[Tuple[int, int, int, in
     out: List[Tuple[int, int, int, int, int]] = []
 
     def far(left: Sequence[int]) -> int:
-        return max((m for m in range(1, max(left) + 1) if sum(min(r, m) for r in left) <= most), default=0)
+        low, high = 0, max(left)
+        while low < high:
+            m = (low + high + 1) // 2
+            low, high = (m, high) if sum(min(r, m) for r in left) <= most else (low, m - 1)
+        return low
 
     if far(rows) >= min(8, max(rows)):
         done = 0
@@ -112,9 +117,14 @@ def chunks_pay(lens: Sequence[int], beside: bool, n_heads: int, n_kv_heads: int,
     by token against chunks: 39 and 38 us for 80 tokens, 46 and 32 for 96, 59 and 37 for 128, 213 and 69 for 512; 16 heads of 64: 23
     and 26, 27 and 26, 35 and 31, 127 and 40.  Many requests: 48 heads, 16 of 80 tokens 311 and 222, four of 512 604 and 199; 48 heads
     of 64 columns that share no keys, 16 of 80 160 and 188, of 128 244 and 198."""
-    parts = [lens]
-    if most is not None:
-        parts = [[min(n, row1 * ops.DELTA_CHUNK) - row0 * ops.DELTA_CHUNK for n in lens[first:first + count]]
+    return _chunks_pay(tuple(lens), beside, n_heads, n_kv_heads, head_dim, v_dim, most)  # (a step's layers ask the same)
+
+
+@functools.lru_cache(maxsize=256)
+def _chunks_pay(lens: Tuple[int, ...], beside: bool, n_heads: int, n_kv_heads: int, head_dim: int, v_dim: int, most: Optional[int]) -> bool:
+    parts: List[Sequence[int]] = [lens]
+    if most is not None and sum(-(-n // ops.DELTA_CHUNK) for n in lens) > most:
+        parts = [[max(0, min(n, row1 * ops.DELTA_CHUNK) - row0 * ops.DELTA_CHUNK) for n in lens[first:first + count]]
                  for first, count, row0, row1, _ in chunk_passes(lens, most)]
     in_chunks = sum(chunk_time(p, n_heads, n_kv_heads, head_dim, v_dim) for p in parts) + (6.0 if beside else 0.0)
     longest = max(lens)
@@ -159,6 +169,9 @@ class GatedDelta(Mixer):
         self.b_col = self.g_col + (self.gate_rank or H * Dv)
         self.a_col = self.b_col + H
         self.proj_rows = self.a_col + (self.decay_rank or H)
+        # scratch of the longest step: its rows, and what one takes
+        self.most_rows, size = self.chunk_scratch(env.max_step_tokens, env.max_step_tokens // CHUNK_MIN_TOKENS)
+        self.row_bytes = size // max(self.most_rows, 1)
 
     def param_specs(self) -> Dict[str, ParamSpec]:
         std = self.spec.get("init_std")
@@ -224,12 +237,14 @@ class GatedDelta(Mixer):
         args = dict(z=z)
         long = [seg.q_len for seg in step.segments if seg.q_len >= CHUNK_MIN_TOKENS] if z is None and h.is_cuda else []
         n_long = len(long)
-        if long:
-            rows, n = self.chunk_scratch(T, n_long)
-            if n and chunks_pay(long, n_long < n_segs, H, self.n_kv_heads, D, Dv, rows):  # (by rows: layers of other sizes have a buffer of their own, and no step asks for more rows)
-                row, most = n // rows, self.chunk_scratch(cap, cap // CHUNK_MIN_TOKENS)[0]
-                args = dict(scratch=ws.get("delta.chunks", (rows, row), torch.uint8, (most, row)), long_from=CHUNK_MIN_TOKENS, n_long=n_long)
-                if rows < T // ops.DELTA_CHUNK + n_long:
+        if long and self.row_bytes:
+            need = T // ops.DELTA_CHUNK + n_long
+            rows = min(need, self.most_rows)
+            if chunks_pay(long, n_long < n_segs, H, self.n_kv_heads, D, Dv, rows):
+                # (by rows: layers of other sizes have a buffer of their own, and no step asks for more rows)
+                args = dict(scratch=ws.get("delta.chunks", (rows, self.row_bytes), torch.uint8, (self.most_rows, self.row_bytes)),
+                            long_from=CHUNK_MIN_TOKENS, n_long=n_long)
+                if rows < need:
                     args["passes"] = chunk_passes(long, rows)
         ops.delta_scan(qkv[:, : self.k_col], qkv[:, self.k_col: self.v_col], qkv[:, self.v_col:],
                        proj[:, self.b_col: self.a_col], a, self.params["A_log"], self.params["dt_bias"],
