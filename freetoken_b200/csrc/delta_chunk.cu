@@ -509,7 +509,7 @@ __device__ __noinline__ void dc_by_token(const DeltaChunkArgs& a, float* state, 
 // A block owns NV value columns of one (request, head).  A thread has a row (a token of K, of Q; a key channel) and 8 or 16 of the
 // columns.  Products, by one thread (columns of NV in tensor memory; each is read before the next is issued, so all use the same):
 //   [K; Q] S      two 16-channel steps of the leading piece each in columns of their own (up to 4), the second and third piece (4, 5)
-//   [T; A T] X    32 tokens each of the leading pieces' product (0, 1), second order (2), third (3)
+//   [T; A T] X    (without the diagonals) 32 tokens each of the leading pieces' product (0, 1), second order (2), third (3)
 //   K^T U         the same
 template <int NV>
 constexpr int dc_threads() { return NV == 64 ? 512 : 256; }

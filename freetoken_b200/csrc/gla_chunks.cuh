@@ -450,7 +450,6 @@ __global__ void __launch_bounds__(2 * D, 256 / D) gla_local_kernel(GlaArgs a) {
     }
     a.decay_prod[((size_t)c * a.H + h) * D + tid] = hi;
   }
-  const bool two = n >= 2;
   // the chunk's contribution: keys decayed to its end, in three pieces; a thread has eight channels of a token of every 16
   {
     constexpr int kPass = kThreads / kLanes;  // tokens at a time
@@ -490,82 +489,71 @@ __global__ void __launch_bounds__(2 * D, 256 / D) gla_local_kernel(GlaArgs a) {
   fence_async_smem();
   tc_fence_before();
   __syncthreads();
-  // Products, two sums of them at a time (2 D columns): the second and third pieces' and the first's of 32 tokens, then the first's of the
-  // other 32.  They are added up in registers, and the two newest tokens', the largest where decays are strong, last and by themselves:
-  // the accumulator cuts off instead of rounding.
-  const int j = (warp & 3) * 32 + lane;  // a value column; 64 channels of it
-  const uint32_t my_tmem = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)((warp >> 2) * 64);
-  const float* k_last = &sh.k[n - 1][(warp >> 2) * 64];
-  auto value = [&](int t) {
-    return __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(sh.v + (j >> 6) * (kGcTokens * 128) + t * 128 + ((((j >> 3) & 7) ^ (t & 7)) << 4) + (j & 7) * 2));
-  };
-  const float v_last = j < 64 * VT ? value(n - 1) : 0.f, v_before = j < 64 * VT && two ? value(n - 2) : 0.f;
-  float* dst = a.carry + (((size_t)c * a.H + h) * D + (warp >> 2) * 64) * a.Dv + j;
-  float acc[64];
+  if (warp == 0) {
+    tc_fence_after();
+    if (elect_one()) {
+      constexpr uint32_t id = instr_desc(D) | kMnMajorA | kMnMajorB;
+      const uint32_t v0 = smem_addr(sh.v), k0 = smem_addr(sh.q);
 #pragma unroll
-  for (int round = 0; round < 2; ++round) {
-    if (warp == 0) {
-      tc_fence_after();
-      if (elect_one()) {
-        constexpr uint32_t id = instr_desc(D) | kMnMajorA | kMnMajorB;
-        const uint32_t v0 = smem_addr(sh.v), k0 = smem_addr(sh.q);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const uint64_t v = smem_desc_mn(v0 + k * 2048, kGcTokens * 128);
-          if (round == 0) {
-            tc_mma(tmem, v, smem_desc_mn(k0 + GcLocal<D, VT>::piece + k * 2048, kGcTokens * 128), id, k != 0);
-            tc_mma(tmem, v, smem_desc_mn(k0 + 2 * GcLocal<D, VT>::piece + k * 2048, kGcTokens * 128), id, 1);
-          }
-          if (k / 2 == round) tc_mma(tmem + (1 - round) * D, v, smem_desc_mn(k0 + k * 2048, kGcTokens * 128), id, k % 2);
-        }
-        tc_commit(&mma_done);
+      for (int k = 0; k < 4; ++k) {
+        const uint64_t v = smem_desc_mn(v0 + k * 2048, kGcTokens * 128);
+        tc_mma(tmem, v, smem_desc_mn(k0 + k * 2048, kGcTokens * 128), id, k != 0);
+        tc_mma(tmem + D, v, smem_desc_mn(k0 + GcLocal<D, VT>::piece + k * 2048, kGcTokens * 128), id, k != 0);
+        tc_mma(tmem + D, v, smem_desc_mn(k0 + 2 * GcLocal<D, VT>::piece + k * 2048, kGcTokens * 128), id, 1);
       }
-      __syncwarp();
-    }
-    if (!mbar_wait(&mma_done, round, &abort_flag)) {
-      if (atomicCAS(&g_gla_status[0], 0, 602) == 0) g_gla_status[1] = blockIdx.x;
-      abort_flag = 1;
+      tc_commit(&mma_done);
     }
     __syncwarp();
-    tc_fence_after();
-#pragma unroll
+  }
+  if (!mbar_wait(&mma_done, 0, &abort_flag)) {
+    if (atomicCAS(&g_gla_status[0], 0, 602) == 0) g_gla_status[1] = blockIdx.x;
+    abort_flag = 1;
+  }
+  __syncwarp();
+  tc_fence_after();
+  {
+    // The two newest tokens' share, the largest where decays are strong, is added last and by itself: the accumulator cuts off instead of
+    // rounding.  (Two sums of 32 tokens, read one after the other, bring states 0 to 2 % closer to 64 bits; with outputs of four sums of 16 a
+    // retention layer of 16 heads of 128 takes 91 us instead of 77 for 572 tokens, most of it code that a block fetches once.)
+    const int j = (warp & 3) * 32 + lane;  // a value column; 64 channels of it
+    const uint32_t my_tmem = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)((warp >> 2) * 64);
+    auto value = [&](int t) {
+      return __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(sh.v + (j >> 6) * (kGcTokens * 128) + t * 128 + ((((j >> 3) & 7) ^ (t & 7)) << 4) + (j & 7) * 2));
+    };
+    const bool two = n >= 2, mine = j < 64 * VT;
+    const float v_last = mine ? value(n - 1) : 0.f, v_before = mine && two ? value(n - 2) : 0.f;
+    const float *k_last = &sh.k[n - 1][(warp >> 2) * 64], *k_before = two ? k_last - LD : k_last;
+    float* dst = a.carry + (((size_t)c * a.H + h) * D + (warp >> 2) * 64) * a.Dv + j;
+#pragma unroll 1
     for (int i = 0; i < 64; i += 8) {
-      float r[2][8];
+      float r[2][8], k[2][8], y[8];
       tmem_ld8_start(my_tmem + i, r[0]);
-      if (round == 0) tmem_ld8_start(my_tmem + D + i, r[1]);
+      tmem_ld8_start(my_tmem + D + i, r[1]);
+#pragma unroll
+      for (int e = 0; e < 8; e += 4) {
+        Vec4<float>::load(k_last + i + e, reinterpret_cast<float (&)[4]>(k[0][e]));
+        Vec4<float>::load(k_before + i + e, reinterpret_cast<float (&)[4]>(k[1][e]));
+      }
       tmem_ld8_finish(r);
-      if (round == 0) {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) acc[i + e] = r[0][e] + r[1][e];
-        continue;
-      }
-      float y[8], k[8];
-#pragma unroll
-      for (int e = 0; e < 8; ++e) y[e] = acc[i + e] + r[0][e];
-      if (two) {
-        Vec4<float>::load(k_last - LD + i, reinterpret_cast<float (&)[4]>(k[0]));
-        Vec4<float>::load(k_last - LD + i + 4, reinterpret_cast<float (&)[4]>(k[4]));
-#pragma unroll
-        for (int e = 0; e < 8; ++e) y[e] = fmaf(k[e], v_before, y[e]);
-      }
-      Vec4<float>::load(k_last + i, reinterpret_cast<float (&)[4]>(k[0]));
-      Vec4<float>::load(k_last + i + 4, reinterpret_cast<float (&)[4]>(k[4]));
-#pragma unroll
-      for (int e = 0; e < 8; ++e) y[e] = fmaf(k[e], v_last, y[e]);
+      for (int e = 0; e < 8; ++e) y[e] = fmaf(k[0][e], v_last, fmaf(k[1][e], v_before, r[0][e] + r[1][e]));
       if (j < a.Dv) {
         if (gc_none(y)) {
+#pragma unroll 1
+          for (int e = 0; e < 8; ++e) {
+            float z = 0.f;
 #pragma unroll
-          for (int e = 0; e < 8; ++e)
-            if (!(fabsf(y[e]) < INFINITY)) y[e] = gc_contribution<D, VT>(sh, (warp >> 2) * 64 + i + e, j, n - 2);
+            for (int f = 0; f < 8; ++f) z = e == f ? y[f] : z;
+            if (fabsf(z) < INFINITY) continue;
+            z = gc_contribution<D, VT>(sh, (warp >> 2) * 64 + i + e, j, n - 2);
+#pragma unroll
+            for (int f = 0; f < 8; ++f) y[f] = e == f ? z : y[f];
+          }
         }
 #pragma unroll
         for (int e = 0; e < 8; ++e) dst[(size_t)(i + e) * a.Dv] = y[e];
       }
       __syncwarp();
-    }
-    if (round == 0) {
-      tc_fence_before();
-      __syncthreads();
     }
   }
   tc_fence_before();
@@ -854,27 +842,22 @@ __global__ void __launch_bounds__(256, 2) gla_out_kernel(GlaArgs a) {
       put8(GoPlace::q, GoPlace::tile, i >> 3, i & 7, qv[u]);
     }
     fence_async_smem();
-#pragma unroll 1
-    for (int pair = 0; pair < 2; ++pair) {  // sums of 16 tokens
-      tc_fence_before();
-      __syncthreads();
-      if (warp == 0) {
-        tc_fence_after();
-        if (elect_one()) {
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+      tc_fence_after();
+      if (elect_one()) {
 #pragma unroll
-          for (int x = 0; x < 2; ++x) {
-            const int k = 2 * pair + x;
-            const uint64_t v = smem_desc_mn(base + GoPlace::v + k * 2048, GoPlace::tile);
-            tc_mma(tmem + x * 64, v, smem_desc(base + GoPlace::q) + 2 * k, id1, 0);
-            tc_mma(tmem + 128, v, smem_desc(base + GoPlace::q + GoPlace::tile) + 2 * k, id2, 1);
-          }
-          tc_commit(&mma_done);
+        for (int k = 0; k < 4; ++k) {
+          const uint64_t v = smem_desc_mn(base + GoPlace::v + k * 2048, GoPlace::tile);
+          tc_mma(tmem + (k >> 1) * 64, v, smem_desc(base + GoPlace::q) + 2 * k, id1, k & 1);
+          tc_mma(tmem + 128, v, smem_desc(base + GoPlace::q + GoPlace::tile) + 2 * k, id2, 1);
         }
-        __syncwarp();
+        tc_commit(&mma_done);
       }
-      wait();
-      if (pair == 0) add_chains();
+      __syncwarp();
     }
+    wait();
     const int j = quad * 32 + lane, odd_from = j < Dv ? first_odd[j] : kGcTokens;
     float* o = a.out + (x.row0 * a.H + h) * Dv + j;
     bool odd = j < Dv && odd_from < n;
