@@ -20,10 +20,10 @@
 // running product.
 //
 // 48 heads of 128 x 128, 2,048 tokens, a decay per channel, cold caches: contributions 212 us, carry 48 and outputs 130 with all products
-// as 32-bit fmas, 179, 50 and 94 now, 328 in a row (one decay a head 294; 16 heads 124 and 98; token by token 226, 99 and 359 with their
-// waits).  The layer 973 -> 690 -> 632 us.  Outputs and states against 64 bits (1,024 tokens; as fmas, now): 1.4e-7 and 0.98e-7, 1.2 and
-// 0.83; where the decays are close to 1 2.8 and 2.0, 1.8 and 1.5; with decays of e^-6 a token, where a result is one token's product,
-// 0.89 and 0.25, 0.86 and 0.25; with one decay of 0.88 for all channels 1.05 and 0.60, 1.02 and 0.62.
+// as 32-bit fmas, 174, 48 and 90 now, 318 in a row (one decay a head 284; 16 heads 118 and 94; token by token 226, 99 and 359 with their
+// waits).  The layer 973 -> 690 -> 634 us.  Outputs and states against 64 bits (1,024 tokens; as fmas, now): 1.4e-7 and 0.98e-7, 1.2 and
+// 0.85; where the decays are close to 1 2.8 and 2.0, 1.8 and 1.5; with decays of e^-6 a token, where a result is one token's product,
+// 0.89 and 0.25, 0.86 and 0.25; with one decay of 0.88 for all channels 1.05 and 0.60, 1.04 and 0.62.
 #pragma once
 #include "tc_common.cuh"
 
@@ -201,7 +201,7 @@ __device__ __noinline__ float gc_contribution(const GcLocal<D, VT>& sh, int d, i
 // What bounds it: loads, decays and the pairs' sums on the fma pipe, one after the other between barriers, with two blocks an SM.  The
 // logits come through shared memory so that the decays are a loop of four instead of 32 copies of the code (a block's first pass
 // 38,000 -> 28,000 cycles).  The contribution, as L^T = V^T K, is on tcgen05, keys in three pieces (split3):
-// 212 -> 179 us against fmas (cold caches).
+// 212 -> 174 us against fmas (cold caches).
 template <int D, int VT>
 __global__ void __launch_bounds__(2 * D, 256 / D) gla_local_kernel(GlaArgs a) {
   constexpr int kThreads = 2 * D, LD = D + 4, kLanes = D / 8;  // lanes a token
