@@ -513,8 +513,9 @@ __global__ void __launch_bounds__(2 * D, 256 / D) gla_local_kernel(GlaArgs a) {
   tc_fence_after();
   {
     // The two newest tokens' share, the largest where decays are strong, is added last and by itself: the accumulator cuts off instead of
-    // rounding.  (Two sums of 32 tokens, read one after the other, bring states 0 to 2 % closer to 64 bits; with outputs of four sums of 16 a
-    // retention layer of 16 heads of 128 takes 91 us instead of 77 for 572 tokens, most of it code that a block fetches once.)
+    // rounding.  (Two sums of 32 tokens, read one after the other, bring states 0 to 2 % closer to 64 bits; with them, with the sum of an
+    // infinity's element written out eight times and with outputs of four sums of 16 a retention layer of 16 heads of 128, 572 tokens took
+    // 91 us instead of 77.)
     const int j = (warp & 3) * 32 + lane;  // a value column; 64 channels of it
     const uint32_t my_tmem = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)((warp >> 2) * 64);
     auto value = [&](int t) {
